@@ -17,7 +17,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(BUILD, "libbg3.so")
 ROOT = os.path.dirname(HERE)
 
-SOURCES = ["bg3_step.cu", "bg3_growth.cu", "bg3_api.cu", "bg3_noalloc.cu", "bg3_serve.cu",
+SOURCES = ["bg3_step.cu", "bg3_block.cu", "bg3_growth.cu", "bg3_api.cu", "bg3_noalloc.cu", "bg3_serve.cu",
            "bg3_selftest.cu", "bg3_serialize.cu", "bg3_hostrng.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC",

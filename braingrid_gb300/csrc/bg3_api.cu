@@ -35,9 +35,16 @@ void launch_growth(const NetDev &h, const NetDev *d_net, int epoch, int add_thre
 void launch_rebuild_maps(const NetDev &h, const NetDev *d_net, cudaStream_t s);
 void launch_scale_weights(const NetDev &h, float f, cudaStream_t s);
 void launch_record(const NetDev &h, const NetDev *d_net, cudaStream_t s);
+bool blk_thin_ok(int Mq);
+void launch_blk_masks(const NetDev &h, const BlkDev &b, cudaStream_t s);
+void launch_blk_ring(const NetDev &h, const BlkDev &b, cudaStream_t s);
+void launch_blk_thin(const NetDev &h, const BlkDev &b, int nt, cudaStream_t s);
+void launch_blk_thin_batch(int syn_kind, const NetDev *nets, const BlkDev *blks, int nets_n,
+                           const int2 *tiles, int n, int pad, int max_mq, int nt, cudaStream_t s);
 }  // namespace bg3
 
 static const int GRAPH_STEPS = 32;  // fused steps captured per CUDA graph replay
+static const int GRAPH_BLOCKS = 16;  // blocks of steps captured per CUDA graph replay
 static const int SMALL_STEPS = 4096;  // steps per launch of a small network (bg3::launch_small)
 
 // kernels one step launches after its neuron pass: delivery (+ post-spike STDP) and the sweep
@@ -62,8 +69,17 @@ struct bg3_net {
     void *flush_buf = nullptr, *scrub_buf = nullptr;
     size_t flush_size = 0;
     cudaGraphExec_t graph = nullptr;
+    int graph_steps = 0;      // steps per block in the captured graph (0: the per-step kernels)
     std::vector<std::tuple<int, int, uint32_t, uint32_t>> exp_keys;  // exp tables this net holds
     uint64_t bytes = 0;                                                 // device bytes allocated
+    // spikes of the last 64 steps, kept as the per-step kernels' ring or the block kernels' masks:
+    // whichever ran last is current, the other is rebuilt when it is needed
+    BlkDev blk = {};
+    bool ring_ok = true, mask_ok = false;
+    // fewest steps between two spikes of a neuron, for the block kernels' STDP ring rule: the
+    // shortest refractory period + 1, or 1 once spike histories were uploaded
+    int min_isi = 1;
+    bool hist_given = false;
 };
 
 #define CK(x)                                                                            \
@@ -90,6 +106,9 @@ static int dalloc(bg3_net *n, T **p, size_t count, int fill = 0)
     *p = (T *)q;
     return BG3_OK;
 }
+
+static size_t blk_act_bytes(size_t Np) { return BLK_ACT_ROWS * (Np / 32) * sizeof(uint32_t); }
+static size_t blk_bytes(size_t Np) { return Np * sizeof(unsigned long long) + blk_act_bytes(Np); }
 
 static void drop_graph(bg3_net *n);
 // The step kernels take the descriptor by value (captured into the step graph); the growth
@@ -120,6 +139,7 @@ static void drop_graph(bg3_net *n)
 {
     if (n->graph) cudaGraphExecDestroy(n->graph);
     n->graph = nullptr;
+    n->graph_steps = 0;
 }
 
 // decay / delay class tables (host copy is the source of truth; pushed on change)
@@ -406,6 +426,11 @@ int bg3_create(const bg3_net_desc *desc, bg3_net **out)
     }
 #undef A
     if ((rc = dalloc(n, &h.history, N * (size_t)max_spikes, 0xff)) != 0) goto fail;
+    if (cudaMalloc((void **)&n->blk.hist, Np * sizeof(*n->blk.hist)) != cudaSuccess ||
+        cudaMalloc((void **)&n->blk.act, blk_act_bytes(Np)) != cudaSuccess) {
+        rc = BG3_ENOMEM;
+        goto fail;
+    }
     if (cudaMalloc((void **)&n->d, sizeof(NetDev)) != cudaSuccess) { rc = BG3_ENOMEM; goto fail; }
     // type constants of createSynapse at this deltaT (Synapses/AllSpikingSynapses.cpp:192-240,
     // AllDSSynapses.cpp:180-218); decay = exp(-deltaT / tau) on the host, as the reference does
@@ -480,10 +505,11 @@ int64_t bg3_net_footprint(const bg3_net_desc *desc)
     if (D.neuron_kind == BG3_NEURON_IZH) b += 6 * N * 4;
     b += N * (uint64_t)ms * 8;                                     // spike history
     b += sizeof(NetDev) + 54 * N;                                  // descriptor, input
+    b += blk_bytes((size_t)Np);                                    // spike masks
     return (int64_t)b;
 }
 
-uint64_t bg3_net_bytes(bg3_net *n) { return n ? n->bytes + sizeof(NetDev) : 0; }
+uint64_t bg3_net_bytes(bg3_net *n) { return n ? n->bytes + sizeof(NetDev) + blk_bytes((size_t)n->h.Np) : 0; }
 
 int bg3_set_device(int32_t device)
 {
@@ -513,6 +539,8 @@ int bg3_destroy(bg3_net *n)
     for (auto &a : n->allocs)
         if (a.first) cudaFree(a.first);
     if (n->d) cudaFree(n->d);
+    if (n->blk.hist) cudaFree(n->blk.hist);
+    if (n->blk.act) cudaFree(n->blk.act);
     if (n->noise_dev) cudaFree(n->noise_dev);
     if (n->flush_buf) cudaFree(n->flush_buf);
     if (n->scrub_buf) cudaFree(n->scrub_buf);
@@ -521,6 +549,33 @@ int bg3_destroy(bg3_net *n)
     if (n->stream) cudaStreamDestroy(n->stream);
     delete n;
     return BG3_OK;
+}
+
+// Fewest steps between two spikes of any neuron with these refractory periods.
+static void set_min_isi(bg3_net *n, const float *Trefract)
+{
+    int m = 1 << 30;
+    for (int i = 0; i < n->h.N; i++) {
+        const double r = (double)(Trefract[i] / n->h.dt) + 0.5;
+        m = std::min(m, r > 0.0 && r < 1e9 ? (int)r + 1 : 1);
+    }
+    n->min_isi = m;
+}
+
+// The spike ring, brought up to date from the masks (queued on the network's stream).
+static int ensure_ring(bg3_net *n)
+{
+    if (n->ring_ok) return BG3_OK;
+    bg3::launch_blk_ring(n->h, n->blk, n->stream);
+    CK(cudaGetLastError());
+    n->ring_ok = true;
+    return BG3_OK;
+}
+// The ring was written from outside the block kernels.
+static void ring_changed(bg3_net *n)
+{
+    n->ring_ok = true;
+    n->mask_ok = false;
 }
 
 // ---- uploads --------------------------------------------------------------------------------
@@ -540,6 +595,8 @@ int bg3_upload_lif(bg3_net *n, const bg3_lif_arrays *a)
         (rc = h2d(n, (uint64_t *)h.history, a->history, N * (size_t)h.max_spikes)))
         return rc;
     CK(cudaStreamSynchronize(n->stream));
+    if (a->history) n->hist_given = true;
+    if (a->Trefract) set_min_isi(n, a->Trefract);
     return BG3_OK;
 }
 
@@ -717,6 +774,7 @@ int bg3_upload_synapses(bg3_net *n, const bg3_synapse_arrays *a, uint64_t step)
         (rc = h2d(n, h.count, count.data(), N)) || (rc = h2d(n, h.ring, ring.data(), ring.size())) ||
         (rc = h2d(n, h.ring_n, ring_n.data(), ring_n.size())))
         return rc;
+    ring_changed(n);
     unsigned long long s64 = step;
     CK(cudaMemcpyAsync(h.step, &s64, sizeof(s64), cudaMemcpyHostToDevice, n->stream));
     CK(cudaMemcpyAsync(h.dstep, &s64, sizeof(s64), cudaMemcpyHostToDevice, n->stream));
@@ -1000,10 +1058,103 @@ int bg3_download_poisson(bg3_net *n, bg3_poisson_arrays *a)
 // next step's neurons, the last sweep without that epilogue.  Runs of interior steps replay a
 // CUDA graph of GRAPH_STEPS (deliver, fused sweep) pairs.  Injected-noise mode: neurons,
 // deliver, sweep for every step, GRAPH_STEPS of them per graph replay.
+// Most steps a network's block may hold: every spike takes at least that many to arrive.
+static int blk_delay_steps(const bg3_net *n)
+{
+    int m = BLK_MAX_STEPS;
+    for (int D : n->ltab) m = std::min(m, D);
+    return m;
+}
+// bit s & 63 for every step s whose spikes may arrive in a block starting at step 0
+static unsigned long long blk_window(const bg3_net *n)
+{
+    const int T = blk_delay_steps(n);
+    unsigned long long w = 0;
+    for (int D : n->ltab)
+        for (int j = 0; j < T; j++) w |= 1ull << ((j - D) & 63);
+    return w;
+}
+
+// Steps per block when the network runs in blocks (bg3_block.cu), 0 when it does not (always
+// with small_max_slots 0, which asks for the per-step kernels): device noise, a thin network (one warp per tile) and delays of two steps or more.  STDP kinds: the
+// host build's spike-time arithmetic (its pre-spike walks read only the destination's own
+// history), and a history ring long enough that the spikes a block adds never overwrite an entry
+// a post-spike walk reads (entries within 3 tau+, at most one per min_isi steps).
+static int blk_steps(const bg3_net *n, const LaunchCfg &c)
+{
+    const NetDev &h = n->h;
+    if (c.small_max_slots == 0 || h.noise_mode != BG3_NOISE_DEVICE || !bg3::sweep_is_thin(h, c) ||
+        !bg3::blk_thin_ok(h.Mq))
+        return 0;
+    if (h.syn_kind >= BG3_SYN_STDP) {
+        if (h.stdp_signed) return 0;
+        float tau = 0.0f;
+        for (const StdpConst &s : h.stdp) tau = std::max(tau, s.taupos);
+        if (!(tau >= 0.0f) || !(tau < 1e3f)) return 0;
+        const int isi = n->hist_given ? 1 : n->min_isi;
+        const double window = 3.0 * (double)tau / (double)h.dt + 1.0;
+        if (window / isi + BLK_MAX_STEPS + 4.0 > (double)h.max_spikes) return 0;
+    }
+    const int T = blk_delay_steps(n);
+    return T >= 2 ? T : 0;
+}
+
+// The spike masks as of the network's current step, for a block to start from.
+static int ensure_masks(bg3_net *n)
+{
+    const unsigned long long w = blk_window(n);
+    if (n->mask_ok && w == n->blk.win) return BG3_OK;
+    int rc = ensure_ring(n);
+    if (rc) return rc;
+    n->blk.win = w;
+    drop_graph(n);  // holds the window
+    bg3::launch_blk_masks(n->h, n->blk, n->stream);
+    CK(cudaGetLastError());
+    n->mask_ok = true;
+    return BG3_OK;
+}
+
+// ceil(nsteps / T) blocks, runs of GRAPH_BLOCKS of them replayed from a CUDA graph.
+static int run_blocks(bg3_net *n, int64_t nsteps, int T)
+{
+    const NetDev &h = n->h;
+    int rc = ensure_masks(n);
+    if (rc) return rc;
+    n->ring_ok = false;
+    if (n->graph && n->graph_steps != T) drop_graph(n);
+    const int64_t blocks = (nsteps + T - 1) / T;
+    int64_t left = nsteps;
+    if (left >= (int64_t)GRAPH_BLOCKS * T && !n->graph) {
+        cudaGraph_t g;
+        CK(cudaStreamBeginCapture(n->stream, cudaStreamCaptureModeThreadLocal));
+        for (int i = 0; i < GRAPH_BLOCKS; i++) bg3::launch_blk_thin(h, n->blk, T, n->stream);
+        CK(cudaStreamEndCapture(n->stream, &g));
+        cudaError_t e = cudaGraphInstantiate(&n->graph, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) { n->graph = nullptr; return BG3_ECUDA; }
+        n->graph_steps = T;
+    }
+    while (n->graph && left >= (int64_t)GRAPH_BLOCKS * T) {
+        CK(cudaGraphLaunch(n->graph, n->stream));
+        left -= (int64_t)GRAPH_BLOCKS * T;
+    }
+    for (; left > 0; left -= T)
+        bg3::launch_blk_thin(h, n->blk, (int)std::min<int64_t>(left, T), n->stream);
+    n->launches += blocks * (h.syn_kind >= BG3_SYN_STDP ? 2 : 1);
+    CK(cudaGetLastError());
+    return BG3_OK;
+}
+
 static int run_steps(bg3_net *n, int64_t nsteps)
 {
     if (nsteps <= 0) return BG3_OK;
     const NetDev &h = n->h;
+    const int T = bg3::small_eligible(h, n->cfg) ? 0 : blk_steps(n, n->cfg);
+    if (T) return run_blocks(n, nsteps, T);
+    int rc = ensure_ring(n);
+    if (rc) return rc;
+    n->mask_ok = false;
+    if (n->graph && n->graph_steps) drop_graph(n);
     if (bg3::small_eligible(h, n->cfg)) {
         // a small network: up to SMALL_STEPS whole steps per launch, one CTA
         for (int64_t left = nsteps; left > 0;) {
@@ -1175,7 +1326,8 @@ int bg3_download_synapses(bg3_net *n, bg3_synapse_arrays *a)
     std::vector<uint32_t> count(N);
     unsigned long long step = 0;
     const bool ds = h.syn_kind == BG3_SYN_DS || h.syn_kind == BG3_SYN_DYNSTDP;
-    int rc;
+    int rc = ensure_ring(n);
+    if (rc) return rc;
     if ((rc = d2h(n, psr.data(), h.psr, S)) || (rc = d2h(n, dc.data(), h.dcls, S / 8)) ||
         (rc = d2h(n, lc.data(), h.lcls, S)) || (rc = d2h(n, ev.data(), h.ev, S)) ||
         (rc = d2h(n, src.data(), h.src, S)) || (rc = d2h(n, st.data(), h.stype, S)) ||
@@ -1456,9 +1608,12 @@ struct bg3_batch {
     NetDev *d_nets = nullptr;
     CUtensorMap *d_maps = nullptr;
     int2 *d_tiles = nullptr;
-    int ntiles = 0, n_thick = 0, max_n = 0, syn_kind = 1;
+    BlkDev *d_blks = nullptr;
+    std::vector<BlkDev> blks;     // as uploaded
+    int ntiles = 0, n_thick = 0, max_n = 0, syn_kind = 1, thin_mq = 0;
     cudaStream_t stream = nullptr;
     cudaGraphExec_t graph = nullptr;
+    int graph_steps = 0;          // steps per block in the captured graph (0: per-step kernels)
     cudaEvent_t ev = nullptr;
     void *flush_buf = nullptr, *scrub_buf = nullptr;
     size_t flush_size = 0;
@@ -1502,6 +1657,9 @@ static int batch_refresh(bg3_batch *b)
     for (auto &t : tiles)
         if (!bg3::sweep_is_thin(b->nets[t.second.x]->h, b->cfg)) tl.push_back(t.second);
     b->n_thick = (int)tl.size();
+    b->thin_mq = 0;
+    for (bg3_net *n : b->nets)
+        if (bg3::sweep_is_thin(n->h, b->cfg)) b->thin_mq = std::max(b->thin_mq, n->h.Mq);
     tl.insert(tl.end(), thin.begin(), thin.end());
     if ((int)tl.size() != b->ntiles) {
         if (b->d_tiles) cudaFree(b->d_tiles);
@@ -1553,7 +1711,8 @@ int bg3_batch_create(bg3_net *const *nets, int32_t count, bg3_batch **out)
         goto fail;
     rc = BG3_ENOMEM;
     if (cudaMalloc(&b->d_nets, count * sizeof(NetDev)) != cudaSuccess ||
-        cudaMalloc(&b->d_maps, 2 * count * sizeof(CUtensorMap)) != cudaSuccess)
+        cudaMalloc(&b->d_maps, 2 * count * sizeof(CUtensorMap)) != cudaSuccess ||
+        cudaMalloc(&b->d_blks, count * sizeof(BlkDev)) != cudaSuccess)
         goto fail;
     for (bg3_net *n : b->nets) cudaStreamSynchronize(n->stream);
     if ((rc = batch_refresh(b)) != 0) goto fail;
@@ -1572,6 +1731,7 @@ int bg3_batch_destroy(bg3_batch *b)
     if (b->graph) cudaGraphExecDestroy(b->graph);
     if (b->d_nets) cudaFree(b->d_nets);
     if (b->d_maps) cudaFree(b->d_maps);
+    if (b->d_blks) cudaFree(b->d_blks);
     if (b->d_tiles) cudaFree(b->d_tiles);
     if (b->flush_buf) cudaFree(b->flush_buf);
     if (b->scrub_buf) cudaFree(b->scrub_buf);
@@ -1600,12 +1760,88 @@ static void batch_interior(bg3_batch *b, int64_t n)
     }
 }
 
+static void batch_drop_graph(bg3_batch *b)
+{
+    if (b->graph) cudaGraphExecDestroy(b->graph);
+    b->graph = nullptr;
+    b->graph_steps = 0;
+}
+
+// Steps per block when every member runs in blocks (the fewest of any), else 0.
+static int batch_blk_steps(const bg3_batch *b)
+{
+    int T = BLK_MAX_STEPS;
+    for (const bg3_net *n : b->nets) T = std::min(T, blk_steps(n, b->cfg));
+    return T;
+}
+
+static void batch_block(bg3_batch *b, int nt)
+{
+    bg3::launch_blk_thin_batch(b->syn_kind, b->d_nets, b->d_blks, (int)b->nets.size(),
+                               b->d_tiles + b->n_thick, b->ntiles - b->n_thick, b->cfg.thin_warps,
+                               b->thin_mq, nt, b->stream);
+}
+
+// Members' rings brought up to date for the per-step kernels (on the members' streams).
+static int batch_rings(bg3_batch *b)
+{
+    for (bg3_net *n : b->nets) {
+        const int rc = ensure_ring(n);
+        if (rc) return rc;
+        n->mask_ok = false;
+    }
+    return BG3_OK;
+}
+
+static int batch_run_blocks(bg3_batch *b, int64_t nsteps, int T)
+{
+    int rc;
+    bool same = b->blks.size() == b->nets.size();
+    for (size_t k = 0; k < b->nets.size(); k++) {
+        if ((rc = ensure_masks(b->nets[k]))) return rc;
+        b->nets[k]->ring_ok = false;
+        same = same && !memcmp(&b->blks[k], &b->nets[k]->blk, sizeof(BlkDev));
+    }
+    if ((rc = batch_order(b, true))) return rc;
+    if (!same) {
+        b->blks.clear();
+        for (bg3_net *n : b->nets) b->blks.push_back(n->blk);
+        CK(cudaMemcpyAsync(b->d_blks, b->blks.data(), b->blks.size() * sizeof(BlkDev),
+                           cudaMemcpyHostToDevice, b->stream));
+    }
+    if (b->graph && b->graph_steps != T) batch_drop_graph(b);
+    const int64_t blocks = (nsteps + T - 1) / T;
+    int64_t left = nsteps;
+    if (left >= (int64_t)GRAPH_BLOCKS * T && !b->graph) {
+        cudaGraph_t g;
+        CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+        for (int i = 0; i < GRAPH_BLOCKS; i++) batch_block(b, T);
+        CK(cudaStreamEndCapture(b->stream, &g));
+        cudaError_t e = cudaGraphInstantiate(&b->graph, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) { b->graph = nullptr; return BG3_ECUDA; }
+        b->graph_steps = T;
+    }
+    while (b->graph && left >= (int64_t)GRAPH_BLOCKS * T) {
+        CK(cudaGraphLaunch(b->graph, b->stream));
+        left -= (int64_t)GRAPH_BLOCKS * T;
+    }
+    for (; left > 0; left -= T) batch_block(b, (int)std::min<int64_t>(left, T));
+    b->launches += blocks * (b->syn_kind >= BG3_SYN_STDP ? 2 : 1);
+    CK(cudaGetLastError());
+    return batch_order(b, false);
+}
+
 int bg3_batch_step(bg3_batch *b, int64_t nsteps)
 {
     if (!b || nsteps < 0) return BG3_EINVAL;
     if (nsteps == 0) return BG3_OK;
-    int rc = batch_order(b, true);
+    const int T = batch_blk_steps(b);
+    if (T) return batch_run_blocks(b, nsteps, T);
+    int rc = batch_rings(b);
     if (rc) return rc;
+    if ((rc = batch_order(b, true))) return rc;
+    if (b->graph && b->graph_steps) batch_drop_graph(b);
     const int M = (int)b->nets.size();
     bg3::launch_neurons_batch(b->d_nets, M, b->max_n, b->stream);
     bg3::launch_deliver_batch(b->syn_kind, b->d_nets, M, b->cfg, b->stream);
@@ -1668,6 +1904,9 @@ int bg3_bench_steps(bg3_net *n, int64_t nsteps, int64_t flush_bytes, float *step
         CK(cudaMemsetAsync(n->scrub_buf, 0, (size_t)flush_bytes + 16, n->stream));
         n->flush_size = (size_t)flush_bytes;
     }
+    const int ring_rc = ensure_ring(n);
+    if (ring_rc) return ring_rc;
+    n->mask_ok = false;
     const NetDev &h = n->h;
     const bool inject = h.noise_mode == BG3_NOISE_INJECT;
     std::vector<cudaEvent_t> ev((size_t)nsteps * 3);
@@ -1733,8 +1972,9 @@ int bg3_batch_bench_steps(bg3_batch *b, int64_t nsteps, int64_t flush_bytes, flo
         CK(cudaMemsetAsync(b->scrub_buf, 0, (size_t)flush_bytes + 16, b->stream));
         b->flush_size = (size_t)flush_bytes;
     }
-    int rc = batch_order(b, true);
+    int rc = batch_rings(b);
     if (rc) return rc;
+    if ((rc = batch_order(b, true))) return rc;
     const int M = (int)b->nets.size();
     std::vector<cudaEvent_t> ev((size_t)nsteps * 2);
     for (auto &e : ev) CK(cudaEventCreate(&e));
@@ -1855,6 +2095,8 @@ struct StateCopy {
 static int state_save(bg3_net *n, StateCopy &sc)
 {
     sc.parts.clear();
+    const int rc = ensure_ring(n);
+    if (rc) return rc;
     for (auto &a : n->allocs)
         if (a.first) sc.parts.push_back(a);
     if (n->noise_dev) sc.parts.push_back(std::make_pair((void *)n->noise_dev, (size_t)n->noise_cap * sizeof(float)));
@@ -1877,6 +2119,7 @@ static int state_save(bg3_net *n, StateCopy &sc)
 
 static int state_load(bg3_net *n, const StateCopy &sc)
 {
+    ring_changed(n);
     size_t off = 0;
     for (auto &p : sc.parts) {
         CK(cudaMemcpyAsync(p.first, (const char *)sc.buf + off, p.second, cudaMemcpyDeviceToDevice, n->stream));
@@ -2245,6 +2488,8 @@ extern "C" {
 int bg3_checkpoint_save(bg3_net *n, void *buf, uint64_t cap, uint64_t *len)
 {
     if (!n || !len) return BG3_EINVAL;
+    const int ring_rc = ensure_ring(n);
+    if (ring_rc) return ring_rc;
     CK(cudaStreamSynchronize(n->stream));
     const NetDev &h = n->h;
     uint64_t arrays = 0, named = 0;
@@ -2393,6 +2638,8 @@ int bg3_checkpoint_load(bg3_net *n, const void *buf, uint64_t len)
     // ---- second phase: nothing above changed the network ----
     CK(cudaStreamSynchronize(n->stream));
     drop_graph(n);
+    ring_changed(n);
+    n->hist_given = true;
 #define BG3_LOAD_ONE(f)                                                                           \
     {                                                                                             \
         if ((rc = aresize(n, h.f, (size_t)as[CKA_##f]))) return rc;                               \

@@ -188,6 +188,20 @@ struct NetDev {
     const float *p_xD[BG3_MAX_PCLS], *p_xF[BG3_MAX_PCLS];
 };
 
+// Spike masks of the block kernels (bg3_block.cu), beside the network's arrays: what the spike
+// ring holds, by neuron instead of by step.  They follow from the ring and are rebuilt from it, so
+// no checkpoint holds them.
+constexpr int BLK_MAX_STEPS = 8;   // most steps advanced per pass over a network's state
+constexpr int BLK_ACT_ROWS = 16;   // blocks start at most 8 steps apart: two rows never meet
+struct BlkDev {
+    unsigned long long *hist;  // [Np] bit s & 63: the neuron fired at step s (last 64 steps)
+    // [BLK_ACT_ROWS][ntiles] row t & 15: the neurons of a 32-neuron tile with a spike that may
+    // arrive in a block starting at step t (any delay class)
+    uint32_t *act;
+    // bit s & 63 for the steps s whose spikes may arrive in a block starting at step 0
+    unsigned long long win;
+};
+
 // device error word bits (mirrored in include/bg3.h)
 enum : uint32_t {
     ERR_HISTORY_OVERFLOW = 1u << 0,
@@ -643,6 +657,29 @@ __device__ __forceinline__ float izh_v_ff(float Vint, float u, float C3, float c
     return Vnew;
 }
 
+// The same expression in integer-pipe binary64 (SoftD); ok = false outside its range.  Not
+// inlined: a launch option, kept out of the step loops' instruction footprint.
+static __device__ __noinline__ float izh_v_soft(float Vint, float u, float C3, float c2sp, bool &ok)
+{
+    // the double constants 0.04, 140.0 and 0.001 as (mantissa, exponent, sign)
+    constexpr SoftD K004 = {0x147ae147ae147bull, -5, 0u};
+    constexpr SoftD K140 = {0x11800000000000ull, 7, 0u};
+    constexpr SoftD K0001 = {0x10624dd2f1a9fcull, -10, 0u};
+    const SoftD vd = sd_from_float(Vint, ok);
+    SoftD t = sd_mul(K004, vd, ok);
+    t = sd_mul(t, vd, ok);
+    t = sd_add(t, sd_from_float(5.0f * Vint, ok), ok);
+    t = sd_add(t, K140, ok);
+    SoftD nu = sd_from_float(u, ok);
+    nu.s ^= 1u;
+    t = sd_add(t, nu, ok);
+    t = sd_mul(sd_from_float(C3, ok), t, ok);
+    const float Vb = sd_to_float(sd_add(vd, t, ok), ok);
+    SoftD w = sd_mul(sd_from_float(Vb, ok), K0001, ok);
+    w = sd_add(w, sd_from_float(c2sp, ok), ok);
+    return sd_to_float(w, ok);
+}
+
 // How a neuron's Izhikevich double expression is evaluated: the integer-pipe restatement, the
 // hardware FP64 pipe, or float-float arithmetic with the FP64 pipe for uncertain roundings (the
 // same bits every way).
@@ -654,17 +691,19 @@ __device__ __forceinline__ int izh_mode(const NetDev &n, int i)
     return IZH_SOFT;
 }
 
+// One step's update of a neuron held in x: Vm, refr and u change there, the spike history and
+// count in memory.
 // mode: IZH_SOFT, IZH_HW or IZH_FF (izh_mode); the same bits every way.  FFOK = false compiles
 // the float-float branch out (IZH_FF then takes the FP64 pipe), for kernels without registers
 // to spare.
 template <bool FFOK = true>
-__device__ __forceinline__ bool neuron_apply(const NetDev &n, int i, const NeuronIn &x, int br,
-                                             float sp, float noise, unsigned long long t,
-                                             int mode = IZH_SOFT)
+__device__ __forceinline__ bool neuron_update(const NetDev &n, int i, NeuronIn &x, int br,
+                                              float sp, float noise, unsigned long long t,
+                                              int mode = IZH_SOFT)
 {
     const bool izh = n.neuron_kind == 1;
     if (br == BR_REFRACTORY) {
-        gst(&n.refr[i], x.refr - 1);
+        x.refr = x.refr - 1;
         return false;
     }
     if (br == BR_FIRE) {
@@ -674,12 +713,12 @@ __device__ __forceinline__ bool neuron_apply(const NetDev &n, int i, const Neuro
         cnt += 1;
         gst(&n.spikeCount[i], cnt);
         if (cnt >= n.max_spikes) set_err(n, ERR_HISTORY_OVERFLOW);
-        gst(&n.refr[i], (int)((double)(x.Trefract / n.dt) + 0.5));
+        x.refr = (int)((double)(x.Trefract / n.dt) + 0.5);
         if (izh) {
-            gst(&n.Vm[i], (float)((double)x.Cc * 0.001));
-            gst(&n.u_izh[i], x.u + x.Dd);
+            x.Vm = (float)((double)x.Cc * 0.001);
+            x.u = x.u + x.Dd;
         } else {
-            gst(&n.Vm[i], n.Vreset[i]);
+            x.Vm = n.Vreset[i];
         }
         return true;
     }
@@ -691,7 +730,6 @@ __device__ __forceinline__ bool neuron_apply(const NetDev &n, int i, const Neuro
         const float u = x.u, C3 = x.C3;
         // Vb = (float)(v + C3 * (0.04 v v + (double)(5 v) + 140 - u)), then
         // Vm = (float)((double)Vb * 0.001 + (double)(C2 sp)), each double operation rounded once
-        // the double constants 0.04, 140.0 and 0.001 as (mantissa, exponent, sign)
         float Vnew;
         bool ffok = false;
         if (FFOK && mode == IZH_FF) {
@@ -700,31 +738,32 @@ __device__ __forceinline__ bool neuron_apply(const NetDev &n, int i, const Neuro
         } else if (mode == IZH_HW || mode == IZH_FF) {
             Vnew = izh_v_fp64(Vint, u, C3, x.C2 * sp);
         } else {
-            constexpr SoftD K004 = {0x147ae147ae147bull, -5, 0u};
-            constexpr SoftD K140 = {0x11800000000000ull, 7, 0u};
-            constexpr SoftD K0001 = {0x10624dd2f1a9fcull, -10, 0u};
             bool ok = true;
-            const SoftD vd = sd_from_float(Vint, ok);
-            SoftD t = sd_mul(K004, vd, ok);
-            t = sd_mul(t, vd, ok);
-            t = sd_add(t, sd_from_float(5.0f * Vint, ok), ok);
-            t = sd_add(t, K140, ok);
-            SoftD nu = sd_from_float(u, ok);
-            nu.s ^= 1u;
-            t = sd_add(t, nu, ok);
-            t = sd_mul(sd_from_float(C3, ok), t, ok);
-            const float Vb = sd_to_float(sd_add(vd, t, ok), ok);
-            SoftD w = sd_mul(sd_from_float(Vb, ok), K0001, ok);
-            w = sd_add(w, sd_from_float(x.C2 * sp, ok), ok);
-            Vnew = sd_to_float(w, ok);
+            Vnew = izh_v_soft(Vint, u, C3, x.C2 * sp, ok);
             if (!ok) Vnew = izh_v_fp64(Vint, u, C3, x.C2 * sp);  // outside the restated range
         }
-        gst(&n.u_izh[i], u + C3 * x.A * (x.B * Vint - u));
-        gst(&n.Vm[i], Vnew);
+        x.u = u + C3 * x.A * (x.B * Vint - u);
+        x.Vm = Vnew;
     } else {
-        gst(&n.Vm[i], x.C1 * x.Vm + x.C2 * sp);
+        x.Vm = x.C1 * x.Vm + x.C2 * sp;
     }
     return false;
+}
+
+// One step's update with the changed state stored.
+template <bool FFOK = true>
+__device__ __forceinline__ bool neuron_apply(const NetDev &n, int i, const NeuronIn &x, int br,
+                                             float sp, float noise, unsigned long long t,
+                                             int mode = IZH_SOFT)
+{
+    NeuronIn y = x;
+    const bool fired = neuron_update<FFOK>(n, i, y, br, sp, noise, t, mode);
+    if (br != BR_INTEGRATE) gst(&n.refr[i], y.refr);
+    if (br != BR_REFRACTORY) {
+        gst(&n.Vm[i], y.Vm);
+        if (n.neuron_kind == 1) gst(&n.u_izh[i], y.u);
+    }
+    return fired;
 }
 
 // ---- external input, applied to the summation point before the neuron update ----------------
@@ -754,9 +793,9 @@ __device__ __forceinline__ int32_t next_isi(const NetDev &n, int i)
 
 // HostSInputRegular::inputStimulus (Inputs/HostSInputRegular.cpp:59-80) and
 // HostSInputPoisson::inputStimulus (Inputs/HostSInputPoisson.cpp:60-94) for neuron i at step t:
-// returns the summation point after the input.
-__device__ __forceinline__ float input_apply(const NetDev &n, int i, const NeuronIn &x,
-                                             unsigned long long t, float sp)
+// returns the summation point after the input; the input synapse's state changes in x.
+__device__ __forceinline__ float input_update(const NetDev &n, int i, NeuronIn &x,
+                                              unsigned long long t, float sp)
 {
     if (n.input_kind == 1) {
         const int cyc = (int)(((unsigned long long)n.reg_c0 + (t - n.reg_t0)) % (unsigned long long)n.reg_cycle);
@@ -769,7 +808,7 @@ __device__ __forceinline__ float input_apply(const NetDev &n, int i, const Neuro
             q |= 1u << ((uint32_t)(t + x.idelay) & 31u);
             c = next_isi(n, i);
         }
-        gst(&n.pois_nisi[i], c);
+        x.nisi = c;
         const uint32_t bit = 1u << ((uint32_t)t & 31u);
         float psr = x.ipsr;
         const float dec = x.idec;
@@ -783,10 +822,24 @@ __device__ __forceinline__ float input_apply(const NetDev &n, int i, const Neuro
             gst(&n.in_ev[i].r, r);
             gst(&n.in_ev[i].last, (uint32_t)t);
         }
-        gst(&n.in_queue[i], q);
+        x.q = q;
         psr = psr * dec;
-        gst(&n.in_psr[i], psr);
+        x.ipsr = psr;
         sp = sp + psr;
+    }
+    return sp;
+}
+
+// One step's input with the changed state stored.
+__device__ __forceinline__ float input_apply(const NetDev &n, int i, const NeuronIn &x,
+                                             unsigned long long t, float sp)
+{
+    NeuronIn y = x;
+    sp = input_update(n, i, y, t, sp);
+    if (n.input_kind == 2 && x.pmask) {
+        gst(&n.pois_nisi[i], y.nisi);
+        gst(&n.in_queue[i], y.q);
+        gst(&n.in_psr[i], y.ipsr);
     }
     return sp;
 }

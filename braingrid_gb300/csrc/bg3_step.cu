@@ -20,6 +20,7 @@
 #include <utility>
 #include "bg3_internal.cuh"
 #include "bg3_ptx.cuh"
+#include "bg3_stdp.cuh"
 
 namespace bg3 {
 
@@ -239,233 +240,6 @@ __global__ void __launch_bounds__(1024) k_neurons_inject_apply(const __grid_cons
         for (int k = 0; k < nb; k++) tot += n.outFill[k];
         *n.noise_cursor = cursor + (unsigned long long)tot;
     }
-}
-
-// ---- STDP ------------------------------------------------------------------------------------
-// AllSTDPSynapses::advanceSynapse / stdpLearning (Synapses/AllSTDPSynapses.cpp:283-472) and the
-// device form advanceSTDPSynapsesDevice (AllSynapsesDeviceFuncs_d.cu:100-380).  The only
-// difference between the two builds is the type of the spike times in the interval arithmetic:
-// uint64_t on the host (a pre-spike walk interval wraps to a huge positive value), int64_t on
-// the device.  Each float / double operation rounds as in the reference; the exp factors come
-// from the host library's tables.
-
-// getSpikeHistory (Neurons/AllSpikingNeurons.cpp:182-188) for off in [-max_spikes, -1];
-// co = spikeCount + spikeCountOffset.
-__device__ __forceinline__ unsigned long long hist_at(const NetDev &n, int i, int co, int off)
-{
-    const int x = (co + n.max_spikes + off) % n.max_spikes;
-    return n.history[(size_t)i * n.max_spikes + x];
-}
-
-// W^mu with mu = 0, the only exponent a network accepts (set_stdp_type refuses others)
-__device__ __forceinline__ float pow_mu(float, float) { return 1.0f; }
-
-// One stdpLearning call with delta = dk steps (dk the signed interval; 0 when not a small count),
-// in two parts.  stdp_inc: the weight change, which W does not enter (W^mu = 1): false when delta
-// lies within the gap (W unchanged, no clamp), else epost * epre * dw in double.  stdp_apply: W
-// plus that change, rounded to float, then the clamps.  So the walks below can find a walk's
-// changes before W is known and apply them in order after.
-__device__ __forceinline__ bool stdp_inc(const StdpConst &c, float delta, float epost, float epre,
-                                         long long dk, double &inc)
-{
-    const double d = (double)delta;
-    float dw;
-    if (d < (double)(-c.gap)) {
-        const double e = (dk < 0 && -dk < (long long)c.dlen_neg) ? c.dneg[-dk] : exp(d / (double)c.tauneg);
-        dw = (float)((double)(pow_mu(0.0f, c.muneg) * c.Aneg) * e);
-    } else if (d > (double)c.gap) {
-        const double e = (dk > 0 && dk < (long long)c.dlen_pos) ? c.dpos[dk] : exp(-d / (double)c.taupos);
-        dw = (float)((double)(pow_mu(0.0f, c.mupos) * c.Apos) * e);
-    } else {
-        return false;
-    }
-    inc = (double)epost * (double)epre * (double)dw;
-    return true;
-}
-__device__ __forceinline__ float stdp_apply(const StdpConst &c, float W, double inc)
-{
-    W = (float)((double)W + inc);
-    if ((c.Wex < 0.0f && W > 0.0f) || (c.Wex > 0.0f && W < 0.0f)) W = 0.0f;
-    if (fabsf(W) > fabsf(c.Wex)) W = c.Wex;
-    return W;
-}
-__device__ __forceinline__ float stdp_learn(const StdpConst &c, float W, float delta, float epost,
-                                            float epre, long long dk)
-{
-    double inc;
-    return stdp_inc(c, delta, epost, epre, dk, inc) ? stdp_apply(c, W, inc) : W;
-}
-
-// A neuron's history entries -1 .. -4 read together (those of them that exist: off >= -ms), so
-// that a walk's first steps do not wait on one load each; hist_get takes the rest from memory.
-struct Hist4 {
-    unsigned long long h0, h1, h2, h3;
-};
-__device__ __forceinline__ void hist_load4(const NetDev &n, int i, int co, Hist4 &c)
-{
-    const int ms = n.max_spikes;
-    c.h0 = hist_at(n, i, co, -1);  // max_spikes >= 1
-    c.h1 = ms >= 2 ? hist_at(n, i, co, -2) : BG3_ULONG_MAX;
-    c.h2 = ms >= 3 ? hist_at(n, i, co, -3) : BG3_ULONG_MAX;
-    c.h3 = ms >= 4 ? hist_at(n, i, co, -4) : BG3_ULONG_MAX;
-}
-// entry off (-ms <= off <= -1)
-__device__ __forceinline__ unsigned long long hist_get(const NetDev &n, int i, int co, int off,
-                                                       const Hist4 &c)
-{
-    return off == -1 ? c.h0 : off == -2 ? c.h1 : off == -3 ? c.h2 : off == -4 ? c.h3
-                                                                    : hist_at(n, i, co, off);
-}
-
-// The fPre branch: a spike from pre arrives at the synapse onto post at step t.  Returns W.
-__device__ float stdp_pre(const NetDev &n, const StdpConst &c, float W, int pre, int post,
-                          unsigned long long t)
-{
-    const int ms = n.max_spikes;
-    const int cpost = n.spikeCount[post] + n.spikeCountOffset[post];
-    if (!n.stdp_signed) {
-        // Every interval (spikeHistory - step) wraps to ~1.8e15 s (or is 0 at step t): each
-        // learning call potentiates by exactly zero and applies the clamps, so only whether one
-        // happens matters: the walk runs while entries -k and -(k+1) are valid.
-        const unsigned long long h1 = hist_at(n, post, cpost, -1);
-        const unsigned long long h2 = hist_at(n, post, cpost, -2);
-        if (hist_at(n, post, cpost, -ms) != BG3_ULONG_MAX) set_err(n, ERR_STDP_RING);
-        bool learn;
-        if (c.useFD) {
-            const unsigned long long h3 = hist_at(n, post, cpost, -3);
-            learn = h1 != BG3_ULONG_MAX && h2 != BG3_ULONG_MAX && (h1 != t || h3 != BG3_ULONG_MAX);
-        } else {
-            learn = h1 != BG3_ULONG_MAX && (h1 != t || h2 != BG3_ULONG_MAX);
-        }
-        if (learn) {
-            // potentiation by (float)(x * exp(-huge)) = +-0; epost * epre >= 0 keeps dw's sign
-            const float dw = (float)((double)(pow_mu(c.Wex - W, c.mupos) * c.Apos) * 0.0);
-            W = (float)((double)W + (double)dw);
-            if ((c.Wex < 0.0f && W > 0.0f) || (c.Wex > 0.0f && W < 0.0f)) W = 0.0f;
-            if (fabsf(W) > fabsf(c.Wex)) W = c.Wex;
-        }
-        return W;
-    }
-    const int cpre = n.spikeCount[pre] + n.spikeCountOffset[pre];
-    Hist4 hp;
-    hist_load4(n, post, cpost, hp);
-    const unsigned long long sp2 = hist_at(n, pre, cpre, -2);
-    float epre = 1.0f;
-    if ((long long)sp2 > 0 && c.useFD)
-        epre = (float)(1.0 - (double)exp_interval(n, t - sp2, true, c.tauspre));
-    for (int off = -1;; --off) {
-        if (off < -ms) { set_err(n, ERR_STDP_RING); break; }
-        const unsigned long long sh = hist_get(n, post, cpost, off, hp);
-        if (sh == BG3_ULONG_MAX) break;
-        const long long dk = (long long)(sh - t);
-        const float delta = (float)dk * n.dt;
-        if ((double)delta <= -3.0 * (double)c.tauneg) break;
-        float epost = 1.0f;
-        if (c.useFD) {
-            if (off - 1 < -ms) { set_err(n, ERR_STDP_RING); break; }
-            const unsigned long long sh2 = hist_get(n, post, cpost, off - 1, hp);
-            if (sh2 == BG3_ULONG_MAX) break;
-            epost = (float)(1.0 - (double)exp_interval(n, sh - sh2, true, c.tauspost));
-        }
-        W = stdp_learn(c, W, delta, epost, epre, dk);
-    }
-    return W;
-}
-
-// The fPost branch: post fired at step t; walk the pre history (both builds agree here).  The
-// walk does not depend on W, so it runs in two parts: stdp_post_prep reads everything it needs
-// (spike counts, histories, tables) and makes its first four steps, keeping their weight changes;
-// stdp_post_finish applies them to W and makes any further steps.  The post-spike pass calls
-// the first before its wait on the delivery of the same step (the one writer of W there).
-constexpr int POST_STEPS = 4;
-struct PostPrep {
-    double inc0, inc1, inc2, inc3;  // the changes of steps 1 .. 4 (those with a bit in mask)
-    float epost;
-    int cpre;
-    int mask;                       // bit k: step k + 1 changed W
-    int next;                       // 0: the walk has ended; else the entry it continues from
-};
-__device__ __forceinline__ void stdp_post_prep(const NetDev &n, const StdpConst &c, int pre,
-                                               int post, int total_delay, unsigned long long t,
-                                               PostPrep &q)
-{
-    const int ms = n.max_spikes;
-    const bool sgn = n.stdp_signed != 0;
-    const int cpost = n.spikeCount[post] + n.spikeCountOffset[post];
-    const int cpre = n.spikeCount[pre] + n.spikeCountOffset[pre];
-    const unsigned long long q2 = hist_at(n, post, cpost, -2);
-    Hist4 hp;
-    hist_load4(n, pre, cpre, hp);
-    float epost = 1.0f;
-    const bool ok = sgn ? ((long long)q2 > 0) : (q2 != BG3_ULONG_MAX);
-    if (ok && c.useFD) epost = (float)(1.0 - (double)exp_interval(n, t - q2, sgn, c.tauspost));
-    q.epost = epost;
-    q.cpre = cpre;
-    q.mask = 0;
-    q.next = 0;
-    q.inc0 = q.inc1 = q.inc2 = q.inc3 = 0.0;
-#pragma unroll
-    for (int k = 0; k < POST_STEPS; k++) {
-        const int off = -1 - k;
-        if (off < -ms) { set_err(n, ERR_STDP_RING); return; }
-        const unsigned long long sh = hist_get(n, pre, cpre, off, hp);
-        if (sh == BG3_ULONG_MAX) return;
-        const unsigned long long dd = t - (unsigned long long)(long long)total_delay - sh;
-        const float delta = (sgn ? (float)(long long)dd : (float)dd) * n.dt;
-        if (delta <= 0.0f || (double)delta >= 3.0 * (double)c.taupos) return;
-        float epre = 1.0f;
-        if (c.useFD) {
-            if (off - 1 < -ms) { set_err(n, ERR_STDP_RING); return; }
-            const unsigned long long sh2 = hist_get(n, pre, cpre, off - 1, hp);
-            if (sh2 == BG3_ULONG_MAX) return;
-            epre = (float)(1.0 - (double)exp_interval(n, sh - sh2, sgn, c.tauspre));
-        }
-        double inc;
-        if (stdp_inc(c, delta, epost, epre, (long long)dd, inc)) {
-            q.mask |= 1 << k;
-            if (k == 0) q.inc0 = inc;
-            else if (k == 1) q.inc1 = inc;
-            else if (k == 2) q.inc2 = inc;
-            else q.inc3 = inc;
-        }
-    }
-    q.next = -1 - POST_STEPS;
-}
-__device__ __forceinline__ float stdp_post_finish(const NetDev &n, const StdpConst &c, float W,
-                                                  int pre, int total_delay, unsigned long long t,
-                                                  const PostPrep &q)
-{
-    if (q.mask & 1) W = stdp_apply(c, W, q.inc0);
-    if (q.mask & 2) W = stdp_apply(c, W, q.inc1);
-    if (q.mask & 4) W = stdp_apply(c, W, q.inc2);
-    if (q.mask & 8) W = stdp_apply(c, W, q.inc3);
-    if (!q.next) return W;
-    const int ms = n.max_spikes;
-    const bool sgn = n.stdp_signed != 0;
-    for (int off = q.next;; --off) {
-        if (off < -ms) { set_err(n, ERR_STDP_RING); break; }
-        const unsigned long long sh = hist_at(n, pre, q.cpre, off);
-        if (sh == BG3_ULONG_MAX) break;
-        const unsigned long long dd = t - (unsigned long long)(long long)total_delay - sh;
-        const float delta = (sgn ? (float)(long long)dd : (float)dd) * n.dt;
-        if (delta <= 0.0f || (double)delta >= 3.0 * (double)c.taupos) break;
-        float epre = 1.0f;
-        if (c.useFD) {
-            if (off - 1 < -ms) { set_err(n, ERR_STDP_RING); break; }
-            const unsigned long long sh2 = hist_at(n, pre, q.cpre, off - 1);
-            if (sh2 == BG3_ULONG_MAX) break;
-            epre = (float)(1.0 - (double)exp_interval(n, sh - sh2, sgn, c.tauspre));
-        }
-        W = stdp_learn(c, W, delta, q.epost, epre, (long long)dd);
-    }
-    return W;
-}
-__device__ float stdp_post(const NetDev &n, const StdpConst &c, float W, int pre, int post,
-                           int total_delay, unsigned long long t)
-{
-    PostPrep q;
-    stdp_post_prep(n, c, pre, post, total_delay, t, q);
-    return stdp_post_finish(n, c, W, pre, total_delay, t, q);
 }
 
 // ---- spike arrival ---------------------------------------------------------------------------

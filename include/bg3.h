@@ -428,8 +428,9 @@ typedef struct {
     int32_t small_max_slots;  /* a network of at most 2,048 neurons whose synapse planes hold at most
                                  this many slots (neurons rounded up to 32 x max synapses rounded up
                                  to 4) runs up to 4,096 whole steps per launch on one CTA, with no
-                                 launch between its passes (default 65,536; 0: never).  Same
-                                 results either way.                                                */
+                                 launch between its passes (default 65,536; 0: never, and no network
+                                 runs several steps per launch: the per-step kernels).  Same results
+                                 either way.                                                        */
 } bg3_launch_cfg;
 int bg3_get_launch(bg3_net *net, bg3_launch_cfg *cfg);
 int bg3_set_launch(bg3_net *net, const bg3_launch_cfg *cfg);

@@ -1,0 +1,128 @@
+"""Blocks of steps (bg3_block.cu) against the per-step kernels, bit for bit: the same network
+advanced by both (small_max_slots 0 keeps a network on the per-step kernels, 1 keeps it off the
+one-launch path of small networks), at sizes around the 32-neuron tiles, the row quads and the
+eight steps of a block, with downloads, epoch ends and single steps in between."""
+import numpy as np
+import pytest
+
+from braingrid_gb300 import lib as bg
+from braingrid_gb300 import netgen
+
+pytestmark = pytest.mark.gpu
+
+STEPS = (1, 8, 7, 9, 131, 3)   # remainders of a block, a graph's worth of blocks
+
+
+def lif(w, h, syn, radius, drive, max_syn, seed=5):
+    spec = netgen.lif_network(w, h, seed=seed)
+    # membranes near threshold: the network fires, and its spikes arrive, from the first steps
+    spec["Vm"] = np.random.RandomState(seed).uniform(13.2e-3, 15.2e-3, spec["N"]).astype(np.float32)
+    net = bg.Network(spec["N"], max_syn, w, h, 0.1, 1e-4, 1000, 4, syn, bg.BG3_NOISE_DEVICE, seed)
+    netgen.configure_lif(net, spec)
+    if syn >= bg.BG3_SYN_STDP:
+        net.set_stdp_constants(**netgen.STDP_ADDITIVE)
+    if radius:
+        netgen.pregrow(net, spec, radius, weight_scale=0.3)
+    rs = np.random.RandomState(seed + 1)
+    if drive == "poisson":
+        arr, lam = netgen.poisson_arrays(spec, 40.0, 9.5)
+        net.input_poisson(lam, seed=seed, step=0, **arr)
+    elif drive == "regular":
+        net.input_regular(np.full(spec["N"], 4e-9, np.float32), rs.randint(0, 40, spec["N"]), 20, 60)
+    return net
+
+
+def izh(w, h, seed=5):
+    net = netgen.make_izh_static(w, h, seed, epoch_duration=0.1)[1]
+    net.set_launch(small_max_slots=0)
+    net.step(900)      # per-step kernels, until STDP and the drive have the network firing
+    net.record()
+    return net
+
+
+def state(net):
+    out = dict(net.download_lif())
+    out.update({"syn_" + k: v for k, v in net.download_synapses().items()})
+    if net.desc.neuron_kind == bg.BG3_NEURON_IZH:
+        out.update({"izh_" + k: v for k, v in net.download_izh().items()})
+    out["step"], out["err"] = net.sim_step, net.error_word
+    return out
+
+
+def same(a, b, what):
+    x, y = state(a), state(b)
+    for k in x:
+        u, v = np.asarray(x[k]), np.asarray(y[k])
+        if u.dtype == np.float32:
+            u, v = u.view(np.uint32), v.view(np.uint32)
+        assert np.array_equal(u, v), "%s: %s differs at %s" % (what, k, np.nonzero(u != v)[0][:5])
+
+
+def advance(make, end="record"):
+    blocks, plain = make(), make()
+    blocks.set_launch(small_max_slots=1)
+    plain.set_launch(small_max_slots=0)
+    spikes = 0
+    for i, n in enumerate(STEPS):
+        b0 = blocks.launches
+        blocks.step(n)
+        plain.step(n)
+        assert blocks.launches - b0 <= 2 * ((n + 7) // 8)     # it did run in blocks
+        if i % 2:
+            same(blocks, plain, "after call %d (%d steps)" % (i, n))
+            spikes = max(spikes, int(blocks.download_lif(fields=("spikeCount",))["spikeCount"].sum()))
+    if end == "growth":
+        blocks.growth(1)
+        plain.growth(1)
+    else:
+        blocks.record()
+        plain.record()
+    # masks -> ring -> masks: per-step kernels for a while, then blocks again
+    blocks.set_launch(small_max_slots=0)
+    blocks.step(5)
+    plain.step(5)
+    blocks.set_launch(small_max_slots=1)
+    blocks.step(40)
+    plain.step(40)
+    same(blocks, plain, "after the epoch end")
+    assert spikes > 0
+    assert blocks.error_word == 0
+    for net in (blocks, plain):
+        net.close()
+
+
+@pytest.mark.parametrize("syn", [bg.BG3_SYN_SPIKING, bg.BG3_SYN_DS, bg.BG3_SYN_STDP, bg.BG3_SYN_DYNSTDP])
+@pytest.mark.parametrize("w,h,radius,drive,max_syn", [
+    (9, 7, 1.2, "none", 30),        # 63 neurons, a partial last quad
+    (13, 5, 1.5, "poisson", 33),    # 65 neurons: one past a tile
+    (8, 4, 0.0, "regular", 4),      # one tile, no synapse
+    (40, 33, 1.9, "poisson", 64),   # the widest rows of a thin tile
+])
+def test_thin_blocks_equal_steps(syn, w, h, radius, drive, max_syn):
+    advance(lambda: lif(w, h, syn, radius, drive, max_syn), end="growth")
+
+
+@pytest.mark.parametrize("w,h", [(9, 7), (13, 5), (60, 41)])
+def test_izhikevich_stdp_blocks_equal_steps(w, h):
+    advance(lambda: izh(w, h))
+
+
+def test_batched_blocks_equal_steps():
+    shapes = [(9, 7), (13, 5), (32, 20), (25, 41)]
+    a, b = [izh(w, h, 20 + w) for w, h in shapes], [izh(w, h, 20 + w) for w, h in shapes]
+    batch = bg.Batch(a)
+    for n in STEPS:
+        batch.step(n)
+        for net in b:
+            net.step(n)
+    batch.sync()
+    for x, y in zip(a, b):
+        same(x, y, "batched")
+    batch.set_launch(small_max_slots=0)     # the batch's per-step kernels, and back
+    batch.step(3)
+    batch.set_launch(small_max_slots=65536)
+    batch.step(21)
+    for x, y in zip(a, b):
+        y.step(24)
+        same(x, y, "batched, after per-step kernels")
+    batch.close()
