@@ -36,6 +36,12 @@ void launch_rebuild_maps(const NetDev &h, const NetDev *d_net, cudaStream_t s);
 void launch_scale_weights(const NetDev &h, float f, cudaStream_t s);
 void launch_record(const NetDev &h, const NetDev *d_net, cudaStream_t s);
 bool blk_thin_ok(int Mq);
+bool blk_dense_ok(int Mq);
+void launch_blk_range(const NetDev &h, const BlkDev &b, cudaStream_t s);
+void launch_blk_dense(const NetDev &h, const BlkDev &b, const CUtensorMap &tp, const CUtensorMap &tc,
+                      int nt, cudaStream_t s);
+void launch_blk_dense_batch(int syn_kind, const NetDev *nets, const BlkDev *blks,
+                            const CUtensorMap *maps, const int2 *tiles, int n, int nt, cudaStream_t s);
 void launch_blk_masks(const NetDev &h, const BlkDev &b, cudaStream_t s);
 void launch_blk_ring(const NetDev &h, const BlkDev &b, cudaStream_t s);
 void launch_blk_thin(const NetDev &h, const BlkDev &b, int nt, cudaStream_t s);
@@ -76,6 +82,7 @@ struct bg3_net {
     // whichever ran last is current, the other is rebuilt when it is needed
     BlkDev blk = {};
     bool ring_ok = true, mask_ok = false;
+    bool range_ok = false;    // blk.range follows the synapses
     // fewest steps between two spikes of a neuron, for the block kernels' STDP ring rule: the
     // shortest refractory period + 1, or 1 once spike histories were uploaded
     int min_isi = 1;
@@ -108,7 +115,14 @@ static int dalloc(bg3_net *n, T **p, size_t count, int fill = 0)
 }
 
 static size_t blk_act_bytes(size_t Np) { return BLK_ACT_ROWS * (Np / 32) * sizeof(uint32_t); }
-static size_t blk_bytes(size_t Np) { return Np * sizeof(unsigned long long) + blk_act_bytes(Np); }
+static size_t blk_range_bytes(size_t Np, int Mq)
+{
+    return bg3::blk_thin_ok(Mq) || !bg3::blk_dense_ok(Mq) ? 0 : Np / 32 * (size_t)Mq * sizeof(uint32_t);
+}
+static size_t blk_bytes(size_t Np, int Mq)
+{
+    return Np * sizeof(unsigned long long) + blk_act_bytes(Np) + blk_range_bytes(Np, Mq);
+}
 
 static void drop_graph(bg3_net *n);
 // The step kernels take the descriptor by value (captured into the step graph); the growth
@@ -427,7 +441,9 @@ int bg3_create(const bg3_net_desc *desc, bg3_net **out)
 #undef A
     if ((rc = dalloc(n, &h.history, N * (size_t)max_spikes, 0xff)) != 0) goto fail;
     if (cudaMalloc((void **)&n->blk.hist, Np * sizeof(*n->blk.hist)) != cudaSuccess ||
-        cudaMalloc((void **)&n->blk.act, blk_act_bytes(Np)) != cudaSuccess) {
+        cudaMalloc((void **)&n->blk.act, blk_act_bytes(Np)) != cudaSuccess ||
+        (blk_range_bytes(Np, h.Mq) &&
+         cudaMalloc((void **)&n->blk.range, blk_range_bytes(Np, h.Mq)) != cudaSuccess)) {
         rc = BG3_ENOMEM;
         goto fail;
     }
@@ -505,11 +521,11 @@ int64_t bg3_net_footprint(const bg3_net_desc *desc)
     if (D.neuron_kind == BG3_NEURON_IZH) b += 6 * N * 4;
     b += N * (uint64_t)ms * 8;                                     // spike history
     b += sizeof(NetDev) + 54 * N;                                  // descriptor, input
-    b += blk_bytes((size_t)Np);                                    // spike masks
+    b += blk_bytes((size_t)Np, (int)((D.max_syn_per_neuron + 3) / 4));  // spike masks, source ranges
     return (int64_t)b;
 }
 
-uint64_t bg3_net_bytes(bg3_net *n) { return n ? n->bytes + sizeof(NetDev) + blk_bytes((size_t)n->h.Np) : 0; }
+uint64_t bg3_net_bytes(bg3_net *n) { return n ? n->bytes + sizeof(NetDev) + blk_bytes((size_t)n->h.Np, n->h.Mq) : 0; }
 
 int bg3_set_device(int32_t device)
 {
@@ -541,6 +557,7 @@ int bg3_destroy(bg3_net *n)
     if (n->d) cudaFree(n->d);
     if (n->blk.hist) cudaFree(n->blk.hist);
     if (n->blk.act) cudaFree(n->blk.act);
+    if (n->blk.range) cudaFree(n->blk.range);
     if (n->noise_dev) cudaFree(n->noise_dev);
     if (n->flush_buf) cudaFree(n->flush_buf);
     if (n->scrub_buf) cudaFree(n->scrub_buf);
@@ -576,6 +593,7 @@ static void ring_changed(bg3_net *n)
 {
     n->ring_ok = true;
     n->mask_ok = false;
+    n->range_ok = false;  // the synapses came with it
 }
 
 // ---- uploads --------------------------------------------------------------------------------
@@ -1076,16 +1094,22 @@ static unsigned long long blk_window(const bg3_net *n)
 }
 
 // Steps per block when the network runs in blocks (bg3_block.cu), 0 when it does not (always
-// with small_max_slots 0, which asks for the per-step kernels): device noise, a thin network (one warp per tile) and delays of two steps or more.  STDP kinds: the
-// host build's spike-time arithmetic (its pre-spike walks read only the destination's own
-// history), and a history ring long enough that the spikes a block adds never overwrite an entry
-// a post-spike walk reads (entries within 3 tau+, at most one per min_isi steps).
+// with small_max_slots 0, which asks for the per-step kernels): device noise and delays of two
+// steps or more.  STDP kinds: a thin network (one warp per tile: their arrivals may have to wait
+// for the destination's own spikes), the host build's spike-time arithmetic (its pre-spike walks
+// read only the destination's own history), and a history ring long enough that the spikes a
+// block adds never overwrite an entry a post-spike walk reads (entries within 3 tau+, at most one
+// per min_isi steps).
+static bool blk_is_thin(const NetDev &h, const LaunchCfg &c)
+{
+    return bg3::sweep_is_thin(h, c) && bg3::blk_thin_ok(h.Mq);
+}
 static int blk_steps(const bg3_net *n, const LaunchCfg &c)
 {
     const NetDev &h = n->h;
-    if (c.small_max_slots == 0 || h.noise_mode != BG3_NOISE_DEVICE || !bg3::sweep_is_thin(h, c) ||
-        !bg3::blk_thin_ok(h.Mq))
-        return 0;
+    if (c.small_max_slots == 0 || h.noise_mode != BG3_NOISE_DEVICE) return 0;
+    const bool thin = blk_is_thin(h, c);
+    if (!thin && (h.syn_kind >= BG3_SYN_STDP || !bg3::blk_dense_ok(h.Mq))) return 0;
     if (h.syn_kind >= BG3_SYN_STDP) {
         if (h.stdp_signed) return 0;
         float tau = 0.0f;
@@ -1103,6 +1127,11 @@ static int blk_steps(const bg3_net *n, const LaunchCfg &c)
 static int ensure_masks(bg3_net *n)
 {
     const unsigned long long w = blk_window(n);
+    if (n->blk.range && !n->range_ok) {
+        bg3::launch_blk_range(n->h, n->blk, n->stream);
+        CK(cudaGetLastError());
+        n->range_ok = true;
+    }
     if (n->mask_ok && w == n->blk.win) return BG3_OK;
     int rc = ensure_ring(n);
     if (rc) return rc;
@@ -1124,10 +1153,15 @@ static int run_blocks(bg3_net *n, int64_t nsteps, int T)
     if (n->graph && n->graph_steps != T) drop_graph(n);
     const int64_t blocks = (nsteps + T - 1) / T;
     int64_t left = nsteps;
+    const bool thin = blk_is_thin(h, n->cfg);
+    auto one = [&](int nt) {
+        if (thin) bg3::launch_blk_thin(h, n->blk, nt, n->stream);
+        else bg3::launch_blk_dense(h, n->blk, n->tm_psr, n->tm_cls, nt, n->stream);
+    };
     if (left >= (int64_t)GRAPH_BLOCKS * T && !n->graph) {
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(n->stream, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < GRAPH_BLOCKS; i++) bg3::launch_blk_thin(h, n->blk, T, n->stream);
+        for (int i = 0; i < GRAPH_BLOCKS; i++) one(T);
         CK(cudaStreamEndCapture(n->stream, &g));
         cudaError_t e = cudaGraphInstantiate(&n->graph, g, 0);
         cudaGraphDestroy(g);
@@ -1138,8 +1172,7 @@ static int run_blocks(bg3_net *n, int64_t nsteps, int T)
         CK(cudaGraphLaunch(n->graph, n->stream));
         left -= (int64_t)GRAPH_BLOCKS * T;
     }
-    for (; left > 0; left -= T)
-        bg3::launch_blk_thin(h, n->blk, (int)std::min<int64_t>(left, T), n->stream);
+    for (; left > 0; left -= T) one((int)std::min<int64_t>(left, T));
     n->launches += blocks * (h.syn_kind >= BG3_SYN_STDP ? 2 : 1);
     CK(cudaGetLastError());
     return BG3_OK;
@@ -1235,6 +1268,7 @@ int bg3_epoch_growth(bg3_net *n, int32_t epoch)
 {
     if (!n || epoch < 0) return BG3_EINVAL;
     bg3::launch_growth(n->h, n->d, epoch, n->cfg.growth_threads, n->stream);
+    n->range_ok = false;
     n->launches += 8;
     CK(cudaGetLastError());
     return BG3_OK;
@@ -1771,13 +1805,22 @@ static void batch_drop_graph(bg3_batch *b)
 static int batch_blk_steps(const bg3_batch *b)
 {
     int T = BLK_MAX_STEPS;
-    for (const bg3_net *n : b->nets) T = std::min(T, blk_steps(n, b->cfg));
+    for (const bg3_net *n : b->nets) {
+        // the tile table's thin part is what the thin kernel takes
+        if (bg3::sweep_is_thin(n->h, b->cfg) != blk_is_thin(n->h, b->cfg)) return 0;
+        T = std::min(T, blk_steps(n, b->cfg));
+    }
     return T;
 }
 
+// The TMA-swept networks' tiles, then the thin ones'; each network is in one of the two.
 static void batch_block(bg3_batch *b, int nt)
 {
-    bg3::launch_blk_thin_batch(b->syn_kind, b->d_nets, b->d_blks, (int)b->nets.size(),
+    if (b->n_thick > 0)
+        bg3::launch_blk_dense_batch(b->syn_kind, b->d_nets, b->d_blks, b->d_maps, b->d_tiles,
+                                    b->n_thick, nt, b->stream);
+    if (b->ntiles > b->n_thick)
+        bg3::launch_blk_thin_batch(b->syn_kind, b->d_nets, b->d_blks, (int)b->nets.size(),
                                b->d_tiles + b->n_thick, b->ntiles - b->n_thick, b->cfg.thin_warps,
                                b->thin_mq, nt, b->stream);
 }
@@ -1827,7 +1870,7 @@ static int batch_run_blocks(bg3_batch *b, int64_t nsteps, int T)
         left -= (int64_t)GRAPH_BLOCKS * T;
     }
     for (; left > 0; left -= T) batch_block(b, (int)std::min<int64_t>(left, T));
-    b->launches += blocks * (b->syn_kind >= BG3_SYN_STDP ? 2 : 1);
+    b->launches += blocks * ((b->n_thick > 0) + (b->ntiles > b->n_thick) * (b->syn_kind >= BG3_SYN_STDP ? 2 : 1));
     CK(cudaGetLastError());
     return batch_order(b, false);
 }

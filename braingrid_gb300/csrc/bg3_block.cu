@@ -71,6 +71,57 @@ __global__ void __launch_bounds__(256) k_blk_ring(const __grid_constant__ NetDev
     }
 }
 
+// End of a tile's block, one lane per destination: the neuron's state and spikes stored, the
+// bitmap word for the block after this one, and from the network's last tile the step counter.
+template <int SYN>
+__device__ __forceinline__ void blk_finish(const NetDev &n, const BlkDev &b, int tile, int d,
+                                           bool valid, const NeuronIn &x, float sp,
+                                           unsigned long long hist, uint32_t fired, int nt,
+                                           unsigned long long t)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned long long t1 = t + (unsigned)nt;
+    if (valid) {
+        gst(&n.sp[d], sp);
+        gst(&n.refr[d], x.refr);
+        gst(&n.Vm[d], x.Vm);
+        if (n.neuron_kind == 1) gst(&n.u_izh[d], x.u);
+        if (n.input_kind == 2 && x.pmask) {
+            gst(&n.pois_nisi[d], x.nisi);
+            gst(&n.in_queue[d], x.q);
+            gst(&n.in_psr[d], x.ipsr);
+        }
+        hist = (hist & ~rotl64((1ull << nt) - 1ull, (unsigned)t)) | rotl64(fired, (unsigned)t);
+        gst(&b.hist[d], hist);
+    }
+    const unsigned w = __ballot_sync(0xffffffffu, (hist & rotl64(b.win, (unsigned)t1)) != 0ull);
+    if (SYN >= 2) {
+        // the neurons that fired, for the post-spike pass: in the ring slot of the block's first
+        // step (the ring's lists are rebuilt from the masks when they are needed)
+        const unsigned m = __ballot_sync(0xffffffffu, fired != 0u);
+        if (m) {
+            const int slot = (int)(t & (BG3_RING - 1));
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&n.ring_n[slot], __popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            at += __popc(m & ((1u << lane) - 1u));
+            if (fired && at < n.N) n.ring[(size_t)slot * n.N + at] = d;
+            else if (fired) set_err(n, ERR_SPIKE_LIST);
+        }
+    }
+    if (lane == 0) {
+        b.act[(t1 & (BLK_ACT_ROWS - 1)) * n.ntiles + tile] = w;
+        if (atomicAdd(n.sweep_done, 1u) == (unsigned)n.ntiles - 1u) {
+            // the network's last tile: every tile has read the step
+            *n.sweep_done = 0u;
+            *n.step = t1;
+            *n.dstep = t1;
+            n.ring_n[t1 & (BG3_RING - 1)] = 0;
+            if (t1 >= 0xffffff00ull) set_err(n, ERR_STEP_RANGE);
+        }
+    }
+}
+
 // ---- thin networks: one warp per tile ---------------------------------------------------------
 // Networks of at most BLK_THIN_QUADS row quads per destination.  The warp keeps its tile's psr in
 // shared memory for the whole block, beside the decay factors (expanded once, so that a step
@@ -295,51 +346,11 @@ __device__ __forceinline__ void blk_thin_tile(const NetDev &n, const BlkDev &b, 
         sp = acc;
     }
     for (int q = 0; q < nq; q++) gst(&P[(size_t)q * 32], s.psr[q * 32 + lane]);
-    // the neuron's state, its spikes, and the bitmap word for the block after this one
-    const unsigned long long t1 = t + (unsigned)nt;
-    if (valid) {
-        gst(&n.sp[d], sp);
-        gst(&n.refr[d], x.refr);
-        gst(&n.Vm[d], x.Vm);
-        if (n.neuron_kind == 1) gst(&n.u_izh[d], x.u);
-        if (n.input_kind == 2 && x.pmask) {
-            gst(&n.pois_nisi[d], x.nisi);
-            gst(&n.in_queue[d], x.q);
-            gst(&n.in_psr[d], x.ipsr);
-        }
-        hist = (hist & ~rotl64((1ull << nt) - 1ull, (unsigned)t)) | rotl64(fired, (unsigned)t);
-        gst(&b.hist[d], hist);
-    }
-    const unsigned w = __ballot_sync(0xffffffffu, (hist & rotl64(b.win, (unsigned)t1)) != 0ull);
-    if (SYN >= 2) {
-        // the neurons that fired, for the post-spike pass: in the ring slot of the block's first
-        // step (the ring's lists are rebuilt from the masks when they are needed)
-        const unsigned m = __ballot_sync(0xffffffffu, fired != 0u);
-        if (m) {
-            const int slot = (int)(t & (BG3_RING - 1));
-            int at = 0;
-            if (lane == 0) at = atomicAdd(&n.ring_n[slot], __popc(m));
-            at = __shfl_sync(0xffffffffu, at, 0);
-            at += __popc(m & ((1u << lane) - 1u));
-            if (fired && at < n.N) n.ring[(size_t)slot * n.N + at] = d;
-            else if (fired) set_err(n, ERR_SPIKE_LIST);
-        }
-    }
-    if (lane == 0) {
-        b.act[(t1 & (BLK_ACT_ROWS - 1)) * n.ntiles + tile] = w;
-        if (atomicAdd(n.sweep_done, 1u) == (unsigned)n.ntiles - 1u) {
-            // the network's last tile: every tile has read the step
-            *n.sweep_done = 0u;
-            *n.step = t1;
-            *n.dstep = t1;
-            n.ring_n[t1 & (BG3_RING - 1)] = 0;
-            if (t1 >= 0xffffff00ull) set_err(n, ERR_STEP_RANGE);
-        }
-    }
+    blk_finish<SYN>(n, b, tile, d, valid, x, sp, hist, fired, nt, t);
 }
 
 template <int SYN>
-__global__ void __launch_bounds__(32 * BLK_THIN_WARPS) k_blk_thin(const __grid_constant__ NetDev n,
+__global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 2) k_blk_thin(const __grid_constant__ NetDev n,
                                                                   const __grid_constant__ BlkDev b,
                                                                   int nt)
 {
@@ -354,7 +365,7 @@ __global__ void __launch_bounds__(32 * BLK_THIN_WARPS) k_blk_thin(const __grid_c
 // network, whose descriptor the block copies into shared memory first.  wsmem: bytes per warp
 // (the batch's widest thin network).
 template <int SYN>
-__global__ void __launch_bounds__(32 * BLK_THIN_WARPS) k_blk_thin_batch(const NetDev *nets,
+__global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 2) k_blk_thin_batch(const NetDev *nets,
                                                                         const BlkDev *blks,
                                                                         const int2 *tiles, int count,
                                                                         int wsmem, int nt)
@@ -442,6 +453,646 @@ __global__ void __launch_bounds__(256) k_blk_post_batch(const NetDev *nets, cons
              (gridDim.x * blockDim.x) >> 5, nt);
 }
 
+// ---- dense networks: one CTA per tile ----------------------------------------------------------
+// Networks of more row quads: the tile's psr and classes stream through shared memory in chunks of
+// 64 rows (3-D TMA boxes, DN_STAGES in flight) and each chunk is scaled and summed for all the
+// block's steps while it is there.
+//   warp 0        issues the loads; then, lane = destination, runs the neurons' steps as the sums
+//                 come in
+//   warps 1-4     arrivals: find the rows whose source has a spike arriving, prepare the psr
+//                 increments (event slots, exp tables), draw the neurons' noise
+//   warps 5, 6    lane = destination, rows in slot order: warp 5 carries a chunk through the
+//                 block's first four steps, warp 6 through the rest and stores it back.  A row is a
+//                 chain of multiplications by its decay; a step's sum is a chain of additions over
+//                 the rows, in the reference's order; four steps a warp interleave four such chains.
+// Finding the arrivals: the range of bitmap words that a row quad's sources span is kept per tile
+// (k_blk_range); only quads with a set word in their range have their sources read.  The rows are
+// taken 16 at a time, by the arrival warps in turn: hits, the sources' masks and the increments go
+// into one of four buffers of step masks and increments, which the sum warps read; groups of 16 rows
+// without a quad to look at, or without a hit in them, take code that reads none.
+constexpr int DN_ROWS = 64, DN_QUADS = 16;
+constexpr int DN_STAGES = 4;
+constexpr int DN_MAX_CHUNKS = 32;   // 2,048 slots per destination
+constexpr int DN_BUFS = 4;
+constexpr int DN_ACT_WORDS = 1280;  // the bitmap row is kept in shared memory up to 40,960 neurons
+constexpr int DN_EV_WARPS = 4;      // = DN_BUFS: buffer k is filled by warp k
+constexpr int DN_THREADS = 32 * (1 + DN_EV_WARPS + 2);
+constexpr int DN_HALF = 4;          // steps of the first sum warp
+constexpr int DN_RANGE_SCAN = 16;   // a quad spanning more bitmap words is always looked at
+constexpr uint32_t DN_CHUNK = DN_ROWS * 32 * 4 + DN_QUADS * 32 * 2;
+
+struct DenseSmem {
+    uint8_t stage[DN_STAGES][DN_CHUNK];              // psr [16 quads][32] float4 | class [16][32] u16
+    float4 binc[DN_BUFS][4][32];                     // increments of 16 rows
+    uint32_t bmsk[DN_BUFS][4][32];                   // step masks, one byte per row
+    uint32_t act[DN_ACT_WORDS];
+    float sum[BLK_MAX_STEPS][32];
+    float noise[BLK_MAX_STEPS][32];
+    float dtab[BG3_MAX_DCLS];
+    int4 src[DN_EV_WARPS][2][4][32];                 // per arrival warp: a group's and the next one's
+    uint32_t lc[DN_EV_WARPS][2][4][32];              // sources and delay classes
+    int32_t ltab[BG3_MAX_DELAYS];
+    uint16_t quads[DN_MAX_CHUNKS];                   // per chunk, the row quads to look at
+    uint32_t groups[4 * DN_MAX_CHUNKS / 32];         // the 16-row groups with such a quad
+    int any[DN_BUFS];                                // the buffer has arrivals; 2: several at a row
+    int issued, failed;
+    uint64_t full[DN_STAGES], half[DN_STAGES], empty[DN_STAGES];
+    uint64_t bfull[DN_BUFS], bempty[DN_BUFS];
+    uint64_t scanned, summed[2], drawn;
+};
+constexpr size_t DN_SMEM = sizeof(DenseSmem);
+
+__device__ __forceinline__ void bar_events()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * DN_EV_WARPS) : "memory");
+}
+
+__device__ __forceinline__ bool dn_wait(const NetDev &n, DenseSmem &s, uint64_t *bar, uint32_t parity)
+{
+    if (mbar_wait(bar, parity)) return true;
+    set_err(n, ERR_TIMEOUT);
+    *(volatile int *)&s.failed = 1;
+    return false;
+}
+
+// The bitmap words that the sources of a tile's row quads span, lo | hi << 16 (lo > hi: no synapse;
+// words past 16 bits: the whole range).  One warp per quad.
+__global__ void __launch_bounds__(256) k_blk_range(const __grid_constant__ NetDev n, uint32_t *range)
+{
+    const int lane = threadIdx.x & 31;
+    const long long total = (long long)n.ntiles * n.Mq;
+    for (long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; i < total;
+         i += ((long long)gridDim.x * blockDim.x) >> 5) {
+        const int tile = (int)(i / n.Mq), q = (int)(i % n.Mq);
+        const int d = tile * 32 + lane;
+        const int left = (d < n.N ? (int)n.count[d] : 0) - 4 * q;
+        uint32_t lo = 0xffffffffu, hi = 0u;
+        if (left > 0) {
+            const int4 v = reinterpret_cast<const int4 *>(n.src)[i * 32 + lane];
+            const uint32_t w[4] = {(uint32_t)v.x >> 5, (uint32_t)v.y >> 5, (uint32_t)v.z >> 5, (uint32_t)v.w >> 5};
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (left > k) {
+                    lo = min(lo, w[k]);
+                    hi = max(hi, w[k]);
+                }
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0) range[i] = lo > hi ? 0x0000ffffu : hi > 0xffffu ? 0xffff0000u : lo | (hi << 16);
+    }
+}
+
+// The lane's rows of quad sources v with a spike that may arrive (bit r: row r).
+__device__ __forceinline__ uint32_t dense_hits(const int4 &v, const uint32_t *act, int left)
+{
+    uint32_t h = 0u;
+    if (left > 0) h |= (act[v.x >> 5] >> (v.x & 31)) & 1u;
+    if (left > 1) h |= ((act[v.y >> 5] >> (v.y & 31)) & 1u) << 1;
+    if (left > 2) h |= ((act[v.z >> 5] >> (v.z & 31)) & 1u) << 2;
+    if (left > 3) h |= ((act[v.w >> 5] >> (v.w & 31)) & 1u) << 3;
+    return h;
+}
+
+// One spike arriving at each of U slots p[u] (m[u]: its step's bit; 0: none), their loads issued
+// together: the psr increments, with the event slots brought up to date
+// (AllSpikingSynapses.cpp:327-334, AllDSSynapses.cpp:227-247).  m[u] is cleared where the synapse did
+// not exist when the spike left, D[u] steps before.
+template <int SYN, int U>
+__device__ __forceinline__ void dense_arrivals(const NetDev &n, const DenseSmem &s, const uint32_t (&p)[U],
+                                               const int (&D)[U], uint32_t (&m)[U], float (&inc)[U],
+                                               unsigned long long t)
+{
+    // the first 16 bytes of a slot (W, u, r, last spike) and the next 8 (birth step, classes)
+    float4 e[U];
+    uint2 f[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+        if (m[u]) {
+            const char *q = reinterpret_cast<const char *>(n.ev) + (size_t)p[u] * sizeof(EvSlot);
+            e[u] = *reinterpret_cast<const float4 *>(q);
+            f[u] = *reinterpret_cast<const uint2 *>(q + 16);
+        }
+    float xr[U], xu[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        if (!m[u]) continue;
+        const uint32_t ta = (uint32_t)t + (uint32_t)(31 - __clz((int)m[u])), last = __float_as_uint(e[u].w);
+        if ((int32_t)(ta - (uint32_t)D[u] - f[u].x) < 0) {
+            m[u] = 0u;
+        } else if (SYN == 1 && last != BG3_NO_SPIKE32) {
+            const int pc = (int)((f[u].y >> 8) & 255u);
+            xr[u] = exp_tab(n, n.p_xD[pc], ta - last, n.p_D[pc]);
+            xu[u] = exp_tab(n, n.p_xF[pc], ta - last, n.p_F[pc]);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        inc[u] = 0.0f;
+        if (!m[u]) continue;
+        const float dec = s.dtab[f[u].y & 255u];
+        if (SYN == 1) {
+            float uu = e[u].y, rr = e[u].z;
+            if (__float_as_uint(e[u].w) != BG3_NO_SPIKE32) {
+                const float Uc = n.p_U[(f[u].y >> 8) & 255u];
+                rr = 1.0f + (rr * (1.0f - uu) - 1.0f) * xr[u];
+                uu = Uc + uu * (1.0f - Uc) * xu[u];
+            }
+            inc[u] = (e[u].x / dec) * uu * rr;
+            // one store of the slot's first half (nothing else writes W during a block)
+            gst(reinterpret_cast<float4 *>(n.ev) + 2 * (size_t)p[u],
+                make_float4(e[u].x, uu, rr,
+                            __uint_as_float((uint32_t)t + (uint32_t)(31 - __clz((int)m[u])))));
+        } else {
+            inc[u] = e[u].x / dec;
+        }
+    }
+}
+
+// The 16 rows of buffer bf where a synapse has several spikes arriving in the block: those arrivals
+// run at their steps.  psr in place, the steps' sums in and out.
+template <int SYN>
+__device__ __noinline__ void dense_late(const NetDev &n, const DenseSmem &s, int tile, int row0, int bf,
+                                        int j0, int nj, unsigned long long t, float4 *ps4,
+                                        const uint16_t *cw, float *acc)
+{
+    const int lane = threadIdx.x & 31, d = tile * 32 + lane;
+    for (int r = 0; r < 16; r++) {
+        const int q = r >> 2, i = r & 3;
+        float *pr = reinterpret_cast<float *>(ps4 + q * 32) + i;
+        const float dec = s.dtab[(cw[q * 32] >> (4 * i)) & 15u];
+        const uint32_t m = (s.bmsk[bf][q][lane] >> (8 * i)) & 255u;
+        const bool many = (m & (m - 1u)) != 0u;
+        float x = *pr;
+        for (int j = 0; j < nj; j++) {
+            if ((m >> (j0 + j)) & 1u) {
+                if (many) {
+                    const uint32_t p = (uint32_t)slot_pos(row0 + r, d, n.Mq);
+                    const unsigned long long tj = t + (unsigned)(j0 + j);
+                    float a;
+                    if (arrival<SYN>(n, p, d, n.src[p], (uint32_t)tj - (uint32_t)n.ltab[n.lcls[p]], tj, a))
+                        x = x + a;
+                } else {
+                    x = x + reinterpret_cast<const float *>(&s.binc[bf][q][lane])[i];
+                }
+            }
+            x = x * dec;
+            acc[j] = acc[j] + x;
+        }
+        *pr = x;
+    }
+}
+
+// Two products in one instruction, each rounded as a single multiplication.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
+        " mul.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}\n"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
+// Four rows through a half block's steps: psr scaled, and added to each step's sum in row order.  The
+// products of a step's four rows are independent of each other, as are the four steps' sums of a
+// row, so neither half of this waits on itself.  HIT: rows may have an arrival, at the step whose
+// bit is set in the row's byte of m (bit j: step j).  FULL: all DN_HALF steps, else nj.
+template <bool FULL, bool HIT>
+__device__ __forceinline__ void dense_quad(float4 &v, const float4 &dc, float (&acc)[DN_HALF], int nj,
+                                           uint32_t m, const float4 &in)
+{
+    float2 p[DN_HALF][2];
+    float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w);
+    const float2 dx = make_float2(dc.x, dc.y), dy = make_float2(dc.z, dc.w);
+#pragma unroll
+    for (int j = 0; j < DN_HALF; j++) {
+        if (!FULL && j >= nj) break;
+        if (HIT) {
+            if (m & (1u << j)) x.x = x.x + in.x;
+            if (m & (0x100u << j)) x.y = x.y + in.y;
+            if (m & (0x10000u << j)) y.x = y.x + in.z;
+            if (m & (0x1000000u << j)) y.y = y.y + in.w;
+        }
+        p[j][0] = x = mul2(x, dx);
+        p[j][1] = y = mul2(y, dy);
+    }
+#pragma unroll
+    for (int j = 0; j < DN_HALF; j++) {
+        if (!FULL && j >= nj) break;
+        acc[j] = acc[j] + p[j][0].x;
+    }
+#pragma unroll
+    for (int j = 0; j < DN_HALF; j++) {
+        if (!FULL && j >= nj) break;
+        acc[j] = acc[j] + p[j][0].y;
+    }
+#pragma unroll
+    for (int j = 0; j < DN_HALF; j++) {
+        if (!FULL && j >= nj) break;
+        acc[j] = acc[j] + p[j][1].x;
+    }
+#pragma unroll
+    for (int j = 0; j < DN_HALF; j++) {
+        if (!FULL && j >= nj) break;
+        acc[j] = acc[j] + p[j][1].y;
+    }
+    v = make_float4(x.x, x.y, y.x, y.y);
+}
+
+// nj steps from j0 on over all chunks: psr scaled in place, a step's sum over the rows in order.
+// last: the second sum warp, which takes chunks from the first one and stores them back.  FULL:
+// nj = DN_HALF.  Measured alone on an SM (cycles a row of 32 destinations, four steps): 16 rows at a
+// time with paired products 17.7, without the pairs 19.6, eight rows at a time 23, eight rows with
+// the next eight loading 36 (more instructions than latency saved).
+template <int SYN, bool FULL>
+__device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem &s, const CUtensorMap *tm_psr,
+                                           int tile, int nch, int nj, int j0, bool last,
+                                           unsigned long long t)
+{
+    const int lane = threadIdx.x & 31;
+    float acc[DN_HALF];
+#pragma unroll
+    for (int j = 0; j < DN_HALF; j++) acc[j] = 0.0f;
+    bool ok = dn_wait(n, s, &s.scanned, 0);
+    int k = 0;  // 16-row groups with a buffer so far
+    for (int c = 0; ok && c < nch; c++) {
+        const int st = c % DN_STAGES;
+        ok = dn_wait(n, s, last ? &s.half[st] : &s.full[st], (uint32_t)((c / DN_STAGES) & 1));
+        if (!ok) break;
+        float4 *ps4 = reinterpret_cast<float4 *>(s.stage[st]) + lane;
+        const uint16_t *cw = reinterpret_cast<const uint16_t *>(s.stage[st] + DN_ROWS * 32 * 4) + lane;
+#pragma unroll 1
+        for (int g = 0; g < 4; g++, ps4 += 4 * 32, cw += 4 * 32) {
+            float4 v[4], dc[4];
+            uint32_t cl[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                v[q] = ps4[q * 32];
+                cl[q] = cw[q * 32];
+            }
+            const bool looked = (s.groups[c >> 3] >> (4 * (c & 7) + g)) & 1u;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                dc[q] = make_float4(s.dtab[cl[q] & 15u], s.dtab[(cl[q] >> 4) & 15u],
+                                    s.dtab[(cl[q] >> 8) & 15u], s.dtab[(cl[q] >> 12) & 15u]);
+            const int bf = k % DN_BUFS;
+            int any = 0;
+            if (looked) {
+                ok = dn_wait(n, s, &s.bfull[bf], (uint32_t)((k / DN_BUFS) & 1));
+                if (!ok) break;
+                k++;
+                any = s.any[bf];
+            }
+            if (any == 0) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) dense_quad<FULL, false>(v[q], dc[q], acc, nj, 0u, v[q]);
+            } else if (any == 1) {
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    dense_quad<FULL, true>(v[q], dc[q], acc, nj, s.bmsk[bf][q][lane] >> j0,
+                                           s.binc[bf][q][lane]);
+            } else {
+                float a[DN_HALF];
+#pragma unroll
+                for (int j = 0; j < DN_HALF; j++) a[j] = acc[j];
+                dense_late<SYN>(n, s, tile, c * DN_ROWS + 16 * g, bf, j0, nj, t, ps4, cw, a);
+#pragma unroll
+                for (int j = 0; j < DN_HALF; j++) acc[j] = a[j];
+            }
+            if (any != 2) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) ps4[q * 32] = v[q];
+            }
+            if (last && looked) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s.bempty[bf]);
+            }
+        }
+        if (!ok) break;
+        fence_async_smem();  // the TMA store (async proxy) must see these writes
+        __syncwarp();
+        if (lane == 0) {
+            if (!last) {
+                mbar_arrive(&s.half[st]);
+            } else {
+                tma_store_3d(tm_psr, 0, c * DN_QUADS, tile, s.stage[st]);
+                bulk_commit();
+                if (c >= 1) {
+                    bulk_wait_read1();
+                    mbar_arrive(&s.empty[(c - 1) % DN_STAGES]);
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (last && lane == 0) bulk_wait_read_all();
+#pragma unroll
+    for (int j = 0; j < DN_HALF; j++)
+        if (j < nj) s.sum[j0 + j][lane] = acc[j];
+    __syncwarp();
+    if (ok && lane == 0) mbar_arrive(&s.summed[last ? 1 : 0]);
+}
+
+// Sources and delay classes (a byte per row) of 16 rows of the lane's destination, of the quads to
+// look at, on their way to shared memory.
+__device__ __forceinline__ void dense_sources(DenseSmem &s, int w, int st, const int4 *S,
+                                              const uint32_t *L, int q0, uint32_t quads, int cnt)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (((quads >> q) & 1u) && cnt > 4 * (q0 + q)) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&s.src[w][st][q][lane])),
+                         "l"(&S[(size_t)(q0 + q) * 32]) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&s.lc[w][st][q][lane])),
+                         "l"(&L[(size_t)(q0 + q) * 32]) : "memory");
+        }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The arrival warps' part.  Warp w: first the quads to look at (all four warps share them out),
+// then every fourth 16-row group with one, the next such group's sources on their way meanwhile.
+template <int SYN>
+__device__ __forceinline__ void dense_events(const NetDev &n, const BlkDev &b, DenseSmem &s, int tile,
+                                             int w, int cnt, int nch, int nt, unsigned long long t)
+{
+    const int lane = threadIdx.x & 31, tid = (int)threadIdx.x - 32;
+    const size_t base = (size_t)tile * n.Mq * 32 + lane;
+    const int4 *S = reinterpret_cast<const int4 *>(n.src) + base;
+    const uint32_t *L = reinterpret_cast<const uint32_t *>(n.lcls) + base;
+    const uint32_t *act = b.act + (t & (BLK_ACT_ROWS - 1)) * n.ntiles;
+    if (n.ntiles <= DN_ACT_WORDS) {
+        for (int i = tid; i < n.ntiles; i += 32 * DN_EV_WARPS) s.act[i] = act[i];
+        act = s.act;
+        bar_events();
+    }
+    // one lane per row quad: is a bitmap word of its sources' range set?
+    for (int q = tid; q < nch * DN_QUADS; q += 32 * DN_EV_WARPS) {
+        const uint32_t rg = q < n.Mq ? b.range[(size_t)tile * n.Mq + q] : 0x0000ffffu;
+        const int lo = (int)(rg & 0xffffu), hi = (int)(rg >> 16);
+        bool look = hi - lo >= DN_RANGE_SCAN;
+        if (!look)
+            for (int i = lo; i <= hi; i++) look = look || act[i] != 0u;
+        // whole warps but for the last, whose lower half may hold the last chunk
+        const uint32_t m = __ballot_sync(q - lane + 32 <= nch * DN_QUADS ? 0xffffffffu : 0xffffu, look);
+        if (lane == 0 || lane == 16) s.quads[q / DN_QUADS] = (uint16_t)(m >> lane);
+    }
+    bar_events();
+    uint32_t mine = 0u;  // groups 32 w .. 32 w + 31
+    if (32 * w + lane < 4 * nch) mine = (s.quads[8 * w + (lane >> 2)] >> (4 * (lane & 3))) & 15u;
+    mine = __ballot_sync(0xffffffffu, mine != 0u);
+    if (lane == 0) s.groups[w] = mine;
+    bar_events();
+    if (lane == 0) mbar_arrive(&s.scanned);
+    // walks the groups; returns this warp's next one, or -1
+    int word = -1, k = 0;
+    uint32_t left = 0u;
+    auto next = [&]() {
+        for (;;) {
+            while (!left) {
+                if (++word == (int)(sizeof(s.groups) / 4)) return -1;
+                left = s.groups[word];
+            }
+            const int g = 32 * word + __ffs((int)left) - 1;
+            left &= left - 1u;
+            if (k++ % DN_BUFS == w) return g;
+        }
+    };
+    int g = next(), used = 0;
+    if (g >= 0) dense_sources(s, w, 0, S, L, 4 * g, s.quads[g >> 2] >> (4 * (g & 3)), cnt);
+    while (g >= 0) {
+        const int st = used & 1;
+        const int gn = next();
+        if (gn >= 0) {
+            dense_sources(s, w, st ^ 1, S, L, 4 * gn, s.quads[gn >> 2] >> (4 * (gn & 3)), cnt);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        // hits, then the hits' sources' masks: the steps of the block at which a spike arrives (each
+        // lane reads only what it copied itself)
+        const uint32_t quads = s.quads[g >> 2] >> (4 * (g & 3));
+        uint32_t h16 = 0u;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if ((quads >> q) & 1u) h16 |= dense_hits(s.src[w][st][q][lane], act, cnt - 4 * (4 * g + q)) << (4 * q);
+        const bool some = __any_sync(0xffffffffu, h16 != 0u);
+        if (used > 0 && !dn_wait(n, s, &s.bempty[w], (uint32_t)((used - 1) & 1))) return;
+        used++;
+        bool many = false, hit = false;
+        if (some) {
+            uint8_t *mb = reinterpret_cast<uint8_t *>(&s.bmsk[w][0][lane]);  // row r: mb[128 (r / 4) + r % 4]
+            const uint8_t *lb = reinterpret_cast<const uint8_t *>(&s.lc[w][st][0][lane]);
+            const int *sb = reinterpret_cast<const int *>(&s.src[w][st][0][lane]);
+            float *ib = reinterpret_cast<float *>(&s.binc[w][0][lane]);
+            const uint32_t p0 = (uint32_t)slot_pos(16 * g, tile * 32 + lane, n.Mq);
+#pragma unroll
+            for (int q = 0; q < 4; q++) s.bmsk[w][q][lane] = 0u;
+            uint32_t one = 0u;
+            while (h16) {
+                constexpr int U = 4;
+                int r[U];
+                unsigned long long hs[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    r[u] = h16 ? __ffs((int)h16) - 1 : -1;
+                    h16 &= h16 - 1u;
+                    if (r[u] >= 0) hs[u] = b.hist[sb[128 * (r[u] >> 2) + (r[u] & 3)]];
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (r[u] >= 0) {
+                        const int D = s.ltab[lb[128 * (r[u] >> 2) + (r[u] & 3)]];
+                        const uint32_t m = (uint32_t)rotr64(hs[u], (unsigned)t - (unsigned)D) & ((1u << nt) - 1u);
+                        if (!m) continue;
+                        mb[128 * (r[u] >> 2) + (r[u] & 3)] = (uint8_t)m;
+                        hit = true;
+                        if (m & (m - 1u)) {
+                            many = true;
+                        } else {
+                            one |= 1u << r[u];
+                            // towards the L1: a batch's loads below then wait for its first time only
+                            asm volatile("prefetch.global.L1 [%0];" ::"l"(&n.ev[p0 + 128u * (r[u] >> 2) + (r[u] & 3)]));
+                        }
+                    }
+            }
+            while (one) {
+                constexpr int U = 2;
+                uint32_t p[U], m[U];
+                int r[U], D[U];
+                float inc[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    m[u] = 0u;
+                    r[u] = -1;
+                    if (one) {
+                        r[u] = __ffs((int)one) - 1;
+                        one &= one - 1u;
+                        r[u] = 128 * (r[u] >> 2) + (r[u] & 3);
+                        m[u] = mb[r[u]];
+                        D[u] = s.ltab[lb[r[u]]];
+                        p[u] = p0 + (uint32_t)r[u];
+                    }
+                }
+                dense_arrivals<SYN, U>(n, s, p, D, m, inc, t);
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (r[u] >= 0) {
+                        mb[r[u]] = (uint8_t)m[u];
+                        ib[r[u]] = inc[u];
+                    }
+            }
+            hit = __any_sync(0xffffffffu, hit);
+            many = __any_sync(0xffffffffu, many);
+        }
+        __syncwarp();
+        if (lane == 0) {
+            s.any[w] = many ? 2 : hit ? 1 : 0;
+            mbar_arrive(&s.bfull[w]);
+        }
+        g = gn;
+    }
+}
+
+template <int SYN>
+__device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
+                                               const CUtensorMap *tm_psr, const CUtensorMap *tm_cls,
+                                               const int tile, const int nt, DenseSmem &s)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int d = tile * 32 + lane;
+    const bool valid = d < n.N;
+    for (int i = threadIdx.x; i < n.n_dcls; i += blockDim.x) s.dtab[i] = n.dtab[i];
+    for (int i = threadIdx.x; i < n.n_delays; i += blockDim.x) s.ltab[i] = n.ltab[i];
+    const int cnt = valid ? (int)n.count[d] : 0;
+    const int nch = (__reduce_max_sync(0xffffffffu, cnt) + DN_ROWS - 1) / DN_ROWS;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < DN_STAGES; i++) {
+            mbar_init(&s.full[i], 1);
+            mbar_init(&s.half[i], 1);
+            mbar_init(&s.empty[i], 1);
+        }
+        for (int i = 0; i < DN_BUFS; i++) {
+            mbar_init(&s.bfull[i], 1);
+            mbar_init(&s.bempty[i], 1);
+        }
+        mbar_init(&s.summed[0], 1);
+        mbar_init(&s.summed[1], 1);
+        mbar_init(&s.scanned, DN_EV_WARPS);
+        mbar_init(&s.drawn, DN_EV_WARPS);
+        fence_mbar_init();
+        s.issued = 0;
+        s.failed = 0;
+    }
+    __syncthreads();
+    pdl_wait();  // the block before has finished
+    pdl_trigger();
+    const unsigned long long t = *n.step;
+
+    if (warp == 0) {  // ------------------------------------------------ loads, then the neurons
+        bool ok = true;
+        if (lane == 0) {
+            for (int c = 0; c < nch; c++) {
+                const int st = c % DN_STAGES;
+                if (c >= DN_STAGES &&
+                    !dn_wait(n, s, &s.empty[st], (uint32_t)((c / DN_STAGES - 1) & 1))) {
+                    ok = false;
+                    break;
+                }
+                mbar_expect_tx(&s.full[st], DN_CHUNK);
+                tma_load_3d(s.stage[st], tm_psr, 0, c * DN_QUADS, tile, &s.full[st]);
+                tma_load_3d(s.stage[st] + DN_ROWS * 32 * 4, tm_cls, 0, c * DN_QUADS, tile, &s.full[st]);
+                *(volatile int *)&s.issued = c + 1;
+            }
+        }
+        NeuronIn x;
+        float sp = 0.0f;
+        unsigned long long hist = 0ull;
+        if (valid) {
+            neuron_load(n, d, x);
+            sp = n.sp[d];
+            hist = b.hist[d];
+        }
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (ok) ok = dn_wait(n, s, &s.drawn, 0);
+        const int mode = izh_mode(n, d);
+        uint32_t fired = 0u;
+#pragma unroll 1
+        for (int j = 0; ok && j < nt; j++) {
+            // step t + j takes the sum of step t + j - 1
+            if (j == 1) ok = dn_wait(n, s, &s.summed[0], 0);
+            if (j == DN_HALF + 1) ok = dn_wait(n, s, &s.summed[1], 0);
+            if (!ok) break;
+            if (j > 0) sp = s.sum[j - 1][lane];
+            if (valid) {
+                const unsigned long long tj = t + (unsigned)j;
+                const int br = neuron_branch(x);
+                const float in = input_update(n, d, x, tj, sp);
+                if (neuron_update(n, d, x, br, in, s.noise[j][lane], tj, mode)) fired |= 1u << j;
+            }
+        }
+        if (ok && nt == 1) ok = dn_wait(n, s, &s.summed[0], 0);
+        if (ok && nt <= DN_HALF + 1) ok = dn_wait(n, s, &s.summed[1], 0);
+        if (ok) {
+            sp = s.sum[nt - 1][lane];
+            blk_finish<SYN>(n, b, tile, d, valid, x, sp, hist, fired, nt, t);
+        }
+    } else if (warp <= DN_EV_WARPS) {  // ------------------------------------------- arrivals
+        const int w = warp - 1;
+        dense_events<SYN>(n, b, s, tile, w, cnt, nch, nt, t);
+        for (int j = w; j < nt; j += DN_EV_WARPS)
+            s.noise[j][lane] = normal_device(n.noise_seed, t + (unsigned)j, d);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s.drawn);
+    } else {  // --------------------------------------------------------------------- sums
+        const bool last = warp == DN_EV_WARPS + 2;
+        if (nt == 2 * DN_HALF)
+            dense_sums<SYN, true>(n, s, tm_psr, tile, nch, DN_HALF, last ? DN_HALF : 0, last, t);
+        else
+            dense_sums<SYN, false>(n, s, tm_psr, tile, nch, last ? max(0, nt - DN_HALF) : min(nt, DN_HALF),
+                               last ? DN_HALF : 0, last, t);
+    }
+    __syncthreads();
+    if (*(volatile int *)&s.failed && threadIdx.x == 0) {
+        // a wait gave up: the loads in flight land before the shared memory goes away
+        const int issued = *(volatile int *)&s.issued;
+        for (int c = max(0, issued - DN_STAGES); c < issued; c++)
+            if (!mbar_wait(&s.full[c % DN_STAGES], (uint32_t)((c / DN_STAGES) & 1))) break;
+    }
+}
+
+template <int SYN>
+__global__ void __launch_bounds__(DN_THREADS, 3) k_blk_dense(const __grid_constant__ NetDev n,
+                                                             const __grid_constant__ BlkDev b,
+                                                             const __grid_constant__ CUtensorMap tm_psr,
+                                                             const __grid_constant__ CUtensorMap tm_cls,
+                                                             int nt)
+{
+    // declared with its alignment and used as it is: arithmetic on the address would hide from the
+    // compiler that it is shared memory, and every access would be a generic one
+    extern __shared__ __align__(128) uint8_t smem_dense[];
+    blk_dense_tile<SYN>(n, b, &tm_psr, &tm_cls, blockIdx.x, nt, *reinterpret_cast<DenseSmem *>(smem_dense));
+}
+
+// Batched form: tiles[b] = (network, tile), heaviest first; maps as in k_sweep_batch.
+template <int SYN>
+__global__ void __launch_bounds__(DN_THREADS, 3) k_blk_dense_batch(const NetDev *nets,
+                                                                   const BlkDev *blks,
+                                                                   const CUtensorMap *maps,
+                                                                   const int2 *tiles, int nt)
+{
+    extern __shared__ __align__(128) uint8_t smem_dense[];
+    __shared__ __align__(16) NetDev s_net;
+    const int2 tr = tiles[blockIdx.x];
+    const uint4 *s4 = reinterpret_cast<const uint4 *>(nets + tr.x);
+    uint4 *d4 = reinterpret_cast<uint4 *>(&s_net);
+    for (int i = threadIdx.x; i < (int)(sizeof(NetDev) / 16); i += blockDim.x) d4[i] = s4[i];
+    const BlkDev b = blks[tr.x];
+    __syncthreads();
+    blk_dense_tile<SYN>(s_net, b, &maps[2 * tr.x], &maps[2 * tr.x + 1], tr.y, nt,
+                        *reinterpret_cast<DenseSmem *>(smem_dense));
+}
+
 // ---- launchers --------------------------------------------------------------------------------
 template <typename... KArgs, typename... Args>
 static void launch_dep(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t s,
@@ -461,6 +1112,12 @@ static void launch_dep(void (*kern)(KArgs...), dim3 grid, int block, size_t smem
 }
 
 bool blk_thin_ok(int Mq) { return Mq <= BLK_THIN_QUADS; }
+void launch_blk_range(const NetDev &h, const BlkDev &b, cudaStream_t s)
+{
+    k_blk_range<<<152 * 8, 256, 0, s>>>(h, b.range);
+}
+
+bool blk_dense_ok(int Mq) { return Mq <= DN_MAX_CHUNKS * DN_QUADS; }
 
 void launch_blk_masks(const NetDev &h, const BlkDev &b, cudaStream_t s)
 {
@@ -512,6 +1169,38 @@ void launch_blk_thin_batch(int syn_kind, const NetDev *nets, const BlkDev *blks,
     if (syn_kind >= 2)
         launch_dep(k_blk_post_batch, dim3(std::max(1, std::min(152, 1216 / std::max(nets_n, 1))), nets_n),
                    256, 0, s, nets, blks, nt);
+}
+
+// The opt-in shared memory size is a property of the kernel on each device: set before every launch
+// (a host-side table write), so that no process-wide flag is needed.
+template <typename K>
+static void allow_smem(K kern)
+{
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_SMEM);
+}
+
+void launch_blk_dense(const NetDev &h, const BlkDev &b, const CUtensorMap &tp, const CUtensorMap &tc,
+                      int nt, cudaStream_t s)
+{
+    if (h.syn_kind == 1) {
+        allow_smem(k_blk_dense<1>);
+        launch_dep(k_blk_dense<1>, h.ntiles, DN_THREADS, DN_SMEM, s, h, b, tp, tc, nt);
+    } else {
+        allow_smem(k_blk_dense<0>);
+        launch_dep(k_blk_dense<0>, h.ntiles, DN_THREADS, DN_SMEM, s, h, b, tp, tc, nt);
+    }
+}
+
+void launch_blk_dense_batch(int syn_kind, const NetDev *nets, const BlkDev *blks,
+                            const CUtensorMap *maps, const int2 *tiles, int n, int nt, cudaStream_t s)
+{
+    if (syn_kind == 1) {
+        allow_smem(k_blk_dense_batch<1>);
+        launch_dep(k_blk_dense_batch<1>, n, DN_THREADS, DN_SMEM, s, nets, blks, maps, tiles, nt);
+    } else {
+        allow_smem(k_blk_dense_batch<0>);
+        launch_dep(k_blk_dense_batch<0>, n, DN_THREADS, DN_SMEM, s, nets, blks, maps, tiles, nt);
+    }
 }
 
 }  // namespace bg3

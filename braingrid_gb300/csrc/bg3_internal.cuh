@@ -198,6 +198,9 @@ struct BlkDev {
     // [BLK_ACT_ROWS][ntiles] row t & 15: the neurons of a 32-neuron tile with a spike that may
     // arrive in a block starting at step t (any delay class)
     uint32_t *act;
+    // [ntiles][Mq] the bitmap words that the sources of a tile's row quad span (k_blk_range); follows
+    // from the synapses, NULL for networks that never run a dense block
+    uint32_t *range;
     // bit s & 63 for the steps s whose spikes may arrive in a block starting at step 0
     unsigned long long win;
 };
@@ -221,6 +224,9 @@ enum : uint32_t {
 // the reference's x86-64 build.  expf of the reference's host library is correctly rounded for
 // almost every argument; evaluating exp in double and rounding once reproduces that.
 __device__ __forceinline__ float exp_cr(float x) { return (float)exp((double)x); }
+// The same out of line, where a table covers all but far intervals: the double exp's code stays out
+// of the step loops.
+static __device__ __noinline__ float exp_far(float x) { return exp_cr(x); }
 __device__ __forceinline__ float acos_cr(float x) { return (float)acos((double)x); }
 __device__ __forceinline__ float sin_cr(float x) { return (float)sin((double)x); }
 
@@ -235,7 +241,7 @@ __device__ __forceinline__ float exp_steps(const NetDev &n, uint32_t k, float ta
             if (n.expc_tau[c] == tau) return __ldg(n.expc_tab[c] + k);
     }
     const float x = (float)k * n.dt;
-    return exp_cr(-x / tau);
+    return exp_far(-x / tau);
 }
 
 // expf(-((float)k * dt) / tau) from the table of a DS parameter class.
@@ -243,7 +249,7 @@ __device__ __forceinline__ float exp_tab(const NetDev &n, const float *tab, uint
 {
     if (tab && k < (uint32_t)BG3_EXP_LEN) return __ldg(tab + k);
     const float x = (float)k * n.dt;
-    return exp_cr(-x / tau);
+    return exp_far(-x / tau);
 }
 
 // AllDSSynapses::changePSR's facilitation / depression update of u and r
@@ -264,7 +270,7 @@ __device__ __forceinline__ float exp_interval(const NetDev &n, unsigned long lon
 {
     if (u < (unsigned long long)BG3_EXP_LEN) return exp_steps(n, (uint32_t)u, tau);
     const float x = (sgn ? (float)(long long)u : (float)u) * n.dt;
-    return exp_cr(-x / tau);
+    return exp_far(-x / tau);
 }
 
 // ---- counter-based normal generator (device noise mode) --------------------------------------
@@ -770,7 +776,8 @@ __device__ __forceinline__ bool neuron_apply(const NetDev &n, int i, const Neuro
 // One Poisson inter-spike interval in steps (HostSInputPoisson.cpp:81-84): exponential with mean
 // lambda ms, rejected while U <= exp(-isi^2 / 32).  Injected draws replay the reference's own
 // sequence; otherwise a Philox stream keyed by (seed, neuron, draw index).
-__device__ __forceinline__ int32_t next_isi(const NetDev &n, int i)
+// Out of line: one draw per interval, not per step.
+static __device__ __noinline__ int32_t next_isi(const NetDev &n, int i)
 {
     const int32_t k = n.isi_cursor[i];
     gst(&n.isi_cursor[i], k + 1);

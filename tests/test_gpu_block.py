@@ -102,6 +102,18 @@ def test_thin_blocks_equal_steps(syn, w, h, radius, drive, max_syn):
     advance(lambda: lif(w, h, syn, radius, drive, max_syn), end="growth")
 
 
+@pytest.mark.parametrize("syn", [bg.BG3_SYN_SPIKING, bg.BG3_SYN_DS])
+@pytest.mark.parametrize("w,h,radius,drive,max_syn", [
+    (9, 7, 6.0, "poisson", 65),     # every pair connected, 62 rows: one chunk and a row
+    (13, 5, 4.0, "none", 130),      # 64 rows at most in use, three chunks allocated
+    (40, 33, 3.4, "none", 190),     # a partial third chunk; bursts: the chunk-by-chunk arrivals
+    (40, 33, 3.4, "poisson", 191),
+    (30, 30, 13.5, "regular", 900), # fifteen chunks, most of the network in every row
+])
+def test_dense_blocks_equal_steps(syn, w, h, radius, drive, max_syn):
+    advance(lambda: lif(w, h, syn, radius, drive, max_syn), end="growth")
+
+
 @pytest.mark.parametrize("w,h", [(9, 7), (13, 5), (60, 41)])
 def test_izhikevich_stdp_blocks_equal_steps(w, h):
     advance(lambda: izh(w, h))
@@ -126,3 +138,40 @@ def test_batched_blocks_equal_steps():
         y.step(24)
         same(x, y, "batched, after per-step kernels")
     batch.close()
+
+
+def test_batched_dense_and_thin_blocks_equal_steps():
+    shapes = [(9, 7, 6.0, 65), (40, 33, 3.4, 190), (13, 5, 1.5, 33), (33, 31, 1.9, 64)]
+    a, b = ([lif(w, h, bg.BG3_SYN_DS, r, "none", m) for w, h, r, m in shapes] for _ in range(2))
+    batch = bg.Batch(a)
+    for net in b:
+        net.set_launch(small_max_slots=0)
+    for n in STEPS:
+        batch.step(n)
+        for net in b:
+            net.step(n)
+    batch.sync()
+    for x, y in zip(a, b):
+        same(x, y, "batched")
+    batch.close()
+
+
+def test_two_spikes_at_one_synapse_in_a_block():
+    """Neurons without a refractory period whose reset lies above the threshold fire on every
+    step, so that each synapse receives several spikes within a block."""
+    for radius, max_syn in ((1.5, 33), (4.0, 130)):
+        nets = []
+        for small in (1, 0):
+            net = lif(13, 5, bg.BG3_SYN_DS, radius, "none", max_syn)
+            v = net.download_lif(fields=("Vthresh", "Vreset", "Trefract"))
+            v["Trefract"][::3] = 0.0
+            v["Vreset"][::3] = v["Vthresh"][::3] + np.float32(1e-3)
+            v["Vthresh"][1::3] -= np.float32(1.0e-3)
+            net.upload_lif(**v)
+            net.set_launch(small_max_slots=small)
+            nets.append(net)
+        for n in (8, 8, 3, 40):
+            for net in nets:
+                net.step(n)
+            same(nets[0], nets[1], "radius %g after %d steps" % (radius, n))
+        assert int(nets[0].download_lif(fields=("spikeCount",))["spikeCount"].max()) > 8
