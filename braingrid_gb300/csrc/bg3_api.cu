@@ -37,11 +37,11 @@ void launch_scale_weights(const NetDev &h, float f, cudaStream_t s);
 void launch_record(const NetDev &h, const NetDev *d_net, cudaStream_t s);
 bool blk_thin_ok(int Mq);
 bool blk_dense_ok(int Mq);
-void launch_blk_range(const NetDev &h, const BlkDev &b, cudaStream_t s);
 void launch_blk_dense(const NetDev &h, const BlkDev &b, const CUtensorMap &tp, const CUtensorMap &tc,
                       int nt, cudaStream_t s);
 void launch_blk_dense_batch(int syn_kind, const NetDev *nets, const BlkDev *blks,
-                            const CUtensorMap *maps, const int2 *tiles, int n, int nt, cudaStream_t s);
+                            const CUtensorMap *maps, const int2 *tiles, int n, const int *dense, int nd,
+                            int max_tiles, int nt, cudaStream_t s);
 void launch_blk_masks(const NetDev &h, const BlkDev &b, cudaStream_t s);
 void launch_blk_ring(const NetDev &h, const BlkDev &b, cudaStream_t s);
 void launch_blk_thin(const NetDev &h, const BlkDev &b, int nt, cudaStream_t s);
@@ -82,7 +82,6 @@ struct bg3_net {
     // whichever ran last is current, the other is rebuilt when it is needed
     BlkDev blk = {};
     bool ring_ok = true, mask_ok = false;
-    bool range_ok = false;    // blk.range follows the synapses
     // fewest steps between two spikes of a neuron, for the block kernels' STDP ring rule: the
     // shortest refractory period + 1, or 1 once spike histories were uploaded
     int min_isi = 1;
@@ -115,13 +114,16 @@ static int dalloc(bg3_net *n, T **p, size_t count, int fill = 0)
 }
 
 static size_t blk_act_bytes(size_t Np) { return BLK_ACT_ROWS * (Np / 32) * sizeof(uint32_t); }
-static size_t blk_range_bytes(size_t Np, int Mq)
+// A dense block's counts, flags and step masks (one allocation, in this order); 0 for networks that
+// never run one.
+static size_t blk_dense_bytes(size_t Np, int Mq)
 {
-    return bg3::blk_thin_ok(Mq) || !bg3::blk_dense_ok(Mq) ? 0 : Np / 32 * (size_t)Mq * sizeof(uint32_t);
+    return bg3::blk_thin_ok(Mq) || !bg3::blk_dense_ok(Mq)
+               ? 0 : (BLK_ACT_ROWS + 4 * (Np / 32)) * sizeof(uint32_t) + Np * (size_t)Mq * 4;
 }
 static size_t blk_bytes(size_t Np, int Mq)
 {
-    return Np * sizeof(unsigned long long) + blk_act_bytes(Np) + blk_range_bytes(Np, Mq);
+    return Np * sizeof(unsigned long long) + blk_act_bytes(Np) + blk_dense_bytes(Np, Mq);
 }
 
 static void drop_graph(bg3_net *n);
@@ -442,10 +444,18 @@ int bg3_create(const bg3_net_desc *desc, bg3_net **out)
     if ((rc = dalloc(n, &h.history, N * (size_t)max_spikes, 0xff)) != 0) goto fail;
     if (cudaMalloc((void **)&n->blk.hist, Np * sizeof(*n->blk.hist)) != cudaSuccess ||
         cudaMalloc((void **)&n->blk.act, blk_act_bytes(Np)) != cudaSuccess ||
-        (blk_range_bytes(Np, h.Mq) &&
-         cudaMalloc((void **)&n->blk.range, blk_range_bytes(Np, h.Mq)) != cudaSuccess)) {
+        (blk_dense_bytes(Np, h.Mq) &&
+         cudaMalloc((void **)&n->blk.actn, blk_dense_bytes(Np, h.Mq)) != cudaSuccess)) {
         rc = BG3_ENOMEM;
         goto fail;
+    }
+    if (n->blk.actn) {
+        n->blk.gflag = n->blk.actn + BLK_ACT_ROWS;
+        n->blk.msk = (uint8_t *)(n->blk.gflag + 4 * (Np / 32));
+        if (cudaMemsetAsync(n->blk.actn, 0, blk_dense_bytes(Np, h.Mq), n->stream) != cudaSuccess) {
+            rc = BG3_ECUDA;
+            goto fail;
+        }
     }
     if (cudaMalloc((void **)&n->d, sizeof(NetDev)) != cudaSuccess) { rc = BG3_ENOMEM; goto fail; }
     // type constants of createSynapse at this deltaT (Synapses/AllSpikingSynapses.cpp:192-240,
@@ -521,7 +531,7 @@ int64_t bg3_net_footprint(const bg3_net_desc *desc)
     if (D.neuron_kind == BG3_NEURON_IZH) b += 6 * N * 4;
     b += N * (uint64_t)ms * 8;                                     // spike history
     b += sizeof(NetDev) + 54 * N;                                  // descriptor, input
-    b += blk_bytes((size_t)Np, (int)((D.max_syn_per_neuron + 3) / 4));  // spike masks, source ranges
+    b += blk_bytes((size_t)Np, (int)((D.max_syn_per_neuron + 3) / 4));  // spike masks, arrival masks
     return (int64_t)b;
 }
 
@@ -557,7 +567,7 @@ int bg3_destroy(bg3_net *n)
     if (n->d) cudaFree(n->d);
     if (n->blk.hist) cudaFree(n->blk.hist);
     if (n->blk.act) cudaFree(n->blk.act);
-    if (n->blk.range) cudaFree(n->blk.range);
+    if (n->blk.actn) cudaFree(n->blk.actn);
     if (n->noise_dev) cudaFree(n->noise_dev);
     if (n->flush_buf) cudaFree(n->flush_buf);
     if (n->scrub_buf) cudaFree(n->scrub_buf);
@@ -593,7 +603,6 @@ static void ring_changed(bg3_net *n)
 {
     n->ring_ok = true;
     n->mask_ok = false;
-    n->range_ok = false;  // the synapses came with it
 }
 
 // ---- uploads --------------------------------------------------------------------------------
@@ -1127,11 +1136,6 @@ static int blk_steps(const bg3_net *n, const LaunchCfg &c)
 static int ensure_masks(bg3_net *n)
 {
     const unsigned long long w = blk_window(n);
-    if (n->blk.range && !n->range_ok) {
-        bg3::launch_blk_range(n->h, n->blk, n->stream);
-        CK(cudaGetLastError());
-        n->range_ok = true;
-    }
     if (n->mask_ok && w == n->blk.win) return BG3_OK;
     int rc = ensure_ring(n);
     if (rc) return rc;
@@ -1173,7 +1177,7 @@ static int run_blocks(bg3_net *n, int64_t nsteps, int T)
         left -= (int64_t)GRAPH_BLOCKS * T;
     }
     for (; left > 0; left -= T) one((int)std::min<int64_t>(left, T));
-    n->launches += blocks * (h.syn_kind >= BG3_SYN_STDP ? 2 : 1);
+    n->launches += blocks * (h.syn_kind >= BG3_SYN_STDP || !thin ? 2 : 1);
     CK(cudaGetLastError());
     return BG3_OK;
 }
@@ -1268,7 +1272,6 @@ int bg3_epoch_growth(bg3_net *n, int32_t epoch)
 {
     if (!n || epoch < 0) return BG3_EINVAL;
     bg3::launch_growth(n->h, n->d, epoch, n->cfg.growth_threads, n->stream);
-    n->range_ok = false;
     n->launches += 8;
     CK(cudaGetLastError());
     return BG3_OK;
@@ -1643,6 +1646,8 @@ struct bg3_batch {
     CUtensorMap *d_maps = nullptr;
     int2 *d_tiles = nullptr;
     BlkDev *d_blks = nullptr;
+    int *d_dense = nullptr;       // indices of the TMA-swept networks
+    int n_dense = 0, dense_tiles = 0;
     std::vector<BlkDev> blks;     // as uploaded
     int ntiles = 0, n_thick = 0, max_n = 0, syn_kind = 1, thin_mq = 0;
     cudaStream_t stream = nullptr;
@@ -1691,9 +1696,18 @@ static int batch_refresh(bg3_batch *b)
     for (auto &t : tiles)
         if (!bg3::sweep_is_thin(b->nets[t.second.x]->h, b->cfg)) tl.push_back(t.second);
     b->n_thick = (int)tl.size();
-    b->thin_mq = 0;
-    for (bg3_net *n : b->nets)
-        if (bg3::sweep_is_thin(n->h, b->cfg)) b->thin_mq = std::max(b->thin_mq, n->h.Mq);
+    b->thin_mq = b->dense_tiles = 0;
+    std::vector<int> dense;
+    for (size_t k = 0; k < b->nets.size(); k++) {
+        const NetDev &h = b->nets[k]->h;
+        if (bg3::sweep_is_thin(h, b->cfg)) {
+            b->thin_mq = std::max(b->thin_mq, h.Mq);
+        } else {
+            dense.push_back((int)k);
+            b->dense_tiles = std::max(b->dense_tiles, h.ntiles);
+        }
+    }
+    b->n_dense = (int)dense.size();
     tl.insert(tl.end(), thin.begin(), thin.end());
     if ((int)tl.size() != b->ntiles) {
         if (b->d_tiles) cudaFree(b->d_tiles);
@@ -1707,6 +1721,8 @@ static int batch_refresh(bg3_batch *b)
     CK(cudaMemcpyAsync(b->d_nets, hd.data(), hd.size() * sizeof(NetDev), cudaMemcpyHostToDevice, b->stream));
     CK(cudaMemcpyAsync(b->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, b->stream));
     CK(cudaMemcpyAsync(b->d_tiles, tl.data(), tl.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
+    if (b->n_dense)
+        CK(cudaMemcpyAsync(b->d_dense, dense.data(), dense.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     CK(cudaStreamSynchronize(b->stream));
     if (b->graph) cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
@@ -1746,7 +1762,8 @@ int bg3_batch_create(bg3_net *const *nets, int32_t count, bg3_batch **out)
     rc = BG3_ENOMEM;
     if (cudaMalloc(&b->d_nets, count * sizeof(NetDev)) != cudaSuccess ||
         cudaMalloc(&b->d_maps, 2 * count * sizeof(CUtensorMap)) != cudaSuccess ||
-        cudaMalloc(&b->d_blks, count * sizeof(BlkDev)) != cudaSuccess)
+        cudaMalloc(&b->d_blks, count * sizeof(BlkDev)) != cudaSuccess ||
+        cudaMalloc(&b->d_dense, count * sizeof(int)) != cudaSuccess)
         goto fail;
     for (bg3_net *n : b->nets) cudaStreamSynchronize(n->stream);
     if ((rc = batch_refresh(b)) != 0) goto fail;
@@ -1766,6 +1783,7 @@ int bg3_batch_destroy(bg3_batch *b)
     if (b->d_nets) cudaFree(b->d_nets);
     if (b->d_maps) cudaFree(b->d_maps);
     if (b->d_blks) cudaFree(b->d_blks);
+    if (b->d_dense) cudaFree(b->d_dense);
     if (b->d_tiles) cudaFree(b->d_tiles);
     if (b->flush_buf) cudaFree(b->flush_buf);
     if (b->scrub_buf) cudaFree(b->scrub_buf);
@@ -1818,7 +1836,7 @@ static void batch_block(bg3_batch *b, int nt)
 {
     if (b->n_thick > 0)
         bg3::launch_blk_dense_batch(b->syn_kind, b->d_nets, b->d_blks, b->d_maps, b->d_tiles,
-                                    b->n_thick, nt, b->stream);
+                                    b->n_thick, b->d_dense, b->n_dense, b->dense_tiles, nt, b->stream);
     if (b->ntiles > b->n_thick)
         bg3::launch_blk_thin_batch(b->syn_kind, b->d_nets, b->d_blks, (int)b->nets.size(),
                                b->d_tiles + b->n_thick, b->ntiles - b->n_thick, b->cfg.thin_warps,
@@ -1870,7 +1888,7 @@ static int batch_run_blocks(bg3_batch *b, int64_t nsteps, int T)
         left -= (int64_t)GRAPH_BLOCKS * T;
     }
     for (; left > 0; left -= T) batch_block(b, (int)std::min<int64_t>(left, T));
-    b->launches += blocks * ((b->n_thick > 0) + (b->ntiles > b->n_thick) * (b->syn_kind >= BG3_SYN_STDP ? 2 : 1));
+    b->launches += blocks * (2 * (b->n_thick > 0) + (b->ntiles > b->n_thick) * (b->syn_kind >= BG3_SYN_STDP ? 2 : 1));
     CK(cudaGetLastError());
     return batch_order(b, false);
 }

@@ -55,7 +55,10 @@ __global__ void __launch_bounds__(256) k_blk_act(const __grid_constant__ NetDev 
     const unsigned long long t = *n.step;
     const bool on = i < n.N && (b.hist[i] & rotl64(b.win, (unsigned)t)) != 0ull;
     const unsigned w = __ballot_sync(0xffffffffu, on);
-    if ((threadIdx.x & 31) == 0 && i < n.Np) b.act[(t & (BLK_ACT_ROWS - 1)) * n.ntiles + (i >> 5)] = w;
+    if ((threadIdx.x & 31) == 0 && i < n.Np) {
+        b.act[(t & (BLK_ACT_ROWS - 1)) * n.ntiles + (i >> 5)] = w;
+        if (b.actn && w) atomicAdd(&b.actn[t & (BLK_ACT_ROWS - 1)], (uint32_t)__popc(w));
+    }
 }
 // the ring lists from hist (ring_n zeroed before)
 __global__ void __launch_bounds__(256) k_blk_ring(const __grid_constant__ NetDev n,
@@ -111,12 +114,15 @@ __device__ __forceinline__ void blk_finish(const NetDev &n, const BlkDev &b, int
     }
     if (lane == 0) {
         b.act[(t1 & (BLK_ACT_ROWS - 1)) * n.ntiles + tile] = w;
+        if (b.actn && w) atomicAdd(&b.actn[t1 & (BLK_ACT_ROWS - 1)], (uint32_t)__popc(w));
         if (atomicAdd(n.sweep_done, 1u) == (unsigned)n.ntiles - 1u) {
             // the network's last tile: every tile has read the step
             *n.sweep_done = 0u;
             *n.step = t1;
             *n.dstep = t1;
             n.ring_n[t1 & (BG3_RING - 1)] = 0;
+            if (b.actn)  // the counts of the blocks that may follow the next one
+                for (int j = 1; j <= BLK_MAX_STEPS; j++) b.actn[(t1 + j) & (BLK_ACT_ROWS - 1)] = 0u;
             if (t1 >= 0xffffff00ull) set_err(n, ERR_STEP_RANGE);
         }
     }
@@ -461,24 +467,30 @@ __global__ void __launch_bounds__(256) k_blk_post_batch(const NetDev *nets, cons
 //                 come in
 //   warps 1-4     arrivals: find the rows whose source has a spike arriving, prepare the psr
 //                 increments (event slots, exp tables), draw the neurons' noise
-//   warps 5, 6    lane = destination, rows in slot order: warp 5 carries a chunk through the
-//                 block's first four steps, warp 6 through the rest and stores it back.  A row is a
-//                 chain of multiplications by its decay; a step's sum is a chain of additions over
-//                 the rows, in the reference's order; four steps a warp interleave four such chains.
-// Finding the arrivals: the range of bitmap words that a row quad's sources span is kept per tile
-// (k_blk_range); only quads with a set word in their range have their sources read.  The rows are
-// taken 16 at a time, by the arrival warps in turn: hits, the sources' masks and the increments go
-// into one of four buffers of step masks and increments, which the sum warps read; groups of 16 rows
-// without a quad to look at, or without a hit in them, take code that reads none.
+//   warp 5        lane = destination, rows in slot order: carries a chunk through the block's steps
+//                 and stores it back.  A row is a chain of multiplications by its decay; a step's sum
+//                 is a chain of additions over the rows, in the reference's order; the steps
+//                 interleave eight such chains.
+// Arrivals reach the tile in one of two ways, by the number of neurons with a spike that may arrive in
+// the block (BlkDev::actn, known when the block starts):
+//   light   (at most N / DN_LIGHT) k_blk_push has taken the spikes out along the outgoing map before:
+//           step masks in a plane of one byte per slot, increments beside the slots' event state, and
+//           a flag per 16 rows.  The arrival warps only collect the flagged rows.
+//   heavy   the arrival warps look up every slot's source in the spike masks and make the increments.
+// Either way 16 rows at a time, by the four warps in turn, into one of four buffers of step masks and
+// increments that the sum warp reads; groups of 16 rows without an arrival take code that reads none.
+// Why two: a pushed arrival costs half a dozen scattered accesses with the whole GPU to hide them, and
+// reads no sources; a pulled one is found among its neighbours in the slot planes, and costs a pass
+// over the sources.
 constexpr int DN_ROWS = 64, DN_QUADS = 16;
 constexpr int DN_STAGES = 4;
 constexpr int DN_MAX_CHUNKS = 32;   // 2,048 slots per destination
 constexpr int DN_BUFS = 4;
+constexpr int DN_GROUP_WORDS = 4 * DN_MAX_CHUNKS / 32;
+constexpr int DN_LIGHT = 128;
 constexpr int DN_ACT_WORDS = 1280;  // the bitmap row is kept in shared memory up to 40,960 neurons
 constexpr int DN_EV_WARPS = 4;      // = DN_BUFS: buffer k is filled by warp k
-constexpr int DN_THREADS = 32 * (1 + DN_EV_WARPS + 2);
-constexpr int DN_HALF = 4;          // steps of the first sum warp
-constexpr int DN_RANGE_SCAN = 16;   // a quad spanning more bitmap words is always looked at
+constexpr int DN_THREADS = 32 * (1 + DN_EV_WARPS + 1);
 constexpr uint32_t DN_CHUNK = DN_ROWS * 32 * 4 + DN_QUADS * 32 * 2;
 
 struct DenseSmem {
@@ -492,13 +504,12 @@ struct DenseSmem {
     int4 src[DN_EV_WARPS][2][4][32];                 // per arrival warp: a group's and the next one's
     uint32_t lc[DN_EV_WARPS][2][4][32];              // sources and delay classes
     int32_t ltab[BG3_MAX_DELAYS];
-    uint16_t quads[DN_MAX_CHUNKS];                   // per chunk, the row quads to look at
-    uint32_t groups[4 * DN_MAX_CHUNKS / 32];         // the 16-row groups with such a quad
-    int any[DN_BUFS];                                // the buffer has arrivals; 2: several at a row
+    uint32_t groups[DN_GROUP_WORDS];                 // the 16-row groups that have a buffer
+    int any[DN_BUFS];                                // bit q: quad q has arrivals; 16: several at a row
     int issued, failed;
-    uint64_t full[DN_STAGES], half[DN_STAGES], empty[DN_STAGES];
+    uint64_t full[DN_STAGES], empty[DN_STAGES];
     uint64_t bfull[DN_BUFS], bempty[DN_BUFS];
-    uint64_t scanned, summed[2], drawn;
+    uint64_t scanned, summed, drawn;
 };
 constexpr size_t DN_SMEM = sizeof(DenseSmem);
 
@@ -513,34 +524,6 @@ __device__ __forceinline__ bool dn_wait(const NetDev &n, DenseSmem &s, uint64_t 
     set_err(n, ERR_TIMEOUT);
     *(volatile int *)&s.failed = 1;
     return false;
-}
-
-// The bitmap words that the sources of a tile's row quads span, lo | hi << 16 (lo > hi: no synapse;
-// words past 16 bits: the whole range).  One warp per quad.
-__global__ void __launch_bounds__(256) k_blk_range(const __grid_constant__ NetDev n, uint32_t *range)
-{
-    const int lane = threadIdx.x & 31;
-    const long long total = (long long)n.ntiles * n.Mq;
-    for (long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; i < total;
-         i += ((long long)gridDim.x * blockDim.x) >> 5) {
-        const int tile = (int)(i / n.Mq), q = (int)(i % n.Mq);
-        const int d = tile * 32 + lane;
-        const int left = (d < n.N ? (int)n.count[d] : 0) - 4 * q;
-        uint32_t lo = 0xffffffffu, hi = 0u;
-        if (left > 0) {
-            const int4 v = reinterpret_cast<const int4 *>(n.src)[i * 32 + lane];
-            const uint32_t w[4] = {(uint32_t)v.x >> 5, (uint32_t)v.y >> 5, (uint32_t)v.z >> 5, (uint32_t)v.w >> 5};
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-                if (left > k) {
-                    lo = min(lo, w[k]);
-                    hi = max(hi, w[k]);
-                }
-        }
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        if (lane == 0) range[i] = lo > hi ? 0x0000ffffu : hi > 0xffffu ? 0xffff0000u : lo | (hi << 16);
-    }
 }
 
 // The lane's rows of quad sources v with a spike that may arrive (bit r: row r).
@@ -609,12 +592,138 @@ __device__ __forceinline__ void dense_arrivals(const NetDev &n, const DenseSmem 
     }
 }
 
+__device__ __forceinline__ bool blk_light(const NetDev &n, const BlkDev &b, unsigned long long t)
+{
+    return (unsigned long long)b.actn[t & (BLK_ACT_ROWS - 1)] * DN_LIGHT <= (unsigned long long)n.N;
+}
+
+// Light blocks: the spikes taken out along the outgoing map.  A block of the grid serves 2,048 neurons
+// (64 bitmap words) and every gridDim.y-th 128-synapse chunk of theirs; it lists the neurons with a
+// spike, and its warps take them in turn, four synapses per lane.  A slot's step mask and increment
+// wait for the tile's arrival warps (dense_collect); a synapse with several spikes in the block keeps
+// only its mask.
+constexpr int PUSH_WORDS = 64, PUSH_THREADS = 256;
+template <int SYN>
+__device__ __forceinline__ void blk_push(const NetDev &n, const BlkDev &b, int bx, int split, int nsplit, int nt)
+{
+    __shared__ int s_list[PUSH_WORDS * 32];
+    __shared__ int s_n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    const unsigned long long t = *n.step;
+    if (!blk_light(n, b, t)) return;
+    if (threadIdx.x < PUSH_WORDS && bx * PUSH_WORDS + (int)threadIdx.x < n.ntiles) {
+        const int word = bx * PUSH_WORDS + (int)threadIdx.x;
+        uint32_t w = b.act[(t & (BLK_ACT_ROWS - 1)) * n.ntiles + word];
+        if (w) {
+            int at = atomicAdd(&s_n, __popc(w));
+            for (; w; w &= w - 1u) s_list[at++] = word * 32 + __ffs((int)w) - 1;
+        }
+    }
+    __syncthreads();
+    const int total = s_n;
+    for (int it = warp; it < total; it += PUSH_THREADS / 32) {
+        const int i = s_list[it];
+        const unsigned long long h = b.hist[i];
+        for (int c = 0; c < n.n_delays; c++) {
+            const int D = n.ltab[c];
+            const uint32_t m = (uint32_t)rotr64(h, (unsigned)t - (unsigned)D) & ((1u << nt) - 1u);
+            if (!m) continue;
+            const bool one = (m & (m - 1u)) == 0u;
+            const uint32_t ta = (uint32_t)t + (uint32_t)(31 - __clz((int)m));
+            const size_t ci = (size_t)c * n.N + i;
+            const uint32_t b0 = n.outBegin[ci], k = n.outCount[ci];
+            for (uint32_t base = (uint32_t)split * 128u; base < k; base += (uint32_t)nsplit * 128u) {
+                constexpr int U = 4;
+                uint32_t p[U];
+                float4 e[U];
+                uint2 f[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const uint32_t j = base + (uint32_t)lane + 32u * u;
+                    p[u] = j < k ? n.outMap[b0 + j] : 0xffffffffu;
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (p[u] != 0xffffffffu) {
+                        const char *q = reinterpret_cast<const char *>(n.ev) + (size_t)p[u] * sizeof(EvSlot);
+                        e[u] = *reinterpret_cast<const float4 *>(q);
+                        f[u] = *reinterpret_cast<const uint2 *>(q + 16);
+                    }
+                float xr[U], xu[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (p[u] == 0xffffffffu || !one) continue;
+                    const uint32_t last = __float_as_uint(e[u].w);
+                    if ((int32_t)(ta - (uint32_t)D - f[u].x) < 0) {
+                        p[u] = 0xffffffffu;  // the synapse did not exist when the spike left
+                    } else if (SYN == 1 && last != BG3_NO_SPIKE32) {
+                        const int pc = (int)((f[u].y >> 8) & 255u);
+                        xr[u] = exp_tab(n, n.p_xD[pc], ta - last, n.p_D[pc]);
+                        xu[u] = exp_tab(n, n.p_xF[pc], ta - last, n.p_F[pc]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (p[u] == 0xffffffffu) continue;
+                    if (one) {
+                        float4 *q = reinterpret_cast<float4 *>(n.ev) + 2 * (size_t)p[u];
+                        const float dec = n.dtab[f[u].y & 255u];
+                        float inc;
+                        if (SYN == 1) {
+                            float uu = e[u].y, rr = e[u].z;
+                            if (__float_as_uint(e[u].w) != BG3_NO_SPIKE32) {
+                                const float Uc = n.p_U[(f[u].y >> 8) & 255u];
+                                rr = 1.0f + (rr * (1.0f - uu) - 1.0f) * xr[u];
+                                uu = Uc + uu * (1.0f - Uc) * xu[u];
+                            }
+                            inc = (e[u].x / dec) * uu * rr;
+                            gst(q, make_float4(e[u].x, uu, rr, __uint_as_float(ta)));
+                        } else {
+                            inc = e[u].x / dec;
+                        }
+                        gst(&n.ev[p[u]].pad1, __float_as_uint(inc));
+                    }
+                    gst(&b.msk[p[u]], (uint8_t)m);
+                    // slot p: tile p / (128 Mq), row quad (p / 128) % Mq; 16 rows a flag
+                    const uint32_t q4 = p[u] >> 7, tile = q4 / (uint32_t)n.Mq, g = (q4 - tile * (uint32_t)n.Mq) >> 2;
+                    atomicOr(&b.gflag[tile * DN_GROUP_WORDS + (g >> 5)], 1u << (g & 31));
+                }
+            }
+        }
+    }
+}
+
+template <int SYN>
+__global__ void __launch_bounds__(PUSH_THREADS) k_blk_push(const __grid_constant__ NetDev n,
+                                                           const __grid_constant__ BlkDev b, int nt)
+{
+    blk_push<SYN>(n, b, blockIdx.x, blockIdx.y, gridDim.y, nt);
+}
+
+// Batched form: grid.z indexes the networks that run dense blocks.
+template <int SYN>
+__global__ void __launch_bounds__(PUSH_THREADS) k_blk_push_batch(const NetDev *nets, const BlkDev *blks,
+                                                                 const int *dense, int nt)
+{
+    __shared__ __align__(16) NetDev s_net;
+    const int k = dense[blockIdx.z];
+    if ((int)blockIdx.x * PUSH_WORDS >= nets[k].ntiles) return;
+    const uint4 *s4 = reinterpret_cast<const uint4 *>(nets + k);
+    uint4 *d4 = reinterpret_cast<uint4 *>(&s_net);
+    for (int i = threadIdx.x; i < (int)(sizeof(NetDev) / 16); i += blockDim.x) d4[i] = s4[i];
+    blk_push<SYN>(s_net, blks[k], blockIdx.x, blockIdx.y, gridDim.y, nt);
+}
+
 // The 16 rows of buffer bf where a synapse has several spikes arriving in the block: those arrivals
 // run at their steps.  psr in place, the steps' sums in and out.
 template <int SYN>
 __device__ __noinline__ void dense_late(const NetDev &n, const DenseSmem &s, int tile, int row0, int bf,
-                                        int j0, int nj, unsigned long long t, float4 *ps4,
-                                        const uint16_t *cw, float *acc)
+                                        int nt, unsigned long long t, float4 *ps4, const uint16_t *cw,
+                                        float *acc)
 {
     const int lane = threadIdx.x & 31, d = tile * 32 + lane;
     for (int r = 0; r < 16; r++) {
@@ -624,11 +733,11 @@ __device__ __noinline__ void dense_late(const NetDev &n, const DenseSmem &s, int
         const uint32_t m = (s.bmsk[bf][q][lane] >> (8 * i)) & 255u;
         const bool many = (m & (m - 1u)) != 0u;
         float x = *pr;
-        for (int j = 0; j < nj; j++) {
-            if ((m >> (j0 + j)) & 1u) {
+        for (int j = 0; j < nt; j++) {
+            if ((m >> j) & 1u) {
                 if (many) {
                     const uint32_t p = (uint32_t)slot_pos(row0 + r, d, n.Mq);
-                    const unsigned long long tj = t + (unsigned)(j0 + j);
+                    const unsigned long long tj = t + (unsigned)j;
                     float a;
                     if (arrival<SYN>(n, p, d, n.src[p], (uint32_t)tj - (uint32_t)n.ltab[n.lcls[p]], tj, a))
                         x = x + a;
@@ -653,88 +762,93 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b)
     return r;
 }
 
-// Four rows through a half block's steps: psr scaled, and added to each step's sum in row order.  The
-// products of a step's four rows are independent of each other, as are the four steps' sums of a
-// row, so neither half of this waits on itself.  HIT: rows may have an arrival, at the step whose
-// bit is set in the row's byte of m (bit j: step j).  FULL: all DN_HALF steps, else nj.
+// x + inc where m has the bit, as one predicated addition (a branch per step and row otherwise).
+template <uint32_t BIT>
+__device__ __forceinline__ void add_if(float &x, uint32_t m, float inc)
+{
+    asm("{\n .reg .pred p;\n .reg .b32 b;\n and.b32 b, %1, %2;\n setp.ne.u32 p, b, 0;\n"
+        " @p add.rn.f32 %0, %0, %3;\n}\n"
+        : "+f"(x) : "r"(m), "n"(BIT), "f"(inc));
+}
+template <int J>
+__device__ __forceinline__ void add_hits(float2 &x, float2 &y, uint32_t m, const float4 &in)
+{
+    add_if<0x1u << J>(x.x, m, in.x);
+    add_if<0x100u << J>(x.y, m, in.y);
+    add_if<0x10000u << J>(y.x, m, in.z);
+    add_if<0x1000000u << J>(y.y, m, in.w);
+}
+
+// Four rows through the block's steps: psr scaled, and added to each step's sum in row order.  The
+// products of a step's four rows are independent of each other, as are the steps' sums of a row, so neither half of this waits on itself.  HIT: rows may have an arrival, at the step whose
+// bit is set in the row's byte of m (bit j: step j).  FULL: nt = BLK_MAX_STEPS.
 template <bool FULL, bool HIT>
-__device__ __forceinline__ void dense_quad(float4 &v, const float4 &dc, float (&acc)[DN_HALF], int nj,
+__device__ __forceinline__ void dense_quad(float4 &v, const float4 &dc, float (&acc)[BLK_MAX_STEPS], int nt,
                                            uint32_t m, const float4 &in)
 {
-    float2 p[DN_HALF][2];
+    float2 p[BLK_MAX_STEPS][2];
     float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w);
     const float2 dx = make_float2(dc.x, dc.y), dy = make_float2(dc.z, dc.w);
 #pragma unroll
-    for (int j = 0; j < DN_HALF; j++) {
-        if (!FULL && j >= nj) break;
+    for (int j = 0; j < BLK_MAX_STEPS; j++) {
         if (HIT) {
-            if (m & (1u << j)) x.x = x.x + in.x;
-            if (m & (0x100u << j)) x.y = x.y + in.y;
-            if (m & (0x10000u << j)) y.x = y.x + in.z;
-            if (m & (0x1000000u << j)) y.y = y.y + in.w;
+            if (j == 0) add_hits<0>(x, y, m, in);
+            if (j == 1) add_hits<1>(x, y, m, in);
+            if (j == 2) add_hits<2>(x, y, m, in);
+            if (j == 3) add_hits<3>(x, y, m, in);
+            if (j == 4) add_hits<4>(x, y, m, in);
+            if (j == 5) add_hits<5>(x, y, m, in);
+            if (j == 6) add_hits<6>(x, y, m, in);
+            if (j == 7) add_hits<7>(x, y, m, in);
         }
         p[j][0] = x = mul2(x, dx);
         p[j][1] = y = mul2(y, dy);
+        // a shorter block keeps psr as of its last step; the sums past it are not used
+        if (!FULL && j == nt - 1) v = make_float4(x.x, x.y, y.x, y.y);
     }
+    if (FULL) v = make_float4(x.x, x.y, y.x, y.y);
 #pragma unroll
-    for (int j = 0; j < DN_HALF; j++) {
-        if (!FULL && j >= nj) break;
-        acc[j] = acc[j] + p[j][0].x;
-    }
+    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = acc[j] + p[j][0].x;
 #pragma unroll
-    for (int j = 0; j < DN_HALF; j++) {
-        if (!FULL && j >= nj) break;
-        acc[j] = acc[j] + p[j][0].y;
-    }
+    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = acc[j] + p[j][0].y;
 #pragma unroll
-    for (int j = 0; j < DN_HALF; j++) {
-        if (!FULL && j >= nj) break;
-        acc[j] = acc[j] + p[j][1].x;
-    }
+    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = acc[j] + p[j][1].x;
 #pragma unroll
-    for (int j = 0; j < DN_HALF; j++) {
-        if (!FULL && j >= nj) break;
-        acc[j] = acc[j] + p[j][1].y;
-    }
-    v = make_float4(x.x, x.y, y.x, y.y);
+    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = acc[j] + p[j][1].y;
 }
 
-// nj steps from j0 on over all chunks: psr scaled in place, a step's sum over the rows in order.
-// last: the second sum warp, which takes chunks from the first one and stores them back.  FULL:
-// nj = DN_HALF.  Measured alone on an SM (cycles a row of 32 destinations, four steps): 16 rows at a
-// time with paired products 17.7, without the pairs 19.6, eight rows at a time 23, eight rows with
-// the next eight loading 36 (more instructions than latency saved).
+// The decay factors of a row quad's four class codes.
+__device__ __forceinline__ float4 dense_decay(const DenseSmem &s, uint32_t c)
+{
+    return make_float4(s.dtab[c & 15u], s.dtab[(c >> 4) & 15u], s.dtab[(c >> 8) & 15u],
+                       s.dtab[(c >> 12) & 15u]);
+}
+
+// The sum warp: the block's steps over all chunks, psr scaled in place, a step's sum over the rows in
+// order.  FULL: nt = BLK_MAX_STEPS.  Measured as one warp on an SM, cycles a row of 32
+// destinations: eight steps 28 with 16 rows at a time and paired products, 33 with eight rows at a
+// time, 42 with four; two warps of four steps each, one after the other, 18 each (and 28 each beside
+// another tile's two).
 template <int SYN, bool FULL>
 __device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem &s, const CUtensorMap *tm_psr,
-                                           int tile, int nch, int nj, int j0, bool last,
-                                           unsigned long long t)
+                                           int tile, int nch, int nt, unsigned long long t)
 {
     const int lane = threadIdx.x & 31;
-    float acc[DN_HALF];
+    float acc[BLK_MAX_STEPS];
 #pragma unroll
-    for (int j = 0; j < DN_HALF; j++) acc[j] = 0.0f;
+    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = 0.0f;
     bool ok = dn_wait(n, s, &s.scanned, 0);
     int k = 0;  // 16-row groups with a buffer so far
     for (int c = 0; ok && c < nch; c++) {
         const int st = c % DN_STAGES;
-        ok = dn_wait(n, s, last ? &s.half[st] : &s.full[st], (uint32_t)((c / DN_STAGES) & 1));
+        ok = dn_wait(n, s, &s.full[st], (uint32_t)((c / DN_STAGES) & 1));
         if (!ok) break;
         float4 *ps4 = reinterpret_cast<float4 *>(s.stage[st]) + lane;
         const uint16_t *cw = reinterpret_cast<const uint16_t *>(s.stage[st] + DN_ROWS * 32 * 4) + lane;
+        const uint32_t groups = s.groups[c >> 3] >> (4 * (c & 7));
 #pragma unroll 1
         for (int g = 0; g < 4; g++, ps4 += 4 * 32, cw += 4 * 32) {
-            float4 v[4], dc[4];
-            uint32_t cl[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                v[q] = ps4[q * 32];
-                cl[q] = cw[q * 32];
-            }
-            const bool looked = (s.groups[c >> 3] >> (4 * (c & 7) + g)) & 1u;
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                dc[q] = make_float4(s.dtab[cl[q] & 15u], s.dtab[(cl[q] >> 4) & 15u],
-                                    s.dtab[(cl[q] >> 8) & 15u], s.dtab[(cl[q] >> 12) & 15u]);
+            const bool looked = (groups >> g) & 1u;
             const int bf = k % DN_BUFS;
             int any = 0;
             if (looked) {
@@ -744,26 +858,43 @@ __device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem &s, const 
                 any = s.any[bf];
             }
             if (any == 0) {
+                float4 v[4], dc[4];
+                uint32_t cl[4];
 #pragma unroll
-                for (int q = 0; q < 4; q++) dense_quad<FULL, false>(v[q], dc[q], acc, nj, 0u, v[q]);
-            } else if (any == 1) {
+                for (int q = 0; q < 4; q++) {
+                    v[q] = ps4[q * 32];
+                    cl[q] = cw[q * 32];
+                }
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    dense_quad<FULL, true>(v[q], dc[q], acc, nj, s.bmsk[bf][q][lane] >> j0,
-                                           s.binc[bf][q][lane]);
-            } else {
-                float a[DN_HALF];
+                for (int q = 0; q < 4; q++) dc[q] = dense_decay(s, cl[q]);
 #pragma unroll
-                for (int j = 0; j < DN_HALF; j++) a[j] = acc[j];
-                dense_late<SYN>(n, s, tile, c * DN_ROWS + 16 * g, bf, j0, nj, t, ps4, cw, a);
-#pragma unroll
-                for (int j = 0; j < DN_HALF; j++) acc[j] = a[j];
-            }
-            if (any != 2) {
+                for (int q = 0; q < 4; q++) dense_quad<FULL, false>(v[q], dc[q], acc, nt, 0u, v[q]);
 #pragma unroll
                 for (int q = 0; q < 4; q++) ps4[q * 32] = v[q];
+            } else if (!(any & 16)) {
+#pragma unroll 1
+                for (int q = 0; q < 4; q += 2) {
+                    float4 v0 = ps4[q * 32], v1 = ps4[(q + 1) * 32];
+                    const float4 d0 = dense_decay(s, cw[q * 32]), d1 = dense_decay(s, cw[(q + 1) * 32]);
+                    if ((any >> q) & 3) {
+                        dense_quad<FULL, true>(v0, d0, acc, nt, s.bmsk[bf][q][lane], s.binc[bf][q][lane]);
+                        dense_quad<FULL, true>(v1, d1, acc, nt, s.bmsk[bf][q + 1][lane], s.binc[bf][q + 1][lane]);
+                    } else {
+                        dense_quad<FULL, false>(v0, d0, acc, nt, 0u, v0);
+                        dense_quad<FULL, false>(v1, d1, acc, nt, 0u, v1);
+                    }
+                    ps4[q * 32] = v0;
+                    ps4[(q + 1) * 32] = v1;
+                }
+            } else {
+                float a[BLK_MAX_STEPS];
+#pragma unroll
+                for (int j = 0; j < BLK_MAX_STEPS; j++) a[j] = acc[j];
+                dense_late<SYN>(n, s, tile, c * DN_ROWS + 16 * g, bf, nt, t, ps4, cw, a);
+#pragma unroll
+                for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = a[j];
             }
-            if (last && looked) {
+            if (looked) {
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&s.bempty[bf]);
             }
@@ -772,36 +903,32 @@ __device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem &s, const 
         fence_async_smem();  // the TMA store (async proxy) must see these writes
         __syncwarp();
         if (lane == 0) {
-            if (!last) {
-                mbar_arrive(&s.half[st]);
-            } else {
-                tma_store_3d(tm_psr, 0, c * DN_QUADS, tile, s.stage[st]);
-                bulk_commit();
-                if (c >= 1) {
-                    bulk_wait_read1();
-                    mbar_arrive(&s.empty[(c - 1) % DN_STAGES]);
-                }
+            tma_store_3d(tm_psr, 0, c * DN_QUADS, tile, s.stage[st]);
+            bulk_commit();
+            if (c >= 1) {
+                bulk_wait_read1();
+                mbar_arrive(&s.empty[(c - 1) % DN_STAGES]);
             }
         }
         __syncwarp();
     }
-    if (last && lane == 0) bulk_wait_read_all();
+    if (lane == 0) bulk_wait_read_all();
 #pragma unroll
-    for (int j = 0; j < DN_HALF; j++)
-        if (j < nj) s.sum[j0 + j][lane] = acc[j];
+    for (int j = 0; j < BLK_MAX_STEPS; j++)
+        if (j < nt) s.sum[j][lane] = acc[j];
     __syncwarp();
-    if (ok && lane == 0) mbar_arrive(&s.summed[last ? 1 : 0]);
+    if (ok && lane == 0) mbar_arrive(&s.summed);
 }
 
-// Sources and delay classes (a byte per row) of 16 rows of the lane's destination, of the quads to
-// look at, on their way to shared memory.
+// Sources and delay classes (a byte per row) of 16 rows of the lane's destination, on their way to
+// shared memory.
 __device__ __forceinline__ void dense_sources(DenseSmem &s, int w, int st, const int4 *S,
-                                              const uint32_t *L, int q0, uint32_t quads, int cnt)
+                                              const uint32_t *L, int q0, int cnt)
 {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int q = 0; q < 4; q++)
-        if (((quads >> q) & 1u) && cnt > 4 * (q0 + q)) {
+        if (cnt > 4 * (q0 + q)) {
             asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&s.src[w][st][q][lane])),
                          "l"(&S[(size_t)(q0 + q) * 32]) : "memory");
             asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&s.lc[w][st][q][lane])),
@@ -810,76 +937,98 @@ __device__ __forceinline__ void dense_sources(DenseSmem &s, int w, int st, const
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// The arrival warps' part.  Warp w: first the quads to look at (all four warps share them out),
-// then every fourth 16-row group with one, the next such group's sources on their way meanwhile.
+// The arrival warps of a light block: the flagged groups' masks and increments, both planes left
+// clean for the next block.
+__device__ __forceinline__ void dense_collect(const NetDev &n, const BlkDev &b, DenseSmem &s, int tile, int w)
+{
+    const int lane = threadIdx.x & 31;
+    if (w < DN_GROUP_WORDS && lane == 0) {
+        const uint32_t f = b.gflag[tile * DN_GROUP_WORDS + w];
+        s.groups[w] = f;
+        if (f) b.gflag[tile * DN_GROUP_WORDS + w] = 0u;
+    }
+    bar_events();
+    if (lane == 0) mbar_arrive(&s.scanned);
+    uint32_t *M = reinterpret_cast<uint32_t *>(b.msk) + (size_t)tile * n.Mq * 32 + lane;
+    EvSlot *E = n.ev + (size_t)tile * n.Mq * 128 + (size_t)lane * 4;
+    int k = 0, used = 0;
+    for (int word = 0; word < DN_GROUP_WORDS; word++)
+        for (uint32_t left = s.groups[word]; left; left &= left - 1u) {
+            if (k++ % DN_BUFS != w) continue;
+            const int g = 32 * word + __ffs((int)left) - 1;
+            uint32_t m[4], any = 0u;
+#pragma unroll
+            for (int q = 0; q < 4; q++) m[q] = 4 * g + q < n.Mq ? M[(size_t)(4 * g + q) * 32] : 0u;
+            if (used > 0 && !dn_wait(n, s, &s.bempty[w], (uint32_t)((used - 1) & 1))) return;
+            used++;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                s.bmsk[w][q][lane] = m[q];
+                if (m[q]) {
+                    M[(size_t)(4 * g + q) * 32] = 0u;
+                    any |= 1u << q;
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const uint32_t mr = (m[q] >> (8 * r)) & 255u;
+                        if (mr & (mr - 1u)) {
+                            any |= 16u;
+                        } else if (mr) {
+                            uint32_t *inc = &E[(size_t)(4 * g + q) * 128 + r].pad1;
+                            reinterpret_cast<float *>(&s.binc[w][q][lane])[r] = __uint_as_float(*inc);
+                            *inc = 0u;
+                        }
+                    }
+                }
+            }
+            any = __reduce_or_sync(0xffffffffu, any);
+            __syncwarp();
+            if (lane == 0) {
+                s.any[w] = (int)any;
+                mbar_arrive(&s.bfull[w]);
+            }
+        }
+}
+
+// The arrival warps of a heavy block: warp w takes every fourth 16-row group, the next one's sources
+// on their way meanwhile.
 template <int SYN>
 __device__ __forceinline__ void dense_events(const NetDev &n, const BlkDev &b, DenseSmem &s, int tile,
                                              int w, int cnt, int nch, int nt, unsigned long long t)
 {
-    const int lane = threadIdx.x & 31, tid = (int)threadIdx.x - 32;
+    const int lane = threadIdx.x & 31, tid = 32 * w + lane;
     const size_t base = (size_t)tile * n.Mq * 32 + lane;
     const int4 *S = reinterpret_cast<const int4 *>(n.src) + base;
     const uint32_t *L = reinterpret_cast<const uint32_t *>(n.lcls) + base;
     const uint32_t *act = b.act + (t & (BLK_ACT_ROWS - 1)) * n.ntiles;
+    if (w < DN_GROUP_WORDS && lane == 0) {
+        const int k = 4 * nch - 32 * w;
+        s.groups[w] = k >= 32 ? 0xffffffffu : k > 0 ? (1u << k) - 1u : 0u;
+    }
     if (n.ntiles <= DN_ACT_WORDS) {
         for (int i = tid; i < n.ntiles; i += 32 * DN_EV_WARPS) s.act[i] = act[i];
         act = s.act;
-        bar_events();
     }
-    // one lane per row quad: is a bitmap word of its sources' range set?
-    for (int q = tid; q < nch * DN_QUADS; q += 32 * DN_EV_WARPS) {
-        const uint32_t rg = q < n.Mq ? b.range[(size_t)tile * n.Mq + q] : 0x0000ffffu;
-        const int lo = (int)(rg & 0xffffu), hi = (int)(rg >> 16);
-        bool look = hi - lo >= DN_RANGE_SCAN;
-        if (!look)
-            for (int i = lo; i <= hi; i++) look = look || act[i] != 0u;
-        // whole warps but for the last, whose lower half may hold the last chunk
-        const uint32_t m = __ballot_sync(q - lane + 32 <= nch * DN_QUADS ? 0xffffffffu : 0xffffu, look);
-        if (lane == 0 || lane == 16) s.quads[q / DN_QUADS] = (uint16_t)(m >> lane);
-    }
-    bar_events();
-    uint32_t mine = 0u;  // groups 32 w .. 32 w + 31
-    if (32 * w + lane < 4 * nch) mine = (s.quads[8 * w + (lane >> 2)] >> (4 * (lane & 3))) & 15u;
-    mine = __ballot_sync(0xffffffffu, mine != 0u);
-    if (lane == 0) s.groups[w] = mine;
     bar_events();
     if (lane == 0) mbar_arrive(&s.scanned);
-    // walks the groups; returns this warp's next one, or -1
-    int word = -1, k = 0;
-    uint32_t left = 0u;
-    auto next = [&]() {
-        for (;;) {
-            while (!left) {
-                if (++word == (int)(sizeof(s.groups) / 4)) return -1;
-                left = s.groups[word];
-            }
-            const int g = 32 * word + __ffs((int)left) - 1;
-            left &= left - 1u;
-            if (k++ % DN_BUFS == w) return g;
-        }
-    };
-    int g = next(), used = 0;
-    if (g >= 0) dense_sources(s, w, 0, S, L, 4 * g, s.quads[g >> 2] >> (4 * (g & 3)), cnt);
-    while (g >= 0) {
+    if (w < 4 * nch) dense_sources(s, w, 0, S, L, 4 * w, cnt);
+    for (int g = w, used = 0; g < 4 * nch; g += DN_BUFS) {
         const int st = used & 1;
-        const int gn = next();
-        if (gn >= 0) {
-            dense_sources(s, w, st ^ 1, S, L, 4 * gn, s.quads[gn >> 2] >> (4 * (gn & 3)), cnt);
+        if (g + DN_BUFS < 4 * nch) {
+            dense_sources(s, w, st ^ 1, S, L, 4 * (g + DN_BUFS), cnt);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         // hits, then the hits' sources' masks: the steps of the block at which a spike arrives (each
         // lane reads only what it copied itself)
-        const uint32_t quads = s.quads[g >> 2] >> (4 * (g & 3));
         uint32_t h16 = 0u;
 #pragma unroll
         for (int q = 0; q < 4; q++)
-            if ((quads >> q) & 1u) h16 |= dense_hits(s.src[w][st][q][lane], act, cnt - 4 * (4 * g + q)) << (4 * q);
+            h16 |= dense_hits(s.src[w][st][q][lane], act, cnt - 4 * (4 * g + q)) << (4 * q);
         const bool some = __any_sync(0xffffffffu, h16 != 0u);
         if (used > 0 && !dn_wait(n, s, &s.bempty[w], (uint32_t)((used - 1) & 1))) return;
         used++;
-        bool many = false, hit = false;
+        uint32_t any = 0u;  // bit q: quad q has an arrival; 16: a row has several
         if (some) {
             uint8_t *mb = reinterpret_cast<uint8_t *>(&s.bmsk[w][0][lane]);  // row r: mb[128 (r / 4) + r % 4]
             const uint8_t *lb = reinterpret_cast<const uint8_t *>(&s.lc[w][st][0][lane]);
@@ -906,9 +1055,9 @@ __device__ __forceinline__ void dense_events(const NetDev &n, const BlkDev &b, D
                         const uint32_t m = (uint32_t)rotr64(hs[u], (unsigned)t - (unsigned)D) & ((1u << nt) - 1u);
                         if (!m) continue;
                         mb[128 * (r[u] >> 2) + (r[u] & 3)] = (uint8_t)m;
-                        hit = true;
+                        any |= 1u << (r[u] >> 2);
                         if (m & (m - 1u)) {
-                            many = true;
+                            any |= 16u;
                         } else {
                             one |= 1u << r[u];
                             // towards the L1: a batch's loads below then wait for its first time only
@@ -942,15 +1091,13 @@ __device__ __forceinline__ void dense_events(const NetDev &n, const BlkDev &b, D
                         ib[r[u]] = inc[u];
                     }
             }
-            hit = __any_sync(0xffffffffu, hit);
-            many = __any_sync(0xffffffffu, many);
+            any = __reduce_or_sync(0xffffffffu, any);
         }
         __syncwarp();
         if (lane == 0) {
-            s.any[w] = many ? 2 : hit ? 1 : 0;
+            s.any[w] = (int)any;
             mbar_arrive(&s.bfull[w]);
         }
-        g = gn;
     }
 }
 
@@ -959,7 +1106,10 @@ __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
                                                const CUtensorMap *tm_psr, const CUtensorMap *tm_cls,
                                                const int tile, const int nt, DenseSmem &s)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // Roles rotate with the block: warp k of every block is issued by the same quarter of its SM, and
+    // the sum warps of the blocks that share an SM (152 apart in a first wave) are the busy ones.
+    const int lane = threadIdx.x & 31;
+    const int warp = (int)(threadIdx.x / 32 + blockIdx.x / 152) % (DN_THREADS / 32);
     const int d = tile * 32 + lane;
     const bool valid = d < n.N;
     for (int i = threadIdx.x; i < n.n_dcls; i += blockDim.x) s.dtab[i] = n.dtab[i];
@@ -969,15 +1119,13 @@ __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
     if (threadIdx.x == 0) {
         for (int i = 0; i < DN_STAGES; i++) {
             mbar_init(&s.full[i], 1);
-            mbar_init(&s.half[i], 1);
             mbar_init(&s.empty[i], 1);
         }
         for (int i = 0; i < DN_BUFS; i++) {
             mbar_init(&s.bfull[i], 1);
             mbar_init(&s.bempty[i], 1);
         }
-        mbar_init(&s.summed[0], 1);
-        mbar_init(&s.summed[1], 1);
+        mbar_init(&s.summed, 1);
         mbar_init(&s.scanned, DN_EV_WARPS);
         mbar_init(&s.drawn, DN_EV_WARPS);
         fence_mbar_init();
@@ -1020,9 +1168,7 @@ __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
 #pragma unroll 1
         for (int j = 0; ok && j < nt; j++) {
             // step t + j takes the sum of step t + j - 1
-            if (j == 1) ok = dn_wait(n, s, &s.summed[0], 0);
-            if (j == DN_HALF + 1) ok = dn_wait(n, s, &s.summed[1], 0);
-            if (!ok) break;
+            if (j == 1 && !(ok = dn_wait(n, s, &s.summed, 0))) break;
             if (j > 0) sp = s.sum[j - 1][lane];
             if (valid) {
                 const unsigned long long tj = t + (unsigned)j;
@@ -1031,26 +1177,22 @@ __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
                 if (neuron_update(n, d, x, br, in, s.noise[j][lane], tj, mode)) fired |= 1u << j;
             }
         }
-        if (ok && nt == 1) ok = dn_wait(n, s, &s.summed[0], 0);
-        if (ok && nt <= DN_HALF + 1) ok = dn_wait(n, s, &s.summed[1], 0);
+        if (ok && nt == 1) ok = dn_wait(n, s, &s.summed, 0);
         if (ok) {
             sp = s.sum[nt - 1][lane];
             blk_finish<SYN>(n, b, tile, d, valid, x, sp, hist, fired, nt, t);
         }
     } else if (warp <= DN_EV_WARPS) {  // ------------------------------------------- arrivals
         const int w = warp - 1;
-        dense_events<SYN>(n, b, s, tile, w, cnt, nch, nt, t);
+        if (blk_light(n, b, t)) dense_collect(n, b, s, tile, w);
+        else dense_events<SYN>(n, b, s, tile, w, cnt, nch, nt, t);
         for (int j = w; j < nt; j += DN_EV_WARPS)
             s.noise[j][lane] = normal_device(n.noise_seed, t + (unsigned)j, d);
         __syncwarp();
         if (lane == 0) mbar_arrive(&s.drawn);
     } else {  // --------------------------------------------------------------------- sums
-        const bool last = warp == DN_EV_WARPS + 2;
-        if (nt == 2 * DN_HALF)
-            dense_sums<SYN, true>(n, s, tm_psr, tile, nch, DN_HALF, last ? DN_HALF : 0, last, t);
-        else
-            dense_sums<SYN, false>(n, s, tm_psr, tile, nch, last ? max(0, nt - DN_HALF) : min(nt, DN_HALF),
-                               last ? DN_HALF : 0, last, t);
+        if (nt == BLK_MAX_STEPS) dense_sums<SYN, true>(n, s, tm_psr, tile, nch, nt, t);
+        else dense_sums<SYN, false>(n, s, tm_psr, tile, nch, nt, t);
     }
     __syncthreads();
     if (*(volatile int *)&s.failed && threadIdx.x == 0) {
@@ -1112,16 +1254,12 @@ static void launch_dep(void (*kern)(KArgs...), dim3 grid, int block, size_t smem
 }
 
 bool blk_thin_ok(int Mq) { return Mq <= BLK_THIN_QUADS; }
-void launch_blk_range(const NetDev &h, const BlkDev &b, cudaStream_t s)
-{
-    k_blk_range<<<152 * 8, 256, 0, s>>>(h, b.range);
-}
-
 bool blk_dense_ok(int Mq) { return Mq <= DN_MAX_CHUNKS * DN_QUADS; }
 
 void launch_blk_masks(const NetDev &h, const BlkDev &b, cudaStream_t s)
 {
     cudaMemsetAsync(b.hist, 0, (size_t)h.Np * sizeof(*b.hist), s);
+    if (b.actn) cudaMemsetAsync(b.actn, 0, BLK_ACT_ROWS * sizeof(*b.actn), s);
     k_blk_scatter<<<dim3(std::min((h.N + 255) / 256, 16), BG3_RING), 256, 0, s>>>(h, b);
     k_blk_act<<<(h.Np + 255) / 256, 256, 0, s>>>(h, b);
 }
@@ -1179,26 +1317,38 @@ static void allow_smem(K kern)
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_SMEM);
 }
 
+// The push grid: 128-synapse chunks over eight blocks, so that a neuron of a thousand synapses is
+// one round of them.
+constexpr int PUSH_SPLIT = 8;
+
 void launch_blk_dense(const NetDev &h, const BlkDev &b, const CUtensorMap &tp, const CUtensorMap &tc,
                       int nt, cudaStream_t s)
 {
+    const dim3 pg((h.ntiles + PUSH_WORDS - 1) / PUSH_WORDS, PUSH_SPLIT);
     if (h.syn_kind == 1) {
         allow_smem(k_blk_dense<1>);
+        launch_dep(k_blk_push<1>, pg, PUSH_THREADS, 0, s, h, b, nt);
         launch_dep(k_blk_dense<1>, h.ntiles, DN_THREADS, DN_SMEM, s, h, b, tp, tc, nt);
     } else {
         allow_smem(k_blk_dense<0>);
+        launch_dep(k_blk_push<0>, pg, PUSH_THREADS, 0, s, h, b, nt);
         launch_dep(k_blk_dense<0>, h.ntiles, DN_THREADS, DN_SMEM, s, h, b, tp, tc, nt);
     }
 }
 
+// dense: the indices of the nd networks that run dense blocks, max_tiles their most tiles.
 void launch_blk_dense_batch(int syn_kind, const NetDev *nets, const BlkDev *blks,
-                            const CUtensorMap *maps, const int2 *tiles, int n, int nt, cudaStream_t s)
+                            const CUtensorMap *maps, const int2 *tiles, int n, const int *dense, int nd,
+                            int max_tiles, int nt, cudaStream_t s)
 {
+    const dim3 pg((max_tiles + PUSH_WORDS - 1) / PUSH_WORDS, PUSH_SPLIT, nd);
     if (syn_kind == 1) {
         allow_smem(k_blk_dense_batch<1>);
+        launch_dep(k_blk_push_batch<1>, pg, PUSH_THREADS, 0, s, nets, blks, dense, nt);
         launch_dep(k_blk_dense_batch<1>, n, DN_THREADS, DN_SMEM, s, nets, blks, maps, tiles, nt);
     } else {
         allow_smem(k_blk_dense_batch<0>);
+        launch_dep(k_blk_push_batch<0>, pg, PUSH_THREADS, 0, s, nets, blks, dense, nt);
         launch_dep(k_blk_dense_batch<0>, n, DN_THREADS, DN_SMEM, s, nets, blks, maps, tiles, nt);
     }
 }

@@ -198,9 +198,10 @@ struct BlkDev {
     // [BLK_ACT_ROWS][ntiles] row t & 15: the neurons of a 32-neuron tile with a spike that may
     // arrive in a block starting at step t (any delay class)
     uint32_t *act;
-    // [ntiles][Mq] the bitmap words that the sources of a tile's row quad span (k_blk_range); follows
-    // from the synapses, NULL for networks that never run a dense block
-    uint32_t *range;
+    // dense blocks only (NULL for networks that never run one):
+    uint32_t *actn;   // [BLK_ACT_ROWS] neurons set in each bitmap row
+    uint8_t *msk;     // [Np * Mq * 4] pushed arrivals of the running block: step mask per slot
+    uint32_t *gflag;  // [ntiles][4] the 16-row groups with such a mask; both 0 between blocks
     // bit s & 63 for the steps s whose spikes may arrive in a block starting at step 0
     unsigned long long win;
 };
