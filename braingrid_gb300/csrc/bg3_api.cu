@@ -36,6 +36,8 @@ void launch_rebuild_maps(const NetDev &h, const NetDev *d_net, cudaStream_t s);
 void launch_scale_weights(const NetDev &h, float f, cudaStream_t s);
 void launch_record(const NetDev &h, const NetDev *d_net, cudaStream_t s);
 bool blk_thin_ok(int Mq);
+bool blk_small_ok(const NetDev &h);
+void launch_blk_small(const NetDev &h, const BlkDev &b, int nsteps, int T, cudaStream_t s);
 bool blk_dense_ok(int Mq);
 void launch_blk_dense(const NetDev &h, const BlkDev &b, const CUtensorMap &tp, const CUtensorMap &tc,
                       int nt, cudaStream_t s);
@@ -1113,12 +1115,16 @@ static bool blk_is_thin(const NetDev &h, const LaunchCfg &c)
 {
     return bg3::sweep_is_thin(h, c) && bg3::blk_thin_ok(h.Mq);
 }
-static int blk_steps(const bg3_net *n, const LaunchCfg &c)
+// small: for the many-blocks launch of a small network, whose warps take tiles of any width.
+static int blk_steps(const bg3_net *n, const LaunchCfg &c, bool small = false)
 {
     const NetDev &h = n->h;
     if (c.small_max_slots == 0 || h.noise_mode != BG3_NOISE_DEVICE) return 0;
-    const bool thin = blk_is_thin(h, c);
-    if (!thin && (h.syn_kind >= BG3_SYN_STDP || !bg3::blk_dense_ok(h.Mq))) return 0;
+    if (small) {
+        if (!bg3::blk_small_ok(h)) return 0;
+    } else if (!blk_is_thin(h, c) && (h.syn_kind >= BG3_SYN_STDP || !bg3::blk_dense_ok(h.Mq))) {
+        return 0;
+    }
     if (h.syn_kind >= BG3_SYN_STDP) {
         if (h.stdp_signed) return 0;
         float tau = 0.0f;
@@ -1186,14 +1192,26 @@ static int run_steps(bg3_net *n, int64_t nsteps)
 {
     if (nsteps <= 0) return BG3_OK;
     const NetDev &h = n->h;
-    const int T = bg3::small_eligible(h, n->cfg) ? 0 : blk_steps(n, n->cfg);
+    int rc;
+    const bool small = bg3::small_eligible(h, n->cfg);
+    const int T = blk_steps(n, n->cfg, small);
+    if (T && small) {
+        // a small network: up to SMALL_STEPS whole steps per launch
+        if ((rc = ensure_masks(n))) return rc;
+        n->ring_ok = false;
+        for (int64_t left = nsteps; left > 0; left -= SMALL_STEPS) {
+            bg3::launch_blk_small(h, n->blk, (int)std::min<int64_t>(left, SMALL_STEPS), T, n->stream);
+            n->launches += 1;
+        }
+        CK(cudaGetLastError());
+        return BG3_OK;
+    }
     if (T) return run_blocks(n, nsteps, T);
-    int rc = ensure_ring(n);
-    if (rc) return rc;
+    if ((rc = ensure_ring(n))) return rc;
     n->mask_ok = false;
     if (n->graph && n->graph_steps) drop_graph(n);
-    if (bg3::small_eligible(h, n->cfg)) {
-        // a small network: up to SMALL_STEPS whole steps per launch, one CTA
+    if (small) {
+        // the same in one CTA, step by step: injected noise, and what does not run in blocks
         for (int64_t left = nsteps; left > 0;) {
             const int k = (int)std::min<int64_t>(left, SMALL_STEPS);
             bg3::launch_small(h, k, n->stream);

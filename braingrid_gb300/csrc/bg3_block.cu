@@ -74,26 +74,17 @@ __global__ void __launch_bounds__(256) k_blk_ring(const __grid_constant__ NetDev
     }
 }
 
-// End of a tile's block, one lane per destination: the neuron's state and spikes stored, the
-// bitmap word for the block after this one, and from the network's last tile the step counter.
+// End of a tile's block, one lane per destination: its spikes (fired: bit j, at step t + j) into the
+// masks, the bitmap word for the block after this one, and for the STDP kinds the list of the
+// neurons that fired.  Returns the updated mask.
 template <int SYN>
-__device__ __forceinline__ void blk_finish(const NetDev &n, const BlkDev &b, int tile, int d,
-                                           bool valid, const NeuronIn &x, float sp,
-                                           unsigned long long hist, uint32_t fired, int nt,
-                                           unsigned long long t)
+__device__ __forceinline__ unsigned long long blk_spikes(const NetDev &n, const BlkDev &b, int tile, int d,
+                                                         bool valid, unsigned long long hist,
+                                                         uint32_t fired, int nt, unsigned long long t)
 {
     const int lane = threadIdx.x & 31;
     const unsigned long long t1 = t + (unsigned)nt;
     if (valid) {
-        gst(&n.sp[d], sp);
-        gst(&n.refr[d], x.refr);
-        gst(&n.Vm[d], x.Vm);
-        if (n.neuron_kind == 1) gst(&n.u_izh[d], x.u);
-        if (n.input_kind == 2 && x.pmask) {
-            gst(&n.pois_nisi[d], x.nisi);
-            gst(&n.in_queue[d], x.q);
-            gst(&n.in_psr[d], x.ipsr);
-        }
         hist = (hist & ~rotl64((1ull << nt) - 1ull, (unsigned)t)) | rotl64(fired, (unsigned)t);
         gst(&b.hist[d], hist);
     }
@@ -115,17 +106,53 @@ __device__ __forceinline__ void blk_finish(const NetDev &n, const BlkDev &b, int
     if (lane == 0) {
         b.act[(t1 & (BLK_ACT_ROWS - 1)) * n.ntiles + tile] = w;
         if (b.actn && w) atomicAdd(&b.actn[t1 & (BLK_ACT_ROWS - 1)], (uint32_t)__popc(w));
-        if (atomicAdd(n.sweep_done, 1u) == (unsigned)n.ntiles - 1u) {
-            // the network's last tile: every tile has read the step
-            *n.sweep_done = 0u;
-            *n.step = t1;
-            *n.dstep = t1;
-            n.ring_n[t1 & (BG3_RING - 1)] = 0;
-            if (b.actn)  // the counts of the blocks that may follow the next one
-                for (int j = 1; j <= BLK_MAX_STEPS; j++) b.actn[(t1 + j) & (BLK_ACT_ROWS - 1)] = 0u;
-            if (t1 >= 0xffffff00ull) set_err(n, ERR_STEP_RANGE);
-        }
     }
+    return hist;
+}
+
+// What the block starting at t1 and the ones after it find cleared: the next list of fired neurons,
+// and the counts of the blocks that may follow the next one.
+__device__ __forceinline__ void blk_clear(const NetDev &n, const BlkDev &b, unsigned long long t1)
+{
+    n.ring_n[t1 & (BG3_RING - 1)] = 0;
+    if (b.actn)
+        for (int j = 1; j <= BLK_MAX_STEPS; j++) b.actn[(t1 + j) & (BLK_ACT_ROWS - 1)] = 0u;
+}
+
+__device__ __forceinline__ void neuron_store(const NetDev &n, int d, const NeuronIn &x, float sp)
+{
+    gst(&n.sp[d], sp);
+    gst(&n.refr[d], x.refr);
+    gst(&n.Vm[d], x.Vm);
+    if (n.neuron_kind == 1) gst(&n.u_izh[d], x.u);
+    if (n.input_kind == 2 && x.pmask) {
+        gst(&n.pois_nisi[d], x.nisi);
+        gst(&n.in_queue[d], x.q);
+        gst(&n.in_psr[d], x.ipsr);
+    }
+}
+
+// The last tile of a network to finish a block advances the step counter (every tile has read it).
+__device__ __forceinline__ void blk_step(const NetDev &n, const BlkDev &b, unsigned long long t1)
+{
+    if ((threadIdx.x & 31) == 0 && atomicAdd(n.sweep_done, 1u) == (unsigned)n.ntiles - 1u) {
+        *n.sweep_done = 0u;
+        *n.step = t1;
+        *n.dstep = t1;
+        blk_clear(n, b, t1);
+        if (t1 >= 0xffffff00ull) set_err(n, ERR_STEP_RANGE);
+    }
+}
+
+template <int SYN>
+__device__ __forceinline__ void blk_finish(const NetDev &n, const BlkDev &b, int tile, int d,
+                                           bool valid, const NeuronIn &x, float sp,
+                                           unsigned long long hist, uint32_t fired, int nt,
+                                           unsigned long long t)
+{
+    if (valid) neuron_store(n, d, x, sp);
+    blk_spikes<SYN>(n, b, tile, d, valid, hist, fired, nt, t);
+    blk_step(n, b, t + (unsigned)nt);
 }
 
 // ---- thin networks: one warp per tile ---------------------------------------------------------
@@ -140,25 +167,25 @@ constexpr int BLK_THIN_QUADS = 16;
 constexpr int BLK_THIN_WARPS = 8;
 __host__ __device__ constexpr size_t blk_thin_smem(int Mq)
 {
-    return (size_t)Mq * 32 * (16 + 16 + 4) + BLK_MAX_STEPS * 32 * 4;
+    return (size_t)Mq * 32 * (16 + 16 + 16 + 4 + 4) + BLK_MAX_STEPS * 32 * 4;
 }
 
 struct ThinSmem {
     float4 *psr, *dec;  // [Mq][32]
-    uint32_t *msk;      // [Mq][32], one byte per row
+    float4 *inc;        // [Mq][32] psr increments of the arrivals that are ready
+    uint32_t *msk;      // [Mq][32] their steps, one byte per row
+    uint32_t *late;     // [Mq][32] the steps of the others
     float *noise;       // [BLK_MAX_STEPS][32]
 };
 
-// A lane's arrivals in the block, made ready before the steps run so that their chains of loads
-// (the source's mask, the event slot, the exp tables) overlap across the warp's lanes: two of
-// them as (row, step, psr increment) in registers.  Any more, two spikes at one synapse, and STDP
-// arrivals whose weight the learning walk could change keep a mask in shared memory and run at
-// their step (thin_late).
+// A lane's arrivals in the block are made ready before the steps run, so that their chains of loads
+// (the source's mask, the event slot, the exp tables) overlap, across the warp's lanes and four
+// rows at a time: the steps and the psr increments in shared memory.  Two spikes at one synapse, and
+// STDP arrivals whose weight the learning walk could change, run at their step (thin_late).
 struct ThinEvents {
-    int key0, key1;             // row | step << 8, -1: none
-    float inc0, inc1;
-    unsigned long long late;    // rows with a mask in shared memory
+    unsigned long long rows;    // rows with an arrival (tiles of up to 64 rows)
     uint32_t steps;             // bit j: something arrives at step j
+    bool late;                  // something is left for its step
 };
 
 // Whether an STDP arrival's learning walk may change W: with the host build's arithmetic the walk
@@ -169,148 +196,202 @@ __device__ __forceinline__ bool stdp_clamps(const StdpConst &c, float W)
            (c.Wex < 0.0f && W > 0.0f) || (c.Wex > 0.0f && W < 0.0f) || !(fabsf(c.Apos) < 1e30f);
 }
 
+// The arrivals at the rows set in `rows` (of the 64 from row r0 on).
 template <int SYN>
-__device__ __forceinline__ void thin_event(const NetDev &n, const BlkDev &b, const ThinSmem &s, int r,
-                                           int d, int nt, unsigned long long t, ThinEvents &e)
+__device__ __forceinline__ void thin_events(const NetDev &n, const BlkDev &b, const ThinSmem &s,
+                                            unsigned long long rows, int r0, int d, int nt,
+                                            unsigned long long t, ThinEvents &e)
 {
     const int lane = threadIdx.x & 31;
-    const uint32_t p = (uint32_t)slot_pos(r, d, n.Mq);
-    const int src = n.src[p];
-    const int D = n.ltab[n.lcls[p]];
-    const uint32_t m = (uint32_t)rotr64(b.hist[src], (unsigned)(t - (unsigned long long)D)) &
-                       ((1u << nt) - 1u);
-    if (!m) return;
-    e.steps |= m;
-    bool late = (m & (m - 1u)) != 0u || e.key1 >= 0;
-    const int j = __ffs((int)m) - 1;
-    const unsigned long long tj = t + (unsigned)j;
-    if (!late && SYN >= 2) {
-        // a walk that finds the ring full sets an error bit: at its step where the ring may fill
-        // within the block
+    constexpr bool DS = SYN == 1 || SYN == 3;
+    constexpr int U = 4;
+    // STDP: a walk that finds the ring full sets an error bit; where the ring may fill within the
+    // block, at its step
+    bool ring_late = false;
+    if (SYN >= 2 && rows) {
         const int co = n.spikeCount[d] + n.spikeCountOffset[d];
-        late = stdp_clamps(n.stdp[n.stype[p]], n.ev[p].W);
-        if (hist_at(n, d, co, nt - n.max_spikes) != BG3_ULONG_MAX) {
-            if (hist_at(n, d, co, -n.max_spikes) != BG3_ULONG_MAX) set_err(n, ERR_STDP_RING);
-            else late = true;
+        ring_late = hist_at(n, d, co, nt - n.max_spikes) != BG3_ULONG_MAX;
+    }
+    while (rows) {
+        int r[U], D[U];
+        uint32_t p[U], m[U];
+        unsigned long long h[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            r[u] = rows ? r0 + __ffsll((long long)rows) - 1 : -1;
+            rows &= rows - 1ull;
+            m[u] = 0u;
+            if (r[u] < 0) continue;
+            p[u] = (uint32_t)slot_pos(r[u], d, n.Mq);
+            D[u] = n.lcls[p[u]];
+            m[u] = (uint32_t)n.src[p[u]];
         }
-    }
-    if (late) {
-        uint8_t *mk = reinterpret_cast<uint8_t *>(&s.msk[(r >> 2) * 32 + lane]) + (r & 3);
-        *mk = (uint8_t)m;
-        e.late |= 1ull << r;
-        return;
-    }
-    float inc;
-    if (!arrival<(SYN == 3 ? 1 : SYN == 2 ? 0 : SYN)>(n, p, d, src, (uint32_t)tj - (uint32_t)D, tj, inc))
-        return;
-    const int key = r | (j << 8);
-    if (e.key0 < 0) {
-        e.key0 = key;
-        e.inc0 = inc;
-    } else {
-        e.key1 = key;
-        e.inc1 = inc;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (r[u] < 0) continue;
+            D[u] = n.ltab[D[u]];
+            h[u] = b.hist[m[u]];
+        }
+        float4 ev[U];
+        uint2 ef[U];
+        int ty[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (r[u] < 0) continue;
+            m[u] = (uint32_t)rotr64(h[u], (unsigned)t - (unsigned)D[u]) & ((1u << nt) - 1u);
+            if (!m[u]) continue;
+            e.steps |= m[u];
+            if (r[u] < 64) e.rows |= 1ull << r[u];
+            const char *q = reinterpret_cast<const char *>(n.ev) + (size_t)p[u] * sizeof(EvSlot);
+            ev[u] = *reinterpret_cast<const float4 *>(q);
+            ef[u] = *reinterpret_cast<const uint2 *>(q + 16);
+            if (SYN >= 2) ty[u] = n.stype[p[u]];
+        }
+        float xr[U], xu[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (!m[u]) continue;
+            bool late = (m[u] & (m[u] - 1u)) != 0u;
+            if (SYN >= 2) {
+                late = late || stdp_clamps(n.stdp[ty[u]], ev[u].x);
+                if (ring_late) {
+                    const int co = n.spikeCount[d] + n.spikeCountOffset[d];
+                    if (hist_at(n, d, co, -n.max_spikes) == BG3_ULONG_MAX) late = true;
+                }
+            }
+            if (late) {
+                reinterpret_cast<uint8_t *>(&s.late[(r[u] >> 2) * 32 + lane])[r[u] & 3] = (uint8_t)m[u];
+                e.late = true;
+                m[u] = 0u;
+                continue;
+            }
+            const uint32_t ta = (uint32_t)t + (uint32_t)(31 - __clz((int)m[u])), last = __float_as_uint(ev[u].w);
+            if ((int32_t)(ta - (uint32_t)D[u] - ef[u].x) < 0) {
+                m[u] = 0u;  // the synapse did not exist when the spike left
+            } else if (DS && last != BG3_NO_SPIKE32) {
+                const int pc = (int)((ef[u].y >> 8) & 255u);
+                xr[u] = exp_tab(n, n.p_xD[pc], ta - last, n.p_D[pc]);
+                xu[u] = exp_tab(n, n.p_xF[pc], ta - last, n.p_F[pc]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (!m[u]) continue;
+            if (SYN >= 2 && ring_late) set_err(n, ERR_STDP_RING);
+            const float dec = n.dtab[ef[u].y & 255u];
+            float inc;
+            if (DS) {
+                float uu = ev[u].y, rr = ev[u].z;
+                if (__float_as_uint(ev[u].w) != BG3_NO_SPIKE32) {
+                    const float Uc = n.p_U[(ef[u].y >> 8) & 255u];
+                    rr = 1.0f + (rr * (1.0f - uu) - 1.0f) * xr[u];
+                    uu = Uc + uu * (1.0f - Uc) * xu[u];
+                }
+                inc = (ev[u].x / dec) * uu * rr;
+                gst(reinterpret_cast<float4 *>(n.ev) + 2 * (size_t)p[u],
+                    make_float4(ev[u].x, uu, rr,
+                                __uint_as_float((uint32_t)t + (uint32_t)(31 - __clz((int)m[u])))));
+            } else {
+                inc = ev[u].x / dec;
+            }
+            reinterpret_cast<uint8_t *>(&s.msk[(r[u] >> 2) * 32 + lane])[r[u] & 3] = (uint8_t)m[u];
+            reinterpret_cast<float *>(&s.inc[(r[u] >> 2) * 32 + lane])[r[u] & 3] = inc;
+        }
     }
 }
 
 // The lane's remaining arrivals of step t + j.
 template <int SYN>
-__device__ __noinline__ void thin_late(const NetDev &n, const ThinSmem &s, int d,
-                                       unsigned long long rows, int j, unsigned long long t)
+__device__ __noinline__ void thin_late(const NetDev &n, const ThinSmem &s, int d, int nq, int j,
+                                       unsigned long long t)
 {
     const int lane = threadIdx.x & 31;
-    while (rows) {
-        const int r = __ffsll((long long)rows) - 1;
-        rows &= rows - 1ull;
-        if (!((s.msk[(r >> 2) * 32 + lane] >> ((r & 3) * 8 + j)) & 1u)) continue;
-        const uint32_t p = (uint32_t)slot_pos(r, d, n.Mq);
-        const int D = n.ltab[n.lcls[p]];
-        float inc;
-        if (arrival<SYN>(n, p, d, n.src[p], (uint32_t)(t + (unsigned)j) - (uint32_t)D,
-                         t + (unsigned)j, inc)) {
-            float *ps = reinterpret_cast<float *>(&s.psr[(r >> 2) * 32 + lane]) + (r & 3);
-            *ps = *ps + inc;
+    for (int q = 0; q < nq; q++) {
+        const uint32_t w = s.late[q * 32 + lane] >> j;
+        for (int k = 0; k < 4; k++) {
+            if (!((w >> (8 * k)) & 1u)) continue;
+            const uint32_t p = (uint32_t)slot_pos(4 * q + k, d, n.Mq);
+            const int D = n.ltab[n.lcls[p]];
+            float inc;
+            if (arrival<SYN>(n, p, d, n.src[p], (uint32_t)(t + (unsigned)j) - (uint32_t)D,
+                             t + (unsigned)j, inc)) {
+                float *ps = reinterpret_cast<float *>(&s.psr[q * 32 + lane]) + k;
+                *ps = *ps + inc;
+            }
         }
     }
 }
 
-template <int SYN>
-__device__ __forceinline__ void blk_thin_tile(const NetDev &n, const BlkDev &b, const int tile,
-                                              const int nt, uint8_t *smem)
+// The ready arrivals of the block's step j onto their psr.
+__device__ __forceinline__ void thin_add(const ThinSmem &s, int q, int k, int j)
+{
+    const int at = q * 32 + ((int)threadIdx.x & 31);
+    if (!((s.msk[at] >> (8 * k + j)) & 1u)) return;
+    float *ps = reinterpret_cast<float *>(&s.psr[at]) + k;
+    *ps = *ps + reinterpret_cast<const float *>(&s.inc[at])[k];
+}
+
+// A tile's neurons and synapses in registers and shared memory.
+struct ThinTile {
+    NeuronIn x;
+    float sp;
+    unsigned long long hist;
+    int cnt, nq;
+};
+
+// nt steps from t on: the arrivals made ready, then step by step the neuron update, the arrivals,
+// decay and sum.  The psr is in shared memory.  DEP: the kernel's grid-dependency wait comes before
+// the first access that needs it (see k_blk_thin).  Returns the steps at which the neuron fired.
+template <int SYN, bool DEP>
+__device__ __forceinline__ uint32_t thin_steps(const NetDev &n, const BlkDev &b, const ThinSmem &s,
+                                               ThinTile &y, int tile, int d, bool valid, int nt,
+                                               unsigned long long t)
 {
     const int lane = threadIdx.x & 31;
-    const int d = tile * 32 + lane;
-    const bool valid = d < n.N;
-    ThinSmem s;
-    s.psr = reinterpret_cast<float4 *>(smem);
-    s.dec = s.psr + n.Mq * 32;
-    s.msk = reinterpret_cast<uint32_t *>(s.dec + n.Mq * 32);
-    s.noise = reinterpret_cast<float *>(s.msk + n.Mq * 32);
-    const int cnt = valid ? (int)n.count[d] : 0;
-    const int nq = (__reduce_max_sync(0xffffffffu, cnt) + 3) >> 2;
-    const size_t base = (size_t)tile * n.Mq * 32 + lane;  // the lane's first row quad
-    const uint16_t *C = reinterpret_cast<const uint16_t *>(n.dcls) + base;
-    for (int q = 0; q < nq; q++) {
-        const uint32_t c = C[(size_t)q * 32];
-        s.dec[q * 32 + lane] = make_float4(n.dtab[c & 15u], n.dtab[(c >> 4) & 15u],
-                                           n.dtab[(c >> 8) & 15u], n.dtab[(c >> 12) & 15u]);
-    }
-    // STDP kinds follow a post-spike pass, which is launched once the block before has finished and
-    // writes nothing but weights: everything else is final, and the wait can come later
-    if (SYN < 2) {
-        pdl_wait();
-        pdl_trigger();
-    }
-    const unsigned long long t = *n.step;
-    NeuronIn x;
-    float sp = 0.0f;
-    unsigned long long hist = 0ull;
-    if (valid) {
-        neuron_load(n, d, x);
-        sp = n.sp[d];
-        hist = b.hist[d];
-    }
-    // psr into shared memory; the slots whose source has a spike in this block's window
-    float4 *P = reinterpret_cast<float4 *>(n.psr) + base;
-    const int4 *S = reinterpret_cast<const int4 *>(n.src) + base;
+    const int4 *S = reinterpret_cast<const int4 *>(n.src) + (size_t)tile * n.Mq * 32 + lane;
     const uint32_t *act = b.act + (t & (BLK_ACT_ROWS - 1)) * n.ntiles;
-    unsigned long long rows = 0ull;
-    for (int q0 = 0; q0 < nq; q0 += 4) {
-        float4 v[4];
-        int4 sr[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (q0 + k < nq) {
-                v[k] = P[(size_t)(q0 + k) * 32];
-                sr[k] = S[(size_t)(q0 + k) * 32];
-            }
-        uint32_t hit = 0u;
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (q0 + k < nq) {
-                s.psr[(q0 + k) * 32 + lane] = v[k];
-                const int left = cnt - 4 * (q0 + k);  // in-use rows from this quad on
-                if (left > 0) hit |= ((act[sr[k].x >> 5] >> (sr[k].x & 31)) & 1u) << (4 * k);
-                if (left > 1) hit |= ((act[sr[k].y >> 5] >> (sr[k].y & 31)) & 1u) << (4 * k + 1);
-                if (left > 2) hit |= ((act[sr[k].z >> 5] >> (sr[k].z & 31)) & 1u) << (4 * k + 2);
-                if (left > 3) hit |= ((act[sr[k].w >> 5] >> (sr[k].w & 31)) & 1u) << (4 * k + 3);
-            }
-        rows |= (unsigned long long)hit << (4 * q0);
-    }
+    ThinEvents e = {0ull, 0u, false};
+    bool waited = !DEP || SYN < 2;
     // the steps' noise draws depend on nothing but the step: four at a time, so that one draw's
     // latency hides another's (inside the step loop each would wait alone)
 #pragma unroll 4
     for (int j = 0; j < nt; j++)
         s.noise[j * 32 + lane] = normal_device(n.noise_seed, t + (unsigned)j, d);
-    if (SYN >= 2) {
+    for (int g0 = 0; g0 < y.nq; g0 += 16) {
+        // the slots whose source has a spike in this block's window, 64 rows at a time
+        unsigned long long rows = 0ull;
+        const int g1 = min(y.nq, g0 + 16);
+        for (int q0 = g0; q0 < g1; q0 += 4) {
+            int4 sr[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (q0 + k < g1) {
+                    sr[k] = S[(size_t)(q0 + k) * 32];
+                    s.msk[(q0 + k) * 32 + lane] = 0u;
+                    s.late[(q0 + k) * 32 + lane] = 0u;
+                }
+            uint32_t hit = 0u;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (q0 + k < g1) {
+                    const int left = y.cnt - 4 * (q0 + k);  // in-use rows from this quad on
+                    if (left > 0) hit |= ((act[sr[k].x >> 5] >> (sr[k].x & 31)) & 1u) << (4 * k);
+                    if (left > 1) hit |= ((act[sr[k].y >> 5] >> (sr[k].y & 31)) & 1u) << (4 * k + 1);
+                    if (left > 2) hit |= ((act[sr[k].z >> 5] >> (sr[k].z & 31)) & 1u) << (4 * k + 2);
+                    if (left > 3) hit |= ((act[sr[k].w >> 5] >> (sr[k].w & 31)) & 1u) << (4 * k + 3);
+                }
+            rows |= (unsigned long long)hit << (4 * (q0 - g0));
+        }
+        if (!waited) {
+            pdl_wait();
+            pdl_trigger();
+            waited = true;
+        }
+        thin_events<SYN>(n, b, s, rows, 4 * g0, d, nt, t, e);
+    }
+    if (!waited) {
         pdl_wait();
         pdl_trigger();
-    }
-    ThinEvents e = {-1, -1, 0.0f, 0.0f, 0ull, 0u};
-    while (rows) {
-        const int r = __ffsll((long long)rows) - 1;
-        rows &= rows - 1ull;
-        thin_event<SYN>(n, b, s, r, d, nt, t, e);
     }
     const uint32_t any = __reduce_or_sync(0xffffffffu, e.steps);
     const int mode = izh_mode(n, d);
@@ -319,24 +400,24 @@ __device__ __forceinline__ void blk_thin_tile(const NetDev &n, const BlkDev &b, 
     for (int j = 0; j < nt; j++) {
         const unsigned long long tj = t + (unsigned)j;
         if (valid) {
-            const int br = neuron_branch(x);
-            const float in = input_update(n, d, x, tj, sp);
-            if (neuron_update(n, d, x, br, in, s.noise[j * 32 + lane], tj, mode)) fired |= 1u << j;
+            const int br = neuron_branch(y.x);
+            const float in = input_update(n, d, y.x, tj, y.sp);
+            if (neuron_update(n, d, y.x, br, in, s.noise[j * 32 + lane], tj, mode)) fired |= 1u << j;
         }
         if ((any >> j) & 1u) {
-            if (e.key0 >> 8 == j) {
-                float *ps = reinterpret_cast<float *>(&s.psr[((e.key0 >> 2) & 63) * 32 + lane]) + (e.key0 & 3);
-                *ps = *ps + e.inc0;
+            if ((e.steps >> j) & 1u) {
+                for (unsigned long long r = e.rows; r; r &= r - 1ull) {
+                    const int k = __ffsll((long long)r) - 1;
+                    thin_add(s, k >> 2, k & 3, j);
+                }
+                for (int q = 16; q < y.nq; q++)  // a small network's wider tile
+                    for (int k = 0; k < 4; k++) thin_add(s, q, k, j);
+                if (e.late) thin_late<SYN>(n, s, d, y.nq, j, t);
             }
-            if (e.key1 >> 8 == j) {
-                float *ps = reinterpret_cast<float *>(&s.psr[((e.key1 >> 2) & 63) * 32 + lane]) + (e.key1 & 3);
-                *ps = *ps + e.inc1;
-            }
-            if (e.late && ((e.steps >> j) & 1u)) thin_late<SYN>(n, s, d, e.late, j, t);
             __syncwarp();
         }
         float acc = 0.0f;
-        for (int q = 0; q < nq; q++) {
+        for (int q = 0; q < y.nq; q++) {
             float4 v = s.psr[q * 32 + lane];
             const float4 c = s.dec[q * 32 + lane];
             v.x = v.x * c.x;
@@ -349,10 +430,89 @@ __device__ __forceinline__ void blk_thin_tile(const NetDev &n, const BlkDev &b, 
             acc = acc + v.z;
             acc = acc + v.w;
         }
-        sp = acc;
+        y.sp = acc;
     }
-    for (int q = 0; q < nq; q++) gst(&P[(size_t)q * 32], s.psr[q * 32 + lane]);
-    blk_finish<SYN>(n, b, tile, d, valid, x, sp, hist, fired, nt, t);
+    return fired;
+}
+
+__device__ __forceinline__ ThinSmem thin_smem(uint8_t *smem, int Mq)
+{
+    ThinSmem s;
+    s.psr = reinterpret_cast<float4 *>(smem);
+    s.dec = s.psr + Mq * 32;
+    s.inc = s.dec + Mq * 32;
+    s.msk = reinterpret_cast<uint32_t *>(s.inc + Mq * 32);
+    s.late = s.msk + Mq * 32;
+    s.noise = reinterpret_cast<float *>(s.late + Mq * 32);
+    return s;
+}
+
+// What the steps do not change: the row counts, and the decay factors into shared memory.
+__device__ __forceinline__ void thin_static(const NetDev &n, const ThinSmem &s, ThinTile &y, int tile)
+{
+    const int lane = threadIdx.x & 31, d = tile * 32 + lane;
+    y.cnt = d < n.N ? (int)n.count[d] : 0;
+    y.nq = (__reduce_max_sync(0xffffffffu, y.cnt) + 3) >> 2;
+    const uint16_t *C = reinterpret_cast<const uint16_t *>(n.dcls) + (size_t)tile * n.Mq * 32 + lane;
+    for (int q = 0; q < y.nq; q++) {
+        const uint32_t c = C[(size_t)q * 32];
+        s.dec[q * 32 + lane] = make_float4(n.dtab[c & 15u], n.dtab[(c >> 4) & 15u],
+                                           n.dtab[(c >> 8) & 15u], n.dtab[(c >> 12) & 15u]);
+    }
+}
+
+// The tile's neurons into registers, its psr into shared memory.
+__device__ __forceinline__ void thin_load(const NetDev &n, const BlkDev &b, const ThinSmem &s, ThinTile &y,
+                                          int tile)
+{
+    const int lane = threadIdx.x & 31, d = tile * 32 + lane;
+    y.sp = 0.0f;
+    y.hist = 0ull;
+    if (d < n.N) {
+        neuron_load(n, d, y.x);
+        y.sp = n.sp[d];
+        y.hist = b.hist[d];
+    }
+    const float4 *P = reinterpret_cast<const float4 *>(n.psr) + (size_t)tile * n.Mq * 32 + lane;
+    for (int q0 = 0; q0 < y.nq; q0 += 4) {
+        float4 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (q0 + k < y.nq) v[k] = P[(size_t)(q0 + k) * 32];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (q0 + k < y.nq) s.psr[(q0 + k) * 32 + lane] = v[k];
+    }
+}
+
+__device__ __forceinline__ void thin_store(const NetDev &n, const ThinSmem &s, const ThinTile &y, int tile)
+{
+    const int lane = threadIdx.x & 31;
+    float4 *P = reinterpret_cast<float4 *>(n.psr) + (size_t)tile * n.Mq * 32 + lane;
+    for (int q = 0; q < y.nq; q++) gst(&P[(size_t)q * 32], s.psr[q * 32 + lane]);
+}
+
+// STDP kinds follow a post-spike pass, which is launched once the block before has finished and
+// writes nothing but weights: everything else is final, and the wait can come as late as the first
+// arrival.
+template <int SYN>
+__device__ __forceinline__ void blk_thin_tile(const NetDev &n, const BlkDev &b, const int tile,
+                                              const int nt, uint8_t *smem)
+{
+    const int d = tile * 32 + ((int)threadIdx.x & 31);
+    const bool valid = d < n.N;
+    const ThinSmem s = thin_smem(smem, n.Mq);
+    ThinTile y;
+    thin_static(n, s, y, tile);
+    if (SYN < 2) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    const unsigned long long t = *n.step;
+    thin_load(n, b, s, y, tile);
+    const uint32_t fired = thin_steps<SYN, true>(n, b, s, y, tile, d, valid, nt, t);
+    thin_store(n, s, y, tile);
+    blk_finish<SYN>(n, b, tile, d, valid, y.x, y.sp, y.hist, fired, nt, t);
 }
 
 template <int SYN>
@@ -409,10 +569,10 @@ __device__ __forceinline__ int count_at(const NetDev &n, int i, unsigned long lo
 }
 
 // One warp per neuron that fired, one lane per synapse.
-__device__ __forceinline__ void blk_post(const NetDev &n, const BlkDev &b, int gw, int nw, int nt)
+__device__ __forceinline__ void blk_post(const NetDev &n, const BlkDev &b, int gw, int nw, int nt,
+                                         unsigned long long t)
 {
     const int lane = threadIdx.x & 31;
-    const unsigned long long t = *n.step - (unsigned)nt;  // the block's first step
     const int slot = (int)(t & (BG3_RING - 1));
     const int m = min(n.ring_n[slot], n.N);
     const int32_t *ids = n.ring + (size_t)slot * n.N;
@@ -442,7 +602,8 @@ __global__ void __launch_bounds__(256) k_blk_post(const __grid_constant__ NetDev
 {
     pdl_wait();
     pdl_trigger();
-    blk_post(n, b, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5, nt);
+    blk_post(n, b, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5, nt,
+             *n.step - (unsigned)nt);
 }
 
 __global__ void __launch_bounds__(256) k_blk_post_batch(const NetDev *nets, const BlkDev *blks,
@@ -456,7 +617,66 @@ __global__ void __launch_bounds__(256) k_blk_post_batch(const NetDev *nets, cons
     pdl_wait();
     pdl_trigger();
     blk_post(s_net, blks[blockIdx.y], (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-             (gridDim.x * blockDim.x) >> 5, nt);
+             (gridDim.x * blockDim.x) >> 5, nt, *s_net.step - (unsigned)nt);
+}
+
+// ---- small networks: many blocks per launch ----------------------------------------------------
+// A network of few tiles is a launch's latency per block of steps and little else, so one launch runs
+// thousands of steps: one warp per tile, which keeps the tile's psr, neurons and masks for the whole
+// launch, in up to eight blocks of one cluster, with a cluster barrier (a block barrier when there is
+// one block) after each block of steps and, for the STDP kinds, another after the post-spike pass.
+// The barriers order the masks, bitmaps and histories that the tiles read of each other.  Four warps
+// a block, one per quarter of its SM, up to 32 tiles: a warp issues alone, and that is its pace.
+__device__ __forceinline__ void small_sync()
+{
+    if (gridDim.x == 1) {
+        __syncthreads();
+    } else {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+}
+
+template <int SYN>
+__global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 1) k_blk_small(const __grid_constant__ NetDev n,
+                                                                      const __grid_constant__ BlkDev b,
+                                                                      int nsteps, int T)
+{
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    const int warp = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
+    const int tile = (int)blockIdx.x * nw + warp, d = tile * 32 + ((int)threadIdx.x & 31);
+    const bool active = tile < n.ntiles, valid = d < n.N, first = blockIdx.x == 0 && threadIdx.x == 0;
+    const ThinSmem s = thin_smem(smem_raw + warp * blk_thin_smem(n.Mq), n.Mq);
+    ThinTile y;
+    unsigned long long t = *n.step;
+    if (active) {
+        thin_static(n, s, y, tile);
+        thin_load(n, b, s, y, tile);
+    }
+    for (int left = nsteps; left > 0;) {
+        const int nt = min(left, T);
+        if (first) blk_clear(n, b, t + (unsigned)nt);
+        if (active) {
+            const uint32_t fired = thin_steps<SYN, false>(n, b, s, y, tile, d, valid, nt, t);
+            y.hist = blk_spikes<SYN>(n, b, tile, d, valid, y.hist, fired, nt, t);
+        }
+        small_sync();
+        if (SYN >= 2) {
+            blk_post(n, b, tile, (int)gridDim.x * nw, nt, t);
+            small_sync();
+        }
+        t += (unsigned)nt;
+        left -= nt;
+    }
+    if (active) {
+        if (valid) neuron_store(n, d, y.x, y.sp);
+        thin_store(n, s, y, tile);
+    }
+    if (first) {
+        *n.step = t;
+        *n.dstep = t;
+        if (t >= 0xffffff00ull) set_err(n, ERR_STEP_RANGE);
+    }
 }
 
 // ---- dense networks: one CTA per tile ----------------------------------------------------------
@@ -1268,6 +1488,55 @@ void launch_blk_ring(const NetDev &h, const BlkDev &b, cudaStream_t s)
 {
     cudaMemsetAsync(h.ring_n, 0, BG3_RING * sizeof(*h.ring_n), s);
     k_blk_ring<<<(h.N + 255) / 256, 256, 0, s>>>(h, b);
+}
+
+// Blocks and warps per block of a small network's launch; 0 blocks when it does not fit a cluster of
+// eight (200 KB of shared memory per block).
+static int small_shape(const NetDev &h, int &warps)
+{
+    const size_t per = blk_thin_smem(h.Mq);
+    const int most = (int)std::min<size_t>(BLK_THIN_WARPS, 200 * 1024 / per);
+    if (most < 1) return 0;
+    warps = std::min(most, h.ntiles <= 32 ? std::min(4, h.ntiles) : BLK_THIN_WARPS);
+    const int blocks = (h.ntiles + warps - 1) / warps;
+    return blocks <= 8 ? blocks : 0;
+}
+bool blk_small_ok(const NetDev &h)
+{
+    int w;
+    return small_shape(h, w) > 0;
+}
+
+template <int SYN>
+static void launch_small_t(const NetDev &h, const BlkDev &b, int nsteps, int T, cudaStream_t s)
+{
+    int w = 1;
+    const int blocks = small_shape(h, w);
+    const size_t sm = (size_t)w * blk_thin_smem(h.Mq);
+    cudaFuncSetAttribute(k_blk_small<SYN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(32 * w);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_blk_small<SYN>, h, b, nsteps, T);
+}
+
+// nsteps steps of a small network, T at a time, in one launch.
+void launch_blk_small(const NetDev &h, const BlkDev &b, int nsteps, int T, cudaStream_t s)
+{
+    switch (h.syn_kind) {
+    case 1: launch_small_t<1>(h, b, nsteps, T, s); break;
+    case 2: launch_small_t<2>(h, b, nsteps, T, s); break;
+    case 3: launch_small_t<3>(h, b, nsteps, T, s); break;
+    default: launch_small_t<0>(h, b, nsteps, T, s); break;
+    }
 }
 
 // At most 44 KB of shared memory per block beside a batch's descriptor (48 KB is what a launch may

@@ -1,6 +1,6 @@
 """Blocks of steps (bg3_block.cu) against the per-step kernels, bit for bit: the same network
 advanced by both (small_max_slots 0 keeps a network on the per-step kernels, 1 keeps it off the
-one-launch path of small networks), at sizes around the 32-neuron tiles, the row quads and the
+one-launch path of small networks, 65,536 takes that path where it is small enough), at sizes around the 32-neuron tiles, the row quads and the
 eight steps of a block, with downloads, epoch ends and single steps in between."""
 import numpy as np
 import pytest
@@ -58,9 +58,9 @@ def same(a, b, what):
         assert np.array_equal(u, v), "%s: %s differs at %s" % (what, k, np.nonzero(u != v)[0][:5])
 
 
-def advance(make, end="record"):
+def advance(make, end="record", small=1):
     blocks, plain = make(), make()
-    blocks.set_launch(small_max_slots=1)
+    blocks.set_launch(small_max_slots=small)
     plain.set_launch(small_max_slots=0)
     spikes = 0
     for i, n in enumerate(STEPS):
@@ -81,7 +81,7 @@ def advance(make, end="record"):
     blocks.set_launch(small_max_slots=0)
     blocks.step(5)
     plain.step(5)
-    blocks.set_launch(small_max_slots=1)
+    blocks.set_launch(small_max_slots=small)
     blocks.step(40)
     plain.step(40)
     same(blocks, plain, "after the epoch end")
@@ -91,6 +91,7 @@ def advance(make, end="record"):
         net.close()
 
 
+@pytest.mark.parametrize("small", [1, 65536])
 @pytest.mark.parametrize("syn", [bg.BG3_SYN_SPIKING, bg.BG3_SYN_DS, bg.BG3_SYN_STDP, bg.BG3_SYN_DYNSTDP])
 @pytest.mark.parametrize("w,h,radius,drive,max_syn", [
     (9, 7, 1.2, "none", 30),        # 63 neurons, a partial last quad
@@ -98,8 +99,8 @@ def advance(make, end="record"):
     (8, 4, 0.0, "regular", 4),      # one tile, no synapse
     (40, 33, 1.9, "poisson", 64),   # the widest rows of a thin tile
 ])
-def test_thin_blocks_equal_steps(syn, w, h, radius, drive, max_syn):
-    advance(lambda: lif(w, h, syn, radius, drive, max_syn), end="growth")
+def test_thin_blocks_equal_steps(small, syn, w, h, radius, drive, max_syn):
+    advance(lambda: lif(w, h, syn, radius, drive, max_syn), end="growth", small=small)
 
 
 @pytest.mark.parametrize("syn", [bg.BG3_SYN_SPIKING, bg.BG3_SYN_DS])
@@ -114,9 +115,16 @@ def test_dense_blocks_equal_steps(syn, w, h, radius, drive, max_syn):
     advance(lambda: lif(w, h, syn, radius, drive, max_syn), end="growth")
 
 
-@pytest.mark.parametrize("w,h", [(9, 7), (13, 5), (60, 41)])
-def test_izhikevich_stdp_blocks_equal_steps(w, h):
-    advance(lambda: izh(w, h))
+@pytest.mark.parametrize("w,h,small", [(9, 7, 1), (13, 5, 65536), (33, 32, 65536), (60, 41, 1)])
+def test_izhikevich_stdp_blocks_equal_steps(w, h, small):
+    advance(lambda: izh(w, h), small=small)
+
+
+@pytest.mark.parametrize("syn", [bg.BG3_SYN_DS, bg.BG3_SYN_DYNSTDP])
+@pytest.mark.parametrize("w,h,radius,max_syn", [(9, 7, 6.0, 65), (13, 5, 4.0, 301), (5, 4, 3.0, 19), (40, 40, 1.2, 37)])
+def test_small_network_blocks_equal_steps(syn, w, h, radius, max_syn):
+    """Rows beyond a thin tile's, one block and eight."""
+    advance(lambda: lif(w, h, syn, radius, "poisson", max_syn), small=65536)
 
 
 def test_batched_blocks_equal_steps():
@@ -161,7 +169,7 @@ def test_two_spikes_at_one_synapse_in_a_block():
     step, so that each synapse receives several spikes within a block."""
     for radius, max_syn in ((1.5, 33), (4.0, 130)):
         nets = []
-        for small in (1, 0):
+        for small in (1, 65536, 0):
             net = lif(13, 5, bg.BG3_SYN_DS, radius, "none", max_syn)
             v = net.download_lif(fields=("Vthresh", "Vreset", "Trefract"))
             v["Trefract"][::3] = 0.0
@@ -173,5 +181,6 @@ def test_two_spikes_at_one_synapse_in_a_block():
         for n in (8, 8, 3, 40):
             for net in nets:
                 net.step(n)
-            same(nets[0], nets[1], "radius %g after %d steps" % (radius, n))
+            same(nets[0], nets[2], "radius %g after %d steps" % (radius, n))
+            same(nets[1], nets[2], "small, radius %g after %d steps" % (radius, n))
         assert int(nets[0].download_lif(fields=("spikeCount",))["spikeCount"].max()) > 8
