@@ -153,6 +153,100 @@ static int d2h(bg3_net *n, T *dst, const T *src, size_t count)
     return BG3_OK;
 }
 
+// ---- downloads through pinned memory -----------------------------------------------------------
+// A copy to pageable memory waits for itself, about 10 us each; a download of several small arrays
+// queues its copies into one pinned buffer instead, waits once and hands them out.  The buffers are
+// shared by all networks of the process (a download holds one for its duration, under no lock):
+// at most STAGE_KEEP of STAGE_BYTES each stay allocated between downloads, and they are freed
+// with the last network.
+static const size_t STAGE_BYTES = 1 << 20;
+static const size_t STAGE_KEEP = 8;
+static std::mutex g_stage_mu;
+static void *g_stage[STAGE_KEEP];     // idle buffers
+static size_t g_stage_n = 0;
+static long long g_stage_nets = 0;    // live networks
+
+static void stage_enter()
+{
+    std::lock_guard<std::mutex> lock(g_stage_mu);
+    g_stage_nets++;
+}
+static void stage_leave()
+{
+    std::lock_guard<std::mutex> lock(g_stage_mu);
+    if (--g_stage_nets > 0) return;
+    while (g_stage_n > 0) cudaFreeHost(g_stage[--g_stage_n]);
+}
+static void *stage_get()
+{
+    {
+        std::lock_guard<std::mutex> lock(g_stage_mu);
+        if (g_stage_n > 0) return g_stage[--g_stage_n];
+    }
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, STAGE_BYTES, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+static void stage_put(void *p)
+{
+    {
+        std::lock_guard<std::mutex> lock(g_stage_mu);
+        if (g_stage_nets > 0 && g_stage_n < STAGE_KEEP) {
+            g_stage[g_stage_n++] = p;
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
+// One download: add() queues arrays, finish() waits for the stream and fills the destinations.  What
+// does not fit the buffer is copied straight to its destination.
+class Fetch {
+  public:
+    explicit Fetch(bg3_net *net) : n(net) {}
+    ~Fetch()
+    {
+        if (!buf) return;
+        if (used) cudaStreamSynchronize(n->stream);  // left early: copies may be in flight
+        stage_put(buf);
+    }
+    template <typename T>
+    int add(T *dst, const T *src, size_t count)
+    {
+        if (!dst || !count) return BG3_OK;
+        const size_t bytes = count * sizeof(T), room = (bytes + 15) & ~(size_t)15;
+        if (room <= STAGE_BYTES - used && !buf) buf = stage_get();
+        if (!buf || room > STAGE_BYTES - used || np == MAX_PARTS) return d2h(n, dst, src, count);
+        CK(cudaMemcpyAsync((char *)buf + used, src, bytes, cudaMemcpyDeviceToHost, n->stream));
+        parts[np++] = Part{(void *)dst, used, bytes};
+        used += room;
+        return BG3_OK;
+    }
+    int finish()
+    {
+        CK(cudaStreamSynchronize(n->stream));
+        for (int i = 0; i < np; i++) memcpy(parts[i].dst, (const char *)buf + parts[i].at, parts[i].bytes);
+        np = 0;
+        used = 0;
+        return BG3_OK;
+    }
+
+  private:
+    struct Part {
+        void *dst;
+        size_t at, bytes;
+    };
+    static constexpr int MAX_PARTS = 16;  // the neuron arrays are 13
+    bg3_net *n;
+    void *buf = nullptr;
+    size_t used = 0;
+    int np = 0;
+    Part parts[MAX_PARTS];
+};
+
 static void drop_graph(bg3_net *n)
 {
     if (n->graph) cudaGraphExecDestroy(n->graph);
@@ -403,6 +497,7 @@ int bg3_create(const bg3_net_desc *desc, bg3_net **out)
         delete n;
         return BG3_ECUDA;
     }
+    stage_enter();
     NetDev &h = n->h;
     memset(&h, 0, sizeof(h));
     const size_t N = (size_t)D.n_neurons;
@@ -577,6 +672,7 @@ int bg3_destroy(bg3_net *n)
         if (n->ev[i]) cudaEventDestroy(n->ev[i]);
     if (n->stream) cudaStreamDestroy(n->stream);
     delete n;
+    stage_leave();
     return BG3_OK;
 }
 
@@ -1336,17 +1432,17 @@ int bg3_download_lif(bg3_net *n, bg3_lif_arrays *a)
     size_t N = n->h.N;
     NetDev &h = n->h;
     int rc;
-    if ((rc = d2h(n, a->Vm, h.Vm, N)) || (rc = d2h(n, a->Vthresh, h.Vthresh, N)) ||
-        (rc = d2h(n, a->Vreset, h.Vreset, N)) || (rc = d2h(n, a->I0, h.I0, N)) ||
-        (rc = d2h(n, a->Inoise, h.Inoise, N)) || (rc = d2h(n, a->C1, h.C1, N)) ||
-        (rc = d2h(n, a->C2, h.C2, N)) || (rc = d2h(n, a->Trefract, h.Trefract, N)) ||
-        (rc = d2h(n, a->summation, h.sp, N)) || (rc = d2h(n, a->nStepsInRefr, h.refr, N)) ||
-        (rc = d2h(n, a->spikeCount, h.spikeCount, N)) ||
-        (rc = d2h(n, a->spikeCountOffset, h.spikeCountOffset, N)) ||
-        (rc = d2h(n, a->history, (const uint64_t *)h.history, N * (size_t)h.max_spikes)))
+    Fetch f(n);
+    if ((rc = f.add(a->Vm, h.Vm, N)) || (rc = f.add(a->Vthresh, h.Vthresh, N)) ||
+        (rc = f.add(a->Vreset, h.Vreset, N)) || (rc = f.add(a->I0, h.I0, N)) ||
+        (rc = f.add(a->Inoise, h.Inoise, N)) || (rc = f.add(a->C1, h.C1, N)) ||
+        (rc = f.add(a->C2, h.C2, N)) || (rc = f.add(a->Trefract, h.Trefract, N)) ||
+        (rc = f.add(a->summation, h.sp, N)) || (rc = f.add(a->nStepsInRefr, h.refr, N)) ||
+        (rc = f.add(a->spikeCount, h.spikeCount, N)) ||
+        (rc = f.add(a->spikeCountOffset, h.spikeCountOffset, N)) ||
+        (rc = f.add(a->history, (const uint64_t *)h.history, N * (size_t)h.max_spikes)))
         return rc;
-    CK(cudaStreamSynchronize(n->stream));
-    return BG3_OK;
+    return f.finish();
 }
 
 int bg3_download_izh(bg3_net *n, bg3_izh_arrays *a)
@@ -1356,12 +1452,12 @@ int bg3_download_izh(bg3_net *n, bg3_izh_arrays *a)
     size_t N = n->h.N;
     NetDev &h = n->h;
     int rc;
-    if ((rc = d2h(n, a->Aconst, h.Aconst, N)) || (rc = d2h(n, a->Bconst, h.Bconst, N)) ||
-        (rc = d2h(n, a->Cconst, h.Cconst, N)) || (rc = d2h(n, a->Dconst, h.Dconst, N)) ||
-        (rc = d2h(n, a->u, h.u_izh, N)) || (rc = d2h(n, a->C3, h.C3, N)))
+    Fetch f(n);
+    if ((rc = f.add(a->Aconst, h.Aconst, N)) || (rc = f.add(a->Bconst, h.Bconst, N)) ||
+        (rc = f.add(a->Cconst, h.Cconst, N)) || (rc = f.add(a->Dconst, h.Dconst, N)) ||
+        (rc = f.add(a->u, h.u_izh, N)) || (rc = f.add(a->C3, h.C3, N)))
         return rc;
-    CK(cudaStreamSynchronize(n->stream));
-    return BG3_OK;
+    return f.finish();
 }
 
 // Rebuilds the reference's delayQueue / delayIdx from the spike ring and birth steps: a spike
@@ -1618,9 +1714,9 @@ int bg3_download_growth(bg3_net *n, float *radii, float *rates)
 {
     if (!n) return BG3_EINVAL;
     int rc;
-    if ((rc = d2h(n, radii, n->h.radii, n->h.N)) || (rc = d2h(n, rates, n->h.rates, n->h.N))) return rc;
-    CK(cudaStreamSynchronize(n->stream));
-    return BG3_OK;
+    Fetch f(n);
+    if ((rc = f.add(radii, n->h.radii, n->h.N)) || (rc = f.add(rates, n->h.rates, n->h.N))) return rc;
+    return f.finish();
 }
 
 int bg3_download_state(bg3_net *n, const bg3_state_view *v)
