@@ -9,6 +9,7 @@
 //                      the row's in-use prefix            (O(N^2) pairs, no N^2 storage)
 //   k_out_count/scan/fill  outgoing CSR rebuild per delay class (createSynapseImap)
 //   k_record_epoch     recorder histograms, rates/radii history, radius clamp, spike-count roll
+#include "bg3_area.cuh"
 #include "bg3_internal.cuh"
 
 namespace bg3 {
@@ -29,32 +30,6 @@ __global__ void k_growth_radii(const NetDev *nets)
     float og = 1.0f - 2.0f / (e + 1.0f);
     float trho = T * n.g_rho;
     n.radii[i] = n.radii[i] + trho * og;
-}
-
-// Frontier distance and overlap area of the pair (i = source, j = dest)
-// (Connections/ConnGrowth.cpp:319-376; dist from Layouts/Layout.cpp:54-69).  Returns 0 for pairs
-// that do not overlap.  Double where the reference promotes (2.0 * r * len, 2.0 * angle, 0.5 *).
-__device__ __forceinline__ float pair_area(float xi, float yi, float ri, float xj, float yj,
-                                           float rj)
-{
-    float dx = xi - xj, dy = yi - yj;
-    float len2 = dx * dx + dy * dy;
-    float len = sqrtf(len2);
-    float delta = len - (ri + rj);
-    if (!(delta < 0.0f)) return 0.0f;
-    float rmin = fminf(ri, rj), rmax = fmaxf(ri, rj);
-    if (len + rmin <= rmax) {
-        const float pi = 3.1415926536f;  // Utils/Global.cpp:90
-        return pi * rmin * rmin;
-    }
-    float r12 = ri * ri, r22 = rj * rj;
-    float cosCBA = (float)((double)(r22 + len2 - r12) / (2.0 * (double)rj * (double)len));
-    float angCBA = acos_cr(cosCBA);
-    float angCBD = (float)(2.0 * (double)angCBA);
-    float cosCAB = (float)((double)(r12 + len2 - r22) / (2.0 * (double)ri * (double)len));
-    float angCAB = acos_cr(cosCAB);
-    float angCAD = (float)(2.0 * (double)angCAB);
-    return (float)(0.5 * (double)(r22 * (angCBD - sin_cr(angCBD)) + r12 * (angCAD - sin_cr(angCAD))));
 }
 
 // Layout::synType (Layouts/Layout.cpp:129-140): II 0, IE 1, EI 2, EE 3.

@@ -2,12 +2,17 @@
 // bg3_internal.cuh) against the hardware on random operands (random signs, mantissas, exponents
 // in [-300, 300]) and operand pairs that nearly cancel, for add, multiply and the conversion to
 // float.  bg3_selftest_izhikevich: the Izhikevich update's double expression evaluated on the
-// integer pipe and in float-float arithmetic, against the FP64 pipe.  bg3_selftest_timeout: the bounded mbarrier wait of the step kernels, run out on purpose.
+// integer pipe and in float-float arithmetic, against the FP64 pipe.  bg3_selftest_overlap: the
+// growth rule's overlap area in float-float arithmetic against the FP64 pipe.  bg3_selftest_timeout: the bounded mbarrier wait of the step kernels, run out on purpose.
 #include "../../include/bg3.h"
+#include "bg3_area.cuh"
 #include "bg3_internal.cuh"
 #include "bg3_ptx.cuh"
 
 namespace {
+
+using bg3::pair_area_ff;
+using bg3::pair_area_fp64;
 
 __device__ __forceinline__ uint64_t mix64(uint64_t x)
 {
@@ -114,6 +119,45 @@ __global__ void k_izh_test(uint64_t n, uint64_t seed, unsigned long long *bad)
         if (local[k]) atomicAdd(&bad[k], local[k]);
 }
 
+// The overlap area of a pair (pair_area_ff) against pair_area_fp64: whole-number distances up to 27
+// on each axis as on the grid, or any up to 2^+-20; radii equal, within a part in 2^4 to 2^20 of
+// each other or of touching (the angles' ends), or independent.
+__global__ void k_area_test(uint64_t n, uint64_t seed, unsigned long long *bad)
+{
+    unsigned long long local[3] = {0, 0, 0};
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t r1 = mix64(seed ^ (2 * i)), r2 = mix64(seed ^ (2 * i + 1));
+        const float f1 = (float)(r1 >> 40) * 0x1p-24f, f2 = (float)((r1 >> 16) & 0xffffffull) * 0x1p-24f;
+        const float f3 = (float)(r2 >> 40) * 0x1p-24f, f4 = (float)((r2 >> 16) & 0xffffffull) * 0x1p-24f;
+        float dx = (float)(r1 & 31ull) - 4.0f, dy = (float)((r1 >> 5) & 31ull) - 4.0f;
+        if ((r2 & 3ull) == 0) {
+            dx = exp2f(40.0f * f3 - 20.0f);
+            dy = dx * f4;
+        }
+        const float len2 = dx * dx + dy * dy, len = sqrtf(len2);
+        const float near = exp2f(-4.0f - 16.0f * f1);
+        float ri = len * (0.3f + 2.0f * f2), rj;
+        switch ((r2 >> 2) & 3ull) {
+        case 0: rj = ri; break;
+        case 1: rj = ri * (1.0f + near); break;
+        case 2: rj = (r2 & 16ull) ? len - ri + near * len : ri + len - near * len; break;
+        default: rj = len * (0.1f + 2.5f * f1);
+        }
+        if (!(len - (ri + rj) < 0.0f) || len + fminf(ri, rj) <= fmaxf(ri, rj)) {
+            local[2]++;
+            continue;
+        }
+        bool ok = false;
+        const float a = pair_area_ff(len, len2, ri, rj, ok);
+        const float hw = pair_area_fp64(len, len2, ri, rj);
+        if (!ok) local[1]++;
+        else if (__float_as_uint(a) != __float_as_uint(hw)) local[0]++;
+    }
+    for (int k = 0; k < 3; k++)
+        if (local[k]) atomicAdd(&bad[k], local[k]);
+}
+
 // A wait that nothing ends: an mbarrier expecting one arrival that never comes, waited on by a
 // warp with the step kernels' bounded wait at limit_ns.  No copy targets the barrier, so the
 // block may leave it pending; the kernel records whether the wait gave up and how long it took,
@@ -188,5 +232,24 @@ extern "C" int bg3_selftest_izhikevich(uint64_t samples, uint64_t seed, uint64_t
     cudaFree(d);
     if (e1 != cudaSuccess || e2 != cudaSuccess) return BG3_ECUDA;
     for (int k = 0; k < 4; k++) counts[k] = h[k];
+    return BG3_OK;
+}
+
+extern "C" int bg3_selftest_overlap(uint64_t samples, uint64_t seed, uint64_t *counts)
+{
+    if (!counts) return BG3_EINVAL;
+    unsigned long long *d = nullptr;
+    if (cudaMalloc(&d, 4 * sizeof(unsigned long long)) != cudaSuccess) return BG3_ENOMEM;
+    if (cudaMemset(d, 0, 4 * sizeof(unsigned long long)) != cudaSuccess) {
+        cudaFree(d);
+        return BG3_ECUDA;
+    }
+    k_area_test<<<152 * 8, 256>>>(samples, seed, d);
+    unsigned long long h[4];
+    const cudaError_t e1 = cudaDeviceSynchronize();
+    const cudaError_t e2 = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e1 != cudaSuccess || e2 != cudaSuccess) return BG3_ECUDA;
+    for (int k = 0; k < 3; k++) counts[k] = h[k];
     return BG3_OK;
 }

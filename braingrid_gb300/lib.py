@@ -163,6 +163,8 @@ def load(build_if_missing=True):
         "bg3_epoch_record": ([vp], ctypes.c_int),
         "bg3_selftest_izhikevich": ([ctypes.c_uint64, ctypes.c_uint64,
                                      ctypes.POINTER(ctypes.c_uint64)], ctypes.c_int),
+        "bg3_selftest_overlap": ([ctypes.c_uint64, ctypes.c_uint64, ctypes.POINTER(ctypes.c_uint64)],
+                                 ctypes.c_int),
         "bg3_selftest_binary64": ([ctypes.c_uint64, ctypes.c_uint64, ctypes.POINTER(ctypes.c_uint64)],
                                   ctypes.c_int),
         "bg3_get_launch": ([vp, ctypes.POINTER(LaunchCfg)], ctypes.c_int),
@@ -786,6 +788,14 @@ def selftest_binary64(samples=1 << 26, seed=1):
     c = (ctypes.c_uint64 * 4)()
     check(load().bg3_selftest_binary64(int(samples), int(seed), c), "bg3_selftest_binary64")
     return tuple(int(x) for x in c)
+
+
+def selftest_overlap(samples=1 << 26, seed=1):
+    """(mismatches, pairs handed to the FP64 pipe, pairs without angles) of the overlap area in
+    float-float arithmetic against the FP64 pipe."""
+    c = (ctypes.c_uint64 * 4)()
+    check(load().bg3_selftest_overlap(int(samples), int(seed), c), "bg3_selftest_overlap")
+    return tuple(int(x) for x in c)[:3]
 
 
 def selftest_izhikevich(samples=1 << 26, seed=1):

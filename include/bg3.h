@@ -395,6 +395,10 @@ int bg3_selftest_binary64(uint64_t samples, uint64_t seed, uint64_t *counts);
  * the FP64 pipe, float-float mismatches, float-float values handed to the FP64 pipe, operand sets
  * outside the integer pipe's restated range.  No counterpart in the reference. */
 int bg3_selftest_izhikevich(uint64_t samples, uint64_t seed, uint64_t *counts);
+/* The growth rule's overlap area (double acos, sin and division per pair) in float-float arithmetic
+ * against the FP64 pipe on `samples` random pairs: counts[0..2] = mismatches, pairs handed to the
+ * FP64 pipe, pairs drawn that need no angle.  No counterpart in the reference. */
+int bg3_selftest_overlap(uint64_t samples, uint64_t seed, uint64_t *counts);
 /* Failure-detection self-test: one warp waits, with the bounded mbarrier wait the step kernels
  * use, on a barrier that nothing completes, for at most limit_ns (1 .. 2e9).  The wait gives up,
  * the kernel returns normally and the context stays usable: *status = BG3_ERR_TIMEOUT, and

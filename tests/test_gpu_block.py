@@ -184,3 +184,13 @@ def test_two_spikes_at_one_synapse_in_a_block():
             same(nets[0], nets[2], "radius %g after %d steps" % (radius, n))
             same(nets[1], nets[2], "small, radius %g after %d steps" % (radius, n))
         assert int(nets[0].download_lif(fields=("spikeCount",))["spikeCount"].max()) > 8
+
+
+@pytest.mark.parametrize("seed", [5, 6])
+def test_overlap_area_matches_fp64(seed):
+    """The overlap area in float-float arithmetic gives the FP64 pipe's bits on equal, close,
+    just touching, nearly contained and independent radii, and hands only the uncertain few back."""
+    n = 1 << 25
+    bad, handed, without = bg.selftest_overlap(samples=n, seed=seed)
+    assert bad == 0
+    assert without < n // 2 and handed < n // 50, (handed, without)
