@@ -1,25 +1,24 @@
 // Per-epoch ConnGrowth pass and recorder, on the device.
 //
-//   k_growth_radii     rates = spikeCount / T; radii += T * rho * outgrowth      (O(N))
-//   k_growth_existing  W of every in-use synapse from the overlap area of its pair (O(S))
-//   k_growth_rmax      the largest radius (one CTA)
+//   k_out_zero         clears the outgoing counts and the largest radius
+//   k_growth_radii     rates = spikeCount / T; radii += T * rho * outgrowth, their maximum (O(N))
+//   k_growth_existing  W of every in-use synapse from the overlap area of its pair, and its count in
+//                      the outgoing map                                              (O(S))
 //   k_growth_add       one CTA per destination scans the sources in ascending order (on the grid
 //                      layout only the window within the largest radius), computes the frontier
 //                      distance / overlap area, and appends the new synapses in source order after
 //                      the row's in-use prefix            (O(N^2) pairs, no N^2 storage)
-//   k_out_count/scan/fill  outgoing CSR rebuild per delay class (createSynapseImap)
+//   k_out_scan/fill    outgoing CSR rebuild per delay class (createSynapseImap); k_out_count where
+//                      no weight pass counts
 //   k_record_epoch     recorder histograms, rates/radii history, radius clamp, spike-count roll
 #include "bg3_area.cuh"
 #include "bg3_internal.cuh"
 
 namespace bg3 {
 
-// ConnGrowth::updateConns (Connections/ConnGrowth.cpp:295-311).
-__global__ void k_growth_radii(const NetDev *nets)
+// ConnGrowth::updateConns (Connections/ConnGrowth.cpp:295-311): the radius after the epoch.
+__device__ __forceinline__ float grow_radius(const NetDev &n, int i)
 {
-    const NetDev &n = nets[0];
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n.N) return;
     float T = n.epoch_duration;
     const int cnt = n.spikeCount[i];
     float rate = (float)cnt / T;
@@ -29,7 +28,21 @@ __global__ void k_growth_radii(const NetDev *nets)
                                                 : exp_cr((n.g_epsilon - rate / n.g_max_rate) / n.g_beta);
     float og = 1.0f - 2.0f / (e + 1.0f);
     float trho = T * n.g_rho;
-    n.radii[i] = n.radii[i] + trho * og;
+    return n.radii[i] = n.radii[i] + trho * og;
+}
+
+// With the largest radius, for the overlap scan's window (cleared by k_out_zero).
+__global__ void k_growth_radii(const NetDev *nets)
+{
+    const NetDev &n = nets[0];
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    float m = 0.0f;  // the radius after the update; negative and NaN count as 0
+    if (i < n.N) m = fmaxf(m, grow_radius(n, i));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    // non-negative floats order as their bits do
+    if ((threadIdx.x & 31) == 0 && m > 0.0f)
+        atomicMax((int *)n.grow_rmax, __float_as_int(m));
 }
 
 // Layout::synType (Layouts/Layout.cpp:129-140): II 0, IE 1, EI 2, EE 3.
@@ -41,39 +54,32 @@ __device__ __forceinline__ float syn_sign(int type) { return (type <= 1) ? -1.0f
 
 // Weight update of existing synapses (ConnGrowth.cpp:420-438):
 // W = area * synSign(type) * SYNAPSE_STRENGTH_ADJUSTMENT (1.0e-8).
-__global__ void k_growth_existing(const NetDev *nets)
+// Bound by the instructions of the areas (pair_area); a warp takes one row quad of a tile, a lane
+// the four slots of its destination, so the destination's position, the quad's planes and the
+// index arithmetic are read once for four areas.  The outgoing map's counts ride along: their
+// atomics return nothing and cost this kernel little, and a pass over the planes of their own 68 us.
+__global__ void __launch_bounds__(256) k_growth_existing(const NetDev *nets)
 {
     const NetDev &n = nets[0];
-    size_t total = (size_t)n.Np * n.Mq * 4;
-    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total;
-         p += (size_t)gridDim.x * blockDim.x) {
-        int d, k;
-        pos_slot(p, n.Mq, k, d);
-        if (d >= n.N || k >= (int)n.count[d]) continue;
-        int s = n.src[p];
-        float a = pair_area(n.xloc[s], n.yloc[s], n.radii[s], n.xloc[d], n.yloc[d], n.radii[d]);
-        if (a < 0.0f) set_err(n, ERR_NEGATIVE_AREA);  // the reference would erase (area >= 0)
-        n.ev[p].W = a * syn_sign(n.stype[p]) * 1.0e-8f;
-    }
-}
-
-// The largest radius after the epoch's radius update (negative radii count as 0), for the
-// overlap scan's window: one CTA.
-__global__ void __launch_bounds__(1024) k_growth_rmax(const NetDev *nets)
-{
-    const NetDev &n = nets[0];
-    __shared__ float wmax[32];
-    float m = 0.0f;
-    for (int i = threadIdx.x; i < n.N; i += blockDim.x) m = fmaxf(m, n.radii[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        m = threadIdx.x < (blockDim.x >> 5) ? wmax[threadIdx.x] : 0.0f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (threadIdx.x == 0) *n.grow_rmax = m;
+    const int lane = threadIdx.x & 31;
+    const uint32_t total = (uint32_t)n.ntiles * (uint32_t)n.Mq;
+    const uint32_t step = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < total; q += step) {
+        const int d = (int)(q / (uint32_t)n.Mq) * 32 + lane, k0 = (int)(q % (uint32_t)n.Mq) * 4;
+        const int cnt = d < n.N ? (int)n.count[d] - k0 : 0;
+        if (cnt <= 0) continue;
+        const size_t p = ((size_t)q * 32 + lane) * 4;
+        const int4 src = *(const int4 *)(n.src + p);
+        const uint32_t type = *(const uint32_t *)(n.stype + p), cls = *(const uint32_t *)(n.lcls + p);
+        const float xd = n.xloc[d], yd = n.yloc[d], rd = n.radii[d];
+#pragma unroll 1
+        for (int j = 0; j < 4 && j < cnt; j++) {
+            const int s = j == 0 ? src.x : j == 1 ? src.y : j == 2 ? src.z : src.w;
+            const float a = pair_area(n.xloc[s], n.yloc[s], n.radii[s], xd, yd, rd);
+            if (a < 0.0f) set_err(n, ERR_NEGATIVE_AREA);  // the reference would erase (area >= 0)
+            n.ev[p + j].W = a * syn_sign((int)((type >> (8 * j)) & 255u)) * 1.0e-8f;
+            atomicAdd(&n.outCount[(size_t)((cls >> (8 * j)) & 255u) * n.N + s], 1u);
+        }
     }
 }
 
@@ -138,6 +144,15 @@ __global__ void __launch_bounds__(ADD_THREADS) k_growth_add(const NetDev *nets)
     const int8_t td = n.ntype[d];
     const unsigned long long t = *n.step;
     const ScanWindow win = scan_window(n, d, rd);
+    // most destinations add nothing: one look at all pairs without order or areas first (a barrier
+    // for each chunk of them instead made this kernel 83 us, now 72, where nothing is added; 10,000 neurons)
+    bool any = false;
+    for (int c = threadIdx.x; c < win.count; c += ADD_THREADS) {
+        const int s = window_source(n, win, c);
+        if ((existing[s >> 5] >> (s & 31)) & 1u) continue;
+        any |= s != d && pair_delta(n.xloc[s], n.yloc[s], n.radii[s], xd, yd, rd) < 0.0f;
+    }
+    if (!__syncthreads_or(any)) return;
     for (int base = 0; base < win.count; base += ADD_THREADS) {
         const int c = base + threadIdx.x;
         const int s = c < win.count ? window_source(n, win, c) : n.N;
@@ -147,7 +162,7 @@ __global__ void __launch_bounds__(ADD_THREADS) k_growth_add(const NetDev *nets)
             a = pair_area(n.xloc[s], n.yloc[s], n.radii[s], xd, yd, rd);
             add = a > 0.0f;
         }
-        // most chunks add nothing (every pair beyond the radii): one barrier, no ordering
+        // most chunks add nothing: one barrier, no ordering
         if (!__syncthreads_or(add)) continue;
         unsigned m = __ballot_sync(0xffffffffu, add);
         if (lane == 0) warp_cnt[warp] = __popc(m);
@@ -183,6 +198,7 @@ __global__ void __launch_bounds__(ADD_THREADS) k_growth_add(const NetDev *nets)
                 e.last = BG3_NO_SPIKE32;
                 e.born = (uint32_t)t;
                 n.ev[p] = e;
+                atomicAdd(&n.outCount[(size_t)n.t_lcls[type] * n.N + s], 1u);
             } else {
                 set_err(n, ERR_ROW_FULL);
             }
@@ -204,6 +220,7 @@ __global__ void k_out_zero(const NetDev *nets)
         n.outCount[i] = 0u;
         n.outFill[i] = 0u;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *n.grow_rmax = 0.0f;
 }
 __global__ void k_out_count(const NetDev *nets)
 {
@@ -217,20 +234,24 @@ __global__ void k_out_count(const NetDev *nets)
             atomicAdd(&n.outCount[(size_t)n.lcls[p] * n.N + n.src[p]], 1u);
     }
 }
-// exclusive scan of outCount into outBegin; one CTA of 1024 threads walks the table in chunks
+// exclusive scan of outCount into outBegin; one CTA of 1024 threads walks the table in chunks, four
+// entries a thread (one entry a thread and as many times the barriers took 21 us for 20,000 entries, now 14)
 __global__ void __launch_bounds__(1024) k_out_scan(const NetDev *nets)
 {
     const NetDev &n = nets[0];
     __shared__ uint32_t wsum[32];
-    __shared__ uint32_t carry;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int total = n.N * n.n_delays;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int b = 0; b < total; b += 1024) {
-        int i = b + threadIdx.x;
-        uint32_t v = (i < total) ? n.outCount[i] : 0u;
-        uint32_t x = v;
+    uint32_t carry = 0;
+    for (int b = 0; b < total; b += 4096) {
+        const int i = b + (int)threadIdx.x * 4;
+        uint32_t v[4], x = 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            v[u] = x;
+            if (i + u < total) x += n.outCount[i + u];
+        }
+        const uint32_t own = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -238,35 +259,50 @@ __global__ void __launch_bounds__(1024) k_out_scan(const NetDev *nets)
         }
         if (lane == 31) wsum[warp] = x;
         __syncthreads();
-        if (warp == 0) {
-            uint32_t w = wsum[lane], z = w;
+        uint32_t z = wsum[lane];  // every warp scans the warps' sums
+        const uint32_t w = z;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t y = __shfl_up_sync(0xffffffffu, z, o);
-                if (lane >= o) z += y;
-            }
-            wsum[lane] = z - w;
+        for (int o = 1; o < 32; o <<= 1) {
+            uint32_t y = __shfl_up_sync(0xffffffffu, z, o);
+            if (lane >= o) z += y;
         }
-        __syncthreads();
-        uint32_t c = carry;
-        if (i < total) n.outBegin[i] = c + wsum[warp] + x - v;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry = c + wsum[31] + x;
+        const uint32_t base = carry + __shfl_sync(0xffffffffu, z - w, warp) + x - own;
+        carry += __shfl_sync(0xffffffffu, z, 31);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (i + u < total) n.outBegin[i + u] = base + v[u];
         __syncthreads();
     }
 }
-__global__ void k_out_fill(const NetDev *nets)
+// A warp takes one row quad of a tile, 32 consecutive slots at a time (eight dests by four rows: the
+// lanes' sources repeat, so their places in the map are close together), and draws its four places
+// at once: one at a time the pass waits for each atomic's return, 86 us over 7.6 M synapses (now 76); four
+// rows of 32 dests at once scatter the stores, 113 us.
+__global__ void __launch_bounds__(256) k_out_fill(const NetDev *nets)
 {
     const NetDev &n = nets[0];
-    size_t total = (size_t)n.Np * n.Mq * 4;
-    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total;
-         p += (size_t)gridDim.x * blockDim.x) {
-        int d, k;
-        pos_slot(p, n.Mq, k, d);
-        if (d >= n.N || k >= (int)n.count[d]) continue;
-        size_t key = (size_t)n.lcls[p] * n.N + n.src[p];
-        uint32_t slot = n.outBegin[key] + atomicAdd(&n.outFill[key], 1u);
-        n.outMap[slot] = (uint32_t)p;
+    const int lane = threadIdx.x & 31;
+    const uint32_t total = (uint32_t)n.ntiles * (uint32_t)n.Mq;
+    const uint32_t step = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < total; q += step) {
+        const int d0 = (int)(q / (uint32_t)n.Mq) * 32 + (lane >> 2);
+        const int k = (int)(q % (uint32_t)n.Mq) * 4 + (lane & 3);
+        const size_t p = (size_t)q * 128 + lane;
+        size_t key[4];
+        uint32_t slot[4];
+        bool on[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int d = d0 + 8 * j;
+            on[j] = d < n.N && k < (int)n.count[d];
+            if (on[j]) key[j] = (size_t)n.lcls[p + 32 * j] * n.N + n.src[p + 32 * j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (on[j]) slot[j] = n.outBegin[key[j]] + atomicAdd(&n.outFill[key[j]], 1u);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (on[j]) n.outMap[slot[j]] = (uint32_t)(p + 32 * j);
     }
 }
 
@@ -300,19 +336,24 @@ __global__ void k_record_epoch(const NetDev *nets, int epoch, bool growth)
     n.spikeCount[i] = 0;
 }
 
+// blocks of eight warps for a warp per row quad of a tile, at most 8 an SM
+static int quad_blocks(const NetDev &h)
+{
+    const long long b = ((long long)h.ntiles * h.Mq + 7) / 8;
+    return (int)(b < 152 * 8 ? (b > 0 ? b : 1) : 152 * 8);
+}
+
 void launch_growth(const NetDev &h, const NetDev *d_net, int epoch, int add_threads, cudaStream_t s)
 {
     int nb = (h.N + 255) / 256;
+    const int sb = quad_blocks(h);
+    k_out_zero<<<nb, 256, 0, s>>>(d_net);
     k_growth_radii<<<nb, 256, 0, s>>>(d_net);
-    int sb = 152 * 8;
     k_growth_existing<<<sb, 256, 0, s>>>(d_net);
-    k_growth_rmax<<<1, 1024, 0, s>>>(d_net);
     size_t smem = (size_t)((h.N + 31) / 32) * sizeof(uint32_t);
     if (add_threads == 128) k_growth_add<128><<<h.N, 128, smem, s>>>(d_net);
     else if (add_threads == 512) k_growth_add<512><<<h.N, 512, smem, s>>>(d_net);
     else k_growth_add<256><<<h.N, 256, smem, s>>>(d_net);
-    k_out_zero<<<nb, 256, 0, s>>>(d_net);
-    k_out_count<<<sb, 256, 0, s>>>(d_net);
     k_out_scan<<<1, 1024, 0, s>>>(d_net);
     k_out_fill<<<sb, 256, 0, s>>>(d_net);
     k_record_epoch<<<nb, 256, 0, s>>>(d_net, epoch, true);
@@ -347,7 +388,7 @@ void launch_rebuild_maps(const NetDev &h, const NetDev *d_net, cudaStream_t s)
     k_out_zero<<<nb, 256, 0, s>>>(d_net);
     k_out_count<<<sb, 256, 0, s>>>(d_net);
     k_out_scan<<<1, 1024, 0, s>>>(d_net);
-    k_out_fill<<<sb, 256, 0, s>>>(d_net);
+    k_out_fill<<<quad_blocks(h), 256, 0, s>>>(d_net);
 }
 
 }  // namespace bg3
