@@ -339,13 +339,63 @@ struct ThinTile {
     int cnt, nq;
 };
 
+// The barrier of a small network's launch: its block, or its cluster of blocks.
+__device__ __forceinline__ void small_sync()
+{
+    if (gridDim.x == 1) {
+        __syncthreads();
+    } else {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+}
+
+// Injected noise in a small network's launch: each step the integrating neurons draw the next values
+// of one stream, from the highest index down, so a neuron's place depends on how many above it draw.
+// A tile's warp sends its count to every block and passes a barrier; one a step, with the counts of
+// alternate steps in alternate rows.  The value's load is then in flight during the synapse step.
+struct SmallDraws {
+    int *cnt;                   // [2][SMALL_MAX_N / 32] in shared memory
+    unsigned long long cursor;  // of the next step's first draw
+    int tiles, row;
+};
+__device__ __forceinline__ float small_draw(const NetDev &n, SmallDraws &z, int tile, bool draws)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t m = __ballot_sync(0xffffffffu, draws);
+    int *cnt = z.cnt + z.row * (SMALL_MAX_N / 32);
+    z.row ^= 1;
+    if (gridDim.x == 1) {
+        if (lane == 0) cnt[tile] = __popc(m);
+    } else if (lane < (int)gridDim.x) {
+        uint32_t at;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;"
+            : "=r"(at)
+            : "r"((uint32_t)__cvta_generic_to_shared(cnt + tile)), "r"((uint32_t)lane));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(__popc(m)) : "memory");
+    }
+    small_sync();
+    int above = 0, all = 0;
+    for (int k = lane; k < z.tiles; k += 32) {
+        all += cnt[k];
+        if (k > tile) above += cnt[k];
+    }
+    above = __reduce_add_sync(0xffffffffu, above);
+    const unsigned long long pos = z.cursor + (unsigned)(above + __popc((m >> lane) >> 1));
+    z.cursor += (unsigned)__reduce_add_sync(0xffffffffu, all);
+    if (!draws) return 0.0f;
+    if (pos < (unsigned long long)n.noise_len) return n.noise_buf[pos];
+    set_err(n, ERR_NOISE_EXHAUSTED);
+    return 0.0f;
+}
+
 // nt steps from t on: the arrivals made ready, then step by step the neuron update, the arrivals,
 // decay and sum.  The psr is in shared memory.  DEP: the kernel's grid-dependency wait comes before
 // the first access that needs it (see k_blk_thin).  Returns the steps at which the neuron fired.
-template <int SYN, bool DEP>
+template <int SYN, bool DEP, bool INJ = false>
 __device__ __forceinline__ uint32_t thin_steps(const NetDev &n, const BlkDev &b, const ThinSmem &s,
                                                ThinTile &y, int tile, int d, bool valid, int nt,
-                                               unsigned long long t)
+                                               unsigned long long t, SmallDraws *z = nullptr)
 {
     const int lane = threadIdx.x & 31;
     const int4 *S = reinterpret_cast<const int4 *>(n.src) + (size_t)tile * n.Mq * 32 + lane;
@@ -354,8 +404,10 @@ __device__ __forceinline__ uint32_t thin_steps(const NetDev &n, const BlkDev &b,
     bool waited = !DEP || SYN < 2;
     // the steps' noise draws depend on nothing but the step: four at a time, so that one draw's
     // latency hides another's (inside the step loop each would wait alone)
+    float drawn = 0.0f;
+    if (INJ) drawn = small_draw(n, *z, tile, valid && neuron_branch(y.x) == BR_INTEGRATE);
 #pragma unroll 4
-    for (int j = 0; j < nt; j++)
+    for (int j = 0; !INJ && j < nt; j++)
         s.noise[j * 32 + lane] = normal_device(n.noise_seed, t + (unsigned)j, d);
     for (int g0 = 0; g0 < y.nq; g0 += 16) {
         // the slots whose source has a spike in this block's window, 64 rows at a time
@@ -402,8 +454,11 @@ __device__ __forceinline__ uint32_t thin_steps(const NetDev &n, const BlkDev &b,
         if (valid) {
             const int br = neuron_branch(y.x);
             const float in = input_update(n, d, y.x, tj, y.sp);
-            if (neuron_update(n, d, y.x, br, in, s.noise[j * 32 + lane], tj, mode)) fired |= 1u << j;
+            const float noise = INJ ? drawn : s.noise[j * 32 + lane];
+            if (neuron_update(n, d, y.x, br, in, noise, tj, mode)) fired |= 1u << j;
         }
+        if (INJ && j + 1 < nt)
+            drawn = small_draw(n, *z, tile, valid && neuron_branch(y.x) == BR_INTEGRATE);
         if ((any >> j) & 1u) {
             if ((e.steps >> j) & 1u) {
                 for (unsigned long long r = e.rows; r; r &= r - 1ull) {
@@ -627,17 +682,7 @@ __global__ void __launch_bounds__(256) k_blk_post_batch(const NetDev *nets, cons
 // one block) after each block of steps and, for the STDP kinds, another after the post-spike pass.
 // The barriers order the masks, bitmaps and histories that the tiles read of each other.  Four warps
 // a block, one per quarter of its SM, up to 32 tiles: a warp issues alone, and that is its pace.
-__device__ __forceinline__ void small_sync()
-{
-    if (gridDim.x == 1) {
-        __syncthreads();
-    } else {
-        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-    }
-}
-
-template <int SYN>
+template <int SYN, bool INJ>
 __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 1) k_blk_small(const __grid_constant__ NetDev n,
                                                                       const __grid_constant__ BlkDev b,
                                                                       int nsteps, int T)
@@ -649,16 +694,21 @@ __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 1) k_blk_small(const __gr
     const ThinSmem s = thin_smem(smem_raw + warp * blk_thin_smem(n.Mq), n.Mq);
     ThinTile y;
     unsigned long long t = *n.step;
+    __shared__ int s_draws[INJ ? 2 * (SMALL_MAX_N / 32) : 1];
+    SmallDraws z = {s_draws, INJ ? *n.noise_cursor : 0ull, (int)gridDim.x * nw, 0};
     if (active) {
         thin_static(n, s, y, tile);
         thin_load(n, b, s, y, tile);
     }
+    if (INJ) small_sync();  // every block has started: its shared memory can be written
     for (int left = nsteps; left > 0;) {
         const int nt = min(left, T);
         if (first) blk_clear(n, b, t + (unsigned)nt);
         if (active) {
-            const uint32_t fired = thin_steps<SYN, false>(n, b, s, y, tile, d, valid, nt, t);
+            const uint32_t fired = thin_steps<SYN, false, INJ>(n, b, s, y, tile, d, valid, nt, t, &z);
             y.hist = blk_spikes<SYN>(n, b, tile, d, valid, y.hist, fired, nt, t);
+        } else if (INJ) {
+            for (int j = 0; j < nt; j++) small_draw(n, z, tile, false);
         }
         small_sync();
         if (SYN >= 2) {
@@ -673,6 +723,7 @@ __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 1) k_blk_small(const __gr
         thin_store(n, s, y, tile);
     }
     if (first) {
+        if (INJ) *n.noise_cursor = z.cursor;
         *n.step = t;
         *n.dstep = t;
         if (t >= 0xffffff00ull) set_err(n, ERR_STEP_RANGE);
@@ -1507,13 +1558,13 @@ bool blk_small_ok(const NetDev &h)
     return small_shape(h, w) > 0;
 }
 
-template <int SYN>
+template <int SYN, bool INJ>
 static void launch_small_t(const NetDev &h, const BlkDev &b, int nsteps, int T, cudaStream_t s)
 {
     int w = 1;
     const int blocks = small_shape(h, w);
     const size_t sm = (size_t)w * blk_thin_smem(h.Mq);
-    cudaFuncSetAttribute(k_blk_small<SYN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_blk_small<SYN, INJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1525,17 +1576,21 @@ static void launch_small_t(const NetDev &h, const BlkDev &b, int nsteps, int T, 
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_blk_small<SYN>, h, b, nsteps, T);
+    cudaLaunchKernelEx(&cfg, k_blk_small<SYN, INJ>, h, b, nsteps, T);
 }
 
 // nsteps steps of a small network, T at a time, in one launch.
 void launch_blk_small(const NetDev &h, const BlkDev &b, int nsteps, int T, cudaStream_t s)
 {
-    switch (h.syn_kind) {
-    case 1: launch_small_t<1>(h, b, nsteps, T, s); break;
-    case 2: launch_small_t<2>(h, b, nsteps, T, s); break;
-    case 3: launch_small_t<3>(h, b, nsteps, T, s); break;
-    default: launch_small_t<0>(h, b, nsteps, T, s); break;
+    switch (h.syn_kind * 2 + (h.noise_mode == 1 ? 1 : 0)) {
+    case 1: launch_small_t<0, true>(h, b, nsteps, T, s); break;
+    case 2: launch_small_t<1, false>(h, b, nsteps, T, s); break;
+    case 3: launch_small_t<1, true>(h, b, nsteps, T, s); break;
+    case 4: launch_small_t<2, false>(h, b, nsteps, T, s); break;
+    case 5: launch_small_t<2, true>(h, b, nsteps, T, s); break;
+    case 6: launch_small_t<3, false>(h, b, nsteps, T, s); break;
+    case 7: launch_small_t<3, true>(h, b, nsteps, T, s); break;
+    default: launch_small_t<0, false>(h, b, nsteps, T, s); break;
     }
 }
 

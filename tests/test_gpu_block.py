@@ -194,3 +194,33 @@ def test_overlap_area_matches_fp64(seed):
     bad, handed, without = bg.selftest_overlap(samples=n, seed=seed)
     assert bad == 0
     assert without < n // 2 and handed < n // 50, (handed, without)
+
+
+@pytest.mark.parametrize("syn", [bg.BG3_SYN_DS, bg.BG3_SYN_DYNSTDP])
+@pytest.mark.parametrize("w,h,radius,max_syn,steps", [
+    (10, 10, 1.5, 30, 300),         # four tiles, one block
+    (9, 7, 6.0, 65, 300),
+    (33, 31, 1.2, 37, 300),         # 32 tiles in eight blocks
+    (45, 45, 0.7, 9, 300),          # 64 tiles, the most
+    (10, 10, 1.5, 30, 40),          # the stream runs out: zeros and the error flag
+])
+def test_small_network_blocks_draw_injected_noise(syn, w, h, radius, max_syn, steps):
+    values = np.random.RandomState(3).standard_normal(w * h * steps).astype(np.float32)
+    nets = []
+    for small in (65536, 0):
+        net = lif(w, h, syn, radius, "poisson", max_syn)
+        net.set_noise_mode(bg.BG3_NOISE_INJECT, 1)
+        net.push_noise(values)
+        net.set_launch(small_max_slots=small)
+        nets.append(net)
+    for n in STEPS:
+        b0 = nets[0].launches
+        for net in nets:
+            net.step(n)
+        assert nets[0].launches - b0 == 1
+        same(nets[0], nets[1], "after %d steps" % n)
+        assert nets[0].noise_pending() == nets[1].noise_pending()
+    assert int(nets[0].download_lif(fields=("spikeCount",))["spikeCount"].sum()) > 0
+    assert (nets[0].error_word != 0) == (steps < sum(STEPS))
+    for net in nets:
+        net.close()
