@@ -110,6 +110,64 @@ __device__ __forceinline__ unsigned long long blk_spikes(const NetDev &n, const 
     return hist;
 }
 
+// One step of a tile's neurons, one lane per destination; true where the neuron fired.  Most steps
+// no neuron of the tile fires and no input spike falls due, and then every lane takes the same
+// straight line, which keeps or replaces its state by selection; the branches of neuron_update and
+// input_update, taken only when some lane needs them, cost 400 cycles a step of which the
+// arithmetic is 60 (and the regular input's 64-bit remainder another 400: its cycle position is
+// carried from step to step here).
+struct StepRun {
+    int mode;           // izh_mode
+    int cyc, until;     // regular input: the cycle position, and the end of the neuron's stimulus
+};
+__device__ __forceinline__ StepRun step_run(const NetDev &n, int d, const NeuronIn &x, unsigned long long t)
+{
+    StepRun r = {izh_mode(n, d), 0, 0};
+    if (n.input_kind == 1) {
+        r.cyc = (int)(((unsigned long long)n.reg_c0 + (t - n.reg_t0)) % (unsigned long long)n.reg_cycle);
+        r.until = (x.reg_shift + n.reg_dur) % n.reg_cycle;
+    }
+    return r;
+}
+__device__ __forceinline__ bool step_neuron(const NetDev &n, int d, bool valid, NeuronIn &x, float sp,
+                                            float noise, unsigned long long t, StepRun &r)
+{
+    const bool izh = n.neuron_kind == 1, poisson = n.input_kind == 2 && x.pmask;
+    const int br = neuron_branch(x), cyc = r.cyc;
+    const int left = x.nisi - 1;
+    bool slow = br == BR_FIRE || (izh && r.mode != IZH_FF);
+    if (poisson) slow = slow || left <= 0 || ((x.q >> ((uint32_t)t & 31u)) & 1u);
+    if (n.input_kind == 1) r.cyc = cyc + 1 == n.reg_cycle ? 0 : cyc + 1;
+    if (__any_sync(0xffffffffu, valid && slow)) {
+        if (!valid) return false;
+        const float in = input_update(n, d, x, t, sp);
+        return neuron_update(n, d, x, br, in, noise, t, r.mode);
+    }
+    if (n.input_kind == 1 && cyc >= x.reg_shift && cyc < r.until) sp = sp + x.reg_value;
+    if (poisson) {
+        x.nisi = left;
+        x.ipsr = x.ipsr * x.idec;
+        sp = sp + x.ipsr;
+    }
+    const bool on = br == BR_INTEGRATE;
+    if (!on) x.refr = x.refr - 1;
+    sp = sp + x.I0;
+    sp = sp + noise * x.Inoise;
+    if (izh) {
+        const float Vint = x.Vm * 1000.0f, u = x.u;
+        bool ok = false;
+        float V = izh_v_ff(Vint, u, x.C3, x.C2 * sp, ok);
+        if (on && valid && !ok) V = izh_v_fp64(Vint, u, x.C3, x.C2 * sp);  // uncertain rounding
+        const float w = u + x.C3 * x.A * (x.B * Vint - u);
+        x.u = on ? w : x.u;
+        x.Vm = on ? V : x.Vm;
+    } else {
+        const float V = x.C1 * x.Vm + x.C2 * sp;
+        x.Vm = on ? V : x.Vm;
+    }
+    return false;
+}
+
 // What the block starting at t1 and the ones after it find cleared: the next list of fired neurons,
 // and the counts of the blocks that may follow the next one.
 __device__ __forceinline__ void blk_clear(const NetDev &n, const BlkDev &b, unsigned long long t1)
@@ -165,17 +223,26 @@ __device__ __forceinline__ void blk_finish(const NetDev &n, const BlkDev &b, int
 // against 3 per synapse; the loads are hidden by the other warps of the SM.
 constexpr int BLK_THIN_QUADS = 16;
 constexpr int BLK_THIN_WARPS = 8;
-__host__ __device__ constexpr size_t blk_thin_smem(int Mq)
+constexpr int BLK_TEAM = 4;           // warps a tile
+// Quads kept: where one warp is a tile's pace it sums four at a time without looking for the last; a
+// warp among many does no work for quads that are not there (packed).
+__host__ __device__ constexpr int thin_quads(int Mq, bool packed)
 {
-    return (size_t)Mq * 32 * (16 + 16 + 16 + 4 + 4) + BLK_MAX_STEPS * 32 * 4;
+    return packed ? Mq : (Mq + 3) & ~3;
+}
+__host__ __device__ constexpr size_t blk_thin_smem(int Mq, int team, bool packed)
+{
+    return (size_t)thin_quads(Mq, packed) * 32 * (16 + 16 + 16 + 4 + 4) + BLK_MAX_STEPS * 32 * 4 +
+           (size_t)(team - 1) * 32 * 16;
 }
 
-struct ThinSmem {
+struct ThinSmem {           // Mq here: thin_quads; zero beyond the last in use
     float4 *psr, *dec;  // [Mq][32]
     float4 *inc;        // [Mq][32] psr increments of the arrivals that are ready
     uint32_t *msk;      // [Mq][32] their steps, one byte per row
     uint32_t *late;     // [Mq][32] the steps of the others
     float *noise;       // [BLK_MAX_STEPS][32]
+    uint4 *found;       // [BLK_TEAM - 1][32] ThinEvents of the other warps of the tile
 };
 
 // A lane's arrivals in the block are made ready before the steps run, so that their chains of loads
@@ -339,6 +406,19 @@ struct ThinTile {
     int cnt, nq;
 };
 
+// A tile's warps: `role` of `size`, and the named barrier they share.  Warp 0 runs the steps; before
+// them every warp draws its share of the noise and makes ready the arrivals of its quads (role, role +
+// size, ...), and it loads those quads.
+template <int SIZE>  // 0: known at run time
+struct Team {
+    int role, given, bar;
+    __device__ __forceinline__ int size() const { return SIZE ? SIZE : given; }
+    __device__ __forceinline__ void sync() const
+    {
+        if (size() > 1) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * size()) : "memory");
+    }
+};
+
 // The barrier of a small network's launch: its block, or its cluster of blocks.
 __device__ __forceinline__ void small_sync()
 {
@@ -392,11 +472,12 @@ __device__ __forceinline__ float small_draw(const NetDev &n, SmallDraws &z, int 
 // nt steps from t on: the arrivals made ready, then step by step the neuron update, the arrivals,
 // decay and sum.  The psr is in shared memory.  DEP: the kernel's grid-dependency wait comes before
 // the first access that needs it (see k_blk_thin).  Returns the steps at which the neuron fired.
-template <int SYN, bool DEP, bool INJ = false>
+template <int SYN, bool DEP, bool INJ, int SIZE>
 __device__ __forceinline__ uint32_t thin_steps(const NetDev &n, const BlkDev &b, const ThinSmem &s,
-                                               ThinTile &y, int tile, int d, bool valid, int nt,
-                                               unsigned long long t, SmallDraws *z = nullptr)
+                                               ThinTile &y, const Team<SIZE> &team, int tile, int d, bool valid,
+                                               int nt, unsigned long long t, SmallDraws *z = nullptr)
 {
+    constexpr bool PACKED = SIZE == 1;  // no quads beyond the last (thin_quads)
     const int lane = threadIdx.x & 31;
     const int4 *S = reinterpret_cast<const int4 *>(n.src) + (size_t)tile * n.Mq * 32 + lane;
     const uint32_t *act = b.act + (t & (BLK_ACT_ROWS - 1)) * n.ntiles;
@@ -405,34 +486,41 @@ __device__ __forceinline__ uint32_t thin_steps(const NetDev &n, const BlkDev &b,
     // the steps' noise draws depend on nothing but the step: four at a time, so that one draw's
     // latency hides another's (inside the step loop each would wait alone)
     float drawn = 0.0f;
-    if (INJ) drawn = small_draw(n, *z, tile, valid && neuron_branch(y.x) == BR_INTEGRATE);
+    if (INJ && team.role == 0)
+        drawn = small_draw(n, *z, tile, valid && neuron_branch(y.x) == BR_INTEGRATE);
+    else if (INJ)
+        small_sync();
 #pragma unroll 4
-    for (int j = 0; !INJ && j < nt; j++)
+    for (int j = team.role; !INJ && j < nt; j += team.size())
         s.noise[j * 32 + lane] = normal_device(n.noise_seed, t + (unsigned)j, d);
     for (int g0 = 0; g0 < y.nq; g0 += 16) {
         // the slots whose source has a spike in this block's window, 64 rows at a time
         unsigned long long rows = 0ull;
-        const int g1 = min(y.nq, g0 + 16);
-        for (int q0 = g0; q0 < g1; q0 += 4) {
+        const int lim = min(y.nq - g0, 16);
+        for (int i0 = team.role; i0 < lim; i0 += 4 * team.size()) {
             int4 sr[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                if (q0 + k < g1) {
-                    sr[k] = S[(size_t)(q0 + k) * 32];
-                    s.msk[(q0 + k) * 32 + lane] = 0u;
-                    s.late[(q0 + k) * 32 + lane] = 0u;
+            for (int k = 0; k < 4; k++) {
+                const int i = i0 + k * team.size();
+                if (i < lim) {
+                    sr[k] = S[(size_t)(g0 + i) * 32];
+                    s.msk[(g0 + i) * 32 + lane] = 0u;
+                    s.late[(g0 + i) * 32 + lane] = 0u;
                 }
-            uint32_t hit = 0u;
+            }
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                if (q0 + k < g1) {
-                    const int left = y.cnt - 4 * (q0 + k);  // in-use rows from this quad on
-                    if (left > 0) hit |= ((act[sr[k].x >> 5] >> (sr[k].x & 31)) & 1u) << (4 * k);
-                    if (left > 1) hit |= ((act[sr[k].y >> 5] >> (sr[k].y & 31)) & 1u) << (4 * k + 1);
-                    if (left > 2) hit |= ((act[sr[k].z >> 5] >> (sr[k].z & 31)) & 1u) << (4 * k + 2);
-                    if (left > 3) hit |= ((act[sr[k].w >> 5] >> (sr[k].w & 31)) & 1u) << (4 * k + 3);
+            for (int k = 0; k < 4; k++) {
+                const int i = i0 + k * team.size();
+                if (i < lim) {
+                    const int left = y.cnt - 4 * (g0 + i);  // in-use rows from this quad on
+                    uint32_t hit = 0u;
+                    if (left > 0) hit |= ((act[sr[k].x >> 5] >> (sr[k].x & 31)) & 1u);
+                    if (left > 1) hit |= ((act[sr[k].y >> 5] >> (sr[k].y & 31)) & 1u) << 1;
+                    if (left > 2) hit |= ((act[sr[k].z >> 5] >> (sr[k].z & 31)) & 1u) << 2;
+                    if (left > 3) hit |= ((act[sr[k].w >> 5] >> (sr[k].w & 31)) & 1u) << 3;
+                    rows |= (unsigned long long)hit << (4 * i);
                 }
-            rows |= (unsigned long long)hit << (4 * (q0 - g0));
+            }
         }
         if (!waited) {
             pdl_wait();
@@ -445,18 +533,29 @@ __device__ __forceinline__ uint32_t thin_steps(const NetDev &n, const BlkDev &b,
         pdl_wait();
         pdl_trigger();
     }
+    if (team.size() > 1) {
+        if (team.role > 0)
+            s.found[(team.role - 1) * 32 + lane] =
+                make_uint4((uint32_t)e.rows, (uint32_t)(e.rows >> 32), e.steps, e.late ? 1u : 0u);
+        team.sync();
+        if (team.role > 0) {
+            for (int j = 1; INJ && j < nt; j++) small_sync();
+            return 0u;
+        }
+        for (int k = 0; k < team.size() - 1; k++) {
+            const uint4 f = s.found[k * 32 + lane];
+            e.rows |= (unsigned long long)f.y << 32 | f.x;
+            e.steps |= f.z;
+            e.late = e.late || f.w != 0u;
+        }
+    }
     const uint32_t any = __reduce_or_sync(0xffffffffu, e.steps);
-    const int mode = izh_mode(n, d);
+    StepRun run = step_run(n, d, y.x, t);
     uint32_t fired = 0u;
 #pragma unroll 1
     for (int j = 0; j < nt; j++) {
-        const unsigned long long tj = t + (unsigned)j;
-        if (valid) {
-            const int br = neuron_branch(y.x);
-            const float in = input_update(n, d, y.x, tj, y.sp);
-            const float noise = INJ ? drawn : s.noise[j * 32 + lane];
-            if (neuron_update(n, d, y.x, br, in, noise, tj, mode)) fired |= 1u << j;
-        }
+        const float noise = INJ ? drawn : s.noise[j * 32 + lane];
+        if (step_neuron(n, d, valid, y.x, y.sp, noise, t + (unsigned)j, run)) fired |= 1u << j;
         if (INJ && j + 1 < nt)
             drawn = small_draw(n, *z, tile, valid && neuron_branch(y.x) == BR_INTEGRATE);
         if ((any >> j) & 1u) {
@@ -472,44 +571,61 @@ __device__ __forceinline__ uint32_t thin_steps(const NetDev &n, const BlkDev &b,
             __syncwarp();
         }
         float acc = 0.0f;
-        for (int q = 0; q < y.nq; q++) {
-            float4 v = s.psr[q * 32 + lane];
-            const float4 c = s.dec[q * 32 + lane];
-            v.x = v.x * c.x;
-            v.y = v.y * c.y;
-            v.z = v.z * c.z;
-            v.w = v.w * c.w;
-            s.psr[q * 32 + lane] = v;
-            acc = acc + v.x;
-            acc = acc + v.y;
-            acc = acc + v.z;
-            acc = acc + v.w;
+        for (int q0 = 0; q0 < y.nq; q0 += 4) {  // four quads' loads before the first is needed
+            float4 v[4], c[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (PACKED && q0 + k >= y.nq) break;
+                v[k] = s.psr[(q0 + k) * 32 + lane];
+                c[k] = s.dec[(q0 + k) * 32 + lane];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (PACKED && q0 + k >= y.nq) break;
+                v[k].x = v[k].x * c[k].x;
+                v[k].y = v[k].y * c[k].y;
+                v[k].z = v[k].z * c[k].z;
+                v[k].w = v[k].w * c[k].w;
+                s.psr[(q0 + k) * 32 + lane] = v[k];
+                acc = acc + v[k].x;
+                acc = acc + v[k].y;
+                acc = acc + v[k].z;
+                acc = acc + v[k].w;
+            }
         }
         y.sp = acc;
     }
     return fired;
 }
 
-__device__ __forceinline__ ThinSmem thin_smem(uint8_t *smem, int Mq)
+__device__ __forceinline__ ThinSmem thin_smem(uint8_t *smem, int Mq, bool packed)
 {
     ThinSmem s;
+    const int quads = thin_quads(Mq, packed);
     s.psr = reinterpret_cast<float4 *>(smem);
-    s.dec = s.psr + Mq * 32;
-    s.inc = s.dec + Mq * 32;
-    s.msk = reinterpret_cast<uint32_t *>(s.inc + Mq * 32);
-    s.late = s.msk + Mq * 32;
-    s.noise = reinterpret_cast<float *>(s.late + Mq * 32);
+    s.dec = s.psr + quads * 32;
+    s.inc = s.dec + quads * 32;
+    s.msk = reinterpret_cast<uint32_t *>(s.inc + quads * 32);
+    s.late = s.msk + quads * 32;
+    s.noise = reinterpret_cast<float *>(s.late + quads * 32);
+    s.found = reinterpret_cast<uint4 *>(s.noise + BLK_MAX_STEPS * 32);
     return s;
 }
 
 // What the steps do not change: the row counts, and the decay factors into shared memory.
-__device__ __forceinline__ void thin_static(const NetDev &n, const ThinSmem &s, ThinTile &y, int tile)
+template <int SIZE>
+__device__ __forceinline__ void thin_static(const NetDev &n, const ThinSmem &s, ThinTile &y,
+                                            const Team<SIZE> &team, int tile)
 {
     const int lane = threadIdx.x & 31, d = tile * 32 + lane;
     y.cnt = d < n.N ? (int)n.count[d] : 0;
     y.nq = (__reduce_max_sync(0xffffffffu, y.cnt) + 3) >> 2;
     const uint16_t *C = reinterpret_cast<const uint16_t *>(n.dcls) + (size_t)tile * n.Mq * 32 + lane;
-    for (int q = 0; q < y.nq; q++) {
+    for (int q = team.role; q < thin_quads(y.nq, SIZE == 1); q += team.size()) {
+        if (q >= y.nq) {
+            s.dec[q * 32 + lane] = s.psr[q * 32 + lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            continue;
+        }
         const uint32_t c = C[(size_t)q * 32];
         s.dec[q * 32 + lane] = make_float4(n.dtab[c & 15u], n.dtab[(c >> 4) & 15u],
                                            n.dtab[(c >> 8) & 15u], n.dtab[(c >> 12) & 15u]);
@@ -517,26 +633,27 @@ __device__ __forceinline__ void thin_static(const NetDev &n, const ThinSmem &s, 
 }
 
 // The tile's neurons into registers, its psr into shared memory.
+template <int SIZE>
 __device__ __forceinline__ void thin_load(const NetDev &n, const BlkDev &b, const ThinSmem &s, ThinTile &y,
-                                          int tile)
+                                          const Team<SIZE> &team, int tile)
 {
     const int lane = threadIdx.x & 31, d = tile * 32 + lane;
     y.sp = 0.0f;
     y.hist = 0ull;
-    if (d < n.N) {
+    if (team.role == 0 && d < n.N) {
         neuron_load(n, d, y.x);
         y.sp = n.sp[d];
         y.hist = b.hist[d];
     }
     const float4 *P = reinterpret_cast<const float4 *>(n.psr) + (size_t)tile * n.Mq * 32 + lane;
-    for (int q0 = 0; q0 < y.nq; q0 += 4) {
+    for (int q0 = team.role; q0 < y.nq; q0 += 4 * team.size()) {
         float4 v[4];
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            if (q0 + k < y.nq) v[k] = P[(size_t)(q0 + k) * 32];
+            if (q0 + k * team.size() < y.nq) v[k] = P[(size_t)(q0 + k * team.size()) * 32];
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            if (q0 + k < y.nq) s.psr[(q0 + k) * 32 + lane] = v[k];
+            if (q0 + k * team.size() < y.nq) s.psr[(q0 + k * team.size()) * 32 + lane] = v[k];
     }
 }
 
@@ -550,42 +667,44 @@ __device__ __forceinline__ void thin_store(const NetDev &n, const ThinSmem &s, c
 // STDP kinds follow a post-spike pass, which is launched once the block before has finished and
 // writes nothing but weights: everything else is final, and the wait can come as late as the first
 // arrival.
-template <int SYN>
-__device__ __forceinline__ void blk_thin_tile(const NetDev &n, const BlkDev &b, const int tile,
-                                              const int nt, uint8_t *smem)
+template <int SYN, int SIZE>
+__device__ __forceinline__ void blk_thin_tile(const NetDev &n, const BlkDev &b, const Team<SIZE> &team,
+                                              const int tile, const int nt, uint8_t *smem)
 {
     const int d = tile * 32 + ((int)threadIdx.x & 31);
     const bool valid = d < n.N;
-    const ThinSmem s = thin_smem(smem, n.Mq);
+    const ThinSmem s = thin_smem(smem, n.Mq, SIZE == 1);
     ThinTile y;
-    thin_static(n, s, y, tile);
+    thin_static(n, s, y, team, tile);
     if (SYN < 2) {
         pdl_wait();
         pdl_trigger();
     }
     const unsigned long long t = *n.step;
-    thin_load(n, b, s, y, tile);
-    const uint32_t fired = thin_steps<SYN, true>(n, b, s, y, tile, d, valid, nt, t);
+    thin_load(n, b, s, y, team, tile);
+    const uint32_t fired = thin_steps<SYN, true, false>(n, b, s, y, team, tile, d, valid, nt, t);
+    if (team.role > 0) return;
     thin_store(n, s, y, tile);
     blk_finish<SYN>(n, b, tile, d, valid, y.x, y.sp, y.hist, fired, nt, t);
 }
 
-template <int SYN>
+template <int SYN, int SIZE>
 __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 2) k_blk_thin(const __grid_constant__ NetDev n,
                                                                   const __grid_constant__ BlkDev b,
                                                                   int nt)
 {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    const int warp = (int)(threadIdx.x >> 5);
-    const int tile = blockIdx.x * (int)(blockDim.x >> 5) + warp;
+    const int per = (int)(blockDim.x >> 5) / SIZE;  // tiles a block
+    const int at = (int)(threadIdx.x >> 5) % per, tile = blockIdx.x * per + at;
+    const Team<SIZE> team = {(int)(threadIdx.x >> 5) / per, SIZE, 1 + at};
     if (tile < n.ntiles)
-        blk_thin_tile<SYN>(n, b, tile, nt, smem_raw + warp * blk_thin_smem(n.Mq));
+        blk_thin_tile<SYN>(n, b, team, tile, nt, smem_raw + at * blk_thin_smem(n.Mq, SIZE, SIZE == 1));
 }
 
 // Batched form: tiles[i] = (network, tile), -1 tiles idle; a block's entries belong to one
 // network, whose descriptor the block copies into shared memory first.  wsmem: bytes per warp
 // (the batch's widest thin network).
-template <int SYN>
+template <int SYN, int SIZE>
 __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 2) k_blk_thin_batch(const NetDev *nets,
                                                                         const BlkDev *blks,
                                                                         const int2 *tiles, int count,
@@ -593,16 +712,17 @@ __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 2) k_blk_thin_batch(const
 {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ __align__(16) NetDev s_net;
-    const int warp = (int)(threadIdx.x >> 5);
-    const int first = blockIdx.x * (int)(blockDim.x >> 5);
-    const int2 tr = first + warp < count ? tiles[first + warp] : make_int2(0, -1);
+    const int per = (int)(blockDim.x >> 5) / SIZE;
+    const int at = (int)(threadIdx.x >> 5) % per, first = blockIdx.x * per;
+    const Team<SIZE> team = {(int)(threadIdx.x >> 5) / per, SIZE, 1 + at};
+    const int2 tr = first + at < count ? tiles[first + at] : make_int2(0, -1);
     const int k = tiles[first].x;
     const uint4 *s4 = reinterpret_cast<const uint4 *>(nets + k);
     uint4 *d4 = reinterpret_cast<uint4 *>(&s_net);
     for (int i = threadIdx.x; i < (int)(sizeof(NetDev) / 16); i += blockDim.x) d4[i] = s4[i];
     const BlkDev b = blks[k];
     __syncthreads();
-    if (tr.y >= 0) blk_thin_tile<SYN>(s_net, b, tr.y, nt, smem_raw + warp * wsmem);
+    if (tr.y >= 0) blk_thin_tile<SYN>(s_net, b, team, tr.y, nt, smem_raw + at * wsmem);
 }
 
 // ---- STDP: learning after a block's post spikes -----------------------------------------------
@@ -685,40 +805,47 @@ __global__ void __launch_bounds__(256) k_blk_post_batch(const NetDev *nets, cons
 template <int SYN, bool INJ>
 __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 1) k_blk_small(const __grid_constant__ NetDev n,
                                                                       const __grid_constant__ BlkDev b,
-                                                                      int nsteps, int T)
+                                                                      int size, int nsteps, int T)
 {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    const int warp = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
-    const int tile = (int)blockIdx.x * nw + warp, d = tile * 32 + ((int)threadIdx.x & 31);
+    const int warp = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5) / size;  // tiles a block
+    // the warps of a tile on different quarters of the SM, and the first warps of four tiles too
+    const Team<0> team = {warp / nw, size, 1 + (warp + warp / nw) % nw};
+    const int at = team.bar - 1, tile = (int)blockIdx.x * nw + at, d = tile * 32 + ((int)threadIdx.x & 31);
     const bool active = tile < n.ntiles, valid = d < n.N, first = blockIdx.x == 0 && threadIdx.x == 0;
-    const ThinSmem s = thin_smem(smem_raw + warp * blk_thin_smem(n.Mq), n.Mq);
+    const ThinSmem s = thin_smem(smem_raw + at * blk_thin_smem(n.Mq, size, false), n.Mq, false);
     ThinTile y;
     unsigned long long t = *n.step;
     __shared__ int s_draws[INJ ? 2 * (SMALL_MAX_N / 32) : 1];
     SmallDraws z = {s_draws, INJ ? *n.noise_cursor : 0ull, (int)gridDim.x * nw, 0};
     if (active) {
-        thin_static(n, s, y, tile);
-        thin_load(n, b, s, y, tile);
+        thin_static(n, s, y, team, tile);
+        thin_load(n, b, s, y, team, tile);
     }
     if (INJ) small_sync();  // every block has started: its shared memory can be written
     for (int left = nsteps; left > 0;) {
         const int nt = min(left, T);
         if (first) blk_clear(n, b, t + (unsigned)nt);
         if (active) {
-            const uint32_t fired = thin_steps<SYN, false, INJ>(n, b, s, y, tile, d, valid, nt, t, &z);
-            y.hist = blk_spikes<SYN>(n, b, tile, d, valid, y.hist, fired, nt, t);
+            const uint32_t fired = thin_steps<SYN, false, INJ>(n, b, s, y, team, tile, d, valid, nt, t, &z);
+            if (team.role == 0)
+                y.hist = blk_spikes<SYN>(n, b, tile, d, valid, y.hist, fired, nt, t);
         } else if (INJ) {
-            for (int j = 0; j < nt; j++) small_draw(n, z, tile, false);
+            for (int j = 0; j < nt; j++) {
+                if (team.role == 0) small_draw(n, z, tile, false);
+                else small_sync();
+            }
         }
         small_sync();
         if (SYN >= 2) {
-            blk_post(n, b, tile, (int)gridDim.x * nw, nt, t);
+            blk_post(n, b, (int)blockIdx.x * (int)(blockDim.x >> 5) + warp,
+                     (int)(gridDim.x * (blockDim.x >> 5)), nt, t);
             small_sync();
         }
         t += (unsigned)nt;
         left -= nt;
     }
-    if (active) {
+    if (active && team.role == 0) {
         if (valid) neuron_store(n, d, y.x, y.sp);
         thin_store(n, s, y, tile);
     }
@@ -1434,19 +1561,14 @@ __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (ok) ok = dn_wait(n, s, &s.drawn, 0);
-        const int mode = izh_mode(n, d);
+        StepRun run = step_run(n, d, x, t);
         uint32_t fired = 0u;
 #pragma unroll 1
         for (int j = 0; ok && j < nt; j++) {
             // step t + j takes the sum of step t + j - 1
             if (j == 1 && !(ok = dn_wait(n, s, &s.summed, 0))) break;
             if (j > 0) sp = s.sum[j - 1][lane];
-            if (valid) {
-                const unsigned long long tj = t + (unsigned)j;
-                const int br = neuron_branch(x);
-                const float in = input_update(n, d, x, tj, sp);
-                if (neuron_update(n, d, x, br, in, s.noise[j][lane], tj, mode)) fired |= 1u << j;
-            }
+            if (step_neuron(n, d, valid, x, sp, s.noise[j][lane], t + (unsigned)j, run)) fired |= 1u << j;
         }
         if (ok && nt == 1) ok = dn_wait(n, s, &s.summed, 0);
         if (ok) {
@@ -1541,42 +1663,41 @@ void launch_blk_ring(const NetDev &h, const BlkDev &b, cudaStream_t s)
     k_blk_ring<<<(h.N + 255) / 256, 256, 0, s>>>(h, b);
 }
 
-// Blocks and warps per block of a small network's launch; 0 blocks when it does not fit a cluster of
-// eight (200 KB of shared memory per block).
-static int small_shape(const NetDev &h, int &warps)
+// Blocks, tiles per block and warps per tile of a small network's launch; 0 blocks when it does not fit
+// a cluster of eight (200 KB of shared memory per block).
+struct SmallShape {
+    int blocks, tiles, team;
+};
+static SmallShape small_shape(const NetDev &h)
 {
-    const size_t per = blk_thin_smem(h.Mq);
-    const int most = (int)std::min<size_t>(BLK_THIN_WARPS, 200 * 1024 / per);
-    if (most < 1) return 0;
-    warps = std::min(most, h.ntiles <= 32 ? std::min(4, h.ntiles) : BLK_THIN_WARPS);
-    const int blocks = (h.ntiles + warps - 1) / warps;
-    return blocks <= 8 ? blocks : 0;
+    SmallShape s = {0, h.ntiles <= 32 ? std::min(4, h.ntiles) : BLK_THIN_WARPS, 1};
+    s.tiles = (int)std::min<size_t>(s.tiles, 200 * 1024 / blk_thin_smem(h.Mq, BLK_TEAM, false));
+    if (s.tiles < 1) return s;
+    s.team = std::min(BLK_TEAM, BLK_THIN_WARPS / s.tiles);
+    s.blocks = (h.ntiles + s.tiles - 1) / s.tiles;
+    if (s.blocks > 8) s.blocks = 0;
+    return s;
 }
-bool blk_small_ok(const NetDev &h)
-{
-    int w;
-    return small_shape(h, w) > 0;
-}
+bool blk_small_ok(const NetDev &h) { return small_shape(h).blocks > 0; }
 
 template <int SYN, bool INJ>
 static void launch_small_t(const NetDev &h, const BlkDev &b, int nsteps, int T, cudaStream_t s)
 {
-    int w = 1;
-    const int blocks = small_shape(h, w);
-    const size_t sm = (size_t)w * blk_thin_smem(h.Mq);
+    const SmallShape p = small_shape(h);
+    const size_t sm = (size_t)p.tiles * blk_thin_smem(h.Mq, p.team, false);
     cudaFuncSetAttribute(k_blk_small<SYN, INJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)blocks;
+    attr[0].val.clusterDim.x = (unsigned)p.blocks;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(32 * w);
+    cfg.gridDim = dim3(p.blocks);
+    cfg.blockDim = dim3(32 * p.tiles * p.team);
     cfg.dynamicSmemBytes = sm;
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_blk_small<SYN, INJ>, h, b, nsteps, T);
+    cudaLaunchKernelEx(&cfg, k_blk_small<SYN, INJ>, h, b, p.team, nsteps, T);
 }
 
 // nsteps steps of a small network, T at a time, in one launch.
@@ -1596,38 +1717,54 @@ void launch_blk_small(const NetDev &h, const BlkDev &b, int nsteps, int T, cudaS
 
 // At most 44 KB of shared memory per block beside a batch's descriptor (48 KB is what a launch may
 // use without opting in), so that several blocks share an SM.
-static int thin_warps_for(int Mq) { return std::max(1, (int)(45056 / blk_thin_smem(Mq))); }
+static int thin_tiles_for(int Mq, int team) { return std::max(1, (int)(45056 / blk_thin_smem(Mq, team, team == 1))); }
 
-// Few tiles: one warp per block, so that they spread over the SMs.
+// Few tiles leave the SMs idle while one warp a tile waits for itself: then four warps a tile, up to
+// TEAM_TILES tiles (four an SM, which its registers hold), and the tiles spread over the SMs.
+constexpr int TEAM_TILES = 4 * 152;
+
+template <int SIZE>
+static void launch_thin_t(const NetDev &h, const BlkDev &b, int nt, cudaStream_t s)
+{
+    const int w = std::max(1, std::min({BLK_THIN_WARPS / SIZE, thin_tiles_for(h.Mq, SIZE), h.ntiles / 152}));
+    const int blocks = (h.ntiles + w - 1) / w, threads = 32 * w * SIZE;
+    const size_t sm = w * blk_thin_smem(h.Mq, SIZE, SIZE == 1);
+    switch (h.syn_kind) {
+    case 1: launch_dep(k_blk_thin<1, SIZE>, blocks, threads, sm, s, h, b, nt); break;
+    case 2: launch_dep(k_blk_thin<2, SIZE>, blocks, threads, sm, s, h, b, nt); break;
+    case 3: launch_dep(k_blk_thin<3, SIZE>, blocks, threads, sm, s, h, b, nt); break;
+    default: launch_dep(k_blk_thin<0, SIZE>, blocks, threads, sm, s, h, b, nt); break;
+    }
+}
 void launch_blk_thin(const NetDev &h, const BlkDev &b, int nt, cudaStream_t s)
 {
-    const int w = std::max(1, std::min({BLK_THIN_WARPS, thin_warps_for(h.Mq), h.ntiles / 152}));
-    const int blocks = (h.ntiles + w - 1) / w;
-    const size_t sm = w * blk_thin_smem(h.Mq);
-    switch (h.syn_kind) {
-    case 1: launch_dep(k_blk_thin<1>, blocks, 32 * w, sm, s, h, b, nt); break;
-    case 2: launch_dep(k_blk_thin<2>, blocks, 32 * w, sm, s, h, b, nt); break;
-    case 3: launch_dep(k_blk_thin<3>, blocks, 32 * w, sm, s, h, b, nt); break;
-    default: launch_dep(k_blk_thin<0>, blocks, 32 * w, sm, s, h, b, nt); break;
-    }
+    if (h.ntiles <= TEAM_TILES) launch_thin_t<BLK_TEAM>(h, b, nt, s);
+    else launch_thin_t<1>(h, b, nt, s);
     if (h.syn_kind >= 2) launch_dep(k_blk_post, 152, 256, 0, s, h, b, nt);
 }
 
-// tiles: n thin entries, each network's run padded to a multiple of `pad` entries; blocks of a
-// divisor of pad warps, so that a block serves one network.
+// tiles: n thin entries, each network's run padded to a multiple of `pad` entries; a block takes a
+// divisor of pad, so that it serves one network.
+template <int SIZE>
+static void launch_thin_batch_t(int syn_kind, const NetDev *nets, const BlkDev *blks, const int2 *tiles, int n,
+                                int pad, int max_mq, int nt, cudaStream_t s)
+{
+    int w = std::min({pad, BLK_THIN_WARPS / SIZE, thin_tiles_for(max_mq, SIZE)});
+    while (pad % w) w--;
+    const int blocks = (n + w - 1) / w, ws = (int)blk_thin_smem(max_mq, SIZE, SIZE == 1), threads = 32 * w * SIZE;
+    const size_t sm = (size_t)w * ws;
+    switch (syn_kind) {
+    case 1: launch_dep(k_blk_thin_batch<1, SIZE>, blocks, threads, sm, s, nets, blks, tiles, n, ws, nt); break;
+    case 2: launch_dep(k_blk_thin_batch<2, SIZE>, blocks, threads, sm, s, nets, blks, tiles, n, ws, nt); break;
+    case 3: launch_dep(k_blk_thin_batch<3, SIZE>, blocks, threads, sm, s, nets, blks, tiles, n, ws, nt); break;
+    default: launch_dep(k_blk_thin_batch<0, SIZE>, blocks, threads, sm, s, nets, blks, tiles, n, ws, nt); break;
+    }
+}
 void launch_blk_thin_batch(int syn_kind, const NetDev *nets, const BlkDev *blks, int nets_n,
                            const int2 *tiles, int n, int pad, int max_mq, int nt, cudaStream_t s)
 {
-    int w = std::min({pad, BLK_THIN_WARPS, thin_warps_for(max_mq)});
-    while (pad % w) w--;
-    const int blocks = (n + w - 1) / w, ws = (int)blk_thin_smem(max_mq);
-    const size_t sm = (size_t)w * ws;
-    switch (syn_kind) {
-    case 1: launch_dep(k_blk_thin_batch<1>, blocks, 32 * w, sm, s, nets, blks, tiles, n, ws, nt); break;
-    case 2: launch_dep(k_blk_thin_batch<2>, blocks, 32 * w, sm, s, nets, blks, tiles, n, ws, nt); break;
-    case 3: launch_dep(k_blk_thin_batch<3>, blocks, 32 * w, sm, s, nets, blks, tiles, n, ws, nt); break;
-    default: launch_dep(k_blk_thin_batch<0>, blocks, 32 * w, sm, s, nets, blks, tiles, n, ws, nt); break;
-    }
+    if (n <= TEAM_TILES) launch_thin_batch_t<BLK_TEAM>(syn_kind, nets, blks, tiles, n, pad, max_mq, nt, s);
+    else launch_thin_batch_t<1>(syn_kind, nets, blks, tiles, n, pad, max_mq, nt, s);
     if (syn_kind >= 2)
         launch_dep(k_blk_post_batch, dim3(std::max(1, std::min(152, 1216 / std::max(nets_n, 1))), nets_n),
                    256, 0, s, nets, blks, nt);
