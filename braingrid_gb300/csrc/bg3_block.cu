@@ -731,16 +731,14 @@ __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 2) k_blk_thin_batch(const
 // where an arrival at the same synapse follows a post spike within the block, its spike was
 // already under way (the source's newest history entry is later than t - delay), and the walk of
 // such a post spike learns nothing; so all of a block's arrivals come before the post spikes that
-// learn.  A walk sees the histories as of its step: entries the block added after it are skipped.
-__device__ __forceinline__ int count_at(const NetDev &n, int i, unsigned long long t)
+// learn.  A walk sees the histories as of its step: the entries the block added after it, counted in
+// the spike masks, are left out.
+__device__ __forceinline__ int count_at(const NetDev &n, int i, unsigned long long hist, int nt,
+                                        unsigned long long t, int j)
 {
-    int co = n.spikeCount[i] + n.spikeCountOffset[i];
-    for (int f = 0; f < BLK_MAX_STEPS; f++) {
-        const unsigned long long h = hist_at(n, i, co, -1);
-        if (h == BG3_ULONG_MAX || h <= t) break;
-        co = co > 0 ? co - 1 : n.max_spikes - 1;
-    }
-    return co;
+    const int co = n.spikeCount[i] + n.spikeCountOffset[i];
+    const int newer = __popc((uint32_t)rotr64(hist, (unsigned)t) & ((1u << nt) - (2u << j)));
+    return co >= newer ? co - newer : co - newer + n.max_spikes;
 }
 
 // One warp per neuron that fired, one lane per synapse.
@@ -754,17 +752,21 @@ __device__ __forceinline__ void blk_post(const NetDev &n, const BlkDev &b, int g
     for (int e = gw; e < m; e += nw) {
         const int d = ids[e];
         const int cnt = (int)n.count[d];
-        const uint32_t fired = (uint32_t)rotr64(b.hist[d], (unsigned)t) & ((1u << nt) - 1u);
+        const unsigned long long hd = b.hist[d];
+        const uint32_t fired = (uint32_t)rotr64(hd, (unsigned)t) & ((1u << nt) - 1u);
         for (int k = lane; k < cnt; k += 32) {
             const size_t p = slot_pos(k, d, n.Mq);
             const StdpConst &c = n.stdp[n.stype[p]];
             const int pre = n.src[p];
             const int delay = n.ltab[n.lcls[p]];
+            const unsigned long long hp = b.hist[pre];
             float W = n.ev[p].W;
             for (uint32_t f = fired; f; f &= f - 1u) {
-                const unsigned long long tj = t + (unsigned)(__ffs((int)f) - 1);
+                const int j = __ffs((int)f) - 1;
+                const unsigned long long tj = t + (unsigned)j;
                 PostPrep q;
-                stdp_post_prep(n, c, pre, d, count_at(n, pre, tj), count_at(n, d, tj), delay, tj, q);
+                stdp_post_prep(n, c, pre, d, count_at(n, pre, hp, nt, t, j), count_at(n, d, hd, nt, t, j), delay,
+                               tj, q);
                 W = stdp_post_finish(n, c, W, pre, delay, tj, q);
             }
             n.ev[p].W = W;

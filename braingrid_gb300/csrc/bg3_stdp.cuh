@@ -17,7 +17,8 @@ namespace bg3 {
 // co = spikeCount + spikeCountOffset.
 __device__ __forceinline__ unsigned long long hist_at(const NetDev &n, int i, int co, int off)
 {
-    const int x = (co + n.max_spikes + off) % n.max_spikes;
+    int x = co + n.max_spikes + off;  // below 3 max_spikes unless the ring has overflowed
+    while (x >= n.max_spikes) x -= n.max_spikes;
     return n.history[(size_t)i * n.max_spikes + x];
 }
 
@@ -25,30 +26,54 @@ __device__ __forceinline__ unsigned long long hist_at(const NetDev &n, int i, in
 __device__ __forceinline__ float pow_mu(float, float) { return 1.0f; }
 
 // One stdpLearning call with delta = dk steps (dk the signed interval; 0 when not a small count),
-// in two parts.  stdp_inc: the weight change, which W does not enter (W^mu = 1): false when delta
-// lies within the gap (W unchanged, no clamp), else epost * epre * dw in double.  stdp_apply: W
-// plus that change, rounded to float, then the clamps.  So the walks below can find a walk's
-// changes before W is known and apply them in order after.
-__device__ __forceinline__ bool stdp_inc(const StdpConst &c, float delta, float epost, float epre,
-                                         long long dk, double &inc)
+// in two parts.  stdp_dw: the weight change before the efficacies, which W does not enter (W^mu =
+// 1); false when delta lies within the gap (W unchanged, no clamp).  stdp_apply: W plus the double
+// product epost * epre * dw, rounded to float, then the clamps.  So the walks below can find a
+// walk's changes before W is known and apply them in order after.
+//
+// The reference promotes to double all along; on this chip's narrow FP64 pipe a post-spike pass of
+// a 30x30 network at 60 Hz waited for little else (500 steps 3.9 ms, now 3.3).  The comparisons need no double: a float against
+// a float is the same comparison in either, and 3 tau, exact in double, is replaced by the float next
+// to it on the far side.  1 - x rounds the same directly and by way of double (53 bits are more than
+// twice 24 and two).  The sum is made in float-float arithmetic where every value within 2^-44 of the
+// change and 2^-46 of the sum rounds the same (its distance from the double chain's value is below an
+// eighth of that), and in double otherwise.  What stays in double is the table's factor.
+__device__ __forceinline__ bool stdp_dw(const StdpConst &c, float delta, long long dk, float &dw)
 {
-    const double d = (double)delta;
-    float dw;
-    if (d < (double)(-c.gap)) {
-        const double e = (dk < 0 && -dk < (long long)c.dlen_neg) ? c.dneg[-dk] : exp(d / (double)c.tauneg);
+    if (delta < -c.gap) {
+        const double e = (dk < 0 && -dk < (long long)c.dlen_neg) ? c.dneg[-dk]
+                                                                  : exp((double)delta / (double)c.tauneg);
         dw = (float)((double)(pow_mu(0.0f, c.muneg) * c.Aneg) * e);
-    } else if (d > (double)c.gap) {
-        const double e = (dk > 0 && dk < (long long)c.dlen_pos) ? c.dpos[dk] : exp(-d / (double)c.taupos);
+    } else if (delta > c.gap) {
+        const double e = (dk > 0 && dk < (long long)c.dlen_pos) ? c.dpos[dk]
+                                                                 : exp(-(double)delta / (double)c.taupos);
         dw = (float)((double)(pow_mu(0.0f, c.mupos) * c.Apos) * e);
     } else {
         return false;
     }
-    inc = (double)epost * (double)epre * (double)dw;
     return true;
 }
-__device__ __forceinline__ float stdp_apply(const StdpConst &c, float W, double inc)
+// W + epost * epre * dw from float-float arithmetic; false where the rounding is not certain, or
+// the product so far from W's range of sizes that its low parts could be lost.
+__device__ __forceinline__ bool stdp_sum_ff(float W, float epost, float epre, float dw, float &out)
 {
-    W = (float)((double)W + inc);
+    const float f = epost * epre;
+    const float g = __fmaf_rn(epost, epre, -f);
+    const float p = f * dw;
+    const float q = __fmaf_rn(g, dw, __fmaf_rn(f, dw, -p));  // epost epre dw = p + q
+    const FF s = ff_two_sum(W, p);
+    const float lo = s.lo + q, err = fabsf(p) * 0x1p-44f + fabsf(s.hi) * 0x1p-46f;
+    const float up = s.hi + (lo + err), dn = s.hi + (lo - err);
+    out = up;
+    return up == dn && fabsf(p) > 0x1p-60f && fabsf(W) < 0x1p+60f && fabsf(p) < 0x1p+60f &&
+           fabsf(s.hi) > fabsf(p) * 0x1p-3f;
+}
+__device__ __forceinline__ float stdp_apply(const StdpConst &c, float W, float epost, float epre, float dw)
+{
+    float s;
+    if (!stdp_sum_ff(W, epost, epre, dw, s))
+        s = (float)((double)W + (double)epost * (double)epre * (double)dw);
+    W = s;
     if ((c.Wex < 0.0f && W > 0.0f) || (c.Wex > 0.0f && W < 0.0f)) W = 0.0f;
     if (fabsf(W) > fabsf(c.Wex)) W = c.Wex;
     return W;
@@ -56,8 +81,8 @@ __device__ __forceinline__ float stdp_apply(const StdpConst &c, float W, double 
 __device__ __forceinline__ float stdp_learn(const StdpConst &c, float W, float delta, float epost,
                                             float epre, long long dk)
 {
-    double inc;
-    return stdp_inc(c, delta, epost, epre, dk, inc) ? stdp_apply(c, W, inc) : W;
+    float dw;
+    return stdp_dw(c, delta, dk, dw) ? stdp_apply(c, W, epost, epre, dw) : W;
 }
 
 // A neuron's history entries -1 .. -4 read together (those of them that exist: off >= -ms), so
@@ -116,20 +141,20 @@ static __device__ float stdp_pre(const NetDev &n, const StdpConst &c, float W, i
     const unsigned long long sp2 = hist_at(n, pre, cpre, -2);
     float epre = 1.0f;
     if ((long long)sp2 > 0 && c.useFD)
-        epre = (float)(1.0 - (double)exp_interval(n, t - sp2, true, c.tauspre));
+        epre = 1.0f - exp_interval(n, t - sp2, true, c.tauspre);
     for (int off = -1;; --off) {
         if (off < -ms) { set_err(n, ERR_STDP_RING); break; }
         const unsigned long long sh = hist_get(n, post, cpost, off, hp);
         if (sh == BG3_ULONG_MAX) break;
         const long long dk = (long long)(sh - t);
         const float delta = (float)dk * n.dt;
-        if ((double)delta <= -3.0 * (double)c.tauneg) break;
+        if (delta <= __fmul_rd(-3.0f, c.tauneg)) break;
         float epost = 1.0f;
         if (c.useFD) {
             if (off - 1 < -ms) { set_err(n, ERR_STDP_RING); break; }
             const unsigned long long sh2 = hist_get(n, post, cpost, off - 1, hp);
             if (sh2 == BG3_ULONG_MAX) break;
-            epost = (float)(1.0 - (double)exp_interval(n, sh - sh2, true, c.tauspost));
+            epost = 1.0f - exp_interval(n, sh - sh2, true, c.tauspost);
         }
         W = stdp_learn(c, W, delta, epost, epre, dk);
     }
@@ -143,7 +168,7 @@ static __device__ float stdp_pre(const NetDev &n, const StdpConst &c, float W, i
 // the first before its wait on the delivery of the same step (the one writer of W there).
 constexpr int POST_STEPS = 4;
 struct PostPrep {
-    double inc0, inc1, inc2, inc3;  // the changes of steps 1 .. 4 (those with a bit in mask)
+    float dw[POST_STEPS], epre[POST_STEPS];  // the changes of steps 1 .. 4 (those with a bit in mask)
     float epost;
     int cpre;
     int mask;                       // bit k: step k + 1 changed W
@@ -161,12 +186,11 @@ __device__ __forceinline__ void stdp_post_prep(const NetDev &n, const StdpConst 
     hist_load4(n, pre, cpre, hp);
     float epost = 1.0f;
     const bool ok = sgn ? ((long long)q2 > 0) : (q2 != BG3_ULONG_MAX);
-    if (ok && c.useFD) epost = (float)(1.0 - (double)exp_interval(n, t - q2, sgn, c.tauspost));
+    if (ok && c.useFD) epost = 1.0f - exp_interval(n, t - q2, sgn, c.tauspost);
     q.epost = epost;
     q.cpre = cpre;
     q.mask = 0;
     q.next = 0;
-    q.inc0 = q.inc1 = q.inc2 = q.inc3 = 0.0;
 #pragma unroll
     for (int k = 0; k < POST_STEPS; k++) {
         const int off = -1 - k;
@@ -175,22 +199,16 @@ __device__ __forceinline__ void stdp_post_prep(const NetDev &n, const StdpConst 
         if (sh == BG3_ULONG_MAX) return;
         const unsigned long long dd = t - (unsigned long long)(long long)total_delay - sh;
         const float delta = (sgn ? (float)(long long)dd : (float)dd) * n.dt;
-        if (delta <= 0.0f || (double)delta >= 3.0 * (double)c.taupos) return;
+        if (delta <= 0.0f || delta >= __fmul_ru(3.0f, c.taupos)) return;
         float epre = 1.0f;
         if (c.useFD) {
             if (off - 1 < -ms) { set_err(n, ERR_STDP_RING); return; }
             const unsigned long long sh2 = hist_get(n, pre, cpre, off - 1, hp);
             if (sh2 == BG3_ULONG_MAX) return;
-            epre = (float)(1.0 - (double)exp_interval(n, sh - sh2, sgn, c.tauspre));
+            epre = 1.0f - exp_interval(n, sh - sh2, sgn, c.tauspre);
         }
-        double inc;
-        if (stdp_inc(c, delta, epost, epre, (long long)dd, inc)) {
-            q.mask |= 1 << k;
-            if (k == 0) q.inc0 = inc;
-            else if (k == 1) q.inc1 = inc;
-            else if (k == 2) q.inc2 = inc;
-            else q.inc3 = inc;
-        }
+        q.epre[k] = epre;
+        if (stdp_dw(c, delta, (long long)dd, q.dw[k])) q.mask |= 1 << k;
     }
     q.next = -1 - POST_STEPS;
 }
@@ -205,10 +223,9 @@ __device__ __forceinline__ float stdp_post_finish(const NetDev &n, const StdpCon
                                                   int pre, int total_delay, unsigned long long t,
                                                   const PostPrep &q)
 {
-    if (q.mask & 1) W = stdp_apply(c, W, q.inc0);
-    if (q.mask & 2) W = stdp_apply(c, W, q.inc1);
-    if (q.mask & 4) W = stdp_apply(c, W, q.inc2);
-    if (q.mask & 8) W = stdp_apply(c, W, q.inc3);
+#pragma unroll
+    for (int k = 0; k < POST_STEPS; k++)
+        if ((q.mask >> k) & 1) W = stdp_apply(c, W, q.epost, q.epre[k], q.dw[k]);
     if (!q.next) return W;
     const int ms = n.max_spikes;
     const bool sgn = n.stdp_signed != 0;
@@ -218,13 +235,13 @@ __device__ __forceinline__ float stdp_post_finish(const NetDev &n, const StdpCon
         if (sh == BG3_ULONG_MAX) break;
         const unsigned long long dd = t - (unsigned long long)(long long)total_delay - sh;
         const float delta = (sgn ? (float)(long long)dd : (float)dd) * n.dt;
-        if (delta <= 0.0f || (double)delta >= 3.0 * (double)c.taupos) break;
+        if (delta <= 0.0f || delta >= __fmul_ru(3.0f, c.taupos)) break;
         float epre = 1.0f;
         if (c.useFD) {
             if (off - 1 < -ms) { set_err(n, ERR_STDP_RING); break; }
             const unsigned long long sh2 = hist_at(n, pre, q.cpre, off - 1);
             if (sh2 == BG3_ULONG_MAX) break;
-            epre = (float)(1.0 - (double)exp_interval(n, sh - sh2, sgn, c.tauspre));
+            epre = 1.0f - exp_interval(n, sh - sh2, sgn, c.tauspre);
         }
         W = stdp_learn(c, W, delta, q.epost, epre, (long long)dd);
     }
