@@ -592,75 +592,42 @@ __device__ __forceinline__ FF ff_fast_two_sum(float a, float b)  // |a| >= |b| o
     const float s = a + b;
     return FF{s, b - (s - a)};
 }
-__device__ __forceinline__ FF ff_add_f(FF a, float b)
-{
-    FF s = ff_two_sum(a.hi, b);
-    s.lo = s.lo + a.lo;
-    return ff_fast_two_sum(s.hi, s.lo);
-}
-__device__ __forceinline__ FF ff_mul_f(FF a, float b)
-{
-    const float p = a.hi * b;
-    float e = __fmaf_rn(a.hi, b, -p);
-    e = __fmaf_rn(a.lo, b, e);
-    return ff_fast_two_sum(p, e);
-}
-// Rounds a float-float value to float when no rounding boundary lies within err of it.
-__device__ __forceinline__ bool ff_round(FF a, float err, float &out)
-{
-    const uint32_t m = __float_as_uint(a.hi) & 0x7fffffffu;
-    if (m < 0x00800001u || m >= 0x7f000000u || !(err < 1e30f)) return false;  // tiny, huge, NaN
-    const float up = __uint_as_float(m + 1u) - __uint_as_float(m);    // gap above |hi|
-    const float dn = __uint_as_float(m) - __uint_as_float(m - 1u);    // gap below |hi|
-    const bool neg = (__float_as_uint(a.hi) >> 31) != 0u;
-    // distances from hi + lo to the midpoints above and below hi (on the real line)
-    const float half_hi = 0.5f * (neg ? dn : up), half_lo = 0.5f * (neg ? up : dn);
-    if (half_hi - a.lo <= err || half_lo + a.lo <= err) return false;
-    out = a.hi;
-    return true;
-}
 
 // (float)(v + C3 (0.04 v v + (double)(5 v) + 140 - u)) and (float)((double)Vb * 0.001 + c2sp)
 // as izh_v_fp64 computes them, from float-float arithmetic: the constants 0.04 and 0.001 as
-// three floats (exact to ~2^-72); every operation of the chain adds at most ~2^-46 of the
-// magnitudes it combines and the reference's seven double roundings ~2^-53 each, so
+// two floats (to ~2^-49); every operation of the chain adds at most ~2^-46 of the magnitudes it
+// combines and the reference's seven double roundings ~2^-53 each, so
 // E = 2^-40 x (|C3| x M + |Vb|), M = 0.04 v^2 + 5 |v| + 140 + |u|, bounds the distance to the
-// reference's double with a wide margin (and likewise for the second expression).
+// reference's double with a wide margin (and likewise for the second expression).  The low parts
+// are only added up, never made small against the high ones again: the last sums round hi + lo -+ E
+// whatever lo's size, and agree where the rounding is certain.  (With every intermediate value made
+// canonical, and the distance to the rounding boundaries taken from the bits, twice the
+// instructions; a 90x90 network's step is a chain of them.)
 __device__ __forceinline__ float izh_v_ff(float Vint, float u, float C3, float c2sp, bool &ok)
 {
-    // the double constants split into three floats each (their sum is the double exactly)
-    constexpr float K04H = (float)0.04, K04M = (float)(0.04 - (double)K04H),
-                    K04L = (float)(0.04 - (double)K04H - (double)K04M);
-    constexpr float K001H = (float)0.001, K001M = (float)(0.001 - (double)K001H),
-                    K001L = (float)(0.001 - (double)K001H - (double)K001M);
-    ok = true;
-    if (!(fabsf(Vint) < 1e4f) || !(fabsf(u) < 1e4f) || !(fabsf(C3) < 1e4f) || !(fabsf(c2sp) < 1e4f)) {
-        ok = false;
-        return 0.0f;
-    }
-    FF t = ff_mul_f(FF{K04H, K04M}, Vint);
-    t.lo = __fmaf_rn(K04L, Vint, t.lo);
-    t = ff_mul_f(t, Vint);
+    constexpr float K04H = (float)0.04, K04M = (float)(0.04 - (double)K04H);
+    constexpr float K001H = (float)0.001, K001M = (float)(0.001 - (double)K001H);
+    // 0.04 v v = p + e
+    const float a = K04H * Vint, ae = __fmaf_rn(K04M, Vint, __fmaf_rn(K04H, Vint, -a));
+    const float p = a * Vint, e = __fmaf_rn(ae, Vint, __fmaf_rn(a, Vint, -p));
     const float v5 = 5.0f * Vint;
-    t = ff_add_f(t, v5);
-    t = ff_add_f(t, 140.0f);
-    t = ff_add_f(t, -u);
-    t = ff_mul_f(t, C3);
-    t = ff_add_f(t, Vint);
+    const FF s1 = ff_two_sum(v5, 140.0f), s2 = ff_two_sum(p, -u), s3 = ff_two_sum(s1.hi, s2.hi);
+    const float lo = (s1.lo + s2.lo) + (s3.lo + e);
+    const float q = s3.hi * C3, qe = __fmaf_rn(lo, C3, __fmaf_rn(s3.hi, C3, -q));
+    const FF t = ff_two_sum(Vint, q);
+    const float tl = t.lo + qe;
     const float M = 0.04f * Vint * Vint + fabsf(v5) + 140.0f + fabsf(u);
-    float Vb;
-    if (!ff_round(t, (fabsf(C3) * M + fabsf(t.hi)) * 0x1p-40f, Vb)) {
-        ok = false;
-        return 0.0f;
-    }
-    FF w = ff_mul_f(FF{K001H, K001M}, Vb);
-    w.lo = __fmaf_rn(K001L, Vb, w.lo);
-    w = ff_add_f(w, c2sp);
-    float Vnew;
-    if (!ff_round(w, (fabsf(Vb) * 0.001f + fabsf(c2sp)) * 0x1p-40f, Vnew)) {
-        ok = false;
-        return 0.0f;
-    }
+    const float err = (fabsf(C3) * M + fabsf(t.hi)) * 0x1p-40f;
+    const float Vb = t.hi + (tl + err);
+    ok = Vb == t.hi + (tl - err);  // false for NaN
+    const float r = K001H * Vb, re = __fmaf_rn(K001M, Vb, __fmaf_rn(K001H, Vb, -r));
+    const FF w = ff_two_sum(r, c2sp);
+    const float wl = w.lo + re, werr = (fabsf(Vb) * 0.001f + fabsf(c2sp)) * 0x1p-40f;
+    const float Vnew = w.hi + (wl + werr);
+    ok = ok && Vnew == w.hi + (wl - werr);
+    // sizes far from float's limits, so that no low part is lost
+    ok = ok && fmaxf(fmaxf(fabsf(Vint), fabsf(u)), fmaxf(fabsf(C3), fabsf(c2sp))) < 1e4f &&
+         fminf(err, werr) > 1e-30f;
     return Vnew;
 }
 
