@@ -155,7 +155,7 @@ static int d2h(bg3_net *n, T *dst, const T *src, size_t count)
 
 // ---- downloads through pinned memory -----------------------------------------------------------
 // A copy to pageable memory waits for itself, about 10 us each; a download of several small arrays
-// queues its copies into one pinned buffer instead, waits once and hands them out.  The buffers are
+// has them written to one pinned buffer instead, waits once and hands them out.  The buffers are
 // shared by all networks of the process (a download holds one for its duration, under no lock):
 // at most STAGE_KEEP of STAGE_BYTES each stay allocated between downloads, and they are freed
 // with the last network.
@@ -202,49 +202,77 @@ static void stage_put(void *p)
     cudaFreeHost(p);
 }
 
-// One download: add() queues arrays, finish() waits for the stream and fills the destinations.  What
-// does not fit the buffer is copied straight to its destination.
+// The arrays of one download, written to pinned memory by the device: one launch for all of them.  A
+// copy each costs 5 to 6 us whatever its size (five arrays of 100 or of 4,225 neurons: 41 us with the
+// wait, in one launch 34); their bytes are next to nothing.
+constexpr int FETCH_PARTS = 16;  // the neuron arrays are 13
+struct FetchList {
+    struct Part {
+        const char *src;
+        char *dst;
+        uint32_t bytes;  // a multiple of four
+    } part[FETCH_PARTS];
+};
+constexpr uint32_t FETCH_BLOCK = 256 * 16 * 2;  // bytes a block takes of a part
+static __global__ void __launch_bounds__(256) k_fetch(const __grid_constant__ FetchList l)
+{
+    const char *src = l.part[blockIdx.y].src;
+    char *dst = l.part[blockIdx.y].dst;
+    const uint32_t bytes = l.part[blockIdx.y].bytes, end = min(bytes, (blockIdx.x + 1) * FETCH_BLOCK);
+    uint32_t at = blockIdx.x * FETCH_BLOCK;
+    if (((uintptr_t)src & 15u) == 0) {  // the staging places are aligned
+        for (uint32_t k = at + threadIdx.x * 16; k + 16 <= end; k += blockDim.x * 16)
+            *(uint4 *)(dst + k) = *(const uint4 *)(src + k);
+        at = max(at, end & ~15u);
+    }
+    for (uint32_t k = at + threadIdx.x * 4; k < end; k += blockDim.x * 4)
+        *(uint32_t *)(dst + k) = *(const uint32_t *)(src + k);
+}
+
+// One download: add() notes arrays, finish() fetches them, waits for the stream and fills the
+// destinations.  What does not fit the buffer is copied straight to its destination.
 class Fetch {
   public:
     explicit Fetch(bg3_net *net) : n(net) {}
     ~Fetch()
     {
-        if (!buf) return;
-        if (used) cudaStreamSynchronize(n->stream);  // left early: copies may be in flight
-        stage_put(buf);
+        if (buf) stage_put(buf);
     }
     template <typename T>
     int add(T *dst, const T *src, size_t count)
     {
+        static_assert(sizeof(T) % 4 == 0, "k_fetch copies words");
         if (!dst || !count) return BG3_OK;
         const size_t bytes = count * sizeof(T), room = (bytes + 15) & ~(size_t)15;
         if (room <= STAGE_BYTES - used && !buf) buf = stage_get();
-        if (!buf || room > STAGE_BYTES - used || np == MAX_PARTS) return d2h(n, dst, src, count);
-        CK(cudaMemcpyAsync((char *)buf + used, src, bytes, cudaMemcpyDeviceToHost, n->stream));
-        parts[np++] = Part{(void *)dst, used, bytes};
+        if (!buf || room > STAGE_BYTES - used || np == FETCH_PARTS) return d2h(n, dst, src, count);
+        list.part[np] = {(const char *)src, (char *)buf + used, (uint32_t)bytes};
+        to[np++] = dst;
+        most = std::max(most, (uint32_t)bytes);
         used += room;
         return BG3_OK;
     }
     int finish()
     {
+        if (np) {
+            k_fetch<<<dim3((most + FETCH_BLOCK - 1) / FETCH_BLOCK, np), 256, 0, n->stream>>>(list);
+            CK(cudaGetLastError());
+        }
         CK(cudaStreamSynchronize(n->stream));
-        for (int i = 0; i < np; i++) memcpy(parts[i].dst, (const char *)buf + parts[i].at, parts[i].bytes);
+        for (int i = 0; i < np; i++) memcpy(to[i], list.part[i].dst, list.part[i].bytes);
         np = 0;
         used = 0;
         return BG3_OK;
     }
 
   private:
-    struct Part {
-        void *dst;
-        size_t at, bytes;
-    };
-    static constexpr int MAX_PARTS = 16;  // the neuron arrays are 13
     bg3_net *n;
     void *buf = nullptr;
     size_t used = 0;
+    uint32_t most = 0;
     int np = 0;
-    Part parts[MAX_PARTS];
+    FetchList list;
+    void *to[FETCH_PARTS];
 };
 
 static void drop_graph(bg3_net *n)
