@@ -246,7 +246,7 @@ struct ThinSmem {           // Mq here: thin_quads; zero beyond the last in use
 };
 
 // A lane's arrivals in the block are made ready before the steps run, so that their chains of loads
-// (the source's mask, the event slot, the exp tables) overlap, across the warp's lanes and four
+// (the source's mask, the event slot, the exp tables) overlap, across the warp's lanes and two
 // rows at a time: the steps and the psr increments in shared memory.  Two spikes at one synapse, and
 // STDP arrivals whose weight the learning walk could change, run at their step (thin_late).
 struct ThinEvents {
@@ -271,7 +271,7 @@ __device__ __forceinline__ void thin_events(const NetDev &n, const BlkDev &b, co
 {
     const int lane = threadIdx.x & 31;
     constexpr bool DS = SYN == 1 || SYN == 3;
-    constexpr int U = 4;
+    constexpr int U = 2;  // four: 3 % more a step on every network timed, 2,000 to 38,000 neurons
     // STDP: a walk that finds the ring full sets an error bit; where the ring may fill within the
     // block, at its step
     bool ring_late = false;
@@ -1473,6 +1473,10 @@ __device__ __forceinline__ void dense_events(const NetDev &n, const BlkDev &b, D
         used++;
         uint32_t any = 0u;  // bit q: quad q has an arrival; 16: a row has several
         if (some) {
+            // Four masks and two arrivals in flight a lane.  The unrolled code runs in full while any lane
+            // has a hit left: with one and one 10,000 neurons at 0.8 Hz take 57 us a block instead of 64,
+            // but 32,400 at 300 Hz 488 instead of 420; four and four cost both a third; both forms, by
+            // the group's hits, gain nothing (63, 444).
             uint8_t *mb = reinterpret_cast<uint8_t *>(&s.bmsk[w][0][lane]);  // row r: mb[128 (r / 4) + r % 4]
             const uint8_t *lb = reinterpret_cast<const uint8_t *>(&s.lc[w][st][0][lane]);
             const int *sb = reinterpret_cast<const int *>(&s.src[w][st][0][lane]);
