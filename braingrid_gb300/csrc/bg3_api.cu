@@ -1207,6 +1207,7 @@ int bg3_download_poisson(bg3_net *n, bg3_poisson_arrays *a)
 }
 
 // ---- hot path -------------------------------------------------------------------------------
+// Blocks of steps (bg3_block.cu) where blk_steps allows them; otherwise step by step.
 // Device-noise mode: neurons(t0), then per step deliver + sweep whose epilogue integrates the
 // next step's neurons, the last sweep without that epilogue.  Runs of interior steps replay a
 // CUDA graph of GRAPH_STEPS (deliver, fused sweep) pairs.  Injected-noise mode: neurons,

@@ -1,4 +1,7 @@
-// Per-step kernels of the spiking hot path.
+// Per-step kernels of the spiking hot path.  Most calls run blocks of steps instead (bg3_block.cu); these
+// remain for delays of less than two steps, injected noise in networks too large for one cluster, dense
+// networks with STDP, the device build's spike-time arithmetic, launch options that ask for them, and the
+// measurement of single steps.
 //
 // One simulation step t on the network's stream:
 //   k_deliver    (t)  spike arrival: for every delay class D, the neurons that fired at step
@@ -1047,7 +1050,9 @@ __global__ void __launch_bounds__(1024) k_sweep_thin_batch(const NetDev *nets, c
 
 bool sweep_is_thin(const NetDev &h, const LaunchCfg &c) { return h.Mq <= c.thin_max_quads; }
 
-// ---- small networks: many steps per launch ----------------------------------------------------
+// ---- small networks: many steps per launch, step by step ---------------------------------------
+// For what k_blk_small (bg3_block.cu) does not take: delays of less than two steps, the device build's
+// spike-time arithmetic, rows too wide for its shared memory.
 // A network of at most SMALL_MAX_N neurons whose synapse planes hold at most the launch
 // configuration's small_max_slots slots is advanced by one CTA through many steps in one launch.
 // Each step runs the passes of a bg3_step call in their order — the neuron pass (device noise as

@@ -431,8 +431,8 @@ typedef struct {
                                  way.                                                                 */
     int32_t small_max_slots;  /* a network of at most 2,048 neurons whose synapse planes hold at most
                                  this many slots (neurons rounded up to 32 x max synapses rounded up
-                                 to 4) runs up to 4,096 whole steps per launch on one CTA, with no
-                                 launch between its passes (default 65,536; 0: never, and no network
+                                 to 4) runs up to 4,096 whole steps per launch in one cluster of up
+                                 to eight CTAs, with no launch between its passes (default 65,536; 0: never, and no network
                                  runs several steps per launch: the per-step kernels).  Same results
                                  either way.                                                        */
 } bg3_launch_cfg;
