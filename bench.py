@@ -591,8 +591,9 @@ def run_growth():
            # evaluates the lens area with 2 acos and 2 sin
            "grown_transcendental_calls": 4 * S,
            "grown_transcendentals_per_s": 4 * S / t_update,
-           "grown_bound": "fp64 (acos and sin of the overlap area evaluated in double; "
-                          "86 % FP64-pipe busy, profiles/k_growth_plain.md)",
+           "grown_bound": "instruction issue of the overlap areas (float-float with certified "
+                          "rounding), scattered writes of the outgoing map "
+                          "(profiles/blocks_of_steps.md)",
            "error_word": err}
     N2, r2, c2, u2, S2, e2 = _growth_passes(200, 200, RADIUS)
     out["served_largest_200x200"] = {
