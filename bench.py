@@ -592,8 +592,7 @@ def run_growth():
            "grown_transcendental_calls": 4 * S,
            "grown_transcendentals_per_s": 4 * S / t_update,
            "grown_bound": "instruction issue of the overlap areas (float-float with certified "
-                          "rounding), scattered writes of the outgoing map "
-                          "(profiles/blocks_of_steps.md)",
+                          "rounding), scattered writes of the outgoing map",
            "error_word": err}
     N2, r2, c2, u2, S2, e2 = _growth_passes(200, 200, RADIUS)
     out["served_largest_200x200"] = {

@@ -17,8 +17,12 @@ namespace bg3 {
 // co = spikeCount + spikeCountOffset.
 __device__ __forceinline__ unsigned long long hist_at(const NetDev &n, int i, int co, int off)
 {
-    int x = co + n.max_spikes + off;  // below 3 max_spikes unless the ring has overflowed
-    while (x >= n.max_spikes) x -= n.max_spikes;
+    // below 3 max_spikes unless the ring has overflowed: no remainder for what two comparisons do
+    const int ms = n.max_spikes;
+    int x = co + ms + off;
+    if (x >= ms) x -= ms;
+    if (x >= ms) x -= ms;
+    if (x >= ms) x %= ms;
     return n.history[(size_t)i * n.max_spikes + x];
 }
 
