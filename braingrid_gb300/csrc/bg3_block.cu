@@ -20,7 +20,7 @@
 // Three forms: thin networks (k_blk_thin, up to 64 slots per neuron), small networks, whose launch
 // runs thousands of steps in one cluster (k_blk_small), and dense ones (k_blk_push, k_blk_dense).
 // A step, in the per-step kernels and here: 90x90 Izhikevich with STDP 13.9 and 2.6 us; 100x100 without
-// synapses 4.1 and 0.74; 30x30 LIF with STDP at 3 Hz 8.3 and 1.6; 100x100 with 7.6 M synapses 14 and 6
+// synapses 4.3 and 0.75; 30x30 LIF with STDP at 3 Hz 8.3 and 1.6; 100x100 with 7.6 M synapses 14 and 6
 // to 8; 180x180 with 23 M at 300 Hz 87 and 55.
 #include <cuda.h>
 #include <algorithm>
