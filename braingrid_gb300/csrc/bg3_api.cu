@@ -1248,7 +1248,9 @@ static int blk_steps(const bg3_net *n, const LaunchCfg &c, bool small = false)
     if (c.small_max_slots == 0 || (h.noise_mode != BG3_NOISE_DEVICE && !small)) return 0;
     if (small) {
         if (!bg3::blk_small_ok(h)) return 0;
-    } else if (!blk_is_thin(h, c) && (h.syn_kind >= BG3_SYN_STDP || !bg3::blk_dense_ok(h.Mq))) {
+    } else if (!blk_is_thin(h, c) && (h.syn_kind >= BG3_SYN_STDP || !n->blk.actn)) {
+        // by width alone a network has the dense blocks' planes or it has not: thin_max_quads below the
+        // width of one that could run thin blocks asks for the TMA sweep, which is a per-step kernel
         return 0;
     }
     if (h.syn_kind >= BG3_SYN_STDP) {

@@ -224,3 +224,35 @@ def test_small_network_blocks_draw_injected_noise(syn, w, h, radius, max_syn, st
     assert (nets[0].error_word != 0) == (steps < sum(STEPS))
     for net in nets:
         net.close()
+
+
+def test_narrow_network_below_the_thin_option():
+    """thin_max_quads below the width of a network that could run thin blocks (10 row quads): the
+    per-step kernels, set by the caller, in a batch, from a checkpoint and by the tuner."""
+    def make():
+        return lif(50, 42, bg.BG3_SYN_DS, 1.55, "poisson", 40)
+    want, a, b, c = make(), make(), make(), make()
+    want.set_launch(small_max_slots=0)
+    a.set_launch(thin_max_quads=1)
+    batch = bg.Batch([b])
+    batch.set_launch(thin_max_quads=9)
+    for n in STEPS:
+        want.step(n)
+        a.step(n)
+        batch.step(n)
+    batch.sync()
+    same(a, want, "set by the caller")
+    same(b, want, "in a batch")
+    batch.close()
+    c.load_checkpoint(a.checkpoint())
+    assert c.launch["thin_max_quads"] == 1
+    for net in (c, want):
+        net.step(41)
+    same(c, want, "from a checkpoint")
+    cfg, ms = c.autotune(steps_per_trial=40)
+    assert ms > 0
+    same(c, want, "after tuning")
+    for net in (c, want):
+        net.step(30)
+    same(c, want, "with the tuned launch")
+    assert int(want.download_lif(fields=("spikeCount",))["spikeCount"].sum()) > 0
