@@ -1806,6 +1806,13 @@ struct bg3_batch {
     LaunchCfg cfg = LAUNCH_DEFAULT;
 };
 
+static void batch_drop_graph(bg3_batch *b)
+{
+    if (b->graph) cudaGraphExecDestroy(b->graph);
+    b->graph = nullptr;
+    b->graph_steps = 0;
+}
+
 static int batch_refresh(bg3_batch *b)
 {
     std::vector<NetDev> hd;
@@ -1870,8 +1877,7 @@ static int batch_refresh(bg3_batch *b)
     if (b->n_dense)
         CK(cudaMemcpyAsync(b->d_dense, dense.data(), dense.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     CK(cudaStreamSynchronize(b->stream));
-    if (b->graph) cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
+    batch_drop_graph(b);
     return BG3_OK;
 }
 
@@ -1925,7 +1931,7 @@ int bg3_batch_destroy(bg3_batch *b)
 {
     if (!b) return BG3_EINVAL;
     if (b->stream) cudaStreamSynchronize(b->stream);
-    if (b->graph) cudaGraphExecDestroy(b->graph);
+    batch_drop_graph(b);
     if (b->d_nets) cudaFree(b->d_nets);
     if (b->d_maps) cudaFree(b->d_maps);
     if (b->d_blks) cudaFree(b->d_blks);
@@ -1956,13 +1962,6 @@ static void batch_interior(bg3_batch *b, int64_t n)
         bg3::launch_sweep_batch(b->d_nets, b->d_maps, b->d_tiles, b->n_thick, b->ntiles - b->n_thick, true, b->cfg, b->stream);
         bg3::launch_deliver_batch(b->syn_kind, b->d_nets, (int)b->nets.size(), b->cfg, b->stream);
     }
-}
-
-static void batch_drop_graph(bg3_batch *b)
-{
-    if (b->graph) cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-    b->graph_steps = 0;
 }
 
 // Steps per block when every member runs in blocks (the fewest of any), else 0.
@@ -2481,8 +2480,7 @@ int bg3_batch_autotune(bg3_batch *b, int32_t steps, bg3_launch_cfg *best, float 
                            b->cfg.izh_hw_every != c.izh_hw_every;
         b->cfg = c;
         if (split && batch_refresh(b) != BG3_OK) return -1.0f;
-        if (b->graph) cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
+        batch_drop_graph(b);
         return time_batch_steps(b, steps);
     };
     float ms = 0.0f;

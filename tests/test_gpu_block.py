@@ -256,3 +256,26 @@ def test_narrow_network_below_the_thin_option():
         net.step(30)
     same(c, want, "with the tuned launch")
     assert int(want.download_lif(fields=("spikeCount",))["spikeCount"].sum()) > 0
+
+
+def test_batch_graphs_of_the_two_forms_are_told_apart():
+    """Blocks, a refresh, a run of single steps long enough for a graph of them (a member that
+    draws injected noise keeps its batch off the blocks), and blocks again without a refresh."""
+    shapes = [(40, 33, 3.4, 190), (33, 31, 1.9, 64)]
+    a, b = ([lif(w, h, bg.BG3_SYN_DS, r, "none", m) for w, h, r, m in shapes] for _ in range(2))
+    for net in b:
+        net.set_launch(small_max_slots=0)
+    batch = bg.Batch(a)
+    batch.step(130)
+    batch.refresh()
+    a[0].set_noise_mode(bg.BG3_NOISE_INJECT, 5)
+    b0 = batch.launches
+    batch.step(40)
+    assert batch.launches - b0 > 40
+    a[0].set_noise_mode(bg.BG3_NOISE_DEVICE, 5)
+    batch.step(300)
+    batch.sync()
+    for net, other in zip(a, b):
+        other.step(470)
+        same(net, other, "batched")
+    batch.close()
