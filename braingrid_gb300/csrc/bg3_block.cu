@@ -1724,14 +1724,15 @@ void launch_blk_ring(const NetDev &h, const BlkDev &b, cudaStream_t s)
 }
 
 // Blocks, tiles per block and warps per tile of a small network's launch; 0 blocks when it does not fit
-// a cluster of eight (200 KB of shared memory per block).
+// a cluster of eight (SMALL_SMEM of shared memory per block).
+constexpr size_t SMALL_SMEM = 200 * 1024;
 struct SmallShape {
     int blocks, tiles, team;
 };
 static SmallShape small_shape(const NetDev &h)
 {
     SmallShape s = {0, h.ntiles <= 32 ? std::min(4, h.ntiles) : BLK_THIN_WARPS, 1};
-    s.tiles = (int)std::min<size_t>(s.tiles, 200 * 1024 / blk_thin_smem(h.Mq, BLK_TEAM, false));
+    s.tiles = (int)std::min<size_t>(s.tiles, SMALL_SMEM / blk_thin_smem(h.Mq, BLK_TEAM, false));
     if (s.tiles < 1) return s;
     s.team = std::min(BLK_TEAM, BLK_THIN_WARPS / s.tiles);
     s.blocks = (h.ntiles + s.tiles - 1) / s.tiles;
@@ -1745,7 +1746,9 @@ static void launch_small_t(const NetDev &h, const BlkDev &b, int nsteps, int T, 
 {
     const SmallShape p = small_shape(h);
     const size_t sm = (size_t)p.tiles * blk_thin_smem(h.Mq, p.team, false);
-    cudaFuncSetAttribute(k_blk_small<SYN, INJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    // the most any network takes, not this one's: the limit belongs to the kernel, and another thread's
+    // wider network may be between this call and its launch
+    cudaFuncSetAttribute(k_blk_small<SYN, INJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SMEM);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;

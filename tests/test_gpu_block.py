@@ -2,6 +2,8 @@
 advanced by both (small_max_slots 0 keeps a network on the per-step kernels, 1 keeps it off the
 one-launch path of small networks, 65,536 takes that path where it is small enough), at sizes around the 32-neuron tiles, the row quads and the
 eight steps of a block, with downloads, epoch ends and single steps in between."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -279,3 +281,30 @@ def test_batch_graphs_of_the_two_forms_are_told_apart():
         other.step(470)
         same(net, other, "batched")
     batch.close()
+
+
+def test_small_networks_of_several_threads():
+    """A narrow and a wide small network stepped at the same time by two threads: every launch is
+    accepted, and each network ends as it does alone."""
+    shapes = [(10, 10, 1.5, 30), (13, 5, 4.0, 301)]    # 8 and 76 row quads
+    nets, alone = ([lif(w, h, bg.BG3_SYN_DS, r, "poisson", m) for w, h, r, m in shapes] for _ in range(2))
+    errors, start = [], threading.Barrier(len(nets))
+
+    def run(net):
+        try:
+            start.wait()
+            for _ in range(3000):
+                net.step(1)
+            net.sync()
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=run, args=(net,)) for net in nets]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for net, other in zip(nets, alone):
+        other.step(3000)
+        same(net, other, "stepped beside another")
