@@ -13,17 +13,21 @@ namespace bg3 {
 // the device.  Each float / double operation rounds as in the reference; the exp factors come
 // from the host library's tables.
 
-// getSpikeHistory (Neurons/AllSpikingNeurons.cpp:182-188) for off in [-max_spikes, -1];
-// co = spikeCount + spikeCountOffset.
-__device__ __forceinline__ unsigned long long hist_at(const NetDev &n, int i, int co, int off)
+// getSpikeHistory (Neurons/AllSpikingNeurons.cpp:182-188) for off in [-max_spikes, -1]; co = spikeCount +
+// spikeCountOffset.  A ring of one or two entries is asked for -2 and -3 all the same (by walks that
+// need a valid entry there to learn): the first place where that is before the ring.
+__host__ __device__ __forceinline__ int hist_index(int co, int ms, int off)
 {
     // below 3 max_spikes unless the ring has overflowed: no remainder for what two comparisons do
-    const int ms = n.max_spikes;
     int x = co + ms + off;
     if (x >= ms) x -= ms;
     if (x >= ms) x -= ms;
     if (x >= ms) x %= ms;
-    return n.history[(size_t)i * n.max_spikes + x];
+    return x > 0 ? x : 0;
+}
+__device__ __forceinline__ unsigned long long hist_at(const NetDev &n, int i, int co, int off)
+{
+    return n.history[(size_t)i * n.max_spikes + hist_index(co, n.max_spikes, off)];
 }
 
 // W^mu with mu = 0, the only exponent a network accepts (set_stdp_type refuses others)
