@@ -84,10 +84,11 @@ struct bg3_net {
     // whichever ran last is current, the other is rebuilt when it is needed
     BlkDev blk = {};
     bool ring_ok = true, mask_ok = false;
-    // fewest steps between two spikes of a neuron, for the block kernels' STDP ring rule: the
-    // shortest refractory period + 1, or 1 once spike histories were uploaded
+    // fewest steps between two spikes of a neuron in the history rings, for the block kernels' STDP
+    // rule: the shortest refractory period + 1 of any in force while steps were made, or 1 once
+    // histories, or what their spacing follows from, were uploaded beside earlier steps
     int min_isi = 1;
-    bool hist_given = false;
+    bool hist_given = false, stepped = false;
 };
 
 #define CK(x)                                                                            \
@@ -704,7 +705,8 @@ int bg3_destroy(bg3_net *n)
     return BG3_OK;
 }
 
-// Fewest steps between two spikes of any neuron with these refractory periods.
+// Fewest steps between two spikes of any neuron with these refractory periods.  Spikes made with
+// earlier, shorter ones may still be in the rings.
 static void set_min_isi(bg3_net *n, const float *Trefract)
 {
     int m = 1 << 30;
@@ -712,7 +714,7 @@ static void set_min_isi(bg3_net *n, const float *Trefract)
         const double r = (double)(Trefract[i] / n->h.dt) + 0.5;
         m = std::min(m, r > 0.0 && r < 1e9 ? (int)r + 1 : 1);
     }
-    n->min_isi = m;
+    n->min_isi = n->stepped ? std::min(n->min_isi, m) : m;
 }
 
 // The spike ring, brought up to date from the masks (queued on the network's stream).
@@ -748,7 +750,10 @@ int bg3_upload_lif(bg3_net *n, const bg3_lif_arrays *a)
         (rc = h2d(n, (uint64_t *)h.history, a->history, N * (size_t)h.max_spikes)))
         return rc;
     CK(cudaStreamSynchronize(n->stream));
-    if (a->history) n->hist_given = true;
+    // once there are spikes, a neuron whose refractory steps are set anew may fire sooner after its
+    // last one, and other counts put the entries in another order
+    if (a->history || (n->stepped && (a->nStepsInRefr || a->spikeCount || a->spikeCountOffset)))
+        n->hist_given = true;
     if (a->Trefract) set_min_isi(n, a->Trefract);
     return BG3_OK;
 }
@@ -1319,6 +1324,7 @@ static int run_blocks(bg3_net *n, int64_t nsteps, int T)
 static int run_steps(bg3_net *n, int64_t nsteps)
 {
     if (nsteps <= 0) return BG3_OK;
+    n->stepped = true;
     const NetDev &h = n->h;
     int rc;
     const bool small = bg3::small_eligible(h, n->cfg);
@@ -1995,6 +2001,7 @@ static int batch_rings(bg3_batch *b)
         const int rc = ensure_ring(n);
         if (rc) return rc;
         n->mask_ok = false;
+        n->stepped = true;
     }
     return BG3_OK;
 }
@@ -2006,6 +2013,7 @@ static int batch_run_blocks(bg3_batch *b, int64_t nsteps, int T)
     for (size_t k = 0; k < b->nets.size(); k++) {
         if ((rc = ensure_masks(b->nets[k]))) return rc;
         b->nets[k]->ring_ok = false;
+        b->nets[k]->stepped = true;
         same = same && !memcmp(&b->blks[k], &b->nets[k]->blk, sizeof(BlkDev));
     }
     if ((rc = batch_order(b, true))) return rc;
@@ -2113,6 +2121,7 @@ int bg3_bench_steps(bg3_net *n, int64_t nsteps, int64_t flush_bytes, float *step
     const int ring_rc = ensure_ring(n);
     if (ring_rc) return ring_rc;
     n->mask_ok = false;
+    n->stepped = true;
     const NetDev &h = n->h;
     const bool inject = h.noise_mode == BG3_NOISE_INJECT;
     std::vector<cudaEvent_t> ev((size_t)nsteps * 3);
@@ -2844,7 +2853,7 @@ int bg3_checkpoint_load(bg3_net *n, const void *buf, uint64_t len)
     CK(cudaStreamSynchronize(n->stream));
     drop_graph(n);
     ring_changed(n);
-    n->hist_given = true;
+    n->hist_given = n->stepped = true;
 #define BG3_LOAD_ONE(f)                                                                           \
     {                                                                                             \
         if ((rc = aresize(n, h.f, (size_t)as[CKA_##f]))) return rc;                               \

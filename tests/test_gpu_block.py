@@ -308,3 +308,37 @@ def test_small_networks_of_several_threads():
     for net, other in zip(nets, alone):
         other.step(3000)
         same(net, other, "stepped beside another")
+
+
+def firing_at_intervals(steps, max_spikes, seed=7):
+    """65 neurons that fire every `steps` steps, in random phases, on STDP synapses."""
+    spec = netgen.lif_network(13, 5, seed=seed)
+    net = bg.Network(spec["N"], 33, 13, 5, (max_spikes + 0.5) * 1e-3, 1e-4, 1000, 9, bg.BG3_SYN_DYNSTDP,
+                     bg.BG3_NOISE_DEVICE, seed)
+    netgen.configure_lif(net, spec)
+    net.set_stdp_constants(**netgen.STDP_ADDITIVE)
+    netgen.pregrow(net, spec, 1.5, weight_scale=0.3)
+    v = net.download_lif(fields=("Vthresh", "Vreset", "Trefract", "Vm"))
+    v["Vreset"] = v["Vthresh"] + np.float32(1e-3)
+    v["Vm"] = v["Vreset"].copy()
+    v["Trefract"][:] = (steps - 1) * 1e-4
+    v["nStepsInRefr"] = np.random.RandomState(seed).randint(0, steps, spec["N"]).astype(np.int32)
+    net.upload_lif(**v)
+    return net
+
+
+@pytest.mark.parametrize("small", [1, 65536])
+def test_longer_refractory_periods_beside_a_dense_history(small):
+    """Spikes seven steps apart, then a pause longer than the delays (a walk ends at a spike that is
+    still under way): the walks of the next spikes read the 3 tau+ before, to the ring's last entry."""
+    nets = [firing_at_intervals(7, 85) for _ in range(2)]
+    nets[0].set_launch(small_max_slots=small)
+    nets[1].set_launch(small_max_slots=0)
+    for net in nets:
+        for _ in range(4):
+            net.step(190)
+            net.record()
+        net.upload_lif(Trefract=np.full(65, 31e-4, np.float32))
+        net.step(40)
+    same(nets[0], nets[1], "longer periods")
+    assert nets[0].max_spikes == 85
