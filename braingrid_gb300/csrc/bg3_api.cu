@@ -89,6 +89,9 @@ struct bg3_net {
     // histories, or what their spacing follows from, were uploaded beside earlier steps
     int min_isi = 1;
     bool hist_given = false, stepped = false;
+    // STDP kinds: steps until every spike under way that the histories may lack has arrived (it came
+    // with uploaded delay queues, or was under way when the histories were replaced)
+    int queued = 0;
 };
 
 #define CK(x)                                                                            \
@@ -754,6 +757,9 @@ int bg3_upload_lif(bg3_net *n, const bg3_lif_arrays *a)
     // last one, and other counts put the entries in another order
     if (a->history || (n->stepped && (a->nStepsInRefr || a->spikeCount || a->spikeCountOffset)))
         n->hist_given = true;
+    // and the histories given may lack spikes under way
+    if (n->stepped && n->h.syn_kind >= BG3_SYN_STDP && (a->history || a->spikeCount || a->spikeCountOffset))
+        n->queued = 31;
     if (a->Trefract) set_min_isi(n, a->Trefract);
     return BG3_OK;
 }
@@ -849,6 +855,7 @@ int bg3_upload_synapses(bg3_net *n, const bg3_synapse_arrays *a, uint64_t step)
     // fired[s] bit j: neuron s fired at step - 1 - j (j < 32), from the queues
     std::vector<uint32_t> fired(N, 0u);
     uint32_t seenU = 0xffffffffu, seenD = 0xffffffffu, seenF = 0xffffffffu;  // last (U, D, F)
+    int due = 0;  // steps until the last of these spikes arrives
     int seenC = 0;
     for (size_t d = 0; d < N; d++) {
         size_t c = 0;
@@ -898,6 +905,7 @@ int bg3_upload_synapses(bg3_net *n, const bg3_synapse_arrays *a, uint64_t step)
                 int o = (b - di) & 31;
                 if (o >= D || (uint64_t)(D - o) > step) return BG3_EINVAL;  // not a past spike
                 fired[a->src[i]] |= 1u << (D - o - 1);
+                due = std::max(due, o + 1);
             }
         }
     }
@@ -933,6 +941,7 @@ int bg3_upload_synapses(bg3_net *n, const bg3_synapse_arrays *a, uint64_t step)
         (rc = h2d(n, h.ring_n, ring_n.data(), ring_n.size())))
         return rc;
     ring_changed(n);
+    n->queued = h.syn_kind >= BG3_SYN_STDP ? due : 0;
     unsigned long long s64 = step;
     CK(cudaMemcpyAsync(h.step, &s64, sizeof(s64), cudaMemcpyHostToDevice, n->stream));
     CK(cudaMemcpyAsync(h.dstep, &s64, sizeof(s64), cudaMemcpyHostToDevice, n->stream));
@@ -1241,7 +1250,8 @@ static unsigned long long blk_window(const bg3_net *n)
 // for the destination's own spikes), the host build's spike-time arithmetic (its pre-spike walks
 // read only the destination's own history), and a history ring long enough that the spikes a
 // block adds never overwrite an entry a post-spike walk reads (entries within 3 tau+, at most one
-// per min_isi steps).
+// per min_isi steps), and no spike under way that the histories may lack (bg3_net::queued): post-spike
+// learning after a block relies on them to hold the spikes that arrive in it.
 static bool blk_is_thin(const NetDev &h, const LaunchCfg &c)
 {
     return bg3::sweep_is_thin(h, c) && bg3::blk_thin_ok(h.Mq);
@@ -1259,7 +1269,7 @@ static int blk_steps(const bg3_net *n, const LaunchCfg &c, bool small = false)
         return 0;
     }
     if (h.syn_kind >= BG3_SYN_STDP) {
-        if (h.stdp_signed) return 0;
+        if (h.stdp_signed || n->queued > 0) return 0;
         float tau = 0.0f;
         for (const StdpConst &s : h.stdp) tau = std::max(tau, s.taupos);
         if (!(tau >= 0.0f) || !(tau < 1e3f)) return 0;
@@ -1321,7 +1331,7 @@ static int run_blocks(bg3_net *n, int64_t nsteps, int T)
     return BG3_OK;
 }
 
-static int run_steps(bg3_net *n, int64_t nsteps)
+static int run_form(bg3_net *n, int64_t nsteps)
 {
     if (nsteps <= 0) return BG3_OK;
     n->stepped = true;
@@ -1414,10 +1424,20 @@ static int run_steps(bg3_net *n, int64_t nsteps)
     return BG3_OK;
 }
 
+// Steps that bg3_net::queued waits for were made.
+static void steps_made(bg3_net *n, int64_t nsteps)
+{
+    n->queued = (int)std::max<int64_t>(0, n->queued - nsteps);
+}
+
 int bg3_step(bg3_net *n, int64_t nsteps)
 {
     if (!n || nsteps < 0) return BG3_EINVAL;
-    return run_steps(n, nsteps);
+    const int64_t first = std::min<int64_t>(nsteps, n->queued);  // in the form blk_steps gives them
+    int rc = run_form(n, first);
+    if (rc) return rc;
+    steps_made(n, first);
+    return run_form(n, nsteps - first);
 }
 
 int bg3_epoch_growth(bg3_net *n, int32_t epoch)
@@ -2046,10 +2066,9 @@ static int batch_run_blocks(bg3_batch *b, int64_t nsteps, int T)
     return batch_order(b, false);
 }
 
-int bg3_batch_step(bg3_batch *b, int64_t nsteps)
+static int batch_run_form(bg3_batch *b, int64_t nsteps)
 {
-    if (!b || nsteps < 0) return BG3_EINVAL;
-    if (nsteps == 0) return BG3_OK;
+    if (nsteps <= 0) return BG3_OK;
     const int T = batch_blk_steps(b);
     if (T) return batch_run_blocks(b, nsteps, T);
     int rc = batch_rings(b);
@@ -2079,6 +2098,18 @@ int bg3_batch_step(bg3_batch *b, int64_t nsteps)
     b->launches += 1 + (step_kernels(b->syn_kind) - 1 + sweeps) * nsteps;
     CK(cudaGetLastError());
     return batch_order(b, false);
+}
+
+int bg3_batch_step(bg3_batch *b, int64_t nsteps)
+{
+    if (!b || nsteps < 0) return BG3_EINVAL;
+    int64_t first = 0;  // as in bg3_step
+    for (bg3_net *n : b->nets) first = std::max<int64_t>(first, n->queued);
+    first = std::min(first, nsteps);
+    int rc = batch_run_form(b, first);
+    if (rc) return rc;
+    for (bg3_net *n : b->nets) steps_made(n, first);
+    return batch_run_form(b, nsteps - first);
 }
 
 int bg3_batch_sync(bg3_batch *b)
@@ -2122,6 +2153,7 @@ int bg3_bench_steps(bg3_net *n, int64_t nsteps, int64_t flush_bytes, float *step
     if (ring_rc) return ring_rc;
     n->mask_ok = false;
     n->stepped = true;
+    steps_made(n, nsteps);
     const NetDev &h = n->h;
     const bool inject = h.noise_mode == BG3_NOISE_INJECT;
     std::vector<cudaEvent_t> ev((size_t)nsteps * 3);
@@ -2189,6 +2221,7 @@ int bg3_batch_bench_steps(bg3_batch *b, int64_t nsteps, int64_t flush_bytes, flo
     }
     int rc = batch_rings(b);
     if (rc) return rc;
+    for (bg3_net *n : b->nets) steps_made(n, nsteps);
     if ((rc = batch_order(b, true))) return rc;
     const int M = (int)b->nets.size();
     std::vector<cudaEvent_t> ev((size_t)nsteps * 2);
@@ -2305,11 +2338,13 @@ int bg3_batch_set_launch(bg3_batch *b, const bg3_launch_cfg *c)
 struct StateCopy {
     void *buf = nullptr;
     std::vector<std::pair<void *, size_t>> parts;
+    int queued = 0;
 };
 
 static int state_save(bg3_net *n, StateCopy &sc)
 {
     sc.parts.clear();
+    sc.queued = n->queued;
     const int rc = ensure_ring(n);
     if (rc) return rc;
     for (auto &a : n->allocs)
@@ -2335,6 +2370,7 @@ static int state_save(bg3_net *n, StateCopy &sc)
 static int state_load(bg3_net *n, const StateCopy &sc)
 {
     ring_changed(n);
+    n->queued = sc.queued;
     size_t off = 0;
     for (auto &p : sc.parts) {
         CK(cudaMemcpyAsync(p.first, (const char *)sc.buf + off, p.second, cudaMemcpyDeviceToDevice, n->stream));
@@ -2854,6 +2890,7 @@ int bg3_checkpoint_load(bg3_net *n, const void *buf, uint64_t len)
     drop_graph(n);
     ring_changed(n);
     n->hist_given = n->stepped = true;
+    n->queued = n->h.syn_kind >= BG3_SYN_STDP ? 31 : 0;  // saved with uploaded spikes under way, perhaps
 #define BG3_LOAD_ONE(f)                                                                           \
     {                                                                                             \
         if ((rc = aresize(n, h.f, (size_t)as[CKA_##f]))) return rc;                               \

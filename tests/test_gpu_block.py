@@ -342,3 +342,35 @@ def test_longer_refractory_periods_beside_a_dense_history(small):
         net.step(40)
     same(nets[0], nets[1], "longer periods")
     assert nets[0].max_spikes == 85
+
+
+@pytest.mark.parametrize("form", [1, 65536, "batch"])
+def test_spikes_put_in_the_delay_queues(form):
+    """Spikes on their way that no history holds: an upload adds them to the delay queues.  A post
+    spike before such an arrival learns from the source's older spikes, and the arrival has the new
+    weight."""
+    nets = [firing_at_intervals(41, 85) for _ in range(2)]
+    nets[0].set_launch(small_max_slots=1 if form == "batch" else form)
+    nets[1].set_launch(small_max_slots=0)
+    batch = bg.Batch(nets[:1]) if form == "batch" else None
+    added = 0
+    for net in nets:
+        run = batch if batch and net is nets[0] else net
+        run.step(200)
+        for _ in range(6):
+            syn = net.download_synapses()
+            used = syn["in_use"].astype(bool)
+            # the sources without a spike under way: one at the last step, of every second of them
+            busy = np.unique(syn["src"][used & (syn["delayQueue"] != 0)])
+            put = used & ~np.isin(syn["src"], busy) & (syn["src"] % 2 == 0)
+            bit = (syn["delayIdx"] + syn["total_delay"] - 1) & 31
+            syn["delayQueue"][put] |= (np.uint32(1) << bit[put].astype(np.uint32))
+            added += int(put.sum())
+            net.upload_synapses(net.sim_step, **syn)
+            if batch and net is nets[0]:
+                batch.refresh()
+            run.step(23)
+    assert added > 0
+    same(nets[0], nets[1], "spikes added")
+    if batch:
+        batch.close()
