@@ -872,9 +872,9 @@ __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 1) k_blk_small(const __gr
 // block's steps while it is there.
 //   warp 0        issues the loads; then, lane = destination, runs the neurons' steps as the sums
 //                 come in
-//   warps 1-4     arrivals: find the rows whose source has a spike arriving, prepare the psr
+//   warps 1-W     arrivals: find the rows whose source has a spike arriving, prepare the psr
 //                 increments (event slots, exp tables), draw the neurons' noise
-//   warp 5        lane = destination, rows in slot order: carries a chunk through the block's steps
+//   warp W + 1    lane = destination, rows in slot order: carries a chunk through the block's steps
 //                 and stores it back.  A row is a chain of multiplications by its decay; a step's sum
 //                 is a chain of additions over the rows, in the reference's order; the steps
 //                 interleave eight such chains.
@@ -884,7 +884,7 @@ __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 1) k_blk_small(const __gr
 //           step masks in a plane of one byte per slot, increments beside the slots' event state, and
 //           a flag per 16 rows.  The arrival warps only collect the flagged rows.
 //   heavy   the arrival warps look up every slot's source in the spike masks and make the increments.
-// Either way 16 rows at a time, by the four warps in turn, into one of four buffers of step masks and
+// Either way 16 rows at a time, by the W warps in turn, into one of W buffers of step masks and
 // increments that the sum warp reads; groups of 16 rows without an arrival take code that reads none.
 // Why two: a pushed arrival costs half a dozen scattered accesses with the whole GPU to hide them, and
 // reads no sources; a pulled one is found among its neighbours in the slot planes, and costs a pass
@@ -892,40 +892,47 @@ __global__ void __launch_bounds__(32 * BLK_THIN_WARPS, 1) k_blk_small(const __gr
 constexpr int DN_ROWS = 64, DN_QUADS = 16;
 constexpr int DN_STAGES = 4;
 constexpr int DN_MAX_CHUNKS = 32;   // 2,048 slots per destination
-constexpr int DN_BUFS = 4;
 constexpr int DN_GROUP_WORDS = 4 * DN_MAX_CHUNKS / 32;
 constexpr int DN_LIGHT = 128;
 constexpr int DN_ACT_WORDS = 1280;  // the bitmap row is kept in shared memory up to 40,960 neurons
-constexpr int DN_EV_WARPS = 4;      // = DN_BUFS: buffer k is filled by warp k
-constexpr int DN_THREADS = 32 * (1 + DN_EV_WARPS + 1);
+constexpr int dn_threads(int W) { return 32 * (1 + W + 1); }
+// Arrival warps a tile, and the blocks an SM then holds: 16, 8 or 4 warps by the tiles there are, one wave
+// of them in each form.  A heavy block's arrivals are chains of loads, and with four warps on an SM of
+// their own one tile's chains took longer than the per-step kernels, which spread them over the GPU.  160
+// steps at 200 to 320 Hz, up to 920 rows a neuron, us with 4 warps, with this choice and step by step:
+// 33x33 (35 tiles) 2782, 1327, 1674; 45x45 2879, 1349, 2259; 60x60 (113) 3052, 1389, 2777; 80x80 (200,
+// eight warps) 3186, 2160, 3599; 100x100 (313, four) 3502, 3524, 4462.
+constexpr int dn_blocks(int W) { return W == 4 ? 3 : W == 8 ? 2 : 1; }
 constexpr uint32_t DN_CHUNK = DN_ROWS * 32 * 4 + DN_QUADS * 32 * 2;
 
+template <int W>  // arrival warps, and buffers: buffer k is filled by warp k
 struct DenseSmem {
     uint8_t stage[DN_STAGES][DN_CHUNK];              // psr [16 quads][32] float4 | class [16][32] u16
-    float4 binc[DN_BUFS][4][32];                     // increments of 16 rows
-    uint32_t bmsk[DN_BUFS][4][32];                   // step masks, one byte per row
+    float4 binc[W][4][32];                           // increments of 16 rows
+    uint32_t bmsk[W][4][32];                         // step masks, one byte per row
     uint32_t act[DN_ACT_WORDS];
     float sum[BLK_MAX_STEPS][32];
     float noise[BLK_MAX_STEPS][32];
     float dtab[BG3_MAX_DCLS];
-    int4 src[DN_EV_WARPS][2][4][32];                 // per arrival warp: a group's and the next one's
-    uint32_t lc[DN_EV_WARPS][2][4][32];              // sources and delay classes
+    int4 src[W][2][4][32];                           // per arrival warp: a group's and the next one's
+    uint32_t lc[W][2][4][32];                        // sources and delay classes
     int32_t ltab[BG3_MAX_DELAYS];
     uint32_t groups[DN_GROUP_WORDS];                 // the 16-row groups that have a buffer
-    int any[DN_BUFS];                                // bit q: quad q has arrivals; 16: several at a row
+    int any[W];                                      // bit q: quad q has arrivals; 16: several at a row
     int issued, failed;
     uint64_t full[DN_STAGES], empty[DN_STAGES];
-    uint64_t bfull[DN_BUFS], bempty[DN_BUFS];
+    uint64_t bfull[W], bempty[W];
     uint64_t scanned, summed, drawn;
 };
-constexpr size_t DN_SMEM = sizeof(DenseSmem);
 
+template <int W>
 __device__ __forceinline__ void bar_events()
 {
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * DN_EV_WARPS) : "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * W) : "memory");
 }
 
-__device__ __forceinline__ bool dn_wait(const NetDev &n, DenseSmem &s, uint64_t *bar, uint32_t parity)
+template <int W>
+__device__ __forceinline__ bool dn_wait(const NetDev &n, DenseSmem<W> &s, uint64_t *bar, uint32_t parity)
 {
     if (mbar_wait(bar, parity)) return true;
     set_err(n, ERR_TIMEOUT);
@@ -948,8 +955,8 @@ __device__ __forceinline__ uint32_t dense_hits(const int4 &v, const uint32_t *ac
 // together: the psr increments, with the event slots brought up to date
 // (AllSpikingSynapses.cpp:327-334, AllDSSynapses.cpp:227-247).  m[u] is cleared where the synapse did
 // not exist when the spike left, D[u] steps before.
-template <int SYN, int U>
-__device__ __forceinline__ void dense_arrivals(const NetDev &n, const DenseSmem &s, const uint32_t (&p)[U],
+template <int SYN, int U, int W>
+__device__ __forceinline__ void dense_arrivals(const NetDev &n, const DenseSmem<W> &s, const uint32_t (&p)[U],
                                                const int (&D)[U], uint32_t (&m)[U], float (&inc)[U],
                                                unsigned long long t)
 {
@@ -1131,8 +1138,8 @@ __global__ void __launch_bounds__(PUSH_THREADS) k_blk_push_batch(const NetDev *n
 
 // The 16 rows of buffer bf where a synapse has several spikes arriving in the block: those arrivals
 // run at their steps.  psr in place, the steps' sums in and out.
-template <int SYN>
-__device__ __noinline__ void dense_late(const NetDev &n, const DenseSmem &s, int tile, int row0, int bf,
+template <int SYN, int W>
+__device__ __noinline__ void dense_late(const NetDev &n, const DenseSmem<W> &s, int tile, int row0, int bf,
                                         int nt, unsigned long long t, float4 *ps4, const uint16_t *cw,
                                         float *acc)
 {
@@ -1229,7 +1236,8 @@ __device__ __forceinline__ void dense_quad(float4 &v, const float4 &dc, float (&
 }
 
 // The decay factors of a row quad's four class codes.
-__device__ __forceinline__ float4 dense_decay(const DenseSmem &s, uint32_t c)
+template <int W>
+__device__ __forceinline__ float4 dense_decay(const DenseSmem<W> &s, uint32_t c)
 {
     return make_float4(s.dtab[c & 15u], s.dtab[(c >> 4) & 15u], s.dtab[(c >> 8) & 15u],
                        s.dtab[(c >> 12) & 15u]);
@@ -1240,8 +1248,8 @@ __device__ __forceinline__ float4 dense_decay(const DenseSmem &s, uint32_t c)
 // destinations: eight steps 28 with 16 rows at a time and paired products, 33 with eight rows at a
 // time, 42 with four; two warps of four steps each, one after the other, 18 each (and 28 each beside
 // another tile's two).
-template <int SYN, bool FULL>
-__device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem &s, const CUtensorMap *tm_psr,
+template <int SYN, bool FULL, int W>
+__device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem<W> &s, const CUtensorMap *tm_psr,
                                            int tile, int nch, int nt, unsigned long long t)
 {
     const int lane = threadIdx.x & 31;
@@ -1260,10 +1268,10 @@ __device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem &s, const 
 #pragma unroll 1
         for (int g = 0; g < 4; g++, ps4 += 4 * 32, cw += 4 * 32) {
             const bool looked = (groups >> g) & 1u;
-            const int bf = k % DN_BUFS;
+            const int bf = k % W;
             int any = 0;
             if (looked) {
-                ok = dn_wait(n, s, &s.bfull[bf], (uint32_t)((k / DN_BUFS) & 1));
+                ok = dn_wait(n, s, &s.bfull[bf], (uint32_t)((k / W) & 1));
                 if (!ok) break;
                 k++;
                 any = s.any[bf];
@@ -1333,7 +1341,8 @@ __device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem &s, const 
 
 // Sources and delay classes (a byte per row) of 16 rows of the lane's destination, on their way to
 // shared memory.
-__device__ __forceinline__ void dense_sources(DenseSmem &s, int w, int st, const int4 *S,
+template <int W>
+__device__ __forceinline__ void dense_sources(DenseSmem<W> &s, int w, int st, const int4 *S,
                                               const uint32_t *L, int q0, int cnt)
 {
     const int lane = threadIdx.x & 31;
@@ -1350,7 +1359,8 @@ __device__ __forceinline__ void dense_sources(DenseSmem &s, int w, int st, const
 
 // The arrival warps of a light block: the flagged groups' masks and increments, both planes left
 // clean for the next block.
-__device__ __forceinline__ void dense_collect(const NetDev &n, const BlkDev &b, DenseSmem &s, int tile, int w)
+template <int W>
+__device__ __forceinline__ void dense_collect(const NetDev &n, const BlkDev &b, DenseSmem<W> &s, int tile, int w)
 {
     const int lane = threadIdx.x & 31;
     if (w < DN_GROUP_WORDS && lane == 0) {
@@ -1358,7 +1368,7 @@ __device__ __forceinline__ void dense_collect(const NetDev &n, const BlkDev &b, 
         s.groups[w] = f;
         if (f) b.gflag[tile * DN_GROUP_WORDS + w] = 0u;
     }
-    bar_events();
+    bar_events<W>();
     if (lane == 0) mbar_arrive(&s.scanned);
     uint32_t *M = reinterpret_cast<uint32_t *>(b.msk) + (size_t)tile * n.Mq * 32 + lane;
     EvSlot *E = n.ev + (size_t)tile * n.Mq * 128 + (size_t)lane * 4;
@@ -1374,7 +1384,7 @@ __device__ __forceinline__ void dense_collect(const NetDev &n, const BlkDev &b, 
             }
             const int g = 32 * word + __ffs((int)left) - 1;
             left &= left - 1u;
-            if (k++ % DN_BUFS == w) return g;
+            if (k++ % W == w) return g;
         }
     };
     auto masks = [&](int g, uint32_t (&m)[4]) {
@@ -1445,8 +1455,8 @@ __device__ __forceinline__ void dense_collect(const NetDev &n, const BlkDev &b, 
     }
 }
 
-template <int SYN>
-__device__ __forceinline__ void dense_events(const NetDev &n, const BlkDev &b, DenseSmem &s, int tile,
+template <int SYN, int W>
+__device__ __forceinline__ void dense_events(const NetDev &n, const BlkDev &b, DenseSmem<W> &s, int tile,
                                              int w, int cnt, int nch, int nt, unsigned long long t)
 {
     const int lane = threadIdx.x & 31, tid = 32 * w + lane;
@@ -1459,16 +1469,16 @@ __device__ __forceinline__ void dense_events(const NetDev &n, const BlkDev &b, D
         s.groups[w] = k >= 32 ? 0xffffffffu : k > 0 ? (1u << k) - 1u : 0u;
     }
     if (n.ntiles <= DN_ACT_WORDS) {
-        for (int i = tid; i < n.ntiles; i += 32 * DN_EV_WARPS) s.act[i] = act[i];
+        for (int i = tid; i < n.ntiles; i += 32 * W) s.act[i] = act[i];
         act = s.act;
     }
-    bar_events();
+    bar_events<W>();
     if (lane == 0) mbar_arrive(&s.scanned);
     if (w < 4 * nch) dense_sources(s, w, 0, S, L, 4 * w, cnt);
-    for (int g = w, used = 0; g < 4 * nch; g += DN_BUFS) {
+    for (int g = w, used = 0; g < 4 * nch; g += W) {
         const int st = used & 1;
-        if (g + DN_BUFS < 4 * nch) {
-            dense_sources(s, w, st ^ 1, S, L, 4 * (g + DN_BUFS), cnt);
+        if (g + W < 4 * nch) {
+            dense_sources(s, w, st ^ 1, S, L, 4 * (g + W), cnt);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -1559,15 +1569,15 @@ __device__ __forceinline__ void dense_events(const NetDev &n, const BlkDev &b, D
     }
 }
 
-template <int SYN>
+template <int SYN, int W>
 __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
                                                const CUtensorMap *tm_psr, const CUtensorMap *tm_cls,
-                                               const int tile, const int nt, DenseSmem &s)
+                                               const int tile, const int nt, DenseSmem<W> &s)
 {
     // Roles rotate with the block: warp k of every block is issued by the same quarter of its SM, and
     // the sum warps of the blocks that share an SM (152 apart in a first wave) are the busy ones.
     const int lane = threadIdx.x & 31;
-    const int warp = (int)(threadIdx.x / 32 + blockIdx.x / 152) % (DN_THREADS / 32);
+    const int warp = (int)(threadIdx.x / 32 + blockIdx.x / 152) % (W + 2);
     const int d = tile * 32 + lane;
     const bool valid = d < n.N;
     for (int i = threadIdx.x; i < n.n_dcls; i += blockDim.x) s.dtab[i] = n.dtab[i];
@@ -1579,13 +1589,13 @@ __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
             mbar_init(&s.full[i], 1);
             mbar_init(&s.empty[i], 1);
         }
-        for (int i = 0; i < DN_BUFS; i++) {
+        for (int i = 0; i < W; i++) {
             mbar_init(&s.bfull[i], 1);
             mbar_init(&s.bempty[i], 1);
         }
         mbar_init(&s.summed, 1);
-        mbar_init(&s.scanned, DN_EV_WARPS);
-        mbar_init(&s.drawn, DN_EV_WARPS);
+        mbar_init(&s.scanned, W);
+        mbar_init(&s.drawn, W);
         fence_mbar_init();
         s.issued = 0;
         s.failed = 0;
@@ -1635,11 +1645,11 @@ __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
             sp = s.sum[nt - 1][lane];
             blk_finish<SYN>(n, b, tile, d, valid, x, sp, hist, fired, nt, t);
         }
-    } else if (warp <= DN_EV_WARPS) {  // ------------------------------------------- arrivals
+    } else if (warp <= W) {  // ------------------------------------------- arrivals
         const int w = warp - 1;
         if (blk_light(n, b, t)) dense_collect(n, b, s, tile, w);
         else dense_events<SYN>(n, b, s, tile, w, cnt, nch, nt, t);
-        for (int j = w; j < nt; j += DN_EV_WARPS)
+        for (int j = w; j < nt; j += W)
             s.noise[j][lane] = normal_device(n.noise_seed, t + (unsigned)j, d);
         __syncwarp();
         if (lane == 0) mbar_arrive(&s.drawn);
@@ -1656,25 +1666,25 @@ __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
     }
 }
 
-template <int SYN>
-__global__ void __launch_bounds__(DN_THREADS, 3) k_blk_dense(const __grid_constant__ NetDev n,
-                                                             const __grid_constant__ BlkDev b,
-                                                             const __grid_constant__ CUtensorMap tm_psr,
-                                                             const __grid_constant__ CUtensorMap tm_cls,
-                                                             int nt)
+template <int SYN, int W>
+__global__ void __launch_bounds__(dn_threads(W), dn_blocks(W)) k_blk_dense(const __grid_constant__ NetDev n,
+                                                                           const __grid_constant__ BlkDev b,
+                                                                           const __grid_constant__ CUtensorMap tm_psr,
+                                                                           const __grid_constant__ CUtensorMap tm_cls,
+                                                                           int nt)
 {
     // declared with its alignment and used as it is: arithmetic on the address would hide from the
     // compiler that it is shared memory, and every access would be a generic one
     extern __shared__ __align__(128) uint8_t smem_dense[];
-    blk_dense_tile<SYN>(n, b, &tm_psr, &tm_cls, blockIdx.x, nt, *reinterpret_cast<DenseSmem *>(smem_dense));
+    blk_dense_tile<SYN>(n, b, &tm_psr, &tm_cls, blockIdx.x, nt, *reinterpret_cast<DenseSmem<W> *>(smem_dense));
 }
 
 // Batched form: tiles[b] = (network, tile), heaviest first; maps as in k_sweep_batch.
-template <int SYN>
-__global__ void __launch_bounds__(DN_THREADS, 3) k_blk_dense_batch(const NetDev *nets,
-                                                                   const BlkDev *blks,
-                                                                   const CUtensorMap *maps,
-                                                                   const int2 *tiles, int nt)
+template <int SYN, int W>
+__global__ void __launch_bounds__(dn_threads(W), dn_blocks(W)) k_blk_dense_batch(const NetDev *nets,
+                                                                                 const BlkDev *blks,
+                                                                                 const CUtensorMap *maps,
+                                                                                 const int2 *tiles, int nt)
 {
     extern __shared__ __align__(128) uint8_t smem_dense[];
     __shared__ __align__(16) NetDev s_net;
@@ -1685,7 +1695,7 @@ __global__ void __launch_bounds__(DN_THREADS, 3) k_blk_dense_batch(const NetDev 
     const BlkDev b = blks[tr.x];
     __syncthreads();
     blk_dense_tile<SYN>(s_net, b, &maps[2 * tr.x], &maps[2 * tr.x + 1], tr.y, nt,
-                        *reinterpret_cast<DenseSmem *>(smem_dense));
+                        *reinterpret_cast<DenseSmem<W> *>(smem_dense));
 }
 
 // ---- launchers --------------------------------------------------------------------------------
@@ -1839,45 +1849,64 @@ void launch_blk_thin_batch(int syn_kind, const NetDev *nets, const BlkDev *blks,
 // The opt-in shared memory size is a property of the kernel on each device: set before every launch
 // (a host-side table write), so that no process-wide flag is needed.
 template <typename K>
-static void allow_smem(K kern)
+static void allow_smem(K kern, size_t bytes)
 {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_SMEM);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // The push grid: 128-synapse chunks over eight blocks, so that a neuron of a thousand synapses is
 // one round of them.
 constexpr int PUSH_SPLIT = 8;
 
+template <int SYN, int W>
+static void launch_dense_t(const NetDev &h, const BlkDev &b, const CUtensorMap &tp, const CUtensorMap &tc,
+                           int nt, cudaStream_t s)
+{
+    allow_smem(k_blk_dense<SYN, W>, sizeof(DenseSmem<W>));
+    launch_dep(k_blk_dense<SYN, W>, h.ntiles, dn_threads(W), sizeof(DenseSmem<W>), s, h, b, tp, tc, nt);
+}
+template <int SYN>
+static void launch_dense_syn(const NetDev &h, const BlkDev &b, const CUtensorMap &tp, const CUtensorMap &tc,
+                             int nt, cudaStream_t s)
+{
+    const dim3 pg((h.ntiles + PUSH_WORDS - 1) / PUSH_WORDS, PUSH_SPLIT);
+    launch_dep(k_blk_push<SYN>, pg, PUSH_THREADS, 0, s, h, b, nt);
+    if (h.ntiles <= 152 * dn_blocks(16)) launch_dense_t<SYN, 16>(h, b, tp, tc, nt, s);
+    else if (h.ntiles <= 152 * dn_blocks(8)) launch_dense_t<SYN, 8>(h, b, tp, tc, nt, s);
+    else launch_dense_t<SYN, 4>(h, b, tp, tc, nt, s);
+}
 void launch_blk_dense(const NetDev &h, const BlkDev &b, const CUtensorMap &tp, const CUtensorMap &tc,
                       int nt, cudaStream_t s)
 {
-    const dim3 pg((h.ntiles + PUSH_WORDS - 1) / PUSH_WORDS, PUSH_SPLIT);
-    if (h.syn_kind == 1) {
-        allow_smem(k_blk_dense<1>);
-        launch_dep(k_blk_push<1>, pg, PUSH_THREADS, 0, s, h, b, nt);
-        launch_dep(k_blk_dense<1>, h.ntiles, DN_THREADS, DN_SMEM, s, h, b, tp, tc, nt);
-    } else {
-        allow_smem(k_blk_dense<0>);
-        launch_dep(k_blk_push<0>, pg, PUSH_THREADS, 0, s, h, b, nt);
-        launch_dep(k_blk_dense<0>, h.ntiles, DN_THREADS, DN_SMEM, s, h, b, tp, tc, nt);
-    }
+    if (h.syn_kind == 1) launch_dense_syn<1>(h, b, tp, tc, nt, s);
+    else launch_dense_syn<0>(h, b, tp, tc, nt, s);
 }
 
 // dense: the indices of the nd networks that run dense blocks, max_tiles their most tiles.
+template <int SYN, int W>
+static void launch_dense_batch_t(const NetDev *nets, const BlkDev *blks, const CUtensorMap *maps,
+                                 const int2 *tiles, int n, int nt, cudaStream_t s)
+{
+    allow_smem(k_blk_dense_batch<SYN, W>, sizeof(DenseSmem<W>));
+    launch_dep(k_blk_dense_batch<SYN, W>, n, dn_threads(W), sizeof(DenseSmem<W>), s, nets, blks, maps, tiles, nt);
+}
+template <int SYN>
+static void launch_dense_batch_syn(const NetDev *nets, const BlkDev *blks, const CUtensorMap *maps,
+                                   const int2 *tiles, int n, const int *dense, int nd, int max_tiles, int nt,
+                                   cudaStream_t s)
+{
+    const dim3 pg((max_tiles + PUSH_WORDS - 1) / PUSH_WORDS, PUSH_SPLIT, nd);
+    launch_dep(k_blk_push_batch<SYN>, pg, PUSH_THREADS, 0, s, nets, blks, dense, nt);
+    if (n <= 152 * dn_blocks(16)) launch_dense_batch_t<SYN, 16>(nets, blks, maps, tiles, n, nt, s);
+    else if (n <= 152 * dn_blocks(8)) launch_dense_batch_t<SYN, 8>(nets, blks, maps, tiles, n, nt, s);
+    else launch_dense_batch_t<SYN, 4>(nets, blks, maps, tiles, n, nt, s);
+}
 void launch_blk_dense_batch(int syn_kind, const NetDev *nets, const BlkDev *blks,
                             const CUtensorMap *maps, const int2 *tiles, int n, const int *dense, int nd,
                             int max_tiles, int nt, cudaStream_t s)
 {
-    const dim3 pg((max_tiles + PUSH_WORDS - 1) / PUSH_WORDS, PUSH_SPLIT, nd);
-    if (syn_kind == 1) {
-        allow_smem(k_blk_dense_batch<1>);
-        launch_dep(k_blk_push_batch<1>, pg, PUSH_THREADS, 0, s, nets, blks, dense, nt);
-        launch_dep(k_blk_dense_batch<1>, n, DN_THREADS, DN_SMEM, s, nets, blks, maps, tiles, nt);
-    } else {
-        allow_smem(k_blk_dense_batch<0>);
-        launch_dep(k_blk_push_batch<0>, pg, PUSH_THREADS, 0, s, nets, blks, dense, nt);
-        launch_dep(k_blk_dense_batch<0>, n, DN_THREADS, DN_SMEM, s, nets, blks, maps, tiles, nt);
-    }
+    if (syn_kind == 1) launch_dense_batch_syn<1>(nets, blks, maps, tiles, n, dense, nd, max_tiles, nt, s);
+    else launch_dense_batch_syn<0>(nets, blks, maps, tiles, n, dense, nd, max_tiles, nt, s);
 }
 
 }  // namespace bg3

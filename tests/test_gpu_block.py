@@ -374,3 +374,72 @@ def test_spikes_put_in_the_delay_queues(form):
     same(nets[0], nets[1], "spikes added")
     if batch:
         batch.close()
+
+
+def few_firing(w, h, syn, period, count, max_syn=260, radius=4.2, seed=9):
+    """`count` neurons fire every `period` steps, the others never (0: all of them, in turn)."""
+    spec = netgen.lif_network(w, h, seed=seed)
+    net = bg.Network(spec["N"], max_syn, w, h, 0.1, 1e-4, 1000, 4, syn, bg.BG3_NOISE_DEVICE, seed)
+    netgen.configure_lif(net, spec)
+    netgen.pregrow(net, spec, radius, weight_scale=0.3)
+    rs = np.random.RandomState(seed)
+    on = np.zeros(spec["N"], bool)
+    on[rs.permutation(spec["N"])[:count or spec["N"]]] = True
+    v = net.download_lif(fields=("Vthresh", "Vreset", "Trefract", "Vm"))
+    v["Vthresh"][~on] = 1.0
+    v["Vreset"][on] = v["Vthresh"][on] + np.float32(1e-3)
+    v["Vm"][on] = v["Vreset"][on]
+    v["Trefract"][:] = np.float32((period - 1) * 1e-4)
+    v["nStepsInRefr"] = rs.randint(0, period, spec["N"]).astype(np.int32)
+    net.upload_lif(**v)
+    return net, on
+
+
+@pytest.mark.parametrize("syn", [bg.BG3_SYN_SPIKING, bg.BG3_SYN_DS])
+@pytest.mark.parametrize("w,h", [(50, 42), (80, 70), (110, 100)])    # 66, 175 and 344 tiles
+@pytest.mark.parametrize("period,share", [(29, 130), (1, 130), (7, 130), (29, 0)])
+def test_dense_blocks_by_tiles_and_arrivals(syn, w, h, period, share):
+    """Tiles of 16, 8 and 4 arrival warps.  A few neurons (fewer than N / 128: pushed arrivals)
+    reach most of a tile's rows with one spike a block, one at every step, or two; or all of
+    them do (arrivals looked up)."""
+    count = w * h // share if share else 0
+    nets = [few_firing(w, h, syn, period, count) for _ in range(2)]
+    nets[1][0].set_launch(small_max_slots=0)
+    for calls in ((8, 8, 3), (16, 5, 8)):
+        for net, _ in nets:
+            for n in calls:
+                net.step(n)
+        same(nets[0][0], nets[1][0], "after calls of %s steps" % (calls,))
+    fired = nets[0][0].download_lif(fields=("spikeCount",))["spikeCount"] > 0
+    on = nets[0][1]
+    assert fired[~on].sum() == 0 and fired[on].all()
+    assert count == 0 or 0 < on.sum() * 128 <= w * h
+    syn_ = nets[0][0].download_synapses()
+    used = syn_["in_use"].astype(bool)
+    if syn == bg.BG3_SYN_DS:
+        # rows that received a spike in more than eight groups of 16 of some neuron's
+        rows = (used & (syn_["lastSpike"] != np.uint64(2**64 - 1))).reshape(w * h, -1)
+        groups = np.add.reduceat(rows, np.arange(0, rows.shape[1], 16), axis=1) > 0
+        tiles = np.array([groups[d:d + 32].any(axis=0).sum() for d in range(0, w * h, 32)])
+        assert tiles.max() > 8
+    for net, _ in nets:
+        net.close()
+
+
+def test_batched_dense_blocks_by_tiles():
+    """Batches of up to 152, up to 304 and more tiles."""
+    for shapes in ([(50, 42)], [(50, 42), (70, 68)], [(50, 42), (70, 68), (80, 70)]):
+        pairs = [[few_firing(w, h, bg.BG3_SYN_DS, 7, c)[0] for w, h in shapes for c in (0,)] for _ in range(2)]
+        batch = bg.Batch(pairs[0])
+        for net in pairs[1]:
+            net.set_launch(small_max_slots=0)
+        for n in (8, 5, 19):
+            batch.step(n)
+            for net in pairs[1]:
+                net.step(n)
+        batch.sync()
+        for x, y in zip(*pairs):
+            same(x, y, "batched")
+        batch.close()
+        for net in pairs[0] + pairs[1]:
+            net.close()
