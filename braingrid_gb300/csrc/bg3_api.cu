@@ -1281,6 +1281,24 @@ static int blk_steps(const bg3_net *n, const LaunchCfg &c, bool small = false)
     return T >= 2 ? T : 0;
 }
 
+// Whether dense blocks of up to T steps are the shorter way to make nsteps steps: a short block costs
+// nearly what a long one does, and step by step the arrivals spread over the whole GPU.  The line is by
+// the rows a destination has (mq quads), the slots there are, and the steps of a block (of an average one
+// where the blocks are few): one on up to 252 rows and 2.5 M slots, two up to twice that, three beyond; a
+// batch, whose tiles share the GPU, is not held to more than two.  us a call in blocks and step by
+// step, near the target rate / at 200 to 330 Hz: 100x100 with 160 rows, one step, 13 and 17 / (60x60) 14 and
+// 15; 150x150 with 160 rows, one step, at 128 Hz 32 and 21, two 37 and 38; 60x60 with 480 rows, one step 19
+// and 18 / 25 and 19, two 21 and 28 / 28 and 33; 100x100 with 960 rows, one step 27 and 25 / 88 and 33, two
+// 30 and 39 / 108 and 61, three 34 and 52 / 126 and 89, four 34 and 65 / 138 and 117, eight 42 and 120 / 173
+// and 228; a batch of 12, one step 130 and 90, two 102 and 150.  Below 32 tiles either way is the launches.
+static bool dense_pays(int64_t nsteps, int T, int mq, int tiles, int most)
+{
+    const int64_t large = std::max<int64_t>(mq / 64, (int64_t)mq * tiles / 20000);
+    const int fewest = std::min(most, 1 + (int)std::min<int64_t>(2, large));
+    const int64_t blocks = (nsteps + T - 1) / T;
+    return tiles < 32 || (blocks > 4 ? T >= fewest : nsteps >= fewest * blocks);
+}
+
 // The spike masks as of the network's current step, for a block to start from.
 static int ensure_masks(bg3_net *n)
 {
@@ -1288,8 +1306,8 @@ static int ensure_masks(bg3_net *n)
     if (n->mask_ok && w == n->blk.win) return BG3_OK;
     int rc = ensure_ring(n);
     if (rc) return rc;
+    if (w != n->blk.win) drop_graph(n);  // holds the window
     n->blk.win = w;
-    drop_graph(n);  // holds the window
     bg3::launch_blk_masks(n->h, n->blk, n->stream);
     CK(cudaGetLastError());
     n->mask_ok = true;
@@ -1338,7 +1356,8 @@ static int run_form(bg3_net *n, int64_t nsteps)
     const NetDev &h = n->h;
     int rc;
     const bool small = bg3::small_eligible(h, n->cfg);
-    const int T = blk_steps(n, n->cfg, small);
+    int T = blk_steps(n, n->cfg, small);
+    if (T && !small && !blk_is_thin(h, n->cfg) && !dense_pays(nsteps, T, h.Mq, h.ntiles, 3)) T = 0;
     if (T && small) {
         // a small network: up to SMALL_STEPS whole steps per launch
         if ((rc = ensure_masks(n))) return rc;
@@ -1353,7 +1372,8 @@ static int run_form(bg3_net *n, int64_t nsteps)
     if (T) return run_blocks(n, nsteps, T);
     if ((rc = ensure_ring(n))) return rc;
     n->mask_ok = false;
-    if (n->graph && n->graph_steps) drop_graph(n);
+    // a call too short to replay a graph leaves that of the blocks for the next one
+    if (n->graph && n->graph_steps && nsteps >= GRAPH_STEPS) drop_graph(n);
     if (small) {
         // the same in one CTA, step by step: what does not run in blocks
         for (int64_t left = nsteps; left > 0;) {
@@ -1819,7 +1839,7 @@ struct bg3_batch {
     int2 *d_tiles = nullptr;
     BlkDev *d_blks = nullptr;
     int *d_dense = nullptr;       // indices of the TMA-swept networks
-    int n_dense = 0, dense_tiles = 0;
+    int n_dense = 0, dense_tiles = 0, dense_mq = 0;  // how many, and the most tiles and row quads of one
     std::vector<BlkDev> blks;     // as uploaded
     int ntiles = 0, n_thick = 0, max_n = 0, syn_kind = 1, thin_mq = 0;
     cudaStream_t stream = nullptr;
@@ -1875,7 +1895,7 @@ static int batch_refresh(bg3_batch *b)
     for (auto &t : tiles)
         if (!bg3::sweep_is_thin(b->nets[t.second.x]->h, b->cfg)) tl.push_back(t.second);
     b->n_thick = (int)tl.size();
-    b->thin_mq = b->dense_tiles = 0;
+    b->thin_mq = b->dense_tiles = b->dense_mq = 0;
     std::vector<int> dense;
     for (size_t k = 0; k < b->nets.size(); k++) {
         const NetDev &h = b->nets[k]->h;
@@ -1884,6 +1904,7 @@ static int batch_refresh(bg3_batch *b)
         } else {
             dense.push_back((int)k);
             b->dense_tiles = std::max(b->dense_tiles, h.ntiles);
+            b->dense_mq = std::max(b->dense_mq, h.Mq);
         }
     }
     b->n_dense = (int)dense.size();
@@ -2070,11 +2091,12 @@ static int batch_run_form(bg3_batch *b, int64_t nsteps)
 {
     if (nsteps <= 0) return BG3_OK;
     const int T = batch_blk_steps(b);
-    if (T) return batch_run_blocks(b, nsteps, T);
+    if (T && (!b->n_thick || dense_pays(nsteps, T, b->dense_mq, b->n_thick, 2)))
+        return batch_run_blocks(b, nsteps, T);
     int rc = batch_rings(b);
     if (rc) return rc;
     if ((rc = batch_order(b, true))) return rc;
-    if (b->graph && b->graph_steps) batch_drop_graph(b);
+    if (b->graph && b->graph_steps && nsteps >= GRAPH_STEPS) batch_drop_graph(b);  // as in run_form
     const int M = (int)b->nets.size();
     bg3::launch_neurons_batch(b->d_nets, M, b->max_n, b->stream);
     bg3::launch_deliver_batch(b->syn_kind, b->d_nets, M, b->cfg, b->stream);

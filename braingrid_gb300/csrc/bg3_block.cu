@@ -1199,16 +1199,16 @@ __device__ __forceinline__ void add_hits(float2 &x, float2 &y, uint32_t m, const
 
 // Four rows through the block's steps: psr scaled, and added to each step's sum in row order.  The
 // products of a step's four rows are independent of each other, as are the steps' sums of a row, so neither half of this waits on itself.  HIT: rows may have an arrival, at the step whose
-// bit is set in the row's byte of m (bit j: step j).  FULL: nt = BLK_MAX_STEPS.
-template <bool FULL, bool HIT>
-__device__ __forceinline__ void dense_quad(float4 &v, const float4 &dc, float (&acc)[BLK_MAX_STEPS], int nt,
+// bit is set in the row's byte of m (bit j: step j).  S: the steps computed, nt of them used; FULL: nt = S.
+template <int S, bool FULL, bool HIT>
+__device__ __forceinline__ void dense_quad(float4 &v, const float4 &dc, float (&acc)[S], int nt,
                                            uint32_t m, const float4 &in)
 {
-    float2 p[BLK_MAX_STEPS][2];
+    float2 p[S][2];
     float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w);
     const float2 dx = make_float2(dc.x, dc.y), dy = make_float2(dc.z, dc.w);
 #pragma unroll
-    for (int j = 0; j < BLK_MAX_STEPS; j++) {
+    for (int j = 0; j < S; j++) {
         if (HIT) {
             if (j == 0) add_hits<0>(x, y, m, in);
             if (j == 1) add_hits<1>(x, y, m, in);
@@ -1226,13 +1226,13 @@ __device__ __forceinline__ void dense_quad(float4 &v, const float4 &dc, float (&
     }
     if (FULL) v = make_float4(x.x, x.y, y.x, y.y);
 #pragma unroll
-    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = acc[j] + p[j][0].x;
+    for (int j = 0; j < S; j++) acc[j] = acc[j] + p[j][0].x;
 #pragma unroll
-    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = acc[j] + p[j][0].y;
+    for (int j = 0; j < S; j++) acc[j] = acc[j] + p[j][0].y;
 #pragma unroll
-    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = acc[j] + p[j][1].x;
+    for (int j = 0; j < S; j++) acc[j] = acc[j] + p[j][1].x;
 #pragma unroll
-    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = acc[j] + p[j][1].y;
+    for (int j = 0; j < S; j++) acc[j] = acc[j] + p[j][1].y;
 }
 
 // The decay factors of a row quad's four class codes.
@@ -1244,18 +1244,18 @@ __device__ __forceinline__ float4 dense_decay(const DenseSmem<W> &s, uint32_t c)
 }
 
 // The sum warp: the block's steps over all chunks, psr scaled in place, a step's sum over the rows in
-// order.  FULL: nt = BLK_MAX_STEPS.  Measured as one warp on an SM, cycles a row of 32
+// order.  S and FULL as in dense_quad.  Measured as one warp on an SM, cycles a row of 32
 // destinations: eight steps 28 with 16 rows at a time and paired products, 33 with eight rows at a
 // time, 42 with four; two warps of four steps each, one after the other, 18 each (and 28 each beside
 // another tile's two).
-template <int SYN, bool FULL, int W>
+template <int SYN, int S, bool FULL, int W>
 __device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem<W> &s, const CUtensorMap *tm_psr,
                                            int tile, int nch, int nt, unsigned long long t)
 {
     const int lane = threadIdx.x & 31;
-    float acc[BLK_MAX_STEPS];
+    float acc[S];
 #pragma unroll
-    for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = 0.0f;
+    for (int j = 0; j < S; j++) acc[j] = 0.0f;
     bool ok = dn_wait(n, s, &s.scanned, 0);
     int k = 0;  // 16-row groups with a buffer so far
     for (int c = 0; ok && c < nch; c++) {
@@ -1287,7 +1287,7 @@ __device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem<W> &s, con
 #pragma unroll
                 for (int q = 0; q < 4; q++) dc[q] = dense_decay(s, cl[q]);
 #pragma unroll
-                for (int q = 0; q < 4; q++) dense_quad<FULL, false>(v[q], dc[q], acc, nt, 0u, v[q]);
+                for (int q = 0; q < 4; q++) dense_quad<S, FULL, false>(v[q], dc[q], acc, nt, 0u, v[q]);
 #pragma unroll
                 for (int q = 0; q < 4; q++) ps4[q * 32] = v[q];
             } else if (!(any & 16)) {
@@ -1296,22 +1296,22 @@ __device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem<W> &s, con
                     float4 v0 = ps4[q * 32], v1 = ps4[(q + 1) * 32];
                     const float4 d0 = dense_decay(s, cw[q * 32]), d1 = dense_decay(s, cw[(q + 1) * 32]);
                     if ((any >> q) & 3) {
-                        dense_quad<FULL, true>(v0, d0, acc, nt, s.bmsk[bf][q][lane], s.binc[bf][q][lane]);
-                        dense_quad<FULL, true>(v1, d1, acc, nt, s.bmsk[bf][q + 1][lane], s.binc[bf][q + 1][lane]);
+                        dense_quad<S, FULL, true>(v0, d0, acc, nt, s.bmsk[bf][q][lane], s.binc[bf][q][lane]);
+                        dense_quad<S, FULL, true>(v1, d1, acc, nt, s.bmsk[bf][q + 1][lane], s.binc[bf][q + 1][lane]);
                     } else {
-                        dense_quad<FULL, false>(v0, d0, acc, nt, 0u, v0);
-                        dense_quad<FULL, false>(v1, d1, acc, nt, 0u, v1);
+                        dense_quad<S, FULL, false>(v0, d0, acc, nt, 0u, v0);
+                        dense_quad<S, FULL, false>(v1, d1, acc, nt, 0u, v1);
                     }
                     ps4[q * 32] = v0;
                     ps4[(q + 1) * 32] = v1;
                 }
             } else {
-                float a[BLK_MAX_STEPS];
+                float a[S];
 #pragma unroll
-                for (int j = 0; j < BLK_MAX_STEPS; j++) a[j] = acc[j];
+                for (int j = 0; j < S; j++) a[j] = acc[j];
                 dense_late<SYN>(n, s, tile, c * DN_ROWS + 16 * g, bf, nt, t, ps4, cw, a);
 #pragma unroll
-                for (int j = 0; j < BLK_MAX_STEPS; j++) acc[j] = a[j];
+                for (int j = 0; j < S; j++) acc[j] = a[j];
             }
             if (looked) {
                 __syncwarp();
@@ -1333,7 +1333,7 @@ __device__ __forceinline__ void dense_sums(const NetDev &n, DenseSmem<W> &s, con
     }
     if (lane == 0) bulk_wait_read_all();
 #pragma unroll
-    for (int j = 0; j < BLK_MAX_STEPS; j++)
+    for (int j = 0; j < S; j++)
         if (j < nt) s.sum[j][lane] = acc[j];
     __syncwarp();
     if (ok && lane == 0) mbar_arrive(&s.summed);
@@ -1654,8 +1654,13 @@ __device__ __forceinline__ void blk_dense_tile(const NetDev &n, const BlkDev &b,
         __syncwarp();
         if (lane == 0) mbar_arrive(&s.drawn);
     } else {  // --------------------------------------------------------------------- sums
-        if (nt == BLK_MAX_STEPS) dense_sums<SYN, true>(n, s, tm_psr, tile, nch, nt, t);
-        else dense_sums<SYN, false>(n, s, tm_psr, tile, nch, nt, t);
+        // a shorter block's chains are shorter where they are written out for its steps: a call of one
+        // step on the 100x100 network at its target rate 52 us with eight, 27 with one; of four 45 and 34
+        if (nt == BLK_MAX_STEPS) dense_sums<SYN, BLK_MAX_STEPS, true>(n, s, tm_psr, tile, nch, nt, t);
+        else if (nt > 4) dense_sums<SYN, BLK_MAX_STEPS, false>(n, s, tm_psr, tile, nch, nt, t);
+        else if (nt > 2) dense_sums<SYN, 4, false>(n, s, tm_psr, tile, nch, nt, t);
+        else if (nt == 2) dense_sums<SYN, 2, true>(n, s, tm_psr, tile, nch, nt, t);
+        else dense_sums<SYN, 1, true>(n, s, tm_psr, tile, nch, nt, t);
     }
     __syncthreads();
     if (*(volatile int *)&s.failed && threadIdx.x == 0) {

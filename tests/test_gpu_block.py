@@ -443,3 +443,46 @@ def test_batched_dense_blocks_by_tiles():
         batch.close()
         for net in pairs[0] + pairs[1]:
             net.close()
+
+
+@pytest.mark.parametrize("w,h,max_syn,radius", [(33, 33, 64, 1.9), (33, 33, 190, 3.4), (60, 60, 600, 6.0)])
+def test_calls_of_few_steps(w, h, max_syn, radius):
+    """Calls that run in blocks and calls too short for them in turn, a graph of blocks kept between
+    them; wide networks take one step as step by step."""
+    nets = [few_firing(w, h, bg.BG3_SYN_DS, 29, 0, max_syn, radius)[0] for _ in range(3)]
+    nets[1].set_launch(small_max_slots=0)
+    batch = bg.Batch(nets[2:])
+    for n in (1, 1, 130, 1, 2, 3, 160, 1, 9, 1, 10, 40, 1, 33, 130):
+        counts = [net.launches for net in nets[:2]]
+        for run in (nets[0], nets[1], batch):
+            run.step(n)
+        if n == 1 and max_syn == 600:
+            assert nets[0].launches - counts[0] == nets[1].launches - counts[1]
+        if n >= 8:
+            assert nets[0].launches - counts[0] < nets[1].launches - counts[1]
+    batch.sync()
+    same(nets[0], nets[1], "plain")
+    same(nets[2], nets[1], "batched")
+    batch.close()
+
+
+@pytest.mark.parametrize("dt", [1.5e-4, 2e-4, 3e-4, 5e-4, 8e-4])
+@pytest.mark.parametrize("w,h,max_syn,radius", [(33, 33, 64, 1.9), (33, 33, 190, 3.4), (60, 60, 600, 6.0)])
+def test_longer_steps_take_shorter_blocks(w, h, max_syn, radius, dt):
+    """Delays of fewer than eight steps: blocks of two to six."""
+    nets = []
+    for small in (1, 0):
+        spec = netgen.lif_network(w, h, seed=5, delta_t=dt)
+        spec["Vm"] = np.random.RandomState(5).uniform(13.2e-3, 15.2e-3, spec["N"]).astype(np.float32)
+        net = bg.Network(spec["N"], max_syn, w, h, 0.1, dt, 1000, 4, bg.BG3_SYN_DS, bg.BG3_NOISE_DEVICE, 5)
+        netgen.configure_lif(net, spec)
+        netgen.pregrow(net, spec, radius, weight_scale=0.3)
+        net.set_launch(small_max_slots=small)
+        nets.append(net)
+    for n in (1, 3, 40, 7, 130):
+        for net in nets:
+            net.step(n)
+    same(nets[0], nets[1], "dt %g" % dt)
+    if max_syn < 600 or dt < 4e-4:      # two steps at a time do not pay on wide rows
+        assert nets[0].launches < nets[1].launches
+    assert int(nets[0].download_lif(fields=("spikeCount",))["spikeCount"].sum()) > 0
