@@ -1359,6 +1359,10 @@ static int run_form(bg3_net *n, int64_t nsteps)
     int rc;
     const bool small = bg3::small_eligible(h, n->cfg);
     int T = blk_steps(n, n->cfg, small);
+    // a cluster's start, with every tile's state on its way into it, is more than one or two steps of a few
+    // tiles in one CTA: 10x10 with 80 rows, calls of one step 12.6 and 8.6 us, of two 12.8 and 11.3, of three
+    // 14.1 and 14.9; 16x16 with 30 rows 9.9 and 8.1, 10.5 and 10.8; 24x24 (18 tiles) one step 10.2 and 11.2
+    if (small && nsteps <= 2 && nsteps * h.ntiles <= 16) T = 0;
     if (T && !small && !blk_is_thin(h, n->cfg) && !dense_pays(nsteps, T, h.Mq, h.ntiles, 3)) T = 0;
     if (T && small) {
         // a small network: up to SMALL_STEPS whole steps per launch

@@ -486,3 +486,27 @@ def test_longer_steps_take_shorter_blocks(w, h, max_syn, radius, dt):
     if max_syn < 600 or dt < 4e-4:      # two steps at a time do not pay on wide rows
         assert nets[0].launches < nets[1].launches
     assert int(nets[0].download_lif(fields=("spikeCount",))["spikeCount"].sum()) > 0
+
+
+@pytest.mark.parametrize("noise", [bg.BG3_NOISE_DEVICE, bg.BG3_NOISE_INJECT])
+@pytest.mark.parametrize("syn", [bg.BG3_SYN_DS, bg.BG3_SYN_DYNSTDP])
+@pytest.mark.parametrize("w,h,radius,max_syn", [(8, 4, 1.5, 30), (16, 16, 1.5, 30), (32, 16, 1.2, 20), (33, 16, 1.2, 20)])
+def test_small_networks_in_calls_of_one_and_two_steps(noise, syn, w, h, radius, max_syn):
+    """1, 8, 16 and 17 tiles: one CTA and the cluster in turn."""
+    nets = []
+    for small in (65536, 0):
+        net = lif(w, h, syn, radius, "poisson", max_syn)
+        if noise == bg.BG3_NOISE_INJECT:
+            net.set_noise_mode(noise, 1)
+            net.push_noise(np.random.RandomState(3).standard_normal(w * h * 120).astype(np.float32))
+        net.set_launch(small_max_slots=small)
+        nets.append(net)
+    for n in (1, 2, 1, 40, 2, 2, 1, 1, 9, 1, 20):
+        b0 = nets[0].launches
+        for net in nets:
+            net.step(n)
+        assert nets[0].launches - b0 == 1
+    same(nets[0], nets[1], "short calls")
+    if noise == bg.BG3_NOISE_INJECT:
+        assert nets[0].noise_pending() == nets[1].noise_pending()
+    assert int(nets[0].download_lif(fields=("spikeCount",))["spikeCount"].sum()) > 0
