@@ -894,7 +894,7 @@ constexpr int DN_STAGES = 4;
 constexpr int DN_MAX_CHUNKS = 32;   // 2,048 slots per destination
 constexpr int DN_GROUP_WORDS = 4 * DN_MAX_CHUNKS / 32;
 constexpr int DN_LIGHT = 128;
-constexpr int DN_ACT_WORDS = 1280;  // the bitmap row is kept in shared memory up to 40,960 neurons
+constexpr int DN_ACT_WORDS = 1216;  // the bitmap row is kept in shared memory up to 38,912 neurons
 constexpr int dn_threads(int W) { return 32 * (1 + W + 1); }
 // Arrival warps a tile, and the blocks an SM then holds: 16, 8 or 4 warps by the tiles there are, one wave
 // of them in each form.  A heavy block's arrivals are chains of loads, and with four warps on an SM of
@@ -924,6 +924,13 @@ struct DenseSmem {
     uint64_t bfull[W], bempty[W];
     uint64_t scanned, summed, drawn;
 };
+// What a batch's block takes: beside this the descriptor's copy, and 1 KB of the SM's 228 that each block has.
+template <int W>
+constexpr bool dn_fits()
+{
+    return dn_blocks(W) * (sizeof(DenseSmem<W>) + (sizeof(NetDev) + 127) / 128 * 128 + 1024) <= 228 * 1024;
+}
+static_assert(dn_fits<4>() && dn_fits<8>() && dn_fits<16>(), "an SM holds dn_blocks(W) blocks");
 
 template <int W>
 __device__ __forceinline__ void bar_events()
