@@ -2415,41 +2415,52 @@ static void state_free(StateCopy &sc)
 }
 
 // Coordinate search over the launch parameters; trial(cfg) returns a time (ms) or < 0 on error.
+// blocks: the network runs blocks of steps.  What only the per-step kernels read is then timed on them
+// (calls too short for a block, and bg3_bench_steps, run them); blocks would time it as noise.
 template <typename Trial>
-static int tune(LaunchCfg &cur, bool thick, bool thin, int mq, bool batch, bool izh, Trial trial,
+static int tune(LaunchCfg &cur, bool thick, bool thin, int mq, bool batch, bool izh, bool blocks, Trial trial,
                 float &best_ms)
 {
     float t = trial(cur);
     if (t < 0) return (int)t;
     best_ms = t;
-    auto try_param = [&](int LaunchCfg::*field, std::initializer_list<int> values) -> int {
-        const int keep = cur.*field;
-        int best_v = keep;
-        for (int v : values) {
-            if (v == keep) continue;
-            cur.*field = v;
-            const float tv = trial(cur);
-            if (tv < 0) return (int)tv;
-            if (tv < best_ms) { best_ms = tv; best_v = v; }
+    float steps_ms = -1.0f;  // the best of the per-step kernels so far
+    auto try_param = [&](int LaunchCfg::*field, std::initializer_list<int> values, bool steps = false) -> int {
+        LaunchCfg c = cur;
+        if (steps && blocks) {
+            c.small_max_slots = 0;
+            if (steps_ms < 0 && (steps_ms = trial(c)) < 0) return (int)steps_ms;
         }
-        cur.*field = best_v;
+        float &best = steps && blocks ? steps_ms : best_ms;
+        for (int v : values) {
+            if (v == cur.*field) continue;
+            const int keep = c.*field;
+            c.*field = v;
+            const float tv = trial(c);
+            if (tv < 0) return (int)tv;
+            if (tv < best) best = tv;
+            else c.*field = keep;
+        }
+        cur.*field = c.*field;
+        if (!steps) steps_ms = -1.0f;  // may be of other kernels now
         return BG3_OK;
     };
     int rc;
-    if (thick && !batch && (rc = try_param(&LaunchCfg::sweep_dests, {16, 32}))) return rc;
-    if (thick && (rc = try_param(&LaunchCfg::sweep_stages, {4, 6, 8}))) return rc;
+    if (thick && !batch && (rc = try_param(&LaunchCfg::sweep_dests, {16, 32}, true))) return rc;
+    if (thick && (rc = try_param(&LaunchCfg::sweep_stages, {4, 6, 8}, true))) return rc;
     if (mq > 4 && mq <= 64 && (rc = try_param(&LaunchCfg::thin_max_quads, {mq - 1, mq}))) return rc;
-    if ((thin || mq <= 64) && (rc = try_param(&LaunchCfg::thin_warps, {4, 8, 16}))) return rc;
-    if ((rc = try_param(&LaunchCfg::deliver_blocks, {152, 304, 608}))) return rc;
-    if ((rc = try_param(&LaunchCfg::deliver_early, {0, 1}))) return rc;
+    if ((thin || mq <= 64) && (rc = try_param(&LaunchCfg::thin_warps, {4, 8, 16}, !batch))) return rc;
+    if ((rc = try_param(&LaunchCfg::deliver_blocks, {152, 304, 608}, true))) return rc;
+    if ((rc = try_param(&LaunchCfg::deliver_early, {0, 1}, true))) return rc;
     if (izh && (rc = try_param(&LaunchCfg::izh_hw_every, {-1, 0, 1, 2, 3, 4}))) return rc;
     return BG3_OK;
 }
 
-// Warm-up long enough to capture the step graph outside the timed region, then steps timed.
+// Warm-up long enough to capture the graph, of single steps or of blocks, outside the timed region.
+constexpr int WARM_STEPS = std::max(GRAPH_STEPS + 3, GRAPH_BLOCKS * BLK_MAX_STEPS);
 static float time_steps(bg3_net *n, int32_t steps)
 {
-    if (bg3_step(n, GRAPH_STEPS + 3) != BG3_OK) return -1.0f;
+    if (bg3_step(n, WARM_STEPS) != BG3_OK) return -1.0f;
     cudaEvent_t a, b;
     if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess) return -1.0f;
     cudaEventRecord(a, n->stream);
@@ -2480,7 +2491,7 @@ int bg3_autotune(bg3_net *n, int32_t steps, int32_t tune_growth, bg3_launch_cfg 
     };
     float ms = 0.0f;
     rc = tune(cur, !bg3::sweep_is_thin(h, cur), bg3::sweep_is_thin(h, cur), h.Mq, false,
-              h.neuron_kind == BG3_NEURON_IZH, trial, ms);
+              h.neuron_kind == BG3_NEURON_IZH, blk_steps(n, cur, bg3::small_eligible(h, cur)) > 0, trial, ms);
     if (rc == BG3_OK && tune_growth) {
         // the overlap pass: one growth pass per candidate block size from the saved state
         float best_g = -1.0f;
@@ -2515,7 +2526,7 @@ int bg3_autotune(bg3_net *n, int32_t steps, int32_t tune_growth, bg3_launch_cfg 
 
 static float time_batch_steps(bg3_batch *b, int32_t steps)
 {
-    if (bg3_batch_step(b, GRAPH_STEPS + 3) != BG3_OK) return -1.0f;
+    if (bg3_batch_step(b, WARM_STEPS) != BG3_OK) return -1.0f;
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return -1.0f;
     cudaEventRecord(e0, b->stream);
@@ -2557,7 +2568,7 @@ int bg3_batch_autotune(bg3_batch *b, int32_t steps, bg3_launch_cfg *best, float 
         return time_batch_steps(b, steps);
     };
     float ms = 0.0f;
-    if (rc == BG3_OK) rc = tune(cur, thick, thin, thin ? 1 << 30 : mq, true, izh, trial, ms);
+    if (rc == BG3_OK) rc = tune(cur, thick, thin, thin ? 1 << 30 : mq, true, izh, batch_blk_steps(b) > 0, trial, ms);
     int rc2 = BG3_OK;
     for (size_t k = 0; k < b->nets.size(); k++) {
         if (sc[k].buf && state_load(b->nets[k], sc[k]) != BG3_OK) rc2 = BG3_ECUDA;

@@ -510,3 +510,22 @@ def test_small_networks_in_calls_of_one_and_two_steps(noise, syn, w, h, radius, 
     if noise == bg.BG3_NOISE_INJECT:
         assert nets[0].noise_pending() == nets[1].noise_pending()
     assert int(nets[0].download_lif(fields=("spikeCount",))["spikeCount"].sum()) > 0
+
+
+def test_tuning_times_the_kernels_that_read_an_option():
+    """A network that runs in blocks: the per-step kernels' options are timed on those (delivery
+    grid and start, thin sweep), the batch's too."""
+    net, twin = (lif(50, 42, bg.BG3_SYN_DS, 1.55, "poisson", 40) for _ in range(2))
+    l0 = net.launches
+    net.autotune(steps_per_trial=50)
+    assert net.launches - l0 > 5 * 2 * 50      # five options off the default, two launches a step
+    batch = bg.Batch([net])
+    l0 = batch.launches
+    batch.autotune(steps_per_trial=50)
+    assert batch.launches - l0 > 3 * 2 * 50
+    assert batch.launch["small_max_slots"] == net.launch["small_max_slots"] == 65536
+    batch.step(40)
+    batch.sync()
+    twin.step(40)
+    same(net, twin, "tuned")
+    batch.close()
