@@ -1470,7 +1470,7 @@ int bg3_epoch_growth(bg3_net *n, int32_t epoch)
 {
     if (!n || epoch < 0) return BG3_EINVAL;
     bg3::launch_growth(n->h, n->d, epoch, n->cfg.growth_threads, n->stream);
-    n->launches += 8;
+    n->launches += 7;
     CK(cudaGetLastError());
     return BG3_OK;
 }

@@ -529,3 +529,10 @@ def test_tuning_times_the_kernels_that_read_an_option():
     twin.step(40)
     same(net, twin, "tuned")
     batch.close()
+
+
+def test_growth_pass_counts_its_launches():
+    net = lif(9, 7, bg.BG3_SYN_DS, 1.2, "none", 30)
+    l0 = net.launches
+    net.growth(1)
+    assert net.launches - l0 == 7
