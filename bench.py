@@ -339,9 +339,20 @@ def run_bg3(args):
             "clocks": clocks,
             "error_word": err,
         }
-        print(json.dumps(line), flush=True)
+        print_line(line)
     if world > 1:
         dist.destroy_process_group()
+
+
+def print_line(line):
+    """The one line of standard output, without the served streams' records of each job (23 KB with
+    64 of them, more than some readers keep of a line); those go to standard error."""
+    short = dict(line)
+    for k, v in line.items():
+        if isinstance(v, dict) and "per_job" in v:
+            short[k] = {a: b for a, b in v.items() if a != "per_job"}
+            print(json.dumps({k: {"per_job": v["per_job"]}}), file=sys.stderr, flush=True)
+    print(json.dumps(short), flush=True)
 
 
 def _alg_gbs(S, N, bytes_per_neuron, seconds_per_step):
