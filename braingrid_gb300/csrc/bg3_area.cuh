@@ -161,9 +161,20 @@ __device__ __forceinline__ float area_cos(float a, float r, float l, bool &ok)
 //   and the larger its cosine M.  At the node i / 128 nearest to m, with cosine c and angle g,
 //   asin(m) = g + asin(m c - M i / 128), the last argument below 1/181 so that its series is the
 //   argument itself and two terms in float.  acos(|x|) is that or pi/2 minus it, acos(x) pi minus that
-//   for x < 0: the largest error seen is 2^-42 of y + 2^-46, and twice that is allowed for.
+//   for x < 0.
 //   sin(2 y) = 2 x s; rounding y to y - lo turned the angle by -2 lo, so
 //   sin(r) = 2 x s - 2 lo cos(2 y); the next term, 2 lo^2 sin(2 y), is below 2^-45 of it.
+//
+//   Errors.  w is exact for x x >= 1/2 and to 2^-48 below.  rsqrt.approx is good to 2^-22.9 and s0 to
+//   2^-22.3, so one correction leaves 2^-44.4, its roundings (three of 2^-24 on a part of 2^-22.3) 2^-44.7:
+//   s to 2^-43.5 of itself.  That moves an asin(s) of a by 2^-43.5 tan a (at most 2^-43.2 a), and by way of
+//   M t, at most 1/2, an asin(|x|) by 2^-44.5.  The products' low parts, the node's and the sums are below
+//   2^-24 and round by 2^-48 each, about five of them; the base's low part, up to 2^-23.5, by 2^-47.5 twice:
+//   2^-45.7 in all, and 2^-47 without a base.  So y is within 2^-43.2 y + 2^-45.7 (2^-47 where y is an asin
+//   itself and may be small) of the angle, and 2^-41 y + 2^-45 is allowed for.  The sine takes 2^-43.5 of
+//   itself from s and twice the angle's error times the cosine: 2^-41.9 where it is near 1, 2^-41.5 of a for a
+//   small a, 2^-42.2 near pi; 2^-41 of it + 2^-42 is allowed for.  (Largest seen in 3e7 random pairs: 0.35
+//   and 0.43 of what is allowed.)
 __device__ __forceinline__ float area_segment(float x, bool &ok)
 {
     const float ax = fabsf(x);
@@ -182,7 +193,9 @@ __device__ __forceinline__ float area_segment(float x, bool &ok)
     const float p1 = m.hi * node.x, p2 = M.hi * t;
     const float e1 = __fmaf_rn(m.lo, node.x, __fmaf_rn(m.hi, node.y, __fmaf_rn(m.hi, node.x, -p1)));
     const float e2 = __fmaf_rn(M.lo, t, __fmaf_rn(M.hi, t, -p2));
-    const FF d = ff_fast_two_sum(p1 - p2, e1 - e2);  // p1 - p2 is exact: within a factor near 2, or p2 = 0
+    // p1 - p2 is exact: within a factor of two, both multiples of its last place at the first node's lower
+    // edge, or p2 = 0
+    const FF d = ff_fast_two_sum(p1 - p2, e1 - e2);
     const float uu = d.hi * d.hi;
     const float tail = __fmaf_rn(d.hi * uu, __fmaf_rn(uu, 0.075f, 0x1.555556p-3f), d.lo);
     FF y = ff_two_sum(node.z, d.hi);
