@@ -3,11 +3,13 @@
 // in [-300, 300]) and operand pairs that nearly cancel, for add, multiply and the conversion to
 // float.  bg3_selftest_izhikevich: the Izhikevich update's double expression evaluated on the
 // integer pipe and in float-float arithmetic, against the FP64 pipe.  bg3_selftest_overlap: the
-// growth rule's overlap area in float-float arithmetic against the FP64 pipe.  bg3_selftest_timeout: the bounded mbarrier wait of the step kernels, run out on purpose.
+// growth rule's overlap area in float-float arithmetic against the FP64 pipe.  bg3_selftest_stdp_sum:
+// the STDP weight sum, likewise.  bg3_selftest_timeout: the bounded mbarrier wait of the step kernels, run out on purpose.
 #include "../../include/bg3.h"
 #include "bg3_area.cuh"
 #include "bg3_internal.cuh"
 #include "bg3_ptx.cuh"
+#include "bg3_stdp.cuh"
 
 namespace {
 
@@ -158,6 +160,39 @@ __global__ void k_area_test(uint64_t n, uint64_t seed, unsigned long long *bad)
         if (local[k]) atomicAdd(&bad[k], local[k]);
 }
 
+// stdp_sum_ff against the double chain: efficacies in [0, 1] (1 - exp, multiples of 2^-24; some 0 or 1),
+// weights of a few nA, changes from 2^-40 of the weight to eight times it, of either sign, or nearly
+// its negative; and sets of any sizes, zeros among them.
+__global__ void k_stdp_sum_test(uint64_t n, uint64_t seed, unsigned long long *bad)
+{
+    unsigned long long local[2] = {0, 0};
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t r1 = mix64(seed ^ (3 * i)), r2 = mix64(seed ^ (3 * i + 1)), r3 = mix64(seed ^ (3 * i + 2));
+        const float f1 = (float)(r1 >> 40) * 0x1p-24f, f2 = (float)((r1 >> 16) & 0xffffffull) * 0x1p-24f;
+        const float f3 = (float)(r2 >> 40) * 0x1p-24f, f4 = (float)((r2 >> 16) & 0xffffffull) * 0x1p-24f;
+        float epost = (r1 & 15ull) == 0 ? 1.0f : (r1 & 15ull) == 1 ? 0.0f : f1;
+        float epre = (r1 & 0xf0ull) == 0 ? 1.0f : f2;
+        float W = (1.0f + f3) * exp2f(-28.0f - (float)(r2 & 7ull));
+        if (r2 & 8ull) W = -W;
+        float dw = (1.0f + f4) * exp2f((float)(r3 & 63ull) * (44.0f / 64.0f) - 41.0f) * W;
+        if (r2 & 16ull) dw = -dw;
+        const int kind = (int)((r3 >> 6) & 7ull);
+        if (kind == 0 && epost * epre > 0x1p-20f) dw = -W / (epost * epre) * (1.0f + (f4 - 0.5f) * 0x1p-18f);
+        if (kind == 1) {
+            W = (r3 & 512ull) ? 0.0f : W * exp2f((f3 - 0.5f) * 200.0f);
+            dw = (r3 & 1024ull) ? 0.0f : dw * exp2f((f4 - 0.5f) * 200.0f);
+        }
+        float a;
+        const bool ok = bg3::stdp_sum_ff(W, epost, epre, dw, a);
+        const float hw = (float)((double)W + (double)epost * (double)epre * (double)dw);
+        if (!ok) local[1]++;
+        else if (__float_as_uint(a) != __float_as_uint(hw)) local[0]++;
+    }
+    for (int k = 0; k < 2; k++)
+        if (local[k]) atomicAdd(&bad[k], local[k]);
+}
+
 // A wait that nothing ends: an mbarrier expecting one arrival that never comes, waited on by a
 // warp with the step kernels' bounded wait at limit_ns.  No copy targets the barrier, so the
 // block may leave it pending; the kernel records whether the wait gave up and how long it took,
@@ -251,5 +286,24 @@ extern "C" int bg3_selftest_overlap(uint64_t samples, uint64_t seed, uint64_t *c
     cudaFree(d);
     if (e1 != cudaSuccess || e2 != cudaSuccess) return BG3_ECUDA;
     for (int k = 0; k < 3; k++) counts[k] = h[k];
+    return BG3_OK;
+}
+
+extern "C" int bg3_selftest_stdp_sum(uint64_t samples, uint64_t seed, uint64_t *counts)
+{
+    if (!counts) return BG3_EINVAL;
+    unsigned long long *d = nullptr;
+    if (cudaMalloc(&d, 2 * sizeof(unsigned long long)) != cudaSuccess) return BG3_ENOMEM;
+    if (cudaMemset(d, 0, 2 * sizeof(unsigned long long)) != cudaSuccess) {
+        cudaFree(d);
+        return BG3_ECUDA;
+    }
+    k_stdp_sum_test<<<152 * 8, 256>>>(samples, seed, d);
+    unsigned long long h[2];
+    const cudaError_t e1 = cudaDeviceSynchronize();
+    const cudaError_t e2 = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e1 != cudaSuccess || e2 != cudaSuccess) return BG3_ECUDA;
+    for (int k = 0; k < 2; k++) counts[k] = h[k];
     return BG3_OK;
 }

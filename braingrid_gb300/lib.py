@@ -165,6 +165,8 @@ def load(build_if_missing=True):
                                      ctypes.POINTER(ctypes.c_uint64)], ctypes.c_int),
         "bg3_selftest_overlap": ([ctypes.c_uint64, ctypes.c_uint64, ctypes.POINTER(ctypes.c_uint64)],
                                  ctypes.c_int),
+        "bg3_selftest_stdp_sum": ([ctypes.c_uint64, ctypes.c_uint64, ctypes.POINTER(ctypes.c_uint64)],
+                                  ctypes.c_int),
         "bg3_selftest_binary64": ([ctypes.c_uint64, ctypes.c_uint64, ctypes.POINTER(ctypes.c_uint64)],
                                   ctypes.c_int),
         "bg3_get_launch": ([vp, ctypes.POINTER(LaunchCfg)], ctypes.c_int),
@@ -796,6 +798,14 @@ def selftest_overlap(samples=1 << 26, seed=1):
     c = (ctypes.c_uint64 * 4)()
     check(load().bg3_selftest_overlap(int(samples), int(seed), c), "bg3_selftest_overlap")
     return tuple(int(x) for x in c)[:3]
+
+
+def selftest_stdp_sum(samples=1 << 26, seed=1):
+    """(mismatches, sums handed to the FP64 pipe) of the STDP weight sum in float-float arithmetic
+    against the FP64 pipe."""
+    c = (ctypes.c_uint64 * 2)()
+    check(load().bg3_selftest_stdp_sum(int(samples), int(seed), c), "bg3_selftest_stdp_sum")
+    return tuple(int(x) for x in c)
 
 
 def selftest_izhikevich(samples=1 << 26, seed=1):

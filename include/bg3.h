@@ -399,6 +399,10 @@ int bg3_selftest_izhikevich(uint64_t samples, uint64_t seed, uint64_t *counts);
  * against the FP64 pipe on `samples` random pairs: counts[0..2] = mismatches, pairs handed to the
  * FP64 pipe, pairs drawn that need no angle.  No counterpart in the reference. */
 int bg3_selftest_overlap(uint64_t samples, uint64_t seed, uint64_t *counts);
+/* The STDP weight sum (W + epost * epre * dw in double, rounded to float) in float-float arithmetic
+ * against the FP64 pipe on `samples` random operand sets: counts[0..1] = mismatches, sums handed to
+ * the FP64 pipe.  No counterpart in the reference. */
+int bg3_selftest_stdp_sum(uint64_t samples, uint64_t seed, uint64_t *counts);
 /* Failure-detection self-test: one warp waits, with the bounded mbarrier wait the step kernels
  * use, on a barrier that nothing completes, for at most limit_ns (1 .. 2e9).  The wait gives up,
  * the kernel returns normally and the context stays usable: *status = BG3_ERR_TIMEOUT, and

@@ -536,3 +536,41 @@ def test_growth_pass_counts_its_launches():
     l0 = net.launches
     net.growth(1)
     assert net.launches - l0 == 7
+
+
+@pytest.mark.parametrize("seed", [5, 6])
+def test_stdp_sum_matches_fp64(seed):
+    """The STDP weight sum in float-float arithmetic gives the FP64 pipe's bits; what is uncertain, or far
+    in size from the weight, is handed back."""
+    n = 1 << 25
+    bad, handed = bg.selftest_stdp_sum(samples=n, seed=seed)
+    assert bad == 0
+    assert handed < 3 * n // 4, handed      # about a third of the changes are below 2^-60
+
+
+@pytest.mark.parametrize("syn", [bg.BG3_SYN_SPIKING, bg.BG3_SYN_DS, bg.BG3_SYN_STDP, bg.BG3_SYN_DYNSTDP])
+def test_thin_blocks_of_one_warp_a_tile(syn):
+    """657 tiles: more than four warps a tile are used for."""
+    nets = [lif(150, 140, syn, 1.5, "poisson", 33) for _ in range(2)]
+    nets[1].set_launch(small_max_slots=0)
+    for n in (8, 3, 130):
+        for net in nets:
+            net.step(n)
+    same(nets[0], nets[1], "one warp a tile")
+    assert nets[0].launches < nets[1].launches
+    assert int(nets[0].download_lif(fields=("spikeCount",))["spikeCount"].sum()) > 0
+    for net in nets:
+        net.close()
+
+
+@pytest.mark.parametrize("w,h", [(197, 196), (200, 197)])   # 1,207 and 1,232 tiles
+def test_dense_blocks_past_the_bitmap_in_shared_memory(w, h):
+    nets = [few_firing(w, h, bg.BG3_SYN_DS, 29, 0, 84, 2.3)[0] for _ in range(2)]
+    nets[1].set_launch(small_max_slots=0)
+    for n in (8, 8, 21):
+        for net in nets:
+            net.step(n)
+    same(nets[0], nets[1], "%dx%d" % (w, h))
+    assert nets[0].launches < nets[1].launches
+    for net in nets:
+        net.close()
