@@ -357,7 +357,9 @@ static int exp_table(bg3_net *n, int kind, float tau, int len, const T **out)
             g_exp.erase(key);
             return BG3_ENOMEM;
         }
-        if (cudaMemcpy(t.dev, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) {
+        // complete before the lock is left: the next network's stream does not wait for this one's
+        if (cudaMemcpyAsync(t.dev, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, n->stream) != cudaSuccess ||
+            cudaStreamSynchronize(n->stream) != cudaSuccess) {
             cudaFree(t.dev);
             g_exp.erase(key);
             return BG3_ECUDA;
@@ -607,10 +609,9 @@ int bg3_create(const bg3_net_desc *desc, bg3_net **out)
         h.t_r0 = 1.0f;
     }
     if ((rc = make_tensor_maps(n)) != 0) goto fail;
-    if (cudaMemcpy(n->d, &h, sizeof(NetDev), cudaMemcpyHostToDevice) != cudaSuccess) {
-        rc = BG3_ECUDA;
-        goto fail;
-    }
+    // on the network's own stream, as every copy is: one on the default stream may still be on its way when
+    // it returns, and would land on top of a later descriptor where other threads keep that stream busy
+    if ((rc = push_desc(n)) != 0) goto fail;
     for (int t = 0; t < 4 && (h.syn_kind == BG3_SYN_DS || h.syn_kind == BG3_SYN_DYNSTDP); t++) {
         const int c = param_class(n, h.t_U[t], h.t_D[t], h.t_F[t]);
         if (c < 0) { rc = c; goto fail; }
@@ -2934,7 +2935,8 @@ int bg3_checkpoint_load(bg3_net *n, const void *buf, uint64_t len)
     {                                                                                             \
         if ((rc = aresize(n, h.f, (size_t)as[CKA_##f]))) return rc;                               \
         if (as[CKA_##f])                                                                          \
-            CK(cudaMemcpy((void *)h.f, ap[CKA_##f], (size_t)as[CKA_##f], cudaMemcpyHostToDevice)); \
+            CK(cudaMemcpyAsync((void *)h.f, ap[CKA_##f], (size_t)as[CKA_##f], cudaMemcpyHostToDevice,  \
+                               n->stream));                                                       \
     }
     BG3_NET_ARRAYS(BG3_LOAD_ONE)
 #undef BG3_LOAD_ONE
@@ -2949,8 +2951,8 @@ int bg3_checkpoint_load(bg3_net *n, const void *buf, uint64_t len)
             n->noise_dev = nullptr;
             return BG3_ENOMEM;
         }
-        CK(cudaMemcpy(n->noise_dev, noise, (size_t)hd.noise_count * sizeof(float),
-                      cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(n->noise_dev, noise, (size_t)hd.noise_count * sizeof(float),
+                           cudaMemcpyHostToDevice, n->stream));
         n->noise_cap = hd.noise_count;
     }
     // the saved scalars with this network's pointers; exp tables of the saved time constants

@@ -574,3 +574,40 @@ def test_dense_blocks_past_the_bitmap_in_shared_memory(w, h):
     assert nets[0].launches < nets[1].launches
     for net in nets:
         net.close()
+
+
+@pytest.mark.parametrize("syn", [bg.BG3_SYN_SPIKING, bg.BG3_SYN_DYNSTDP])
+def test_networks_do_not_wait_for_the_default_stream(syn):
+    """A network made, grown, saved and loaded while the program's default stream is busy: nothing
+    of it comes after later calls, or has to wait."""
+    torch = pytest.importorskip("torch")
+    twin = lif(13, 5, syn, 1.5, "none", 40)          # and the process's shared tables
+    torch.cuda.synchronize()
+    busy = torch.cuda.Event()
+    torch.cuda._sleep(1 << 30)                        # half a second on the default stream
+    busy.record()
+    net = lif(13, 5, syn, 1.5, "none", 40)
+    net.step(100)
+    net.record()
+    net.sync()
+    early = not busy.query()
+    buf = twin.checkpoint()                           # through the default stream: waits
+    torch.cuda.synchronize()
+    assert early
+    twin.step(100)
+    twin.record()
+    net.growth(2)
+    twin.growth(2)
+    for n in (net, twin):
+        n.step(30)
+    same(net, twin, "made beside a busy default stream")
+    loaded = lif(13, 5, syn, 1.5, "none", 40)
+    torch.cuda._sleep(1 << 28)
+    loaded.load_checkpoint(buf)
+    loaded.step(100)
+    loaded.record()
+    loaded.growth(2)
+    loaded.step(30)
+    loaded.sync()
+    torch.cuda.synchronize()
+    same(loaded, twin, "loaded beside a busy default stream")
