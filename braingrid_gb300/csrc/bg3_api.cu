@@ -58,6 +58,8 @@ static const int SMALL_STEPS = 4096;  // steps per launch of a small network (bg
 // kernels one step launches after its neuron pass: delivery (+ post-spike STDP) and the sweep
 static inline int step_kernels(int syn_kind) { return syn_kind >= BG3_SYN_STDP ? 3 : 2; }
 
+static const int HIST_EMPTY = 1 << 30;
+
 struct bg3_net {
     bg3_net_desc desc;
     NetDev h;                 // host copy of the device descriptor
@@ -84,11 +86,12 @@ struct bg3_net {
     // whichever ran last is current, the other is rebuilt when it is needed
     BlkDev blk = {};
     bool ring_ok = true, mask_ok = false;
-    // fewest steps between two spikes of a neuron in the history rings, for the block kernels' STDP
-    // rule: the shortest refractory period + 1 of any in force while steps were made, or 1 once
-    // histories, or what their spacing follows from, were uploaded beside earlier steps
-    int min_isi = 1;
-    bool hist_given = false, stepped = false;
+    // fewest steps between two spikes of a neuron, for the block kernels' STDP rule: of those in the
+    // history rings (HIST_EMPTY: none) and of those to come (the shortest refractory period + 1)
+    int ring_isi = HIST_EMPTY, refr_isi = 1;
+    // the rings may not hold each neuron's last spikes in order with the unused entries before them:
+    // uploads can put in anything, which the walks then find at other steps than a block looks
+    bool hist_odd = false;
     // STDP kinds: steps until every spike under way that the histories may lack has arrived (it came
     // with uploaded delay queues, or was under way when the histories were replaced)
     int queued = 0;
@@ -709,16 +712,55 @@ int bg3_destroy(bg3_net *n)
     return BG3_OK;
 }
 
-// Fewest steps between two spikes of any neuron with these refractory periods.  Spikes made with
-// earlier, shorter ones may still be in the rings.
-static void set_min_isi(bg3_net *n, const float *Trefract)
+// Fewest steps between two spikes of any neuron with these refractory periods.
+static int refractory_isi(const bg3_net *n, const float *Trefract)
 {
-    int m = 1 << 30;
+    int m = HIST_EMPTY;
     for (int i = 0; i < n->h.N; i++) {
         const double r = (double)(Trefract[i] / n->h.dt) + 0.5;
         m = std::min(m, r > 0.0 && r < 1e9 ? (int)r + 1 : 1);
     }
-    n->min_isi = n->stepped ? std::min(n->min_isi, m) : m;
+    return m;
+}
+// Fewest steps between two entries of any neuron's history (HIST_EMPTY: no two), 0 where one is out of
+// order: backwards from the newest, times fall, and nothing follows an unused entry.
+static int history_isi(const bg3_net *n, const uint64_t *hist, const int32_t *count, const int32_t *offset)
+{
+    const int ms = n->h.max_spikes;
+    uint64_t least = HIST_EMPTY;
+    for (int i = 0; i < n->h.N; i++) {
+        const uint64_t *h = hist + (size_t)i * ms;
+        int at = (int)((((int64_t)count[i] + offset[i]) % ms + ms) % ms);
+        uint64_t newer = BG3_ULONG_MAX;
+        bool used = true, first = true;
+        for (int k = 0; k < ms; k++) {
+            at = at ? at - 1 : ms - 1;
+            const uint64_t t = h[at];
+            used = used && t != BG3_ULONG_MAX;
+            if (!used && t == BG3_ULONG_MAX) continue;
+            if (!used || t >= newer) return 0;
+            if (!first) least = std::min(least, newer - t);
+            newer = t;
+            first = false;
+        }
+    }
+    return (int)least;
+}
+// The rings as uploaded or loaded.  One interval, from the newest entry to the next spike, is not in
+// them; the rule has room for it.
+static void history_given(bg3_net *n, const uint64_t *hist, const int32_t *count, const int32_t *offset)
+{
+    if (n->h.syn_kind < BG3_SYN_STDP) return;
+    const int isi = history_isi(n, hist, count, offset);
+    n->hist_odd = isi == 0;
+    n->ring_isi = isi;
+}
+// Steps that bg3_net::queued waits for, and whose spikes the rings take.
+static void steps_made(bg3_net *n, int64_t nsteps)
+{
+    if (nsteps <= 0) return;
+    n->queued = (int)std::max<int64_t>(0, n->queued - nsteps);
+    n->ring_isi = std::min(n->ring_isi, n->refr_isi);
 }
 
 // The spike ring, brought up to date from the masks (queued on the network's stream).
@@ -754,14 +796,18 @@ int bg3_upload_lif(bg3_net *n, const bg3_lif_arrays *a)
         (rc = h2d(n, (uint64_t *)h.history, a->history, N * (size_t)h.max_spikes)))
         return rc;
     CK(cudaStreamSynchronize(n->stream));
-    // once there are spikes, a neuron whose refractory steps are set anew may fire sooner after its
-    // last one, and other counts put the entries in another order
-    if (a->history || (n->stepped && (a->nStepsInRefr || a->spikeCount || a->spikeCountOffset)))
-        n->hist_given = true;
-    // and the histories given may lack spikes under way
-    if (n->stepped && n->h.syn_kind >= BG3_SYN_STDP && (a->history || a->spikeCount || a->spikeCountOffset))
-        n->queued = 31;
-    if (a->Trefract) set_min_isi(n, a->Trefract);
+    if (a->Trefract) n->refr_isi = refractory_isi(n, a->Trefract);
+    if (h.syn_kind < BG3_SYN_STDP) return BG3_OK;
+    const bool spikes = n->ring_isi != HIST_EMPTY || n->hist_odd;
+    const bool parts = a->history || a->spikeCount || a->spikeCountOffset;
+    if (a->history && a->spikeCount && a->spikeCountOffset) {
+        history_given(n, a->history, a->spikeCount, a->spikeCountOffset);
+    } else {
+        // the entries apart from what places them; or a spike may follow its neuron's last one sooner
+        n->hist_odd = n->hist_odd || a->history || (parts && spikes);
+        if (a->nStepsInRefr && spikes) n->ring_isi = 1;
+    }
+    if (parts && spikes) n->queued = 31;  // the new histories may lack spikes under way
     return BG3_OK;
 }
 
@@ -1251,7 +1297,7 @@ static unsigned long long blk_window(const bg3_net *n)
 // for the destination's own spikes), the host build's spike-time arithmetic (its pre-spike walks
 // read only the destination's own history), and a history ring long enough that the spikes a
 // block adds never overwrite an entry a post-spike walk reads (entries within 3 tau+, at most one
-// per min_isi steps), and no spike under way that the histories may lack (bg3_net::queued): post-spike
+// per ring_isi or refr_isi steps), histories in order, and no spike under way that the histories may lack (bg3_net::queued): post-spike
 // learning after a block relies on them to hold the spikes that arrive in it.
 static bool blk_is_thin(const NetDev &h, const LaunchCfg &c)
 {
@@ -1270,11 +1316,11 @@ static int blk_steps(const bg3_net *n, const LaunchCfg &c, bool small = false)
         return 0;
     }
     if (h.syn_kind >= BG3_SYN_STDP) {
-        if (h.stdp_signed || n->queued > 0) return 0;
+        if (h.stdp_signed || n->queued > 0 || n->hist_odd) return 0;
         float tau = 0.0f;
         for (const StdpConst &s : h.stdp) tau = std::max(tau, s.taupos);
         if (!(tau >= 0.0f) || !(tau < 1e3f)) return 0;
-        const int isi = n->hist_given ? 1 : n->min_isi;
+        const int isi = std::max(1, std::min(n->ring_isi, n->refr_isi));
         const double window = 3.0 * (double)tau / (double)h.dt + 1.0;
         if (window / isi + BLK_MAX_STEPS + 4.0 > (double)h.max_spikes) return 0;
     }
@@ -1355,7 +1401,6 @@ static int run_blocks(bg3_net *n, int64_t nsteps, int T)
 static int run_form(bg3_net *n, int64_t nsteps)
 {
     if (nsteps <= 0) return BG3_OK;
-    n->stepped = true;
     const NetDev &h = n->h;
     int rc;
     const bool small = bg3::small_eligible(h, n->cfg);
@@ -1451,19 +1496,13 @@ static int run_form(bg3_net *n, int64_t nsteps)
     return BG3_OK;
 }
 
-// Steps that bg3_net::queued waits for were made.
-static void steps_made(bg3_net *n, int64_t nsteps)
-{
-    n->queued = (int)std::max<int64_t>(0, n->queued - nsteps);
-}
-
 int bg3_step(bg3_net *n, int64_t nsteps)
 {
     if (!n || nsteps < 0) return BG3_EINVAL;
     const int64_t first = std::min<int64_t>(nsteps, n->queued);  // in the form blk_steps gives them
     int rc = run_form(n, first);
     if (rc) return rc;
-    steps_made(n, first);
+    steps_made(n, nsteps);
     return run_form(n, nsteps - first);
 }
 
@@ -2049,7 +2088,6 @@ static int batch_rings(bg3_batch *b)
         const int rc = ensure_ring(n);
         if (rc) return rc;
         n->mask_ok = false;
-        n->stepped = true;
     }
     return BG3_OK;
 }
@@ -2061,7 +2099,6 @@ static int batch_run_blocks(bg3_batch *b, int64_t nsteps, int T)
     for (size_t k = 0; k < b->nets.size(); k++) {
         if ((rc = ensure_masks(b->nets[k]))) return rc;
         b->nets[k]->ring_ok = false;
-        b->nets[k]->stepped = true;
         same = same && !memcmp(&b->blks[k], &b->nets[k]->blk, sizeof(BlkDev));
     }
     if ((rc = batch_order(b, true))) return rc;
@@ -2137,7 +2174,7 @@ int bg3_batch_step(bg3_batch *b, int64_t nsteps)
     first = std::min(first, nsteps);
     int rc = batch_run_form(b, first);
     if (rc) return rc;
-    for (bg3_net *n : b->nets) steps_made(n, first);
+    for (bg3_net *n : b->nets) steps_made(n, nsteps);
     return batch_run_form(b, nsteps - first);
 }
 
@@ -2181,7 +2218,6 @@ int bg3_bench_steps(bg3_net *n, int64_t nsteps, int64_t flush_bytes, float *step
     const int ring_rc = ensure_ring(n);
     if (ring_rc) return ring_rc;
     n->mask_ok = false;
-    n->stepped = true;
     steps_made(n, nsteps);
     const NetDev &h = n->h;
     const bool inject = h.noise_mode == BG3_NOISE_INJECT;
@@ -2367,13 +2403,14 @@ int bg3_batch_set_launch(bg3_batch *b, const bg3_launch_cfg *c)
 struct StateCopy {
     void *buf = nullptr;
     std::vector<std::pair<void *, size_t>> parts;
-    int queued = 0;
+    int queued = 0, ring_isi = 0;
 };
 
 static int state_save(bg3_net *n, StateCopy &sc)
 {
     sc.parts.clear();
     sc.queued = n->queued;
+    sc.ring_isi = n->ring_isi;
     const int rc = ensure_ring(n);
     if (rc) return rc;
     for (auto &a : n->allocs)
@@ -2400,6 +2437,7 @@ static int state_load(bg3_net *n, const StateCopy &sc)
 {
     ring_changed(n);
     n->queued = sc.queued;
+    n->ring_isi = sc.ring_isi;
     size_t off = 0;
     for (auto &p : sc.parts) {
         CK(cudaMemcpyAsync(p.first, (const char *)sc.buf + off, p.second, cudaMemcpyDeviceToDevice, n->stream));
@@ -2929,7 +2967,18 @@ int bg3_checkpoint_load(bg3_net *n, const void *buf, uint64_t len)
     CK(cudaStreamSynchronize(n->stream));
     drop_graph(n);
     ring_changed(n);
-    n->hist_given = n->stepped = true;
+    {
+        // copies: the buffer's arrays lie at any address
+        std::vector<float> refract(N);
+        std::vector<int32_t> count(N), offset(N);
+        std::vector<uint64_t> hist(n->h.syn_kind >= BG3_SYN_STDP ? N * (uint64_t)h.max_spikes : 0);
+        memcpy(refract.data(), ap[CKA_Trefract], N * sizeof(float));
+        memcpy(count.data(), ap[CKA_spikeCount], N * sizeof(int32_t));
+        memcpy(offset.data(), ap[CKA_spikeCountOffset], N * sizeof(int32_t));
+        memcpy(hist.data(), ap[CKA_history], hist.size() * sizeof(uint64_t));
+        n->refr_isi = refractory_isi(n, refract.data());
+        history_given(n, hist.data(), count.data(), offset.data());
+    }
     n->queued = n->h.syn_kind >= BG3_SYN_STDP ? 31 : 0;  // saved with uploaded spikes under way, perhaps
 #define BG3_LOAD_ONE(f)                                                                           \
     {                                                                                             \

@@ -611,3 +611,46 @@ def test_networks_do_not_wait_for_the_default_stream(syn):
     loaded.sync()
     torch.cuda.synchronize()
     same(loaded, twin, "loaded beside a busy default stream")
+
+
+@pytest.mark.parametrize("small", [1, 65536])
+def test_histories_out_of_order(small):
+    """Offsets that put the next entries two places before the ring's end, unused, with the valid
+    ones after them: the ring's fullness, which an arrival flags, comes with the third spike, where a ring
+    in order would be almost empty."""
+    nets = [firing_at_intervals(41, 700) for _ in range(2)]
+    nets[0].set_launch(small_max_slots=small)
+    nets[1].set_launch(small_max_slots=0)
+    for net in nets:
+        net.step(200)
+        count = net.download_lif(fields=("spikeCount",))["spikeCount"]
+        assert count.min() > 2 and count.max() < 8
+        net.upload_lif(spikeCountOffset=(698 - count).astype(np.int32))
+        for n in (40, 5, 100):
+            net.step(n)
+    same(nets[0], nets[1], "out of order")
+    assert nets[0].error_word != 0
+
+
+@pytest.mark.parametrize("form", ["upload", "checkpoint"])
+def test_a_resumed_stdp_network_runs_in_blocks(form):
+    """Histories in order, uploaded or loaded, have the spacing that is found in them."""
+    nets = [firing_at_intervals(41, 60) for _ in range(3)]
+    for net in nets:
+        net.set_launch(small_max_slots=1)
+    nets[1].set_launch(small_max_slots=0)
+    for net in nets[:2]:
+        net.step(300)
+        net.record()
+        net.step(100)
+    if form == "upload":
+        nets[2].upload_lif(**nets[0].download_lif())
+        nets[2].upload_synapses(nets[0].sim_step, **nets[0].download_synapses())
+    else:
+        nets[2].load_checkpoint(nets[0].checkpoint())
+    l0 = nets[2].launches
+    for net in nets:
+        net.step(331)
+    assert nets[2].launches - l0 < 31 * 4 + 2 * 40     # step by step while spikes are under way, then blocks
+    same(nets[0], nets[1], "went on")
+    same(nets[2], nets[1], "resumed")
