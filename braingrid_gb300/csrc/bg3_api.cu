@@ -86,6 +86,7 @@ struct bg3_net {
     // whichever ran last is current, the other is rebuilt when it is needed
     BlkDev blk = {};
     bool ring_ok = true, mask_ok = false;
+    int short_calls = 0;  // calls of one or two steps in a row on a small network's masks
     // fewest steps between two spikes of a neuron, for the block kernels' STDP rule: of those in the
     // history rings (HIST_EMPTY: none) and of those to come (the shortest refractory period + 1)
     int ring_isi = HIST_EMPTY, refr_isi = 1;
@@ -1408,7 +1409,12 @@ static int run_form(bg3_net *n, int64_t nsteps)
     // a cluster's start, with every tile's state on its way into it, is more than one or two steps of a few
     // tiles in one CTA: 10x10 with 80 rows, calls of one step 12.6 and 8.6 us, of two 12.8 and 11.3, of three
     // 14.1 and 14.9; 16x16 with 30 rows 9.9 and 8.1, 10.5 and 10.8; 24x24 (18 tiles) one step 10.2 and 11.2
-    if (small && nsteps <= 2 && nsteps * h.ntiles <= 16) T = 0;
+    // (from the fourth such call in a row where the masks are current: their ring costs 5 us)
+    if (small && nsteps <= 2 && nsteps * h.ntiles <= 16) {
+        if (n->ring_ok || ++n->short_calls > 3) T = 0;
+    } else {
+        n->short_calls = 0;
+    }
     if (T && !small && !blk_is_thin(h, n->cfg) && !dense_pays(nsteps, T, h.Mq, h.ntiles, 3)) T = 0;
     if (T && small) {
         // a small network: up to SMALL_STEPS whole steps per launch
