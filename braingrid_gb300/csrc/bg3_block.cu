@@ -25,6 +25,7 @@
 #include <cuda.h>
 #include <algorithm>
 #include <utility>
+#define BG3_RARE __noinline__
 #include "bg3_internal.cuh"
 #include "bg3_ptx.cuh"
 #include "bg3_stdp.cuh"

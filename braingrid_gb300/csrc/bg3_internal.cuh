@@ -225,9 +225,13 @@ enum : uint32_t {
 // the reference's x86-64 build.  expf of the reference's host library is correctly rounded for
 // almost every argument; evaluating exp in double and rounding once reproduces that.
 __device__ __forceinline__ float exp_cr(float x) { return (float)exp((double)x); }
-// The same out of line, where a table covers all but far intervals: the double exp's code stays out
-// of the step loops.
-static __device__ __noinline__ float exp_far(float x) { return exp_cr(x); }
+// Code that few steps reach (an exp past its table, an interval's draw, the integer-pipe arithmetic): out
+// of line in the block kernels' step loops (bg3_block.cu), inline in the per-step kernels, where a call
+// costs the registers it may change: the fused sweeps spilled 28 bytes with calls, 18.7 us instead of 18.1 (100x100, driven).
+#ifndef BG3_RARE
+#define BG3_RARE __forceinline__
+#endif
+static __device__ BG3_RARE float exp_far(float x) { return exp_cr(x); }
 __device__ __forceinline__ float acos_cr(float x) { return (float)acos((double)x); }
 __device__ __forceinline__ float sin_cr(float x) { return (float)sin((double)x); }
 
@@ -631,9 +635,8 @@ __device__ __forceinline__ float izh_v_ff(float Vint, float u, float C3, float c
     return Vnew;
 }
 
-// The same expression in integer-pipe binary64 (SoftD); ok = false outside its range.  Not
-// inlined: a launch option, kept out of the step loops' instruction footprint.
-static __device__ __noinline__ float izh_v_soft(float Vint, float u, float C3, float c2sp, bool &ok)
+// The same expression in integer-pipe binary64 (SoftD); ok = false outside its range.
+static __device__ BG3_RARE float izh_v_soft(float Vint, float u, float C3, float c2sp, bool &ok)
 {
     // the double constants 0.04, 140.0 and 0.001 as (mantissa, exponent, sign)
     constexpr SoftD K004 = {0x147ae147ae147bull, -5, 0u};
@@ -744,8 +747,7 @@ __device__ __forceinline__ bool neuron_apply(const NetDev &n, int i, const Neuro
 // One Poisson inter-spike interval in steps (HostSInputPoisson.cpp:81-84): exponential with mean
 // lambda ms, rejected while U <= exp(-isi^2 / 32).  Injected draws replay the reference's own
 // sequence; otherwise a Philox stream keyed by (seed, neuron, draw index).
-// Out of line: one draw per interval, not per step.
-static __device__ __noinline__ int32_t next_isi(const NetDev &n, int i)
+static __device__ BG3_RARE int32_t next_isi(const NetDev &n, int i)
 {
     const int32_t k = n.isi_cursor[i];
     gst(&n.isi_cursor[i], k + 1);
