@@ -58,7 +58,7 @@ static const int SMALL_STEPS = 4096;  // steps per launch of a small network (bg
 // kernels one step launches after its neuron pass: delivery (+ post-spike STDP) and the sweep
 static inline int step_kernels(int syn_kind) { return syn_kind >= BG3_SYN_STDP ? 3 : 2; }
 
-static const int HIST_EMPTY = 1 << 30;
+static const int HIST_EMPTY = 0x3f3f3f3f;  // four equal bytes, for cudaMemsetAsync
 
 struct bg3_net {
     bg3_net_desc desc;
@@ -123,7 +123,8 @@ static int dalloc(bg3_net *n, T **p, size_t count, int fill = 0)
     return BG3_OK;
 }
 
-static size_t blk_act_bytes(size_t Np) { return BLK_ACT_ROWS * (Np / 32) * sizeof(uint32_t); }
+// the bitmap rows, and a word for k_hist_isi
+static size_t blk_act_bytes(size_t Np) { return (BLK_ACT_ROWS * (Np / 32) + 1) * sizeof(uint32_t); }
 // A dense block's counts, flags and step masks (one allocation, in this order); 0 for networks that
 // never run one.
 static size_t blk_dense_bytes(size_t Np, int Mq)
@@ -723,38 +724,49 @@ static int refractory_isi(const bg3_net *n, const float *Trefract)
     }
     return m;
 }
-// Fewest steps between two entries of any neuron's history (HIST_EMPTY: no two), 0 where one is out of
-// order: backwards from the newest, times fall, and nothing follows an unused entry.
-static int history_isi(const bg3_net *n, const uint64_t *hist, const int32_t *count, const int32_t *offset)
+// Fewest steps between two entries of any neuron's history (*least HIST_EMPTY before: no two), 0 where one
+// is out of order: backwards from the newest, times fall, and nothing follows an unused entry.  A warp a
+// neuron, 32 entries at a time.
+static __global__ void __launch_bounds__(256) k_hist_isi(const unsigned long long *hist, const int32_t *count,
+                                                         const int32_t *offset, int N, int ms, int *least)
 {
-    const int ms = n->h.max_spikes;
-    uint64_t least = HIST_EMPTY;
-    for (int i = 0; i < n->h.N; i++) {
-        const uint64_t *h = hist + (size_t)i * ms;
-        int at = (int)((((int64_t)count[i] + offset[i]) % ms + ms) % ms);
-        uint64_t newer = BG3_ULONG_MAX;
-        bool used = true, first = true;
-        for (int k = 0; k < ms; k++) {
-            at = at ? at - 1 : ms - 1;
-            const uint64_t t = h[at];
-            used = used && t != BG3_ULONG_MAX;
-            if (!used && t == BG3_ULONG_MAX) continue;
-            if (!used || t >= newer) return 0;
-            if (!first) least = std::min(least, newer - t);
-            newer = t;
-            first = false;
+    const int lane = threadIdx.x & 31, i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (i >= N) return;
+    const unsigned long long *h = hist + (size_t)i * ms;
+    const int at0 = (int)((((long long)count[i] + offset[i]) % ms + ms) % ms);  // one past the newest
+    unsigned long long newer = BG3_ULONG_MAX;  // the entry before this lane's, none before the newest
+    bool ended = false;
+    int isi = HIST_EMPTY;
+    for (int k0 = 0; k0 < ms; k0 += 32) {
+        const int k = k0 + lane, at = at0 - 1 - k;
+        const unsigned long long t = k < ms ? h[at < 0 ? at + ms : at] : BG3_ULONG_MAX;
+        unsigned long long b = __shfl_up_sync(0xffffffffu, t, 1);
+        if (lane == 0) b = newer;
+        if (t != BG3_ULONG_MAX) {
+            if (ended || t >= b || (k > 0 && b == BG3_ULONG_MAX)) isi = 0;
+            else if (k > 0) isi = (int)min((unsigned long long)isi, b - t);
         }
+        newer = __shfl_sync(0xffffffffu, t, 31);
+        ended = ended || __any_sync(0xffffffffu, t == BG3_ULONG_MAX);
     }
-    return (int)least;
+    isi = __reduce_min_sync(0xffffffffu, isi);
+    if (lane == 0 && isi < HIST_EMPTY) atomicMin(least, isi);
 }
-// The rings as uploaded or loaded.  One interval, from the newest entry to the next spike, is not in
+// The rings after an upload or a load.  One interval, from the newest entry to the next spike, is not in
 // them; the rule has room for it.
-static void history_given(bg3_net *n, const uint64_t *hist, const int32_t *count, const int32_t *offset)
+static int histories_given(bg3_net *n)
 {
-    if (n->h.syn_kind < BG3_SYN_STDP) return;
-    const int isi = history_isi(n, hist, count, offset);
+    const NetDev &h = n->h;
+    int *least = (int *)(n->blk.act + BLK_ACT_ROWS * h.ntiles), isi = 0;
+    CK(cudaMemsetAsync(least, HIST_EMPTY & 255, sizeof(int), n->stream));
+    k_hist_isi<<<(h.N + 7) / 8, 256, 0, n->stream>>>(h.history, h.spikeCount, h.spikeCountOffset, h.N,
+                                                     h.max_spikes, least);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&isi, least, sizeof(int), cudaMemcpyDeviceToHost, n->stream));
+    CK(cudaStreamSynchronize(n->stream));
     n->hist_odd = isi == 0;
     n->ring_isi = isi;
+    return BG3_OK;
 }
 // Steps that bg3_net::queued waits for, and whose spikes the rings take.
 static void steps_made(bg3_net *n, int64_t nsteps)
@@ -796,19 +808,16 @@ int bg3_upload_lif(bg3_net *n, const bg3_lif_arrays *a)
         (rc = h2d(n, h.spikeCountOffset, a->spikeCountOffset, N)) ||
         (rc = h2d(n, (uint64_t *)h.history, a->history, N * (size_t)h.max_spikes)))
         return rc;
+    // STDP kinds: what their blocks take for granted of the histories
+    const bool stdp = h.syn_kind >= BG3_SYN_STDP, parts = a->history || a->spikeCount || a->spikeCountOffset;
+    const bool spikes = n->ring_isi != HIST_EMPTY || n->hist_odd;
+    if (stdp && parts && (rc = histories_given(n))) return rc;
     CK(cudaStreamSynchronize(n->stream));
     if (a->Trefract) n->refr_isi = refractory_isi(n, a->Trefract);
-    if (h.syn_kind < BG3_SYN_STDP) return BG3_OK;
-    const bool spikes = n->ring_isi != HIST_EMPTY || n->hist_odd;
-    const bool parts = a->history || a->spikeCount || a->spikeCountOffset;
-    if (a->history && a->spikeCount && a->spikeCountOffset) {
-        history_given(n, a->history, a->spikeCount, a->spikeCountOffset);
-    } else {
-        // the entries apart from what places them; or a spike may follow its neuron's last one sooner
-        n->hist_odd = n->hist_odd || a->history || (parts && spikes);
-        if (a->nStepsInRefr && spikes) n->ring_isi = 1;
+    if (stdp && spikes) {
+        if (parts) n->queued = 31;  // the histories may lack spikes under way
+        if (a->nStepsInRefr && !a->history) n->ring_isi = 1;  // a spike may follow its neuron's last one sooner
     }
-    if (parts && spikes) n->queued = 31;  // the new histories may lack spikes under way
     return BG3_OK;
 }
 
@@ -2974,16 +2983,9 @@ int bg3_checkpoint_load(bg3_net *n, const void *buf, uint64_t len)
     drop_graph(n);
     ring_changed(n);
     {
-        // copies: the buffer's arrays lie at any address
-        std::vector<float> refract(N);
-        std::vector<int32_t> count(N), offset(N);
-        std::vector<uint64_t> hist(n->h.syn_kind >= BG3_SYN_STDP ? N * (uint64_t)h.max_spikes : 0);
+        std::vector<float> refract(N);  // the buffer's arrays lie at any address
         memcpy(refract.data(), ap[CKA_Trefract], N * sizeof(float));
-        memcpy(count.data(), ap[CKA_spikeCount], N * sizeof(int32_t));
-        memcpy(offset.data(), ap[CKA_spikeCountOffset], N * sizeof(int32_t));
-        memcpy(hist.data(), ap[CKA_history], hist.size() * sizeof(uint64_t));
         n->refr_isi = refractory_isi(n, refract.data());
-        history_given(n, hist.data(), count.data(), offset.data());
     }
     n->queued = n->h.syn_kind >= BG3_SYN_STDP ? 31 : 0;  // saved with uploaded spikes under way, perhaps
 #define BG3_LOAD_ONE(f)                                                                           \
@@ -2995,6 +2997,7 @@ int bg3_checkpoint_load(bg3_net *n, const void *buf, uint64_t len)
     }
     BG3_NET_ARRAYS(BG3_LOAD_ONE)
 #undef BG3_LOAD_ONE
+    if (h.syn_kind >= BG3_SYN_STDP && (rc = histories_given(n))) return rc;
     if (n->noise_dev) cudaFree(n->noise_dev);
     n->noise_dev = nullptr;
     n->noise_cap = 0;
