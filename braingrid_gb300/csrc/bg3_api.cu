@@ -1345,7 +1345,7 @@ static int blk_steps(const bg3_net *n, const LaunchCfg &c, bool small = false)
 // batch, whose tiles share the GPU, is not held to more than two.  us a call in blocks and step by
 // step, near the target rate / at 200 to 330 Hz: 100x100 with 160 rows, one step, 13 and 17 / (60x60) 14 and
 // 15; 150x150 with 160 rows, one step, at 128 Hz 32 and 21, two 37 and 38; 60x60 with 480 rows, one step 19
-// and 18 / 25 and 19, two 21 and 28 / 28 and 33; 100x100 with 960 rows, one step 27 and 25 / 88 and 33, two
+// and 18 / 25 and 19, two 18 and 26 / 32 and 31; 100x100 with 960 rows, one step 27 and 25 / 88 and 33, two
 // 30 and 39 / 108 and 61, three 34 and 52 / 126 and 89, four 34 and 65 / 138 and 117, eight 42 and 120 / 173
 // and 228; a batch of 12, two steps 79 and 150.  Many blocks in a row, where step by step
 // no call begins and ends, want one step more: 200 steps of 100x100 in blocks of three 2705 and 2939 / 11600

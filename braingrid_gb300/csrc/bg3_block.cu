@@ -897,13 +897,15 @@ constexpr int DN_GROUP_WORDS = 4 * DN_MAX_CHUNKS / 32;
 constexpr int DN_LIGHT = 128;
 constexpr int DN_ACT_WORDS = 1216;  // the bitmap row is kept in shared memory up to 38,912 neurons
 constexpr int dn_threads(int W) { return 32 * (1 + W + 1); }
-// Arrival warps a tile, and the blocks an SM then holds: 16, 8 or 4 warps by the tiles there are, one wave
-// of them in each form.  A heavy block's arrivals are chains of loads, and with four warps on an SM of
-// their own one tile's chains took longer than the per-step kernels, which spread them over the GPU.  160
-// steps at 200 to 320 Hz, up to 920 rows a neuron, us with 4 warps, with this choice and step by step:
-// 33x33 (35 tiles) 2782, 1327, 1674; 45x45 2879, 1349, 2259; 60x60 (113) 3052, 1389, 2777; 80x80 (200,
-// eight warps) 3186, 2160, 3599; 100x100 (313, four) 3502, 3524, 4462.
-constexpr int dn_blocks(int W) { return W == 4 ? 3 : W == 8 ? 2 : 1; }
+// Arrival warps a tile, and the blocks an SM then holds: eight where there is at most a tile an SM, else
+// four.  A heavy block's arrivals are chains of loads, and with four warps on an SM of their own one tile's
+// chains took longer than the per-step kernels, which spread them over the GPU.  160 steps at 200 to
+// 320 Hz, up to 920 rows a neuron, us with four warps, with eight and step by step: 33x33 (35 tiles) 2782,
+// 1710, 1676; 45x45 2879, 1784, 2223; 60x60 (113) 3052, 1907, 2746; 80x80 (200, four) 3276 and 3615; 100x100
+// (313, four) 3524 and 4462.  Sixteen: 1327, 1349 and 1389, but such a block takes an SM, and 36 networks of
+// 30x30 to 100x100 on streams of their own, near silent, took 55 us a step (eight 42, four 38; a batch 38).
+constexpr int DN_FEW = 152;
+constexpr int dn_blocks(int W) { return W == 4 ? 3 : 2; }
 constexpr uint32_t DN_CHUNK = DN_ROWS * 32 * 4 + DN_QUADS * 32 * 2;
 
 template <int W>  // arrival warps, and buffers: buffer k is filled by warp k
@@ -931,7 +933,7 @@ constexpr bool dn_fits()
 {
     return dn_blocks(W) * (sizeof(DenseSmem<W>) + (sizeof(NetDev) + 127) / 128 * 128 + 1024) <= 228 * 1024;
 }
-static_assert(dn_fits<4>() && dn_fits<8>() && dn_fits<16>(), "an SM holds dn_blocks(W) blocks");
+static_assert(dn_fits<4>() && dn_fits<8>(), "an SM holds dn_blocks(W) blocks");
 
 template <int W>
 __device__ __forceinline__ void bar_events()
@@ -1884,8 +1886,7 @@ static void launch_dense_syn(const NetDev &h, const BlkDev &b, const CUtensorMap
 {
     const dim3 pg((h.ntiles + PUSH_WORDS - 1) / PUSH_WORDS, PUSH_SPLIT);
     launch_dep(k_blk_push<SYN>, pg, PUSH_THREADS, 0, s, h, b, nt);
-    if (h.ntiles <= 152 * dn_blocks(16)) launch_dense_t<SYN, 16>(h, b, tp, tc, nt, s);
-    else if (h.ntiles <= 152 * dn_blocks(8)) launch_dense_t<SYN, 8>(h, b, tp, tc, nt, s);
+    if (h.ntiles <= DN_FEW) launch_dense_t<SYN, 8>(h, b, tp, tc, nt, s);
     else launch_dense_t<SYN, 4>(h, b, tp, tc, nt, s);
 }
 void launch_blk_dense(const NetDev &h, const BlkDev &b, const CUtensorMap &tp, const CUtensorMap &tc,
@@ -1910,8 +1911,7 @@ static void launch_dense_batch_syn(const NetDev *nets, const BlkDev *blks, const
 {
     const dim3 pg((max_tiles + PUSH_WORDS - 1) / PUSH_WORDS, PUSH_SPLIT, nd);
     launch_dep(k_blk_push_batch<SYN>, pg, PUSH_THREADS, 0, s, nets, blks, dense, nt);
-    if (n <= 152 * dn_blocks(16)) launch_dense_batch_t<SYN, 16>(nets, blks, maps, tiles, n, nt, s);
-    else if (n <= 152 * dn_blocks(8)) launch_dense_batch_t<SYN, 8>(nets, blks, maps, tiles, n, nt, s);
+    if (n <= DN_FEW) launch_dense_batch_t<SYN, 8>(nets, blks, maps, tiles, n, nt, s);
     else launch_dense_batch_t<SYN, 4>(nets, blks, maps, tiles, n, nt, s);
 }
 void launch_blk_dense_batch(int syn_kind, const NetDev *nets, const BlkDev *blks,

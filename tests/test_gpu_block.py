@@ -399,7 +399,7 @@ def few_firing(w, h, syn, period, count, max_syn=260, radius=4.2, seed=9):
 @pytest.mark.parametrize("w,h", [(50, 42), (80, 70), (110, 100)])    # 66, 175 and 344 tiles
 @pytest.mark.parametrize("period,share", [(29, 130), (1, 130), (7, 130), (29, 0)])
 def test_dense_blocks_by_tiles_and_arrivals(syn, w, h, period, share):
-    """Tiles of 16, 8 and 4 arrival warps.  A few neurons (fewer than N / 128: pushed arrivals)
+    """Networks of one tile an SM and of more.  A few neurons (fewer than N / 128: pushed arrivals)
     reach most of a tile's rows with one spike a block, one at every step, or two; or all of
     them do (arrivals looked up)."""
     count = w * h // share if share else 0
